@@ -18,8 +18,8 @@ namespace geye {
 geye_status run_frame(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step, float thresh, float overlap,
                       const float *const *h_ascore_init);
 geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step);
-geye_status run_hog(geye_ctx *ctx, Plan &P);
-geye_status run_conv(geye_ctx *ctx, Plan &P, ModelPlan &mp);
+geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats);
+geye_status run_conv(geye_ctx *ctx, Plan &P);
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp);
 geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh);
 geye_status run_ascore(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, const float *h_init);

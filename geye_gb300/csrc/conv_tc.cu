@@ -594,13 +594,16 @@ __global__ void k_root_sum(const RootSumJob *__restrict__ jobs, float *__restric
   }
 }
 
-// feature planes for a standalone call: [pos][32] float -> NQ planes [ncell + pad][16 B]
+// feature planes for a standalone call: float planes (feat_stride) -> NQ planes [ncell + pad][16 B]
 template <int NQ>
-__global__ void k_feat_planes(const float *__restrict__ feat, int ncell, uint8_t *__restrict__ planes) {
+__global__ void k_feat_planes(const float *__restrict__ feat, int fs0, int fs1, uint8_t *__restrict__ planes) {
+  const int ncell = fs0 * fs1;
+  const size_t plane_f = (size_t)feat_stride(fs0) * fs1;
   const size_t plane = ((size_t)ncell + kTcPlanePad) * 16;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncell + kTcPlanePad; i += gridDim.x * blockDim.x) {
+    const float *src = feat + (size_t)(i / fs0) * feat_stride(fs0) + i % fs0;
     float f[32];
-    for (int c = 0; c < 32; c++) f[c] = i < ncell ? feat[(size_t)i * kFeatPad + c] : 0.f;
+    for (int c = 0; c < 32; c++) f[c] = i < ncell && c < kFeat ? src[c * plane_f] : 0.f;
     tc_store_planes<NQ>(f, planes, plane, i);
   }
 }
@@ -1390,8 +1393,8 @@ geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, con
   GEYE_TRY(d_err->alloc(ctx, 16));
   CUDA_TRY(cudaMemsetAsync(d_err->p, 0, 16, ctx->stream));
   const int grid = std::max(1, std::min((ncell + kTcPlanePad + 255) / 256, 1024));
-  if (NQ == 4) k_feat_planes<4><<<grid, 256, 0, ctx->stream>>>(d_feat, ncell, planes->as<uint8_t>());
-  else k_feat_planes<2><<<grid, 256, 0, ctx->stream>>>(d_feat, ncell, planes->as<uint8_t>());
+  if (NQ == 4) k_feat_planes<4><<<grid, 256, 0, ctx->stream>>>(d_feat, a0, a1, planes->as<uint8_t>());
+  else k_feat_planes<2><<<grid, 256, 0, ctx->stream>>>(d_feat, a0, a1, planes->as<uint8_t>());
   launch_conv_tc(NQ, d_jobs->as<TcJob>(), d_chunks->as<int4>(), (int)chunks.size(), d_cols->as<TcCol>(),
                  planes->as<uint8_t>(), d_bank->as<uint8_t>(), stages, tps, d_out, d_err->as<int>(), smem, ctx->stream);
   CUDA_TRY(cudaGetLastError());

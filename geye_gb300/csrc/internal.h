@@ -3,7 +3,7 @@
 // Device layouts (all spatial maps column-major like the reference, so a
 // level's stage output is a plain copy):
 //   image level l:   3 float planes [c][w][h]                (x*h + y)
-//   feature level l: [pos][32] float, pos = x*fs0 + y, channel 31 = 0
+//   feature level l: 31 float planes [x][feat_stride(fs0)]
 //   conv/DT/score maps: [x][y] float (int for argmax), per (level, filter)
 // Every per-frame buffer lives in one arena sized when a plan is built.
 #pragma once
@@ -20,7 +20,10 @@
 namespace geye {
 
 constexpr int kFeat = 31;       // HOG channels
-constexpr int kFeatPad = 32;    // channel stride in device feature buffers
+// Float features of a level: 31 planes [x][y] (the reference layout) with columns of
+// feat_stride(fs0) floats, so that every column starts on a 16-byte boundary.
+__host__ __device__ inline int feat_stride(int fs0) { return (fs0 + 3) & ~3; }
+__host__ __device__ inline size_t feat_words(int fs0, int fs1) { return (size_t)kFeat * feat_stride(fs0) * fs1; }
 constexpr int kMaxParts = 32;   // parts per component supported by the kernels
 constexpr int kTcPlanePad = 128;   // cells after each bf16 feature plane (reach of a 128-position tile)
 
@@ -67,7 +70,7 @@ struct HogJob {
   int b0, b1;              // histogram blocks (rows, cols)
   int hist_off;            // [18][b1*b0] then norm [b1*b0] at hist_off + 18*b1*b0
   int fs0, fs1;            // output cells
-  int feat_off;            // [pos][32] float
+  int feat_off;            // float planes (feat_stride)
   int feat16_off;          // tensor-core planes (offset in 2-byte units), -1 = not written
   int feat16lo_off;        // BF16 remainder planes (root levels in BF16 mode), -1 = none
   int fast;                // 1 (tensor-core modes): float normalisation factors computed per cell,
@@ -86,14 +89,24 @@ struct HogPixJob {         // (bin, magnitude) of the pixels of one image
   int mag_off, bin_off;    // float magnitudes; u8 bins at (uint8_t *)(arena + bin_off)
 };
 
-struct ConvJob {           // a block of outputs of one (level, filter group)
-  int feat_off, a0, a1;    // feature level [pos][32], dims
-  int filt_base;           // first filter index in the model's filter table
-  int n_filt;              // filters in the group (same size)
+constexpr int kConvGroup = 4;   // filters per FP32 convolution job
+
+struct ConvJob {           // FP32 maps of one level for up to kConvGroup filters of one size
+  int feat_off, a0, a1;    // feature level, dims
+  int n_filt;
+  int bank_off;            // the group's taps in the bank (in pairs)
+  int out_off[kConvGroup];    // float offset of each output map
   int b0, b1;              // filter dims
   int c0, c1;              // output dims
-  int out_off;             // output of filter g at out_off + g*c0*c1
-  int tiles_y, tiles_x;    // output tiles of this job
+  // the launch shape (conv_shape): channels split over the warps or not, a warp's lanes
+  // along y and x, the block's warps along y, tiles, filter columns per stage, padded
+  // filter rows, rows of a staged column
+  int split, ty, tx, wy, tiles_y, tiles_x, xb, b0p, RP;
+  int cost;                // of one tile, relative (the launch starts the dearest first)
+};
+struct ConvBank {          // the groups' taps as the FP32 kernel reads them, built with the jobs
+  std::vector<float> taps;
+  std::map<std::vector<const float *>, int> at;   // a group's filters (host) -> its place, in pairs
 };
 
 // tensor-core convolution (conv_tc.cu)
@@ -259,16 +272,21 @@ constexpr int kBatchCells = 256;   // corners / cells per item (a thread each)
 // one stage (phase: the resize phase) over n items
 void launch_batch_front(int stage, const BatchFrame *d_frames, const BatchItem *d_items, int n, int phase,
                         cudaStream_t s);
-// corners: run the corner-factor pass (jobs with fast = 0 read its factors)
+// corners: run the corner-factor pass (jobs with fast = 0 read its factors); floats: write the float planes
 void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int n_vote_blocks, int max_b0,
                 int max_b1, const HogPixJob *d_pix, int n_pix, int max_xe, float *arena, void *arena16,
-                bool corners, cudaStream_t s);   // arena16: base of the tensor-core planes (bytes)
+                bool corners, bool floats, cudaStream_t s);   // arena16: base of the tensor-core planes (bytes)
 void launch_to_ref_layout(const float *feat, int fs0, int fs1, float *out, cudaStream_t s);
 void launch_flip_feat(const float *feat, int n0, int n1, float *out, cudaStream_t s);
 void launch_from_ref_layout(const float *ref, int fs0, int fs1, float *feat, cudaStream_t s);
-void launch_conv_fp32(const ConvJob *d_jobs, int n_jobs, int max_tiles_y, int max_tiles_x, const float *filters,
-                      const int *filt_off, const float *arena_in, float *arena_out, int max_b0, int max_b1,
-                      int max_group, cudaStream_t s, int cr = 4);
+// jobs for filters of one size [31][b1][b0] (host memory) over one level (J: its features and the
+// filter dims), in groups of equal length; false when they are too large for shared memory one by one
+bool conv_fp32_jobs(ConvJob J, const std::vector<const float *> &filters, const std::vector<int> &out_off,
+                    ConvBank &bank, std::vector<ConvJob> &jobs);
+// (job, tile) of every block, dearest first; returns the launch's shared memory
+size_t conv_fp32_blocks(std::vector<ConvJob> &jobs, std::vector<int2> &blocks);
+void launch_conv_fp32(const ConvJob *d_jobs, const int2 *d_blocks, int n_blocks, size_t smem, const float *d_bank,
+                      const float *arena_in, float *arena_out, cudaStream_t s);
 // (job, first line) of every DT block, pass 1 (columns) and pass 2 (rows), largest maps first
 // DT tiles of about `elems` outputs per block (kDtElems by default; a plan
 // tunes it on its first frame's maps among kDtElemsChoices)

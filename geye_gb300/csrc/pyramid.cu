@@ -377,9 +377,9 @@ __global__ void __launch_bounds__(kVoteThreads, 4) k_hog_vote(const HogJob *__re
   hog_vote_one(jobs[blk.x], arena, blk.y * kVoteThreads + threadIdx.x, hist_s);
 }
 
-// 31 features per output cell (featurepyramid.cpp:421-487), written as 32
-// floats [pos][32] (channel 31 = 0), plus an optional copy as the tensor-core
-// convolution's channel planes (tc_planes.h).
+// 31 features per output cell (featurepyramid.cpp:421-487), written as float
+// planes (feat_stride) and in the tensor-core modes as the convolution's channel
+// planes (tc_planes.h).
 // Normalisation factor of every corner of 2x2 histogram blocks,
 // 1 / sqrt(e(x,y) + e(x,y+1) + e(x+1,y) + e(x+1,y+1) + 0.0001) in the reference's
 // expression (float sum, double root and division, rounded to float), once per
@@ -404,13 +404,12 @@ __global__ void k_hog_norm(const HogJob *__restrict__ jobs, float *__restrict__ 
 
 // output cell i of one level
 __device__ __forceinline__ void hog_feat_one(const HogJob &J, float *__restrict__ arena,
-                                             uint8_t *__restrict__ arena16, int i) {
+                                             uint8_t *__restrict__ arena16, int i, bool floats) {
   const int ncell = J.fs0 * J.fs1;
   const int b0 = J.b0, nb = J.b0 * J.b1;
   const float *hist = arena + J.hist_off;
   const float *N = arena + J.corner_off;
   const int C0 = J.fs0 + 1;
-  float *feat = arena + J.feat_off;
   {
     const int y = i % J.fs0, x = i / J.fs0;
     float n1, n2, n3, n4;
@@ -468,9 +467,12 @@ __device__ __forceinline__ void hog_feat_one(const HogJob &J, float *__restrict_
       out[30] = (float)(0.2357 * (double)t4);
     }
     out[31] = 0.f;
-    float4 *dst = reinterpret_cast<float4 *>(feat + (size_t)i * kFeatPad);
+    if (floats) {   // (the tensor-core modes' frames read only the channel planes below)
+      float *dst = arena + J.feat_off + (size_t)x * feat_stride(J.fs0) + y;
+      const size_t plane = (size_t)feat_stride(J.fs0) * J.fs1;
 #pragma unroll
-    for (int q = 0; q < 8; q++) dst[q] = make_float4(out[4 * q], out[4 * q + 1], out[4 * q + 2], out[4 * q + 3]);
+      for (int c = 0; c < kFeat; c++) dst[c * plane] = out[c];
+    }
     if (J.feat16_off >= 0 && arena16) {   // planes for the tensor-core convolution
       uint8_t *planes = arena16 + 2 * (size_t)J.feat16_off;
       const size_t plane = ((size_t)ncell + kTcPlanePad) * 16;
@@ -481,11 +483,12 @@ __device__ __forceinline__ void hog_feat_one(const HogJob &J, float *__restrict_
   }
 }
 
-__global__ void k_hog_feat(const HogJob *__restrict__ jobs, float *__restrict__ arena, uint8_t *__restrict__ arena16) {
+__global__ void k_hog_feat(const HogJob *__restrict__ jobs, float *__restrict__ arena, uint8_t *__restrict__ arena16,
+                           bool floats) {
   const HogJob J = jobs[blockIdx.y];
   const int ncell = J.fs0 * J.fs1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncell; i += gridDim.x * blockDim.x)
-    hog_feat_one(J, arena, arena16, i);
+    hog_feat_one(J, arena, arena16, i, floats);
 }
 
 // ----------------------------------------------------------------------------
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(256) k_batch_front(const BatchFrame *__restric
     } else {
       const HogJob J = F.hog[I.job];
       const int i = I.chunk * kBatchCells + tid;
-      if (i < J.fs0 * J.fs1) hog_feat_one(J, F.arena, F.arena16, i);
+      if (i < J.fs0 * J.fs1) hog_feat_one(J, F.arena, F.arena16, i, !J.fast);
     }
   }
 }
@@ -551,7 +554,7 @@ void hog_vote_blocks(const std::vector<HogJob> &jobs, std::vector<int2> &blocks)
 
 void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int n_vote_blocks, int max_b0,
                 int max_b1, const HogPixJob *d_pix, int n_pix, int max_xe, float *arena, void *arena16,
-                bool corners, cudaStream_t s) {
+                bool corners, bool floats, cudaStream_t s) {
   if (n_jobs <= 0) return;
   dim3 g0((max_xe + kPixWarps - 1) / kPixWarps, n_pix);
   k_hog_pix<<<g0, kPixWarps * 32, 0, s>>>(d_pix, arena);
@@ -561,25 +564,23 @@ void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int
   if (bx > 512) bx = 512;
   dim3 g2(bx, n_jobs);
   if (corners) k_hog_norm<<<g2, 256, 0, s>>>(d_jobs, arena);
-  k_hog_feat<<<g2, 256, 0, s>>>(d_jobs, arena, reinterpret_cast<uint8_t *>(arena16));
+  k_hog_feat<<<g2, 256, 0, s>>>(d_jobs, arena, reinterpret_cast<uint8_t *>(arena16), floats);
 }
 
 // ----------------------------------------------------------------------------
-// layout conversion between the device feature layout [pos][32] and the
-// reference layout [31][fs1][fs0] (stage entry points only)
+// between the device feature planes and the reference layout [31][fs1][fs0]
+// (stage entry points only): they differ in the columns' padding
 // ----------------------------------------------------------------------------
-__global__ void k_to_ref(const float *__restrict__ feat, int ncell, float *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncell * kFeat; i += gridDim.x * blockDim.x) {
-    const int f = i / ncell, pos = i % ncell;
-    out[i] = feat[(size_t)pos * kFeatPad + f];
-  }
+__global__ void k_to_ref(const float *__restrict__ feat, int fs0, int ncols, float *__restrict__ out) {
+  const int S0 = feat_stride(fs0), n = ncols * fs0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    out[i] = feat[(size_t)(i / fs0) * S0 + i % fs0];
 }
 
-__global__ void k_from_ref(const float *__restrict__ ref, int ncell, float *__restrict__ feat) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncell * kFeatPad; i += gridDim.x * blockDim.x) {
-    const int pos = i / kFeatPad, f = i % kFeatPad;
-    feat[i] = f < kFeat ? ref[(size_t)f * ncell + pos] : 0.f;
-  }
+__global__ void k_from_ref(const float *__restrict__ ref, int fs0, int ncols, float *__restrict__ feat) {
+  const int S0 = feat_stride(fs0), n = ncols * fs0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    feat[(size_t)(i / fs0) * S0 + i % fs0] = ref[i];
 }
 
 // flip_feat (get_boxes.cpp:121-178): output channel c, column x is source
@@ -607,13 +608,13 @@ void launch_flip_feat(const float *feat, int n0, int n1, float *out, cudaStream_
 void launch_to_ref_layout(const float *feat, int fs0, int fs1, float *out, cudaStream_t s) {
   int n = fs0 * fs1 * kFeat;
   if (n <= 0) return;
-  k_to_ref<<<(n + 255) / 256 < 2048 ? (n + 255) / 256 : 2048, 256, 0, s>>>(feat, fs0 * fs1, out);
+  k_to_ref<<<std::min((n + 255) / 256, 2048), 256, 0, s>>>(feat, fs0, fs1 * kFeat, out);
 }
 
 void launch_from_ref_layout(const float *ref, int fs0, int fs1, float *feat, cudaStream_t s) {
-  int n = fs0 * fs1 * kFeatPad;
+  int n = fs0 * fs1 * kFeat;
   if (n <= 0) return;
-  k_from_ref<<<(n + 255) / 256 < 2048 ? (n + 255) / 256 : 2048, 256, 0, s>>>(ref, fs0 * fs1, feat);
+  k_from_ref<<<std::min((n + 255) / 256, 2048), 256, 0, s>>>(ref, fs0, fs1 * kFeat, feat);
 }
 
 }  // namespace geye

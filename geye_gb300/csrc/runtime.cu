@@ -249,6 +249,41 @@ static void feature_dims(int h, int w, int sbin, int &b0, int &b1, int &fs0, int
 // ----------------------------------------------------------------------------
 // plan construction
 // ----------------------------------------------------------------------------
+// The maps of a list of filters (sizes sz) over one feature level: their places in the
+// arena, and in FP32 mode the jobs that fill them.
+static geye_status conv_level(geye_ctx *ctx, Plan &P, ModelPlan &mp, ArenaAlloc &A, const LevelInfo &L,
+                              const std::vector<int> &sz, const std::vector<std::vector<float>> &filters, int n,
+                              const char *too_large, std::vector<int> &out_off) {
+  out_off.assign(n, -1);
+  std::map<std::pair<int, int>, std::vector<int>> by_size;
+  for (int i = 0; i < n; i++) {
+    const int b0 = sz[3 * i], b1 = sz[3 * i + 1], c0 = L.fs0 - b0 + 1, c1 = L.fs1 - b1 + 1;
+    if (c0 < 1 || c1 < 1) { set_error(too_large); return GEYE_ERR_UNSUPPORTED; }
+    out_off[i] = A.take((size_t)c0 * c1);
+    by_size[{b0, b1}].push_back(i);
+    mp.conv_flops += 2.0 * c0 * c1 * b0 * b1 * kFeat;
+    mp.conv_bytes += 4.0 * c0 * c1;
+  }
+  if (n) mp.conv_bytes += 128.0 * L.fs0 * L.fs1;
+  if (ctx->conv_mode != GEYE_CONV_FP32 && !P.from_features) return GEYE_OK;
+  for (auto &g : by_size) {
+    ConvJob J{};
+    J.feat_off = L.feat_off; J.a0 = L.fs0; J.a1 = L.fs1;
+    J.b0 = g.first.first; J.b1 = g.first.second;
+    std::vector<const float *> w;
+    std::vector<int> o;
+    for (int i : g.second) {
+      w.push_back(filters[i].data());
+      o.push_back(out_off[i]);
+    }
+    if (!conv_fp32_jobs(J, w, o, P.conv_bank, P.conv_jobs)) {
+      set_error("filter too large for the FP32 convolution");
+      return GEYE_ERR_UNSUPPORTED;
+    }
+  }
+  return GEYE_OK;
+}
+
 static geye_status build_model_plan(geye_ctx *ctx, Plan &P, geye_model *mdl, int LEN_m, ArenaAlloc &A) {
   const HostModel &m = mdl->h;
   auto mp = std::make_unique<ModelPlan>();
@@ -262,76 +297,25 @@ static geye_status build_model_plan(geye_ctx *ctx, Plan &P, geye_model *mdl, int
   mp->part_d0.assign((size_t)LEN_m * std::max(NoP, 1), 0);
   mp->part_d1.assign((size_t)LEN_m * std::max(NoP, 1), 0);
   mp->skipped.assign(LEN_m, 1);
-  int filt_parts_base = m.NoR;
   for (int level = interval; level < LEN_m; level++) {
     const LevelInfo &L = P.lv[level];
     if (L.fs0 + 2 * m.pady < m.max_Y || L.fs1 + 2 * m.padx < m.max_X) continue;   // fconvsMT.cpp:425
     mp->skipped[level] = 0;
-    // roots: filter c for component c, grouped by size
-    std::vector<int> done(NoC, 0);
-    for (int c = 0; c < NoC; c++) {
-      if (done[c]) continue;
-      const int b0 = m.root_size[3 * c], b1 = m.root_size[3 * c + 1];
-      std::vector<int> grp;
-      for (int c2 = c; c2 < NoC && (int)grp.size() < 8; c2++)
-        if (!done[c2] && m.root_size[3 * c2] == b0 && m.root_size[3 * c2 + 1] == b1 && (grp.empty() || c2 == grp.back() + 1))
-          grp.push_back(c2);
-      const int c0 = L.fs0 - b0 + 1, c1 = L.fs1 - b1 + 1;
-      if (c0 < 1 || c1 < 1) { set_error("root filter larger than a kept feature level"); return GEYE_ERR_UNSUPPORTED; }
-      ConvJob J{};
-      J.feat_off = L.feat_off; J.a0 = L.fs0; J.a1 = L.fs1;
-      J.filt_base = grp[0]; J.n_filt = (int)grp.size(); J.b0 = b0; J.b1 = b1; J.c0 = c0; J.c1 = c1;
-      J.out_off = A.take((size_t)c0 * c1 * grp.size());
-      J.tiles_y = (c0 + 31) / 32; J.tiles_x = (c1 + 15) / 16;
-      for (size_t g = 0; g < grp.size(); g++) {
-        const int cc = grp[g];
-        done[cc] = 1;
-        mp->root_map_off[level * NoC + cc] = J.out_off + (int)g * c0 * c1;
-        mp->root_r0[level * NoC + cc] = c0;
-        mp->root_r1[level * NoC + cc] = c1;
-        mp->conv_flops += 2.0 * c0 * c1 * b0 * b1 * kFeat;
-      }
-      mp->root_jobs.push_back(J);
-      mp->root_max_b0 = std::max(mp->root_max_b0, b0);
-      mp->root_max_b1 = std::max(mp->root_max_b1, b1);
-      mp->root_max_g = std::max(mp->root_max_g, J.n_filt);
-      mp->root_tiles_y = std::max(mp->root_tiles_y, J.tiles_y);
-      mp->root_tiles_x = std::max(mp->root_tiles_x, J.tiles_x);
-      mp->conv_bytes += 128.0 * L.fs0 * L.fs1 + 4.0 * c0 * c1 * grp.size();
-    }
-    // parts at L = level - interval
+    // roots (filter c for component c) at this level, parts at level - interval
     const int Lv = level - interval;
+    std::vector<int> out_off;
+    GEYE_TRY(conv_level(ctx, P, *mp, A, L, m.root_size, m.rootfilter, NoC, "root filter larger than a kept feature level", out_off));
+    for (int c = 0; c < NoC; c++) {
+      mp->root_map_off[level * NoC + c] = out_off[c];
+      mp->root_r0[level * NoC + c] = L.fs0 - m.root_size[3 * c] + 1;
+      mp->root_r1[level * NoC + c] = L.fs1 - m.root_size[3 * c + 1] + 1;
+    }
     const LevelInfo &PL = P.lv[Lv];
-    std::vector<int> pdone(NoP, 0);
+    GEYE_TRY(conv_level(ctx, P, *mp, A, PL, m.part_size, m.partfilter, NoP, "part filter larger than its feature level", out_off));
     for (int p = 0; p < NoP; p++) {
-      if (pdone[p]) continue;
-      const int b0 = m.part_size[3 * p], b1 = m.part_size[3 * p + 1];
-      std::vector<int> grp;
-      for (int p2 = p; p2 < NoP && (int)grp.size() < 8; p2++)
-        if (!pdone[p2] && m.part_size[3 * p2] == b0 && m.part_size[3 * p2 + 1] == b1 && (grp.empty() || p2 == grp.back() + 1))
-          grp.push_back(p2);
-      const int c0 = PL.fs0 - b0 + 1, c1 = PL.fs1 - b1 + 1;
-      if (c0 < 1 || c1 < 1) { set_error("part filter larger than its feature level"); return GEYE_ERR_UNSUPPORTED; }
-      ConvJob J{};
-      J.feat_off = PL.feat_off; J.a0 = PL.fs0; J.a1 = PL.fs1;
-      J.filt_base = filt_parts_base + grp[0]; J.n_filt = (int)grp.size(); J.b0 = b0; J.b1 = b1; J.c0 = c0; J.c1 = c1;
-      J.out_off = A.take((size_t)c0 * c1 * grp.size());
-      J.tiles_y = (c0 + 31) / 32; J.tiles_x = (c1 + 15) / 16;
-      for (size_t g = 0; g < grp.size(); g++) {
-        const int pp = grp[g];
-        pdone[pp] = 1;
-        mp->part_map_off[Lv * NoP + pp] = J.out_off + (int)g * c0 * c1;
-        mp->part_d0[Lv * NoP + pp] = c0;
-        mp->part_d1[Lv * NoP + pp] = c1;
-        mp->conv_flops += 2.0 * c0 * c1 * b0 * b1 * kFeat;
-      }
-      mp->part_jobs.push_back(J);
-      mp->part_max_b0 = std::max(mp->part_max_b0, b0);
-      mp->part_max_b1 = std::max(mp->part_max_b1, b1);
-      mp->part_max_g = std::max(mp->part_max_g, J.n_filt);
-      mp->part_tiles_y = std::max(mp->part_tiles_y, J.tiles_y);
-      mp->part_tiles_x = std::max(mp->part_tiles_x, J.tiles_x);
-      mp->conv_bytes += 128.0 * PL.fs0 * PL.fs1 / std::max(1.0, (double)NoP / grp.size()) + 4.0 * c0 * c1 * grp.size();
+      mp->part_map_off[Lv * NoP + p] = out_off[p];
+      mp->part_d0[Lv * NoP + p] = PL.fs0 - m.part_size[3 * p] + 1;
+      mp->part_d1[Lv * NoP + p] = PL.fs1 - m.part_size[3 * p + 1] + 1;
     }
     // DT per (component, part) and score jobs per component
     for (int c = 0; c < NoC; c++) {
@@ -402,8 +386,6 @@ static geye_status build_model_plan(geye_ctx *ctx, Plan &P, geye_model *mdl, int
     }
   }
   if (mp->dt_max_d0 > 1100 || mp->dt_max_d1 > 1100) { set_error("frame too large for the DT kernels"); return GEYE_ERR_UNSUPPORTED; }
-  GEYE_TRY(upload(ctx, mp->d_root_jobs, mp->root_jobs));
-  GEYE_TRY(upload(ctx, mp->d_part_jobs, mp->part_jobs));
   GEYE_TRY(upload(ctx, mp->d_dt_jobs, mp->dt_jobs));
   {
     std::vector<int2> b1, b2;
@@ -519,7 +501,7 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
     L.sbin = l < interval ? sbin2 : sbin;
     int b0, b1;
     feature_dims(L.img_h, L.img_w, L.sbin, b0, b1, L.fs0, L.fs1);
-    L.feat_off = A.take((size_t)std::max(L.fs0 * L.fs1, 1) * kFeatPad);
+    L.feat_off = A.take(std::max<size_t>(feat_words(L.fs0, L.fs1), 1));
     if (tc_planes) {   // tc_planes planes [fs0*fs1 + kTcPlanePad][16 B]
       size_t o = (P.arena16_elems + 63) & ~size_t(63);
       L.feat16_off = (int)o;
@@ -596,107 +578,16 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
   return GEYE_OK;
 }
 
-// FP32 conv shape tuner: job tables for rows per thread cr (4 or 8) and groups
-// of at most gmax filters, split from the plan's groups (maps of a group are
-// contiguous, so a split group writes the same places); each candidate is timed
-// on the plan's arena (CUDA events after one untimed launch), the fastest kept.
-// Every shape gives the same bits.
-static void conv_jobs_for(const std::vector<ConvJob> &in, int cr, int gmax, std::vector<ConvJob> &out, int &mty,
-                          int &mtx, int &mg) {
-  out.clear();
-  mty = mtx = 0;
-  mg = 1;
-  for (const ConvJob &J : in)
-    for (int k = 0; k < J.n_filt; k += gmax) {
-      ConvJob C = J;
-      C.filt_base = J.filt_base + k;
-      C.n_filt = std::min(gmax, J.n_filt - k);
-      C.out_off = J.out_off + k * J.c0 * J.c1;
-      C.tiles_y = (J.c0 + 8 * cr - 1) / (8 * cr);
-      C.tiles_x = (J.c1 + 15) / 16;
-      mty = std::max(mty, C.tiles_y);
-      mtx = std::max(mtx, C.tiles_x);
-      mg = std::max(mg, C.n_filt);
-      out.push_back(C);
-    }
-}
-
-static geye_status tune_conv_fp32(geye_ctx *ctx, Plan &P, ModelPlan &mp) {
-  geye_model *m = mp.model;
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  CUDA_TRY(cudaEventCreate(&e0));
-  CUDA_TRY(cudaEventCreate(&e1));
-  geye_status st = GEYE_OK;
-  for (int kind = 0; kind < 2 && st == GEYE_OK; kind++) {
-    std::vector<ConvJob> &jobs = kind ? mp.part_jobs : mp.root_jobs;
-    if (jobs.empty()) continue;
-    const int b0 = kind ? mp.part_max_b0 : mp.root_max_b0, b1 = kind ? mp.part_max_b1 : mp.root_max_b1;
-    float best = 0.f;
-    std::vector<ConvJob> best_jobs;
-    int best_cr = 4, bty = 0, btx = 0, bg = 1, best_i = 0;
-    // a geometry this model was tuned at before reuses the choice without timing
-    const std::string key = std::string(kind ? "fp32p:" : "fp32r:") + std::to_string(P.width) + "x" +
-                            std::to_string(P.height) + "/" + std::to_string(mp.LEN);
-    int only = -1;
-    {
-      std::lock_guard<std::mutex> lk(m->tc_mu);
-      auto it = m->tc_tuned.find(key);
-      if (it != m->tc_tuned.end()) only = it->second.first;
-    }
-    for (int ci = 0; ci < 4; ci++) {
-      if (only >= 0 && ci != only) continue;
-      const int cr = ci < 2 ? 4 : 8, gmax = ci % 2 ? 4 : 8;
-      {
-        std::vector<ConvJob> cand;
-        int mty, mtx, mg;
-        conv_jobs_for(jobs, cr, gmax, cand, mty, mtx, mg);
-        DevBuf d;
-        st = upload(ctx, d, cand);
-        if (st != GEYE_OK) break;
-        auto launch = [&]() {
-          launch_conv_fp32(d.as<ConvJob>(), (int)cand.size(), mty, mtx, m->d_filters, m->d_filt_off,
-                           P.arena.as<float>(), P.arena.as<float>(), b0, b1, mg, ctx->stream, cr);
-        };
-        launch();
-        if (cudaEventRecord(e0, ctx->stream) != cudaSuccess) { st = GEYE_ERR_CUDA; break; }
-        for (int r = 0; r < 3; r++) launch();
-        float ms = 0.f;
-        cudaError_t e = cudaEventRecord(e1, ctx->stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-        if (e != cudaSuccess) {
-          set_error(std::string("FP32 conv tuning: ") + cudaGetErrorString(e));
-          st = GEYE_ERR_CUDA;
-          break;
-        }
-        if (best_jobs.empty() || ms < best) {
-          best = ms;
-          best_jobs = cand;
-          best_cr = cr; bty = mty; btx = mtx; bg = mg; best_i = ci;
-        }
-      }
-    }
-    if (st != GEYE_OK) break;
-    if (only < 0) {
-      std::lock_guard<std::mutex> lk(m->tc_mu);
-      m->tc_tuned[key] = {best_i, best / 3.0f};
-    }
-    jobs = best_jobs;
-    if (kind) {
-      mp.part_cr = best_cr; mp.part_tiles_y = bty; mp.part_tiles_x = btx; mp.part_max_g = bg;
-      st = upload(ctx, mp.d_part_jobs, mp.part_jobs);
-    } else {
-      mp.root_cr = best_cr; mp.root_tiles_y = bty; mp.root_tiles_x = btx; mp.root_max_g = bg;
-      st = upload(ctx, mp.d_root_jobs, mp.root_jobs);
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  return st;
-}
-
 static geye_status finish_plan(geye_ctx *ctx, Plan &P, ArenaAlloc &A) {
+  if (!P.conv_jobs.empty()) {
+    std::vector<int2> blocks;
+    P.conv_smem = conv_fp32_blocks(P.conv_jobs, blocks);
+    P.conv_nblocks = (int)blocks.size();
+    GEYE_TRY(upload(ctx, P.d_conv_jobs, P.conv_jobs));
+    GEYE_TRY(upload(ctx, P.d_conv_blocks, blocks));
+    GEYE_TRY(upload(ctx, P.d_conv_bank, P.conv_bank.taps));
+    P.conv_bank = ConvBank();
+  }
   P.arena_words = A.words + 64;
   GEYE_TRY(P.arena.alloc(ctx, P.arena_words * 4));
   if (P.arena16_elems) {
@@ -798,10 +689,7 @@ static geye_status get_frame_plan(geye_ctx *ctx, geye_model *const *models, int 
   if (ctx->conv_mode != GEYE_CONV_FP32) GEYE_TRY(plan_tc(ctx, *P, A));
   GEYE_TRY(finish_plan(ctx, *P, A));
   // after the arena exists: the tile shapes are tuned on it
-  if (ctx->conv_mode != GEYE_CONV_FP32)
-    GEYE_TRY(build_tc_plan(ctx, *P));
-  else
-    for (auto &mp : P->models) GEYE_TRY(tune_conv_fp32(ctx, *P, *mp));
+  if (ctx->conv_mode != GEYE_CONV_FP32) GEYE_TRY(build_tc_plan(ctx, *P));
   GEYE_TRY(P->d_bgr.alloc(ctx, (size_t)width * height * 3 + 64));
   if (ctx->plans.size() > 32) ctx->plans.clear();
   *out = P.get();
@@ -861,32 +749,22 @@ geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_
   return run_resize(ctx, P);
 }
 
-geye_status run_hog(geye_ctx *ctx, Plan &P) {
+// floats: also write the float feature planes (the FP32 convolution and calc_f_pyramid read them)
+geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats) {
   const bool fast = !P.hog_jobs.empty() && P.hog_jobs[0].fast;
   launch_hog(P.d_hog_jobs.as<HogJob>(), (int)P.hog_jobs.size(), P.d_hog_vote_blocks.as<int2>(), P.hog_vote_nblocks,
              P.hog_max_b0, P.hog_max_b1, P.d_pix_jobs.as<HogPixJob>(), (int)P.pix_jobs.size(), P.pix_max_xe,
-             P.arena.as<float>(), P.arena16.p, !fast, ctx->stream);
+             P.arena.as<float>(), P.arena16.p, !fast, floats, ctx->stream);
   ctx->launches += 3;   // pixels, votes, corner norms, features
   return check_launch(ctx, "hog");
 }
 
-// FP32 conv of one model (the tensor-core modes convolve every model at once: run_conv_tc)
-geye_status run_conv(geye_ctx *ctx, Plan &P, ModelPlan &mp) {
-  geye_model *m = mp.model;
-  float *arena = P.arena.as<float>();
-  if (!mp.root_jobs.empty()) {
-    launch_conv_fp32(mp.d_root_jobs.as<ConvJob>(), (int)mp.root_jobs.size(), mp.root_tiles_y, mp.root_tiles_x,
-                     m->d_filters, m->d_filt_off, arena, arena, mp.root_max_b0, mp.root_max_b1, mp.root_max_g,
-                     ctx->stream, mp.root_cr);
-    GEYE_TRY(check_launch(ctx, "root conv"));
-  }
-  if (!mp.part_jobs.empty()) {
-    launch_conv_fp32(mp.d_part_jobs.as<ConvJob>(), (int)mp.part_jobs.size(), mp.part_tiles_y, mp.part_tiles_x,
-                     m->d_filters, m->d_filt_off, arena, arena, mp.part_max_b0, mp.part_max_b1, mp.part_max_g,
-                     ctx->stream, mp.part_cr);
-    GEYE_TRY(check_launch(ctx, "part conv"));
-  }
-  return GEYE_OK;
+// FP32 convolution of every model, roots and parts (the tensor-core modes: run_conv_tc)
+geye_status run_conv(geye_ctx *ctx, Plan &P) {
+  if (!P.conv_nblocks) return GEYE_OK;
+  launch_conv_fp32(P.d_conv_jobs.as<ConvJob>(), P.d_conv_blocks.as<int2>(), P.conv_nblocks, P.conv_smem,
+                   P.d_conv_bank.as<float>(), P.arena.as<float>(), P.arena.as<float>(), ctx->stream);
+  return check_launch(ctx, "conv");
 }
 
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp) {
@@ -1087,24 +965,21 @@ static geye_status run_body(geye_ctx *ctx, Plan &P, float thresh, float overlap)
   StageTimer T(ctx);
   if (!ctx->front_external) GEYE_TRY(run_resize(ctx, P));
   T.mark(1);
-  if (!ctx->front_external) GEYE_TRY(run_hog(ctx, P));
+  if (!ctx->front_external) GEYE_TRY(run_hog(ctx, P, ctx->conv_mode == GEYE_CONV_FP32));
   T.mark(2);
   const bool tc = ctx->conv_mode != GEYE_CONV_FP32;
-  if (tc) GEYE_TRY(run_conv_tc(ctx, P));   // every model's filters in one launch
+  GEYE_TRY(tc ? run_conv_tc(ctx, P) : run_conv(ctx, P));   // every model's filters in one launch
   if (ctx->timing || P.models.size() < 2) {   // stage by stage (per-stage times)
-    if (!tc)
-      for (auto &mp : P.models) GEYE_TRY(run_conv(ctx, P, *mp));
     T.mark(3);
     for (auto &mp : P.models) GEYE_TRY(run_dt(ctx, P, *mp));
     T.mark(4);
     for (size_t mi = 0; mi < P.models.size(); mi++) GEYE_TRY(run_score(ctx, P, *P.models[mi], (int)mi, thresh));
   } else {
-    // each model's conv -> DT -> score chain reads only the shared features and
-    // writes only its own maps and records: models 1.. run on the side stream
-    // beside model 0 (their kernels take the context's stream, swapped while
-    // they are issued), joined before NMS
+    // each model's DT -> score chain reads only the conv maps and writes only its
+    // own maps and records: models 1.. run on the side stream beside model 0
+    // (their kernels take the context's stream, swapped while they are issued),
+    // joined before NMS
     auto chain = [&](size_t mi) -> geye_status {
-      if (!tc) GEYE_TRY(run_conv(ctx, P, *P.models[mi]));
       GEYE_TRY(run_dt(ctx, P, *P.models[mi]));
       return run_score(ctx, P, *P.models[mi], (int)mi, thresh);
     };
@@ -1269,7 +1144,7 @@ geye_status features_plan(geye_ctx *ctx, geye_model *model, const int *ftsize, c
     L.fs1 = ftsize[2 * l + 1];
     L.scale = scales[l];
     L.sbin = l < m.interval ? m.sbin / 2 : m.sbin;
-    L.feat_off = A.take((size_t)std::max(L.fs0 * L.fs1, 1) * kFeatPad);
+    L.feat_off = A.take(std::max<size_t>(feat_words(L.fs0, L.fs1), 1));
   }
   GEYE_TRY(build_model_plan(ctx, *P, model, n_levels, A));
   GEYE_TRY(finish_plan(ctx, *P, A));

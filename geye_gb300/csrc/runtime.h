@@ -63,7 +63,7 @@ constexpr int kSortLevelsUsed = 48, kNmsRoundsUsed = 49;
 // d_small[kNmsNeed + m]: model m's kept set was resolved again in the quicksort's order
 constexpr int kNmsNeed = 160;
 void note_sort_levels(geye_ctx *ctx, Plan &P, int used, int rounds);
-// tensor-core fconvsMT of one feature map ([pos][32] float on the device) for the stage entry point
+// tensor-core fconvsMT of one feature map (float planes on the device) for the stage entry point
 geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, const float *const *filters,
                          const int *b_dims, int n_filters, float *d_out, const std::vector<int> &out_off,
                          std::vector<std::unique_ptr<DevBuf>> &tmp);
@@ -95,7 +95,7 @@ struct LevelInfo {
   int fs0 = 0, fs1 = 0;       // features
   int sbin = 0;
   float scale = 0.f;          // scales[] entry
-  int feat_off = -1;          // [pos][32]
+  int feat_off = -1;          // float planes
   int feat16_off = -1;        // tensor-core planes, 2-byte units
   int feat16lo_off = -1;      // BF16 remainder planes (root levels, BF16 mode), 2-byte units
   int hist_off = -1;
@@ -104,17 +104,13 @@ struct LevelInfo {
 struct ModelPlan {
   geye_model *model = nullptr;
   int LEN = 0;                          // levels this model uses
-  std::vector<ConvJob> root_jobs, part_jobs;
-  int root_max_b0 = 0, root_max_b1 = 0, root_max_g = 1, root_tiles_y = 0, root_tiles_x = 0;
-  int part_max_b0 = 0, part_max_b1 = 0, part_max_g = 1, part_tiles_y = 0, part_tiles_x = 0;
-  int root_cr = 4, part_cr = 4;   // FP32 conv rows per thread (tuned per plan)
   std::vector<DtJob> dt_jobs;
   int dt_max_d0 = 0, dt_max_d1 = 0;
   std::vector<ScoreJob> score_jobs;
   int score_max_r = 0;
   int cap = 0;                          // max detections (sum of root map sizes)
   // device copies
-  DevBuf d_root_jobs, d_part_jobs, d_dt_jobs, d_score_jobs, d_counts;
+  DevBuf d_dt_jobs, d_score_jobs, d_counts;
   DevBuf d_dt_blocks1, d_dt_blocks2;    // DT tiles of every map (dt_block_lists)
   int dt_nblocks1 = 0, dt_nblocks2 = 0;
   int dt_elems = kDtElems;              // outputs per DT block: tuned on the plan's first frame (tune_dt)
@@ -188,6 +184,12 @@ struct Plan {
   int pix_max_xe = 0;
   std::vector<std::unique_ptr<ModelPlan>> models;
   TcPlan tc;                             // BF16 / FP8 modes
+  // FP32 mode: the filter groups of every model and level, one launch
+  std::vector<ConvJob> conv_jobs;
+  ConvBank conv_bank;
+  DevBuf d_conv_jobs, d_conv_blocks, d_conv_bank;
+  int conv_nblocks = 0;
+  size_t conv_smem = 0;
   // memory
   size_t arena_words = 0, arena16_elems = 0;
   DevBuf arena, arena16;

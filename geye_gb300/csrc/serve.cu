@@ -425,9 +425,10 @@ namespace geye {
 size_t plan_device_bytes(const Plan &P) {
   size_t b = P.arena.bytes + P.arena16.bytes + P.d_bgr.bytes + P.d_boxes.bytes + P.d_kept_boxes.bytes +
              P.d_nms_f.bytes + P.d_nms_i.bytes + P.d_small.bytes + P.d_ascore.bytes + P.d_result.bytes;
+  b += P.d_conv_jobs.bytes + P.d_conv_blocks.bytes + P.d_conv_bank.bytes;
   b += P.tc.d_bank.bytes + P.tc.d_jobs.bytes + P.tc.d_chunks.bytes + P.tc.d_cols.bytes + P.tc.d_sums.bytes;
   for (auto &mp : P.models)
-    b += mp->d_root_jobs.bytes + mp->d_part_jobs.bytes + mp->d_dt_jobs.bytes + mp->d_score_jobs.bytes +
+    b += mp->d_dt_jobs.bytes + mp->d_score_jobs.bytes +
          mp->d_dt_blocks1.bytes + mp->d_dt_blocks2.bytes + mp->d_score_blocks.bytes +
          mp->d_counts.bytes + mp->d_as_col.bytes + mp->d_as_row.bytes;
   return b;

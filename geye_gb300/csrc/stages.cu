@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -12,8 +13,8 @@
 
 namespace geye {
 geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step);
-geye_status run_hog(geye_ctx *ctx, Plan &P);
-geye_status run_conv(geye_ctx *ctx, Plan &P, ModelPlan &mp);
+geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats);
+geye_status run_conv(geye_ctx *ctx, Plan &P);
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp);
 geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh);
 geye_status run_ascore(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, const float *h_init);
@@ -166,7 +167,7 @@ geye_status geye_calc_feature(geye_ctx *ctx, const float *src, const int *isize,
   HogPixJob X{};
   X.img_off = 0; X.h = h; X.w = w; X.xe = b1 * sbin - 1; X.ye = b0 * sbin - 1; X.Y = X.ye + 1;
   const size_t n_pix = (size_t)(X.xe + 1) * X.Y;
-  const size_t mag_off = ((feat_off + (size_t)fs0 * fs1 * kFeatPad + 31) & ~size_t(31));
+  const size_t mag_off = ((feat_off + feat_words(fs0, fs1) + 31) & ~size_t(31));
   const size_t bin_off = ((mag_off + n_pix + 31) & ~size_t(31));
   const size_t corner_off = ((bin_off + (n_pix + 3) / 4 + 31) & ~size_t(31));
   X.mag_off = (int)mag_off; X.bin_off = (int)bin_off;
@@ -186,7 +187,7 @@ geye_status geye_calc_feature(geye_ctx *ctx, const float *src, const int *isize,
   hog_vote_blocks(std::vector<HogJob>{J}, vb);
   int2 *d_vb;
   GEYE_TRY(S.put(vb.data(), vb.size(), &d_vb));
-  launch_hog(d_j, 1, d_vb, (int)vb.size(), b0, b1, d_x, 1, X.xe, arena, nullptr, true, ctx->stream);
+  launch_hog(d_j, 1, d_vb, (int)vb.size(), b0, b1, d_x, 1, X.xe, arena, nullptr, true, true, ctx->stream);
   launch_to_ref_layout(arena + feat_off, fs0, fs1, out, ctx->stream);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(feat, out, sizeof(float) * (size_t)fs0 * fs1 * kFeat, cudaMemcpyDeviceToHost, ctx->stream));
@@ -206,7 +207,7 @@ geye_status geye_calc_f_pyramid(geye_ctx *ctx, geye_model *model, const uint8_t 
   CUDA_TRY(cudaMemcpy2DAsync(P->d_bgr.p, (size_t)3 * width, bgr, width_step, (size_t)3 * width, height,
                              cudaMemcpyHostToDevice, ctx->stream));
   GEYE_TRY(run_pyramid(ctx, *P, P->d_bgr.as<uint8_t>(), 3 * width));
-  GEYE_TRY(run_hog(ctx, *P));
+  GEYE_TRY(run_hog(ctx, *P, true));
   const int LEN = P->models[0]->LEN;
   size_t total = 0;
   for (int l = 0; l < LEN; l++) total += (size_t)P->lv[l].fs0 * P->lv[l].fs1 * kFeat;
@@ -267,7 +268,7 @@ geye_status geye_get_boxes(geye_ctx *ctx, geye_model *model, const float *featur
   }
   ModelPlan &mp = *P->models[0];
   CUDA_TRY(cudaMemsetAsync(P->d_small.p, 0, 4096, ctx->stream));
-  GEYE_TRY(run_conv(ctx, *P, mp));
+  GEYE_TRY(run_conv(ctx, *P));
   GEYE_TRY(run_dt(ctx, *P, mp));
   GEYE_TRY(run_score(ctx, *P, mp, 0, thresh));
   if (a_score && img_width > 0 && img_height > 0) GEYE_TRY(run_ascore(ctx, *P, mp, 0, thresh, a_score));
@@ -407,46 +408,50 @@ geye_status geye_fconv(geye_ctx *ctx, const float *feat, const int *a_dims, cons
   ARG_CHECK(a0 > 0 && a1 > 0, "empty feature map");
   CUDA_TRY(cudaSetDevice(ctx->device));
   Scratch S(ctx);
-  const size_t cells = (size_t)a0 * a1;
-  float *d_ref, *arena, *d_filt;
-  int *d_off;
-  GEYE_TRY(S.put(feat, cells * kFeat, &d_ref));
-  std::vector<float> all;
-  std::vector<int> off;
-  std::vector<ConvJob> jobs;
+  const size_t words = (feat_words(a0, a1) + 31) & ~size_t(31);   // the features, then the maps
+  float *d_ref, *arena;
+  GEYE_TRY(S.put(feat, (size_t)a0 * a1 * kFeat, &d_ref));
+  std::vector<int> out_off;
   size_t out_words = 0;
-  int mb0 = 0, mb1 = 0, mty = 0, mtx = 0;
   for (int i = 0; i < n_filters; i++) {
     const int b0 = b_dims[2 * i], b1 = b_dims[2 * i + 1];
     ARG_CHECK(b0 > 0 && b1 > 0 && b0 <= a0 && b1 <= a1, "filter larger than the feature map");
-    off.push_back((int)all.size());
-    all.insert(all.end(), filters[i], filters[i] + (size_t)b0 * b1 * kFeat);
-    ConvJob J{};
-    J.feat_off = 0; J.a0 = a0; J.a1 = a1; J.filt_base = i; J.n_filt = 1; J.b0 = b0; J.b1 = b1;
-    J.c0 = a0 - b0 + 1; J.c1 = a1 - b1 + 1;
-    J.out_off = (int)(cells * kFeatPad + out_words);
-    J.tiles_y = (J.c0 + 31) / 32; J.tiles_x = (J.c1 + 15) / 16;
-    out_words += (size_t)J.c0 * J.c1;
-    mb0 = std::max(mb0, b0); mb1 = std::max(mb1, b1);
-    mty = std::max(mty, J.tiles_y); mtx = std::max(mtx, J.tiles_x);
-    jobs.push_back(J);
+    out_off.push_back((int)(words + out_words));
+    out_words += (size_t)(a0 - b0 + 1) * (a1 - b1 + 1);
   }
-  GEYE_TRY(S.get(cells * kFeatPad + out_words, &arena));
-  GEYE_TRY(S.put(all.data(), all.size(), &d_filt));
-  GEYE_TRY(S.put(off.data(), off.size(), &d_off));
-  ConvJob *d_jobs;
-  GEYE_TRY(S.put(jobs.data(), jobs.size(), &d_jobs));
+  GEYE_TRY(S.get(words + out_words, &arena));
   launch_from_ref_layout(d_ref, a0, a1, arena, ctx->stream);
   if (ctx->conv_mode != GEYE_CONV_FP32) {
-    std::vector<int> out_off;
-    for (auto &J : jobs) out_off.push_back(J.out_off);
     std::vector<std::unique_ptr<DevBuf>> tmp;
     GEYE_TRY(conv_tc_maps(ctx, arena, a0, a1, filters, b_dims, n_filters, arena, out_off, tmp));
   } else {
-    launch_conv_fp32(d_jobs, (int)jobs.size(), mty, mtx, d_filt, d_off, arena, arena, mb0, mb1, 1, ctx->stream);
+    std::map<std::pair<int, int>, std::vector<int>> by_size;
+    for (int i = 0; i < n_filters; i++) by_size[{b_dims[2 * i], b_dims[2 * i + 1]}].push_back(i);
+    std::vector<ConvJob> jobs;
+    ConvBank bank;
+    for (auto &f : by_size) {
+      ConvJob J{};
+      J.a0 = a0; J.a1 = a1; J.b0 = f.first.first; J.b1 = f.first.second;
+      std::vector<const float *> w;
+      std::vector<int> o;
+      for (int i : f.second) { w.push_back(filters[i]); o.push_back(out_off[i]); }
+      if (!conv_fp32_jobs(J, w, o, bank, jobs)) {
+        set_error("filter too large for the FP32 convolution");
+        return GEYE_ERR_UNSUPPORTED;
+      }
+    }
+    std::vector<int2> blocks;
+    const size_t smem = conv_fp32_blocks(jobs, blocks);
+    float *d_bank;
+    ConvJob *d_jobs;
+    int2 *d_blocks;
+    GEYE_TRY(S.put(bank.taps.data(), bank.taps.size(), &d_bank));
+    GEYE_TRY(S.put(jobs.data(), jobs.size(), &d_jobs));
+    GEYE_TRY(S.put(blocks.data(), blocks.size(), &d_blocks));
+    launch_conv_fp32(d_jobs, d_blocks, (int)blocks.size(), smem, d_bank, arena, arena, ctx->stream);
   }
   CUDA_TRY(cudaGetLastError());
-  CUDA_TRY(cudaMemcpyAsync(out, arena + cells * kFeatPad, sizeof(float) * out_words, cudaMemcpyDeviceToHost,
+  CUDA_TRY(cudaMemcpyAsync(out, arena + words, sizeof(float) * out_words, cudaMemcpyDeviceToHost,
                            ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return GEYE_OK;
