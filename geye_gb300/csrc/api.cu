@@ -325,17 +325,16 @@ geye_status geye_model_reset_scales(geye_model *m) {
 // ---------------------------------------------------------------------------
 // whole path
 // ---------------------------------------------------------------------------
-static geye_status fetch_model_result(geye_ctx *ctx, Plan &P, int mi, geye_result *out, int *D_out,
-                                      float **kept_out) {
+static geye_status fetch_model_result(geye_ctx *ctx, Plan &P, int mi, geye_result *out, int *D_out) {
   int counts[4] = {0, 0, 0, 0};
   CUDA_TRY(cudaMemcpyAsync(&counts[0], P.d_small.as<int>() + mi, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaMemcpyAsync(&counts[1], P.d_small.as<int>() + 32 + mi, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   if (mi == 0)
-    CUDA_TRY(cudaMemcpyAsync(&counts[2], P.d_small.as<int>() + kSortLevelsUsed, 2 * sizeof(int),
-                             cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(&counts[2], P.d_small.as<int>() + kSortLevelsUsed, sizeof(int), cudaMemcpyDeviceToHost,
+                             ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   const int D = counts[0], K = counts[1];
-  if (mi == 0 && !P.from_features) note_sort_levels(ctx, P, counts[2], counts[3]);
+  if (mi == 0 && !P.from_features) note_sort_levels(ctx, P, counts[2]);
   if (D_out) *D_out = D;
   P.last_D[mi] = D;
   P.last_K[mi] = K;
@@ -362,13 +361,6 @@ static geye_status fetch_model_result(geye_ctx *ctx, Plan &P, int mi, geye_resul
       CUDA_TRY(cudaMemcpyAsync(out->score, res + 10 * P.max_cap, sizeof(float) * K, cudaMemcpyDeviceToHost, ctx->stream));
     }
   }
-  if (kept_out) {
-    const int GL = P.models[mi]->model->gl();
-    *kept_out = (float *)malloc(sizeof(float) * (size_t)std::max(K, 1) * GL);
-    if (K > 0)
-      CUDA_TRY(cudaMemcpyAsync(*kept_out, P.d_kept_boxes.as<float>() + (size_t)mi * P.max_cap * P.gl,
-                               sizeof(float) * (size_t)K * GL, cudaMemcpyDeviceToHost, ctx->stream));
-  }
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return GEYE_OK;
 }
@@ -389,7 +381,7 @@ geye_status geye_detect_multi(geye_ctx *ctx, geye_model *const *models, int n_mo
     for (int i = 0; i < n_models; i++) init[i] = a_scores[i];
   GEYE_TRY(run_frame(ctx, *P, P->d_bgr.as<uint8_t>(), 3 * width, thresh, overlap, init.data()));
   for (int i = 0; i < n_models; i++) {
-    GEYE_TRY(fetch_model_result(ctx, *P, i, &out[i], nullptr, nullptr));
+    GEYE_TRY(fetch_model_result(ctx, *P, i, &out[i], nullptr));
     if (a_scores && a_scores[i])
       CUDA_TRY(cudaMemcpyAsync(a_scores[i], P->d_ascore.as<float>() + (size_t)i * width * height,
                                sizeof(float) * (size_t)width * height, cudaMemcpyDeviceToHost, ctx->stream));
@@ -426,7 +418,7 @@ geye_status geye_detect_device(geye_ctx *ctx, geye_model *const *models, int n_m
 geye_status geye_fetch_result(geye_ctx *ctx, int model_index, geye_result *out, int *n_boxes_before_nms) {
   ARG_CHECK(ctx && ctx->last_plan, "no device-resident run to fetch");
   ARG_CHECK(model_index >= 0 && model_index < (int)ctx->last_plan->models.size(), "model index out of range");
-  return fetch_model_result(ctx, *ctx->last_plan, model_index, out, n_boxes_before_nms, nullptr);
+  return fetch_model_result(ctx, *ctx->last_plan, model_index, out, n_boxes_before_nms);
 }
 
 }  // extern "C"

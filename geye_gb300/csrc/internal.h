@@ -309,8 +309,8 @@ void launch_ascore_normalize(float *a_score, int n, const unsigned *max_bits, cu
 void launch_nms(const float *boxes, const int *d_num, int n_models, int GL, float overlap, int cap,
                 float *scratch_f, int *scratch_i, float *out, int *d_kept, int *err, cudaStream_t s);
 // pipeline NMS (nms_sort.cu, nms_batch.cu): per model nms_model_words(cap) ints
-// of scratch and 5 * cap floats (the boxes in sorted order)
-constexpr int kNmsBatch = 256;     // boxes resolved per round
+// of scratch and 10 * cap floats (the boxes in sorted order, the picks')
+constexpr int kNmsBatch = 512;     // boxes resolved per round
 constexpr int kNmsSegS = 16384;    // sort segments finished in shared memory (one block, ~203 KB)
 constexpr int kNmsTile = 4096;     // elements per block in the sort's grid-wide partitions
 __host__ __device__ inline int nms_big_cap(int cap) { return cap / kNmsSegS + 2; }
@@ -322,32 +322,35 @@ constexpr int kNmsLevels = 7;      // their sparse-table levels (spans of 1..64 
 // scan short when a model has a million boxes
 __host__ __device__ inline int nms_rs_tile(int cap) { return cap <= (1 << 18) ? 1024 : 4096; }
 __host__ __device__ inline int nms_rs_tiles(int cap) { return (cap + nms_rs_tile(cap) - 1) / nms_rs_tile(cap); }
-// summary bitmap: one bit per word of the alive bitmap
-__host__ __device__ inline int nms_summary_words(int cap) { return ((cap + 31) / 32 + 31) / 32 + 1; }
 __host__ __device__ inline size_t nms_model_words(int cap) {
-  const size_t w = 8 * (size_t)cap + 64 + 5 * kNmsBatch + 4 * (size_t)nms_big_cap(cap) +
-                   2 * (size_t)nms_tile_cap(cap) + 256 * (size_t)nms_rs_tiles(cap) + nms_summary_words(cap) +
-                   2 * kNmsLevels * kNmsCells * (kNmsBatch / 32);
+  const size_t w = 8 * (size_t)cap + 64 + 4 * (size_t)nms_big_cap(cap) + 2 * (size_t)nms_tile_cap(cap) +
+                   4 * 256 * (size_t)nms_rs_tiles(cap);
   return (w + 31) & ~(size_t)31;
 }
+// what the results are made from: per model its regression coefficients [comp][x1, y1, x2, y2][ML],
+// part count and ratio; out: 11 * cap ints per model (point, or_point, type, scale, score)
+struct NmsResults {
+  struct Model {
+    const float *coef;
+    int np;
+    float ratio;
+  } m[16];
+  int *out;
+  int img_w, img_h;
+};
 // diag (optional): per model m, diag[8m+1..8m+5] = sort segments left to the fallback, batches, picks,
-// whether the finish kernel ran rounds itself, whether the quicksort order was needed
-// levels, lv_used: as for launch_nms_sort (nms_common.h); rounds: resolve/pass
-// rounds launched before the finish kernel (<= 0: kNmsRounds), *rounds_used
-// (optional) gets the batches the frame took, the finish kernel's included
+// 0, whether the quicksort order was needed
+// levels, lv_used: as for launch_nms_sort (nms_common.h)
 // need: n_models ints, zero on entry; order: kNmsOrderKey (the scores in
 // key order, the quicksort's order only for the models that need it: need[m]
 // raised) or kNmsOrderQuicksort (the quicksort's order for every model)
-constexpr int kNmsRounds = 8, kNmsMaxRounds = 64;
 constexpr int kNmsOrderKey = 0, kNmsOrderQuicksort = 1;
 // aux: null for plain launches on s; when s is capturing a graph, a second
 // stream that captures the body of the quicksort-order pass's if node
-// extent: box coordinates in [0, extent) spread over the pick masks' cells
-// (any value is exact; boxes outside share the edge cells)
 cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
-                             float extent, int cap, int *si, float *sf, float *out, int *d_kept, int *err,
-                             long long *diag, int levels, int *lv_used, int rounds, int *rounds_used, int *need,
-                             int order, cudaStream_t s, cudaStream_t aux);
+                             int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
+                             long long *diag, int levels, int *lv_used, int *need, int order, cudaStream_t s,
+                             cudaStream_t aux);
 int nms_sort_levels(int cap);   // the default number of grid-wide sort levels for cap boxes
 void launch_new_rects(const float *kept, const int *d_kept, int GL, int np, const float *coef, int img_w,
                       int img_h, float ratio, int *point, int *or_point, int *type, float *scale, float *score,

@@ -3,101 +3,117 @@
 // Same kept set as nms.cu (CAR_TRACKING/nms.cpp:70-217): the reference's Hoare
 // quicksort order for equal scores, greedy suppression by intersection over
 // the smaller area or containment, and a box that is alone when its turn comes
-// never emitted.  The greedy loop is restated so that most of it runs on every
-// SM:
+// never emitted.
 //
-//  1. the order: score order from the radix sort (nms_radix.cu), checked for
+//  1. The order: score order from the radix sort (nms_radix.cu), checked for
 //     the cases where the quicksort's order among equal scores could change
-//     the kept set; the models that raise them go through steps 2-4 again in
-//     the quicksort's order (nms_sort.cu).
-//  2. k_nms_gather: the boxes in sorted order (structure of arrays), an alive
-//     bitmap over sorted positions and its summary (one bit per word).
-//  3. Rounds of two kernels, each a no-op for a model that is done:
-//     k_nms_resolve (one block per model) takes the first kBatch alive boxes
-//     in sorted order (found through the summary), computes for each member
-//     which earlier members suppress it (pairs whose cell spans overlap) and
-//     decides the members in parallel rounds: a member is picked when every
-//     earlier member that suppresses it is decided and none is picked, and
-//     removed when an earlier pick suppresses it -- the sequential loop's
-//     decisions, since every box before the batch is already resolved.  It
-//     then lists its picks by image cell on each axis.
-//     k_nms_pass (grid) tests every other alive box against the picks that
-//     share a row cell and a column cell with it, in pick order; the first
-//     pick that suppresses it is the one the sequential loop would have
-//     removed it with.
-//  4. k_nms_finish (one block per model) runs any remaining rounds itself,
-//     drops the final pick if it suppressed nothing (the reference's
-//     `while (cnum > 0)` with cnum = NUM-1 never takes a box that is alone at
-//     its turn) and writes the kept records in input order.
+//     the kept set; the models that raise them go through step 2 again in
+//     the quicksort's order (nms_sort.cu, k_nms_gather).
+//  2. k_nms_greedy, a cluster of kCluster blocks per model, walks the boxes in
+//     that order, a chunk at a time:
+//       - the cluster tests the chunk's boxes against the picks so far that can
+//         suppress them (found by image cell).  Which of several does is of no
+//         account, but for the last pick of all (step 3): it counts only for
+//         boxes that no earlier one removed;
+//       - rounds over the boxes left alive: every block alike takes the first
+//         kBatch of them; the blocks share the tests of every pair of those, a
+//         bit per pair, written into the first block's shared memory; that
+//         block walks them in order, a bit of each in registers: the first
+//         undecided one is picked and its row of suppressed members struck out
+//         -- the sequential loop's decisions, since every box before the batch
+//         is resolved.  Boxes of the chunk still alive are tested against the
+//         new picks.
+//     A chunk is sized so that about a batch of it survives: a few hundred boxes
+//     at the head of the order, most of them at its end.
+//     Where there are more than kWhole boxes it stops after the first kPrefix:
+//     by then nearly every pick is made.  k_nms_rest tests the others over the
+//     whole grid, and a second cluster launch takes the few survivors.
+//  3. The first block drops the final pick if it suppressed nothing (the
+//     reference's `while (cnum > 0)` with cnum = NUM-1 never takes a box that is
+//     alone at its turn) and writes the results in input order.
+//
+// What bounds it is latency: rounds depend on one another, and so do the steps
+// of a round (L2 reads of a thousand cycles, cluster barriers of 1200, the walk's
+// 200 a pick).  Tried before, 640x480 car+person, NMS stage: 256 members a round
+// resolved by one block, a pass of all alive boxes over the grid, 285 us; 512
+// members, the pair tests by 32 blocks handing over by a ticket, 155 us; one
+// cluster kernel for all rounds with a pass of all alive boxes each, 147 us;
+// this form 157 us (320x240 car: 135 -> 73, 1280x720: 575 -> 399, 1280x720 trained-like:
+// 280 -> 170, 1920x1080 with a model in the quicksort's order: 2414 -> 1833).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "nms_common.h"
+#include "rects.h"
 
 namespace geye {
 
-constexpr int kSortNT = kNmsNT;   // threads of the resolve and finish blocks
+namespace cg = cooperative_groups;
+
+constexpr int kCluster = 16;         // blocks per model (8 where a device cannot place 16)
+constexpr int kResNT = 512, kResWarps = kResNT / 32;
 constexpr int kBatch = kNmsBatch;
-constexpr int kBW = kBatch / 32;   // words of a suppression row
-constexpr int kPassNT = 256;
-constexpr int kRankSortMax = 4096; // kept boxes ordered by ranking in shared memory up to this many
+constexpr int kBW = kBatch / 32;     // words of a suppression row
+constexpr int kPickGroup = 256;      // picks per table of a pass
+constexpr int kGW = kPickGroup / 32;
+constexpr int kPassNT = 256;         // k_nms_gather's blocks
+constexpr int kPrefix = 1 << 16;     // boxes that the first launch takes where there are more than kWhole (the rest
+constexpr int kWhole = 160000;       // of up to 100 000 costs the cluster less than two launches more)
+constexpr int kWinWords = 4 * kResNT;   // words of a chunk's window
+constexpr int kMaxChunk = 32 * (kWinWords - 2);   // with the run at its end
+constexpr int kChunkCap = 60000;
+static_assert(kBatch == kResNT, "a thread per member");
 
 // ---------------------------------------------------------------------------
-// 2. sorted boxes and the alive bitmap
+// the boxes in the quicksort's order (the radix sort brings its own)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kPassNT) k_nms_gather(const float *__restrict__ boxes_all, int GL, int cap, int *si,
                                                         float *sf) {
   const int m = blockIdx.y;
   Slots S = slots(si, sf, m, cap);
   const float *boxes = boxes_all + (size_t)m * cap * GL;
-  const int D = S.st->D;
   const int r = blockIdx.x * kPassNT + threadIdx.x;
-  if (r < D) {
+  if (r < S.st->D) {
     const float *P = boxes + (size_t)S.ord[r] * GL;
     S.y1[r] = P[0]; S.x1[r] = P[1]; S.y2[r] = P[2]; S.x2[r] = P[3];
     S.ar[r] = (P[3] - P[1] + 1.0) * (P[2] - P[0] + 1.0);   // nms.cpp's area expression
   }
-  const unsigned bal = __ballot_sync(0xffffffffu, r < D);
-  const int nwords = (D + 31) >> 5;
-  if ((threadIdx.x & 31) == 0 && (r >> 5) < nwords) S.bits[r >> 5] = bal;
-  // summary: every word below nwords starts with an alive box
-  if (r < (nwords + 31) >> 5) {
-    const int n = min(32, nwords - 32 * r);
-    S.sbits[r] = n == 32 ? ~0u : (1u << n) - 1u;
-  }
 }
 
-// clears the alive bits `clear` of word w (more than one thread may clear bits
-// of the same word); the last clear of a word clears its summary bit
-__device__ __forceinline__ void clear_alive(const Slots &S, int w, unsigned clear) {
-  const unsigned old = atomicAnd(&S.bits[w], ~clear);
-  if (old != 0u && (old & ~clear) == 0u) atomicAnd(&S.sbits[w >> 5], ~(1u << (w & 31)));
-}
-
-// cell of a coordinate on one axis of the pick masks (monotone; NaN to cell 0)
+// cell of a coordinate on one axis of the pick tables (monotone; NaN to cell 0); inv: cells per pixel (.x: y axis, .y: x axis)
 __device__ __forceinline__ int nms_cell(float v, float inv) {
   return (int)fminf(fmaxf(v * inv, 0.0f), (float)(kNmsCells - 1));
 }
 
-// ---------------------------------------------------------------------------
-// 3a. resolve the next batch (whole block)
-// ---------------------------------------------------------------------------
-struct ResolveSmem {
-  int mem_pos[kBatch + 1];
-  int wl[kBatch + 1];    // non-empty words of the alive bitmap holding the members
-  int run_end[kBatch];   // key order: last member with the same score
-  unsigned key[kBatch + 1];   // key order: the candidates' keys
-  float my[5][kBatch];
-  unsigned cm[2][kNmsCells][kBW];   // the picks by cell, built for the pass
-  unsigned und[kBW], pk_bits[kBW];  // undecided and picked members
-  int killed_any[kBatch];           // member (a pick) removed a member alive at its turn
-  unsigned span[kBatch];            // member's cell span (bytes y0, y1, x0, x1)
-  int pick_mem[kBatch];
-  int pick_any[kBatch];
-  int wtot[kSortNT / 32];
-  int nb, nw, np, last_word, done;
+__device__ __forceinline__ unsigned sorted_key(const Slots &S, int pos) {
+  return reinterpret_cast<const unsigned *>(S.val)[pos];
+}
+
+struct PickTable {   // see pick_table
+  unsigned covers[2][kGW][kNmsCells];
+  unsigned in_span[2][kNmsLevels][kGW][kNmsCells];
 };
 
-// exclusive block scan of c (kSortNT threads); *tot gets the sum
+struct GreedySmem {
+  union {
+    unsigned adj[kBatch * kBW];   // the members' rows (the first block's)
+    PickTable table;
+    int idx[kBatch * kBW];        // at the end: the kept boxes
+  };
+  float4 pk[kBatch];              // the tested picks' boxes and areas
+  float pka[kBatch];
+  float my[5][kBatch];            // members' boxes
+  int item[kBatch + 1], pos[kBatch + 1];   // members' items and sorted positions
+  unsigned key[kBatch + 1];       // key order: the candidates' keys
+  int pick_mem[kBatch];
+  int pick_any[kBatch];           // the pick removed a member alive at its turn
+  int wtot[kResWarps];
+  int total[kCluster];            // (the first block's) the blocks' survivors
+  int nb, np, tot;
+};
+
+// exclusive block scan of c (kResNT threads); *tot gets the sum
 __device__ __forceinline__ int block_excl_scan(int c, int *tot, int *wtot) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int inc = c;
@@ -110,7 +126,8 @@ __device__ __forceinline__ int block_excl_scan(int c, int *tot, int *wtot) {
   if (lane == 31) wtot[warp] = inc;
   __syncthreads();
   int before = inc - c, t = 0;
-  for (int k = 0; k < kSortNT / 32; k++) {
+#pragma unroll
+  for (int k = 0; k < kResWarps; k++) {
     const int v = wtot[k];
     if (k < warp) before += v;
     t += v;
@@ -119,495 +136,497 @@ __device__ __forceinline__ int block_excl_scan(int c, int *tot, int *wtot) {
   return before;
 }
 
-__device__ __forceinline__ unsigned sorted_key(const Slots &S, int pos) {
-  return reinterpret_cast<const unsigned *>(S.val)[pos];
-}
-
-// Returns with R.np picks in R.pick_mem, the batch's picks appended to S.picks
-// and written to S.bp, the members cleared from the bitmap and the state
-// advanced; R.done set when no alive box was left.
-// KEY_ORDER (positions in nms_radix.cu's order): a run of equal scores never
-// straddles two batches (the batch ends before a run that the next alive box
-// continues), and *need is raised where the order inside a run could matter:
-// a pick that suppresses an alive member of its own run, or a run longer than
-// a batch.
-template <bool KEY_ORDER>
-__device__ void resolve_batch(Slots &S, float overlap, float cell_inv, ResolveSmem &R, int *need) {
-  constexpr int want = kBatch + (KEY_ORDER ? 1 : 0);   // key order: one more, to see the run at the boundary
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  BatchState &st = *S.st;
-  const int nwords = st.nwords;
-  if (threadIdx.x == 0) R.nw = 0;
-  __syncthreads();
-  // members: the first `want` alive sorted positions from scan_word on, found
-  // through the summary (words before scan_word hold no alive box): the first
-  // `want` non-empty words, then the first `want` alive bits of those
-  const int nsw = (nwords + 31) >> 5;
-  for (int sb = st.scan_word >> 5; sb < nsw; sb += kSortNT) {
-    const int have = R.nw;   // uniform: written before the last barrier
-    if (have >= want) break;
-    const int j = sb + threadIdx.x;
-    const unsigned sw = j < nsw ? S.sbits[j] : 0u;
-    int tot;
-    int rank = have + block_excl_scan(__popc(sw), &tot, R.wtot);
-    unsigned rem = sw;
-    while (rem && rank < want) {
-      R.wl[rank++] = (j << 5) + __ffs(rem) - 1;
-      rem &= rem - 1;
-    }
-    __syncthreads();   // everyone has read R.nw
-    if (threadIdx.x == 0) R.nw = min(want, have + tot);
-    __syncthreads();
-  }
-  const int nw = R.nw;
-  {
-    const int w = threadIdx.x < nw ? R.wl[threadIdx.x] : 0;
-    const unsigned word = threadIdx.x < nw ? S.bits[w] : 0u;
-    int tot;
-    int rank = block_excl_scan(__popc(word), &tot, R.wtot);
-    unsigned rem = word;
-    while (rem && rank < want) {
-      const int r = (w << 5) + __ffs(rem) - 1;
-      R.mem_pos[rank] = r;
-      if (KEY_ORDER) R.key[rank] = sorted_key(S, r);
-      rank++;
-      rem &= rem - 1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int nb = min(want, tot);
-      // every alive box is a member: the summary was exhausted and held no more than a batch
-      const bool all_taken = nw < want && tot <= kBatch;
-      if (KEY_ORDER && nb == want) {   // an alive box follows the batch: end before its run
-        const unsigned kb = R.key[kBatch];
-        int lo = 0, hi = kBatch;   // first candidate with key kb (keys ascend): in [lo, hi]
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (R.key[mid] < kb) lo = mid + 1;
-          else hi = mid;
-        }
-        nb = lo;
-        if (nb == 0) {   // a run longer than a batch
-          *need = 1;
-          nb = kBatch;
-        }
-      }
-      R.nb = nb;
-      R.last_word = (all_taken || nb == 0) ? nwords : (R.mem_pos[nb - 1] >> 5);
-    }
-    __syncthreads();
-  }
-  const int nb = R.nb;
-  // members' boxes
-  if (threadIdx.x < nb) {
-    const int r = R.mem_pos[threadIdx.x];
-    R.my[0][threadIdx.x] = S.y1[r];
-    R.my[1][threadIdx.x] = S.x1[r];
-    R.my[2][threadIdx.x] = S.y2[r];
-    R.my[3][threadIdx.x] = S.x2[r];
-    R.my[4][threadIdx.x] = S.ar[r];
-    if (KEY_ORDER) {   // last member with this key (keys ascend)
-      const unsigned k = R.key[threadIdx.x];
-      int lo = threadIdx.x, hi = nb - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (R.key[mid] == k) lo = mid;
-        else hi = mid - 1;
-      }
-      R.run_end[threadIdx.x] = lo;
-    }
-  }
-  __syncthreads();
-  // The batch's decisions, in parallel rounds.  Four threads per member j
-  // hold its column (bit i of word w: member i < j suppresses j; thread q of
-  // the group: words q and q + 4).  A round decides every undecided member
-  // that an earlier pick suppresses (removed) or whose earlier suppressors
-  // are all decided and none picked (picked): the sequential walk's decision
-  // for it, since the members before it are decided as the walk would.  The
-  // first undecided member is always decided, so the rounds end.
-  const int nwm = (nb + 31) >> 5;
-  const int gj = threadIdx.x >> 2, gq = threadIdx.x & 3;
-  // each member's cell span, widened by two pixels (bytes y0, y1, x0, x1): two
-  // boxes that can suppress each other have overlapping spans on both axes
-  if (threadIdx.x < nb) {
-    const int i = threadIdx.x;
-    const int y0 = nms_cell(fminf(R.my[0][i], R.my[2][i]) - 2.0f, cell_inv);
-    const int y1 = nms_cell(fmaxf(R.my[0][i], R.my[2][i]) + 2.0f, cell_inv);
-    const int x0 = nms_cell(fminf(R.my[1][i], R.my[3][i]) - 2.0f, cell_inv);
-    const int x1 = nms_cell(fmaxf(R.my[1][i], R.my[3][i]) + 2.0f, cell_inv);
-    R.span[i] = (unsigned)y0 | ((unsigned)y1 << 8) | ((unsigned)x0 << 16) | ((unsigned)x1 << 24);
-  }
-  __syncthreads();
-  unsigned col[2] = {0u, 0u};
-  if (gj < nb) {
-    const float b0 = R.my[0][gj], b1 = R.my[1][gj], b2 = R.my[2][gj], b3 = R.my[3][gj], b4 = R.my[4][gj];
-    const unsigned sj = R.span[gj];
-    const int jy0 = sj & 255, jy1 = (sj >> 8) & 255, jx0 = (sj >> 16) & 255, jx1 = sj >> 24;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int w = gq + 4 * h;
-      const int i0 = 32 * w, i1 = min(i0 + 32, gj);
-      unsigned word = 0u;
-      for (int i = i0; i < i1; i++) {
-        const unsigned si_ = R.span[i];
-        if ((int)(si_ & 255) > jy1 || (int)((si_ >> 8) & 255) < jy0 || (int)((si_ >> 16) & 255) > jx1 ||
-            (int)(si_ >> 24) < jx0)
-          continue;
-        if (supp(R.my[0][i], R.my[1][i], R.my[2][i], R.my[3][i], R.my[4][i], b0, b1, b2, b3, b4, overlap))
-          word |= 1u << (i - i0);
-      }
-      col[h] = word;
-    }
-  }
-  if (threadIdx.x < kBW) {
-    const int w = threadIdx.x;
-    R.und[w] = w < nwm ? ((w == nwm - 1 && (nb & 31)) ? (1u << (nb & 31)) - 1u : ~0u) : 0u;
-    R.pk_bits[w] = 0u;
-  }
-  if (threadIdx.x < kBatch) R.killed_any[threadIdx.x] = 0;
-  __syncthreads();
-  for (int round = 0; round <= kBatch; round++) {
-    const bool mine_und = gj < nb && ((R.und[gj >> 5] >> (gj & 31)) & 1u);
-    int hp = ((col[0] & R.pk_bits[gq]) | (col[1] & R.pk_bits[gq + 4])) != 0u;
-    int hu = ((col[0] & R.und[gq]) | (col[1] & R.und[gq + 4])) != 0u;
-    hp |= __shfl_xor_sync(0xffffffffu, hp, 1);
-    hp |= __shfl_xor_sync(0xffffffffu, hp, 2);
-    hu |= __shfl_xor_sync(0xffffffffu, hu, 1);
-    hu |= __shfl_xor_sync(0xffffffffu, hu, 2);
-    const bool decide = mine_und && (hp || !hu), pick = decide && !hp;
-    __syncthreads();   // every group has read the round's state
-    if (gq == 0 && decide) {
-      atomicAnd(&R.und[gj >> 5], ~(1u << (gj & 31)));
-      if (pick) atomicOr(&R.pk_bits[gj >> 5], 1u << (gj & 31));
-    }
-    __syncthreads();
-    unsigned left = 0u;
-#pragma unroll
-    for (int w = 0; w < kBW; w++) left |= R.und[w];
-    if (!left) break;
-  }
-  // a removed member's first suppressor among the picks removed it in the
-  // walk: that pick suppressed a box alive at its turn (its flag); in key
-  // order, a pick that removes a member of its own run of equal scores needs
-  // the quicksort's order
-  {
-    const bool removed = gj < nb && !((R.pk_bits[gj >> 5] >> (gj & 31)) & 1u);
-    const unsigned h0 = removed ? col[0] & R.pk_bits[gq] : 0u, h1 = removed ? col[1] & R.pk_bits[gq + 4] : 0u;
-    int wfirst = h0 ? gq : (h1 ? gq + 4 : 64);   // smallest word with a suppressing pick
-    wfirst = min(wfirst, __shfl_xor_sync(0xffffffffu, wfirst, 1));
-    wfirst = min(wfirst, __shfl_xor_sync(0xffffffffu, wfirst, 2));
-    const unsigned hw = wfirst == gq ? h0 : (wfirst == gq + 4 ? h1 : 0u);
-    if (hw) {
-      const int killer = 32 * wfirst + __ffs(hw) - 1;
-      R.killed_any[killer] = 1;
-      if (KEY_ORDER && R.key[killer] == R.key[gj]) *need = 1;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < nb && ((R.pk_bits[threadIdx.x >> 5] >> (threadIdx.x & 31)) & 1u)) {
-    int rank = __popc(R.pk_bits[threadIdx.x >> 5] & ((1u << (threadIdx.x & 31)) - 1u));
-    for (int w = 0; w < (threadIdx.x >> 5); w++) rank += __popc(R.pk_bits[w]);
-    R.pick_mem[rank] = threadIdx.x;
-    R.pick_any[rank] = R.killed_any[threadIdx.x];
-  }
-  if (threadIdx.x == 0) {
-    int np = 0;
-    for (int w = 0; w < kBW; w++) np += __popc(R.pk_bits[w]);
-    R.np = np;
-  }
-  __syncthreads();
-  const int np = R.np, base = st.npicks;
-  for (int k = threadIdx.x; k < np; k += kSortNT) {
-    const int i = R.pick_mem[k];
-    S.picks[base + k] = R.mem_pos[i];
-    S.flag[base + k] = R.pick_any[k];
-    for (int c = 0; c < 5; c++) S.bp[c * kBatch + k] = R.my[c][i];
-  }
-  // the picks by cell for the pass (the suppression rows are free now): a
-  // pick is listed on every cell of its span widened by two pixels, so a box
-  // that it can suppress (positive overlap, or containment) shares a row and a
-  // column cell with it
-  unsigned *cm = &R.cm[0][0][0];   // [axis][cell][kBW]
-  for (int k = threadIdx.x; k < 2 * kNmsCells * kBW; k += kSortNT) cm[k] = 0u;
-  __syncthreads();
-  for (int k = threadIdx.x; k < np; k += kSortNT) {
-    const int i = R.pick_mem[k];
-    const unsigned bit = 1u << (k & 31);
-    for (int a = 0; a < 2; a++) {   // a = 0: y (my[0], my[2]); 1: x (my[1], my[3])
-      const float lo = fminf(R.my[a][i], R.my[a + 2][i]) - 2.0f, hi = fmaxf(R.my[a][i], R.my[a + 2][i]) + 2.0f;
-      const int c1 = nms_cell(hi, cell_inv);
-      for (int c = nms_cell(lo, cell_inv); c <= c1; c++) atomicOr(&cm[(a * kNmsCells + c) * kBW + (k >> 5)], bit);
-    }
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < 2 * kNmsCells * kBW; k += kSortNT) S.cmask[k] = cm[k];
-  for (int k = threadIdx.x; k < nb; k += kSortNT) {
-    const int r = R.mem_pos[k];
-    clear_alive(S, r >> 5, 1u << (r & 31));   // every member is resolved
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    st.npicks = base + np;
-    st.npb = np;
-    st.scan_word = R.last_word;
-    st.batches += 1;
-    // done once no alive box is left: none found, or this batch took every
-    // one up to the end of the bitmap (its pass would test nothing)
-    if (nb == 0 || R.last_word >= nwords) st.done = 1;
-    R.done = nb == 0;
-  }
-  __syncthreads();
-}
-
-template <bool KEY_ORDER>
-__global__ void __launch_bounds__(kSortNT) k_nms_resolve(int cap, int *si, float *sf, float overlap, float cell_inv,
-                                                         int *need) {
-  __shared__ ResolveSmem R;
-  Slots S = slots(si, sf, blockIdx.x, cap);
-  if (S.st->done) return;
-  resolve_batch<KEY_ORDER>(S, overlap, cell_inv, R, need ? need + blockIdx.x : nullptr);
-}
-
 // ---------------------------------------------------------------------------
-// 3b. test the alive boxes against the batch's picks (warps own bitmap words):
-// each alive box is removed by the first pick, in pick order, that suppresses
-// it, and that pick is flagged; sparse words take a box at a time against 32
-// picks a step, dense ones a pick at a time against 32 boxes a step
+// tests against picks
 // ---------------------------------------------------------------------------
-__device__ void pass_words(Slots &S, const float (*pk)[kBatch], int np, int pick_base, float overlap, int gwarp,
-                           int nwarps) {
+// Which picks can suppress a box.  With an overlap of a half or more, a pick and a box where one suppresses the other
+// share more than half of the smaller one's area, so more than half of its width and of its height, so its centre:
+// the pick covers the box's centre, or the box the pick's.  (Boxes of the pipeline are proper, so containment is an
+// overlap; two pixels of slack cover the + 1 of the reference's widths and every rounding.)  With a smaller
+// overlap they only share a cell on each axis.
+//
+// The table of np <= kPickGroup picks by cell: `covers` lists a pick on every cell of its widened span, `in_span` what
+// a box's span is looked up in (half: the picks' centres; else their spans again) with the unions over 2^l cells,
+// so that a span is the union of two entries.  A warp per axis and word of picks, two cells a lane.
+__device__ __forceinline__ void pick_table(PickTable &T, const float4 *pk, int np, float2 cell_inv, bool half) {
   const int lane = threadIdx.x & 31;
-  const int nwords = S.st->nwords;
-  for (int w = S.st->scan_word + gwarp; w < nwords; w += nwarps) {
-    const unsigned word = S.bits[w];
-    if (!word) continue;
-    const int r = (w << 5) + lane;
-    const bool mine = (word >> lane) & 1u;
-    const float e0 = mine ? S.y1[r] : 0.f, e1 = mine ? S.x1[r] : 0.f, e2 = mine ? S.y2[r] : 0.f,
-                e3 = mine ? S.x2[r] : 0.f, e4 = mine ? S.ar[r] : 0.f;
-    if (2 * __popc(word) * ((np + 31) >> 5) > np) {
-      // dense word: a lane per box walks the picks in order (about np steps for
-      // the warp instead of one 32-pick step per box and pick chunk)
-      int first = -1;
-      if (mine)
-        for (int t = 0; t < np; t++)
-          if (supp(pk[0][t], pk[1][t], pk[2][t], pk[3][t], pk[4][t], e0, e1, e2, e3, e4, overlap)) {
-            first = t;
-            break;
-          }
-      const unsigned gone = __ballot_sync(0xffffffffu, first >= 0);
-      if (first >= 0) S.flag[pick_base + first] = 1;
-      if (lane == 0 && gone) clear_alive(S, w, gone);
-      continue;
+  static_assert(kNmsCells == 64, "two cells a lane");
+  for (int e = threadIdx.x >> 5; e < 2 * ((np + 31) >> 5); e += kResWarps) {
+    const int a = e & 1, k = e >> 1;   // a = 0: y (my[0], my[2]); 1: x (my[1], my[3])
+    int c0 = kNmsCells, c1 = -1, d0 = kNmsCells, d1 = -1;
+    if (32 * k + lane < np) {
+      const float4 p = pk[32 * k + lane];
+      const float lo = (a ? fminf(p.y, p.w) : fminf(p.x, p.z)) - 2.0f, hi = (a ? fmaxf(p.y, p.w) : fmaxf(p.x, p.z)) + 2.0f;
+      const float inv = a ? cell_inv.y : cell_inv.x;
+      c0 = nms_cell(lo, inv);
+      c1 = nms_cell(hi, inv);
+      const float mid = 0.5f * (lo + hi);
+      d0 = half ? nms_cell(mid - 2.0f, inv) : c0;
+      d1 = half ? nms_cell(mid + 2.0f, inv) : c1;
     }
-    unsigned out = word, rem = word;
-    while (rem) {
-      const int b = __ffs(rem) - 1;
-      rem &= rem - 1;
-      const float b0 = __shfl_sync(0xffffffffu, e0, b), b1 = __shfl_sync(0xffffffffu, e1, b);
-      const float b2 = __shfl_sync(0xffffffffu, e2, b), b3 = __shfl_sync(0xffffffffu, e3, b);
-      const float b4 = __shfl_sync(0xffffffffu, e4, b);
-      for (int t0 = 0; t0 < np; t0 += 32) {
-        const int t = t0 + lane;
-        const bool s = t < np && supp(pk[0][t], pk[1][t], pk[2][t], pk[3][t], pk[4][t], b0, b1, b2, b3, b4, overlap);
-        const unsigned bal = __ballot_sync(0xffffffffu, s);
-        if (bal) {
-          out &= ~(1u << b);
-          if (lane == 0) S.flag[pick_base + t0 + __ffs(bal) - 1] = 1;
-          break;
-        }
+    unsigned u0 = 0u, u1 = 0u, v0 = 0u, v1 = 0u;   // cells lane and lane + 32
+#pragma unroll 8
+    for (int b = 0; b < 32; b++) {
+      const int lo = __shfl_sync(0xffffffffu, c0, b), hi = __shfl_sync(0xffffffffu, c1, b);
+      const int l2 = __shfl_sync(0xffffffffu, d0, b), h2 = __shfl_sync(0xffffffffu, d1, b);
+      u0 |= (unsigned)(lo <= lane && lane <= hi) << b;
+      u1 |= (unsigned)(lo <= lane + 32 && lane + 32 <= hi) << b;
+      v0 |= (unsigned)(l2 <= lane && lane <= h2) << b;
+      v1 |= (unsigned)(l2 <= lane + 32 && lane + 32 <= h2) << b;
+    }
+    T.covers[a][k][lane] = u0;
+    T.covers[a][k][lane + 32] = u1;
+#pragma unroll
+    for (int l = 0; l < kNmsLevels; l++) {
+      if (l > 0) {   // the cell 2^(l-1) further, the last one at most
+        const int d = 1 << (l - 1);
+        const unsigned s0 = __shfl_sync(0xffffffffu, v0, (lane + d) & 31), s1 = __shfl_sync(0xffffffffu, v1, (lane + d) & 31);
+        const unsigned top = __shfl_sync(0xffffffffu, v1, 31);
+        v0 |= lane + d < 32 ? s0 : s1;
+        v1 |= lane + d < 32 ? s1 : top;
       }
+      T.in_span[a][l][k][lane] = v0;
+      T.in_span[a][l][k][lane + 32] = v1;
     }
-    if (lane == 0 && out != word) clear_alive(S, w, word & ~out);
   }
 }
 
-// The round's pass: a lane per alive box of a word, testing only the picks
-// that share a row cell and a column cell with it (the union of the picks
-// listed on its cell span, per axis, from a sparse table of spans of 2^l
-// cells), in pick order; the first that suppresses it removes it and is
-// flagged.
-struct PassSmem {
-  float pk[5][kBatch];
-  unsigned tab[2][kNmsLevels][kNmsCells][kBW];
-};
-
-__global__ void __launch_bounds__(kPassNT) k_nms_pass(int cap, int *si, float *sf, float overlap, float cell_inv) {
-  __shared__ PassSmem Z;
-  Slots S = slots(si, sf, blockIdx.y, cap);
-  const BatchState &st = *S.st;
-  if (st.done) return;
-  const int np = st.npb;
-  if (np <= 0) return;
-  const int nwarps = gridDim.x * (kPassNT / 32);
-  const int w_first = st.scan_word + blockIdx.x * (kPassNT / 32);
-  const int nwords = st.nwords;
-  {
-    // a block whose words hold no alive box leaves before it builds the tables
-    // (only this block's warps change its words, so the check stays true)
-    bool any = false;
-    for (int k = threadIdx.x; !any; k += kPassNT) {
-      const int w = w_first + (k & (kPassNT / 32 - 1)) + (k / (kPassNT / 32)) * nwarps;
-      if (w >= nwords) break;
-      any = S.bits[w] != 0u;
-    }
-    if (!__syncthreads_or(any)) return;
-  }
+// One of the table's picks that suppresses a box, or -1; pick `last` only where no other one does.
+__device__ __forceinline__ int suppressor(const PickTable &T, const float4 *pk, const float *pka, int np, int last,
+                                          float e0, float e1, float e2, float e3, float e4, float overlap,
+                                          float2 cell_inv, bool half) {
   const int nwm = (np + 31) >> 5;
-  for (int k = threadIdx.x; k < np; k += kPassNT)
-    for (int c = 0; c < 5; c++) Z.pk[c][k] = S.bp[c * kBatch + k];
-  for (int e = threadIdx.x; e < 2 * kNmsCells * nwm; e += kPassNT) {
-    const int a = e / (kNmsCells * nwm), rem = e - a * kNmsCells * nwm, c = rem / nwm, k = rem - c * nwm;
-    Z.tab[a][0][c][k] = S.cmask[(a * kNmsCells + c) * kBW + k];
-  }
-  __syncthreads();
-  for (int l = 1; l < kNmsLevels; l++) {
-    for (int e = threadIdx.x; e < 2 * kNmsCells * nwm; e += kPassNT) {
-      const int a = e / (kNmsCells * nwm), rem = e - a * kNmsCells * nwm, c = rem / nwm, k = rem - c * nwm;
-      Z.tab[a][l][c][k] = Z.tab[a][l - 1][c][k] | Z.tab[a][l - 1][min(c + (1 << (l - 1)), kNmsCells - 1)][k];
+  const int cy0 = nms_cell(fminf(e0, e2) - 2.0f, cell_inv.x), cy1 = nms_cell(fmaxf(e0, e2) + 2.0f, cell_inv.x);
+  const int cx0 = nms_cell(fminf(e1, e3) - 2.0f, cell_inv.y), cx1 = nms_cell(fmaxf(e1, e3) + 2.0f, cell_inv.y);
+  const int ly = 31 - __clz(cy1 - cy0 + 1), lx = 31 - __clz(cx1 - cx0 + 1);
+  const unsigned *y0p = &T.in_span[0][ly][0][cy0], *y1p = &T.in_span[0][ly][0][cy1 - (1 << ly) + 1];
+  const unsigned *x0p = &T.in_span[1][lx][0][cx0], *x1p = &T.in_span[1][lx][0][cx1 - (1 << lx) + 1];
+  const unsigned *cy = &T.covers[0][0][nms_cell(0.5f * (e0 + e2), cell_inv.x)];
+  const unsigned *cx = &T.covers[1][0][nms_cell(0.5f * (e1 + e3), cell_inv.y)];
+  bool by_last = false;
+  for (int k = 0; k < nwm; k++) {
+    const int o = k * kNmsCells;
+    unsigned cand = (y0p[o] | y1p[o]) & (x0p[o] | x1p[o]);
+    if (half) cand |= cy[o] & cx[o];
+    while (cand) {
+      const int t = (k << 5) + __ffs(cand) - 1;
+      cand &= cand - 1;
+      const float4 p = pk[t];
+      if (supp(p.x, p.y, p.z, p.w, pka[t], e0, e1, e2, e3, e4, overlap)) {
+        if (t != last) return t;
+        by_last = true;
+      }
     }
-    __syncthreads();
   }
+  return by_last ? last : -1;
+}
+
+// Words of the item bitmap [w0, w1], a run of them per warp (gw of nw), against the table's np picks (pick numbers from
+// pick_base on), a lane per box, four words' boxes in flight.  first: the alive items are [c0, c1) (nothing is read
+// from the bitmap), else the bitmap's.  last: the newest pick's place in the table (its flag is raised when it removes a
+// box: only the last of all picks' is read, and any other's would be raised by thousands).  list: the items' sorted positions (null: the item itself).
+__device__ __forceinline__ void test_words(const Slots &S, const PickTable &T, const float4 *pk, const float *pka, int np,
+                                           int pick_base, int last, const int *list, int w0, int w1, bool first, int c0,
+                                           int c1, float overlap, float2 cell_inv, int gw, int nw) {
   const int lane = threadIdx.x & 31;
-  const int pick_base = st.npicks - np;
-  for (int w = w_first + (threadIdx.x >> 5); w < nwords; w += nwarps) {
-    const unsigned word = S.bits[w];
-    if (!word) continue;
-    const int r = (w << 5) + lane;
-    int first = -1;
-    if ((word >> lane) & 1u) {
-      const float e0 = S.y1[r], e1 = S.x1[r], e2 = S.y2[r], e3 = S.x2[r], e4 = S.ar[r];
-      const int cy0 = nms_cell(fminf(e0, e2), cell_inv), cy1 = nms_cell(fmaxf(e0, e2), cell_inv);
-      const int cx0 = nms_cell(fminf(e1, e3), cell_inv), cx1 = nms_cell(fmaxf(e1, e3), cell_inv);
-      const int ly = 31 - __clz(cy1 - cy0 + 1), lx = 31 - __clz(cx1 - cx0 + 1);
-      const int cy2 = cy1 - (1 << ly) + 1, cx2 = cx1 - (1 << lx) + 1;
-      for (int k = 0; k < nwm && first < 0; k++) {
-        unsigned cand = (Z.tab[0][ly][cy0][k] | Z.tab[0][ly][cy2][k]) & (Z.tab[1][lx][cx0][k] | Z.tab[1][lx][cx2][k]);
-        while (cand) {
-          const int t = (k << 5) + __ffs(cand) - 1;
-          cand &= cand - 1;
-          if (supp(Z.pk[0][t], Z.pk[1][t], Z.pk[2][t], Z.pk[3][t], Z.pk[4][t], e0, e1, e2, e3, e4, overlap)) {
-            first = t;
-            break;
-          }
+  const bool half = overlap >= 0.5f;
+  const int run = max(1, min(32, (w1 - w0 + nw) / nw));
+  for (int wb = w0 + gw * run; wb <= w1; wb += nw * run) {
+    const int w = wb + lane;
+    unsigned mine = 0u;
+    if (lane < run && w <= w1) {
+      if (first) {   // items c0 .. c1 of word w
+        const int lo = c0 - 32 * w, hi = c1 - 32 * w;
+        mine = (lo <= 0 ? ~0u : ~0u << lo) & (hi >= 32 ? ~0u : (1u << hi) - 1u);
+      } else {
+        mine = __ldcg(&S.bits[w]);
+      }
+    }
+    unsigned some = __ballot_sync(0xffffffffu, mine != 0u), left = mine;
+    while (some) {
+      int wi[4];
+      unsigned alive[4];
+      float e[4][5];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        wi[u] = some ? __ffs(some) - 1 : -1;
+        some &= some - 1;   // (0 stays 0)
+        alive[u] = __shfl_sync(0xffffffffu, mine, wi[u] & 31);
+        if (wi[u] >= 0 && ((alive[u] >> lane) & 1u)) {
+          const int q = ((wb + wi[u]) << 5) + lane, r = list ? list[q] : q;
+          e[u][0] = S.y1[r]; e[u][1] = S.x1[r]; e[u][2] = S.y2[r]; e[u][3] = S.x2[r]; e[u][4] = S.ar[r];
         }
       }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (wi[u] < 0) break;
+        int k = -1;
+        if ((alive[u] >> lane) & 1u)
+          k = suppressor(T, pk, pka, np, last, e[u][0], e[u][1], e[u][2], e[u][3], e[u][4], overlap,
+                         cell_inv, half);
+        const unsigned gone = __ballot_sync(0xffffffffu, k >= 0);
+        if (k >= 0 && k == last) S.flag[pick_base + k] = 1;
+        if (lane == wi[u]) left &= ~gone;
+      }
     }
-    const unsigned gone = __ballot_sync(0xffffffffu, first >= 0);
-    if (first >= 0) S.flag[pick_base + first] = 1;
-    if (lane == 0 && gone) {   // this warp owns word w in this kernel
-      const unsigned left = word & ~gone;
-      S.bits[w] = left;
-      if (!left) atomicAnd(&S.sbits[w >> 5], ~(1u << (w & 31)));
-    }
+    if (lane < run && w <= w1 && (first || left != mine)) S.bits[w] = left;
   }
 }
 
+// items [c0, c1) (bitmap words w0 .. w1) against the picks [p0, p1), by the warps gw of nw; first: all of
+// them are alive before it (else those in the bitmap)
+__device__ __forceinline__ void test_chunk(const Slots &S, PickTable &T, float4 *pk, float *pka, int p0, int p1,
+                                           const int *list, int w0, int w1, int c0, int c1, float overlap,
+                                           float2 cell_inv, int gw, int nw, bool first = true) {
+  int k0 = p0;
+  do {
+    const int np = min(kPickGroup, p1 - k0);
+    __syncthreads();   // the last table is free
+    if (threadIdx.x < np) {
+      pk[threadIdx.x] = __ldcg(&S.pb[k0 + threadIdx.x]);
+      pka[threadIdx.x] = __ldcg(&S.pa[k0 + threadIdx.x]);
+    }
+    __syncthreads();
+    if (np > 0) pick_table(T, pk, np, cell_inv, overlap >= 0.5f);
+    __syncthreads();
+    test_words(S, T, pk, pka, np, k0, p1 - 1 - k0, list, w0, w1, first && k0 == p0, c0, c1, overlap, cell_inv, gw, nw);
+    k0 += kPickGroup;
+  } while (k0 < p1);
+}
+
 // ---------------------------------------------------------------------------
-// 4. remaining rounds, final-pick rule, kept records in input order
+// rounds over a chunk's survivors
 // ---------------------------------------------------------------------------
-// KEY_ORDER: the key-order pass (writes every model's result; raises need[m]
-// where the quicksort order could differ).  Otherwise the quicksort-order pass:
-// with need given, only the models that raised it (their result replaces the
-// key-order one); without, every model.
+// The batch: the first kBatch alive items of words [w0, w1] with their boxes, by the whole block (R.nb of them; R.tot:
+// the alive items).  The bitmap is read past L1: other blocks of the cluster have changed it.
+// KEY_ORDER (positions in nms_radix.cu's order): a run of equal scores never straddles two batches (the batch ends
+// before a run that the next alive box continues); a run longer than a batch is cut and raises *need (any block may
+// write it: the value is the same).
 template <bool KEY_ORDER>
-__global__ void __launch_bounds__(kSortNT) k_nms_finish(const float *__restrict__ boxes_all, int GL, int cap,
-                                                        int *si, float *sf, float overlap, float *out_all,
-                                                        int *d_kept, int *err, long long *diag, int *rounds_used,
-                                                        int *need, float cell_inv) {
-  __shared__ ResolveSmem R;
-  __shared__ float pk[5][kBatch];
-  __shared__ int wcnt[kSortNT / 32];
-  const int m = blockIdx.x;
-  if (!KEY_ORDER && need && !need[m]) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  Slots S = slots(si, sf, m, cap);
-  BatchState &st = *S.st;
-  const float *boxes = boxes_all + (size_t)m * cap * GL;
-  float *out = out_all + (size_t)m * cap * GL;
-  const int D = st.D;
-  if (!st.done) {
-    if (threadIdx.x == 0) st.fallback = 1;
-    for (int it = 0;; it++) {
-      if (it > D + 1) {   // every round resolves at least one box
-        if (threadIdx.x == 0) atomicOr(err, 2);
-        break;
-      }
-      resolve_batch<KEY_ORDER>(S, overlap, cell_inv, R, need ? need + m : nullptr);
-      if (R.done) break;
-      const int np = R.np;
-      for (int k = threadIdx.x; k < np; k += kSortNT)
-        for (int c = 0; c < 5; c++) pk[c][k] = R.my[c][R.pick_mem[k]];
-      __syncthreads();
-      pass_words(S, pk, np, st.npicks - np, overlap, warp, kSortNT / 32);
-      __syncthreads();
+__device__ __forceinline__ void select_members(const Slots &S, GreedySmem &R, const int *list, int w0, int w1, int *need) {
+  constexpr int want = kBatch + (KEY_ORDER ? 1 : 0);   // key order: one more, to see the run at the boundary
+  const int per = (w1 - w0 + kResNT) / kResNT;         // words per thread: at most four
+  unsigned word[4];
+  int cnt = 0;
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const int w = w0 + threadIdx.x * per + u;
+    word[u] = u < per && w <= w1 ? __ldcg(&S.bits[w]) : 0u;
+    cnt += __popc(word[u]);
+  }
+  int tot;
+  int rank = block_excl_scan(cnt, &tot, R.wtot);
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+    for (unsigned rem = word[u]; rem && rank < want; rem &= rem - 1)
+      R.item[rank++] = ((w0 + threadIdx.x * per + u) << 5) + __ffs(rem) - 1;
+  __syncthreads();
+  for (int k = threadIdx.x; k < min(want, tot); k += kResNT) {
+    const int r = list ? list[R.item[k]] : R.item[k];
+    R.pos[k] = r;
+    if (KEY_ORDER) R.key[k] = sorted_key(S, r);
+    if (k < kBatch) {
+      R.my[0][k] = S.y1[r];
+      R.my[1][k] = S.x1[r];
+      R.my[2][k] = S.y2[r];
+      R.my[3][k] = S.x2[r];
+      R.my[4][k] = S.ar[r];
     }
   }
-  const int npk = st.npicks;
-  // the last pick shares its score with another pick: which of them is last is the quicksort's call
-  if (KEY_ORDER && threadIdx.x == 0 && npk >= 2 && sorted_key(S, S.picks[npk - 1]) == sorted_key(S, S.picks[npk - 2]))
-    need[m] = 1;
-  const int K = npk - ((npk > 0 && S.flag[npk - 1] == 0) ? 1 : 0);
-  int written = 0;
-  if (K <= kRankSortMax) {
-    // few kept boxes: their input indices ranked in shared memory (all distinct)
-    static_assert(sizeof(ResolveSmem) >= sizeof(int) * kRankSortMax, "rank buffer");
-    int *idx = reinterpret_cast<int *>(&R);   // the round's buffers are free now
-    for (int k = threadIdx.x; k < K; k += kSortNT) idx[k] = S.ord[S.picks[k]];
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += kSortNT) {
-      const int v = idx[k];
-      int rank = 0;
-      for (int j = 0; j < K; j++) rank += idx[j] < v;
-      const float *P = boxes + (size_t)v * GL;
-      float *Q = out + (size_t)rank * GL;
-      for (int t = 0; t < GL; t++) Q[t] = P[t];
-    }
-    written = K;
-  } else {
-    int *keep = S.Rpos;
-    for (int i = threadIdx.x; i < D; i += kSortNT) keep[i] = 0;
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += kSortNT) keep[S.ord[S.picks[k]]] = 1;
-    __syncthreads();
-    for (int base = 0; base < D; base += kSortNT) {
-      const int i = base + threadIdx.x;
-      const int f = i < D && keep[i];
-      const unsigned bal = __ballot_sync(0xffffffffu, f);
-      if (lane == 0) wcnt[warp] = __popc(bal);
-      __syncthreads();
-      int before = 0, tot = 0;
-      for (int w = 0; w < kSortNT / 32; w++) {
-        const int c = wcnt[w];
-        if (w < warp) before += c;
-        tot += c;
-      }
-      if (f) {
-        const float *P = boxes + (size_t)i * GL;
-        float *Q = out + (size_t)(written + before + __popc(bal & ((1u << lane) - 1))) * GL;
-        for (int t = 0; t < GL; t++) Q[t] = P[t];
-      }
-      written += tot;
-      __syncthreads();
-    }
-  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    d_kept[m] = written;
-    if (rounds_used) atomicMax(rounds_used, st.batches);   // batches this frame took, grid rounds and any here
-    if (diag) {
-      diag[8 * m + 2] = st.batches;
-      diag[8 * m + 3] = npk;
-      diag[8 * m + 4] = st.fallback;
-      diag[8 * m + 5] = need ? need[m] : 1;
+    int nb = min(kBatch, tot);
+    if (KEY_ORDER && tot > kBatch && R.key[kBatch - 1] == R.key[kBatch]) {   // end before the run that goes on
+      const unsigned kb = R.key[kBatch];
+      int lo = 0, hi = kBatch;   // first candidate with key kb (keys ascend)
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (R.key[mid] < kb) lo = mid + 1;
+        else hi = mid;
+      }
+      nb = lo;
+      if (nb == 0) {   // a run longer than a batch
+        *need = 1;
+        nb = kBatch;
+      }
     }
+    R.nb = nb;
+    R.tot = tot;
+  }
+  __syncthreads();
+}
+
+// Row i of the pairs (bit j of word w: member j = 32 w + lane > i is suppressed by member i) by one warp
+__device__ __forceinline__ void pair_row(const GreedySmem &R, int i, float overlap, unsigned *row) {
+  const int lane = threadIdx.x & 31, nb = R.nb;
+  const float a0 = R.my[0][i], a1 = R.my[1][i], a2 = R.my[2][i], a3 = R.my[3][i], a4 = R.my[4][i];
+  unsigned mine = 0u;
+#pragma unroll 4
+  for (int w = i >> 5; 32 * w < nb; w++) {
+    const int j = 32 * w + lane;
+    const bool s = j > i && j < nb &&
+                   supp(a0, a1, a2, a3, a4, R.my[0][j], R.my[1][j], R.my[2][j], R.my[3][j], R.my[4][j], overlap);
+    const unsigned bal = __ballot_sync(0xffffffffu, s);
+    if (lane == w) mine = bal;
+  }
+  if (lane < kBW) row[lane] = mine;
+}
+
+// The batch's decisions from its rows (R.adj), by the first block: R.np picks in R.pick_mem, appended to S.picks
+// and S.pb, the members cleared from the bitmap.  In key order *need is raised where the order inside a run of equal scores
+// matters: a pick that removes a member of its own run.
+template <bool KEY_ORDER>
+__device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, int base, int *need) {
+  const int nb = R.nb, lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    // the undecided members in registers, every lane alike (one wide broadcast read a pick; warp votes in this
+    // loop measured 640 cycles a pick, this 170)
+    unsigned und[kBW];
+#pragma unroll
+    for (int w = 0; w < kBW; w++) und[w] = nb >= 32 * w + 32 ? ~0u : nb > 32 * w ? (1u << (nb - 32 * w)) - 1u : 0u;
+    int np = 0;
+#pragma unroll
+    for (int w = 0; w < kBW; w++)
+      while (und[w]) {   // its first member: nobody before it suppresses it
+        const int i = 32 * w + __ffs(und[w]) - 1;
+        const uint4 *row = reinterpret_cast<const uint4 *>(R.adj + i * kBW);
+        unsigned gone = 0u;
+#pragma unroll
+        for (int q = w / 4; q < kBW / 4; q++) {
+          const uint4 v = row[q];
+          gone |= (und[4 * q] & v.x) | (und[4 * q + 1] & v.y) | (und[4 * q + 2] & v.z) | (und[4 * q + 3] & v.w);
+          und[4 * q] &= ~v.x; und[4 * q + 1] &= ~v.y; und[4 * q + 2] &= ~v.z; und[4 * q + 3] &= ~v.w;
+        }
+        und[w] &= und[w] - 1u;
+        R.pick_mem[np] = i;
+        R.pick_any[np++] = gone != 0u;
+      }
+    if (lane == 0) R.np = np;
+  }
+  __syncthreads();
+  const int np = R.np;
+  if (KEY_ORDER)
+    for (int k = threadIdx.x; k < np; k += kResNT) {
+      // members of the pick's own run that it removed: suppressed by it and by no pick before it
+      const int i = R.pick_mem[k];
+      for (int j = i + 1; j < nb && R.key[j] == R.key[i]; j++) {
+        if (!((R.adj[i * kBW + (j >> 5)] >> (j & 31)) & 1u)) continue;
+        bool alive = true;
+        for (int q = 0; q < k && alive; q++) alive = !((R.adj[R.pick_mem[q] * kBW + (j >> 5)] >> (j & 31)) & 1u);
+        if (alive) *need = 1;
+      }
+    }
+  for (int k = threadIdx.x; k < np; k += kResNT) {
+    const int i = R.pick_mem[k];
+    S.picks[base + k] = R.pos[i];
+    S.flag[base + k] = R.pick_any[k];
+    S.pb[base + k] = make_float4(R.my[0][i], R.my[1][i], R.my[2][i], R.my[3][i]);
+    S.pa[base + k] = R.my[4][i];
+  }
+  for (int k = threadIdx.x; k < nb; k += kResNT)   // every member is resolved
+    atomicAnd(&S.bits[R.item[k] >> 5], ~(1u << (R.item[k] & 31)));
+}
+
+// ---------------------------------------------------------------------------
+// final-pick rule, the kept boxes in input order (whole block, the model done)
+// ---------------------------------------------------------------------------
+template <bool KEY_ORDER>
+__device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int m, int npk, int batches, const float *boxes,
+                                             int GL, int cap, const NmsResults &res, int *d_kept, long long *diag,
+                                             int *need, cudaGraphConditionalHandle cond, bool has_cond) {
+  const int D = S.st->D;
+  // (the flags are read past L1: other blocks of the cluster have set them)
+  const int K = npk - ((npk > 0 && __ldcg(&S.flag[npk - 1]) == 0) ? 1 : 0);
+  // the last pick shares its score with another pick: which of them is last is the quicksort's call
+  if (KEY_ORDER && threadIdx.x == kResNT - 1 && npk >= 2 &&
+      sorted_key(S, __ldcg(&S.picks[npk - 1])) == sorted_key(S, __ldcg(&S.picks[npk - 2])))
+    need[m] = 1;
+  // the kept boxes' input indices (all distinct) in ascending order
+  int *keep = S.Rpos;
+  int *idx = R.idx;   // the round's buffers are free now
+  constexpr int kRankMax = 2 * kResNT;
+  if (K <= kRankMax) {   // ranked in shared memory
+    for (int k = threadIdx.x; k < ((K + 3) & ~3); k += kResNT) idx[k] = k < K ? S.ord[__ldcg(&S.picks[k])] : 0x7fffffff;
+    __syncthreads();
+    keep = idx + kRankMax;
+    for (int k = threadIdx.x; k < K; k += kResNT) {
+      const int v = idx[k];
+      int r = 0;
+#pragma unroll 4
+      for (int j = 0; j < K; j += 4) {
+        const int4 u = *reinterpret_cast<const int4 *>(idx + j);
+        r += (u.x < v) + (u.y < v) + (u.z < v) + (u.w < v);
+      }
+      keep[r] = v;
+    }
+  } else {   // many: marked by input index, then packed
+    int *mark = S.Lpos;   // (the list of items is done with)
+    for (int i = threadIdx.x; i < D; i += kResNT) mark[i] = 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < K; k += kResNT) mark[S.ord[__ldcg(&S.picks[k])]] = 1;
+    __syncthreads();
+    int written = 0;
+    for (int base = 0; base < D; base += kResNT) {
+      const int i = base + threadIdx.x;
+      const int f = i < D && mark[i];
+      int tot;
+      const int r = block_excl_scan(f, &tot, R.wtot);
+      if (f) keep[written + r] = i;
+      written += tot;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    d_kept[m] = K;
+    if (KEY_ORDER && has_cond && *(volatile int *)&need[m]) cudaGraphSetConditional(cond, 1);
+    if (diag) {
+      diag[8 * m + 2] = batches;
+      diag[8 * m + 3] = npk;
+      diag[8 * m + 5] = need ? *(volatile int *)&need[m] : 1;
+    }
+  }
+  // the results (get_new_rects), four threads a box
+  const NmsResults::Model &Q = res.m[m];
+  int *out = res.out + (size_t)m * cap * 11;
+  for (int e = threadIdx.x; e < 4 * K; e += kResNT) {
+    const int k = e >> 2, c = e & 3;
+    const float *P = boxes + (size_t)keep[k] * GL;
+    const int v = new_rect_side(P, GL, Q.np, Q.coef, res.img_w, res.img_h, c);
+    out[4 * k + c] = v;
+    out[4 * (size_t)cap + 4 * k + c] = (int)((float)v / Q.ratio);
+    // type, scale, score
+    if (c < 3) out[(8 + c) * (size_t)cap + k] = c == 0 ? (int)P[GL - 3] : __float_as_int(P[c == 1 ? GL - 1 : GL - 2]);
   }
 }
 
-// sets an if node's condition: some model raised need
-__global__ void k_nms_need(cudaGraphConditionalHandle h, const int *need, int n_models) {
-  unsigned any = 0;
-  for (int m = 0; m < n_models; m++) any |= need[m] ? 1u : 0u;
-  cudaGraphSetConditional(h, any);
+// The first key-order item at or after c1 whose score differs from the one before it, at most hi (every warp alike)
+__device__ __forceinline__ int run_end(const Slots &S, const int *list, int c1, int hi) {
+  const int lane = threadIdx.x & 31;
+  const unsigned k = sorted_key(S, list ? list[c1 - 1] : c1 - 1);
+  while (c1 < hi) {
+    const int q = c1 + lane;
+    const unsigned other = __ballot_sync(0xffffffffu, q >= hi || sorted_key(S, list ? list[q] : q) != k);
+    if (other) return c1 + __ffs(other) - 1;
+    c1 += 32;
+  }
+  return hi;
+}
+
+// The greedy rounds of a model (see the top of the file).  KEY_ORDER: the key-order pass (every model; raises need[m]
+// where the quicksort order could differ).  Otherwise the quicksort-order pass: with need given, only the models that
+// raised it are not done (their result replaces the key-order one); without, every model.
+// rest = false: all the boxes, or the first kPrefix of more than kWhole; true: the survivors that k_nms_rest left of
+// the others.
+template <bool KEY_ORDER>
+__global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restrict__ boxes_all, int GL, int cap, int *si,
+                                                       float *sf, float overlap, float2 cell_inv,
+                                                       const __grid_constant__ NmsResults res, int *d_kept,
+                                                       long long *diag, int *need, cudaGraphConditionalHandle cond,
+                                                       bool has_cond, bool rest) {
+  extern __shared__ __align__(16) unsigned char res_sm[];
+  GreedySmem &R = *reinterpret_cast<GreedySmem *>(res_sm);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int m = blockIdx.y, rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
+  const int warp = threadIdx.x >> 5, gw = rank * kResWarps + warp, nw = blocks * kResWarps;
+  Slots S = slots(si, sf, m, cap);
+  const BatchState st = *S.st;
+  if (st.done) return;   // (the same in every block: it is written behind a cluster barrier)
+  int *need_m = need ? need + m : nullptr;
+  GreedySmem *R0 = cluster.map_shared_rank(&R, 0);
+  cluster.sync();   // every block has started: its shared memory can be written
+  const int *list = nullptr;
+  int n = st.D, np = st.npicks, tested = 0;
+  if (!rest) {
+    if (st.D > kWhole) n = KEY_ORDER ? run_end(S, nullptr, kPrefix, st.D) : kPrefix;
+  } else {
+    // the alive bits of the words from st.next on as a list of sorted positions, in order: a stretch of words per block
+    const int wa = st.next >> 5, nwords = ((st.D + 31) >> 5) - wa;
+    const int share = (nwords + blocks - 1) / blocks, per = (share + kResNT - 1) / kResNT;
+    const int b0 = wa + rank * share, b1 = min(wa + nwords, b0 + share);
+    const int t0 = b0 + threadIdx.x * per, t1 = min(b1, t0 + per);
+    int cnt = 0, tot;
+    for (int w = t0; w < t1; w++) cnt += __popc(__ldcg(&S.bits[w]));
+    int at = block_excl_scan(cnt, &tot, R.wtot);
+    if (threadIdx.x == 0) R0->total[rank] = tot;
+    cluster.sync();
+    n = 0;
+    for (int b = 0; b < blocks; b++) {
+      const int v = R0->total[b];
+      if (b < rank) at += v;
+      n += v;
+    }
+    for (int w = t0; w < t1; w++)
+      for (unsigned rem = __ldcg(&S.bits[w]); rem; rem &= rem - 1) S.Lpos[at++] = (w << 5) + __ffs(rem) - 1;
+    list = S.Lpos;
+    tested = np;
+    cluster.sync();   // the list is complete, the bitmap free
+  }
+  int chunk = kBatch, batches = st.batches;
+  for (int c0 = 0; c0 < n;) {
+    int c1 = min(c0 + chunk, n);
+    if (KEY_ORDER && c1 < n) {   // not inside a run of equal scores
+      const int lim = min(n, c0 + kMaxChunk);
+      c1 = run_end(S, list, c1, lim);
+      if (c1 == lim && c1 < n && run_end(S, list, c1, c1 + 1) > c1) {   // a run of that length is cut
+        if (threadIdx.x == 0) *need_m = 1;
+      }
+    }
+    const int w0 = c0 >> 5, w1 = (c1 - 1) >> 5;
+    test_chunk(S, R.table, R.pk, R.pka, tested, np, list, w0, w1, c0, c1, overlap, cell_inv, gw, nw);
+    cluster.sync();   // the bitmap is complete
+    int left = 0;
+    for (int round = 0;; round++) {
+      select_members<KEY_ORDER>(S, R, list, w0, w1, need_m);
+      if (round == 0) left = R.tot;
+      if (R.tot == 0) break;
+      for (int k = 0; k * nw < R.nb; k++) {   // rows g, then 2G - 1 - g, ...: long and short ones in turn
+        const int i = k * nw + ((k & 1) ? nw - 1 - gw : gw);
+        if (i < R.nb) pair_row(R, i, overlap, R0->adj + i * kBW);
+      }
+      cluster.sync();   // the rows are in the first block
+      if (rank == 0) decide_members<KEY_ORDER>(S, R, np, need_m);
+      cluster.sync();   // the picks are in the first block and in S, the members cleared
+      const int added = R0->np;
+      batches++;
+      if (R.tot > R.nb) {   // the rest of the chunk against the new picks
+        test_chunk(S, R.table, R.pk, R.pka, np, np + added, list, w0, w1, 0, 0, overlap, cell_inv, gw, nw, false);
+        cluster.sync();
+      }
+      np += added;
+      if (R.tot <= R.nb) break;
+    }
+    cluster.sync();   // (the first block's picks have been read)
+    // the head leaves about a tenth of what follows alive, and the picks thin every next stretch out further:
+    // eight times the chunk leaves a batch or two (twice after one that left more)
+    chunk = min((left > 2 * kBatch ? 2 : 8) * chunk, kChunkCap);
+    c0 = c1;
+  }
+  if (!rest && n < st.D) {
+    if (rank == 0 && threadIdx.x == 0) {
+      S.st->npicks = np;
+      S.st->batches = batches;
+      S.st->next = n;
+    }
+    return;
+  }
+  if (rank == 0) {
+    if (threadIdx.x == 0) S.st->done = 1;
+    finish_model<KEY_ORDER>(S, R, m, np, batches, boxes_all + (size_t)m * cap * GL, GL, cap, res, d_kept, diag, need,
+                            cond, has_cond);
+  }
+}
+
+// The boxes from st.next on against every pick so far, over the grid
+__global__ void __launch_bounds__(kResNT) k_nms_rest(int cap, int *si, float *sf, float overlap, float2 cell_inv) {
+  __shared__ PickTable T;
+  __shared__ float4 pk[kPickGroup];
+  __shared__ float pka[kPickGroup];
+  Slots S = slots(si, sf, blockIdx.y, cap);
+  const BatchState st = *S.st;
+  if (st.done) return;
+  const int w0 = st.next >> 5, w1 = (st.D - 1) >> 5;
+  test_chunk(S, T, pk, pka, 0, st.npicks, nullptr, w0, w1, st.next, st.D, overlap, cell_inv,
+             blockIdx.x * kResWarps + (threadIdx.x >> 5), gridDim.x * kResWarps);
 }
 
 // Inside a stream capture: a handle for a conditional node of the graph s is
@@ -652,55 +671,103 @@ static cudaError_t end_conditional(cudaStream_t aux) {
   return cudaGetLastError();   // a launch inside the body
 }
 
-// gather, the greedy rounds and the finish, in the order the sort left in (val, ord)
-template <bool KEY_ORDER>
-static void launch_greedy(const float *boxes, int n_models, int GL, float overlap, float cell_inv, int cap, int *si,
-                          float *sf, float *out, int *d_kept, int *err, long long *diag, int rounds,
-                          int *rounds_used, int *need, cudaStream_t s) {
-  k_nms_gather<<<dim3((cap + kPassNT - 1) / kPassNT, n_models), kPassNT, 0, s>>>(boxes, GL, cap, si, sf);
-  const int words = (cap + 31) / 32;
-  const int pass_blocks = std::max(1, std::min((words + kPassNT / 32 - 1) / (kPassNT / 32), 512));
-  for (int r = 0; r < rounds; r++) {
-    k_nms_resolve<KEY_ORDER><<<n_models, kSortNT, 0, s>>>(cap, si, sf, overlap, cell_inv, need);
-    k_nms_pass<<<dim3(pass_blocks, n_models), kPassNT, 0, s>>>(cap, si, sf, overlap, cell_inv);
+// blocks per model: kCluster where the device can place such a cluster, else the portable 8
+template <class K>
+static int cluster_blocks(K *kernel, size_t smem) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return 8;
   }
-  k_nms_finish<KEY_ORDER><<<n_models, kSortNT, 0, s>>>(boxes, GL, cap, si, sf, overlap, out, d_kept, err, diag,
-                                                       rounds_used, need, cell_inv);
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(kCluster);
+  c.blockDim = dim3(kResNT);
+  c.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {(unsigned)kCluster, 1, 1};
+  c.attrs = &at;
+  c.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &c) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return 8;
+  }
+  return kCluster;
+}
+
+// the greedy rounds and the results, in the order the sort left in (val, ord)
+template <bool KEY_ORDER>
+static cudaError_t launch_greedy(const float *boxes, int n_models, int GL, float overlap, float2 cell_inv, int cap, int *si,
+                                 float *sf, const NmsResults &res, int *d_kept, long long *diag, int *need,
+                                 cudaGraphConditionalHandle cond, bool has_cond, cudaStream_t s) {
+  static SmemAttr attr;
+  cudaError_t e = raise_smem(attr, k_nms_greedy<KEY_ORDER>, sizeof(GreedySmem));
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t c = {};
+  const int blocks = cluster_blocks(k_nms_greedy<KEY_ORDER>, sizeof(GreedySmem));
+  c.gridDim = dim3(blocks, n_models);
+  c.blockDim = dim3(kResNT);
+  c.dynamicSmemBytes = sizeof(GreedySmem);
+  c.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {(unsigned)blocks, 1, 1};
+  c.attrs = &at;
+  c.numAttrs = 1;
+  for (const bool rest : {false, true}) {
+    if (rest) {
+      if (cap <= kWhole) break;
+      k_nms_rest<<<dim3(std::max(304 / n_models, 1), n_models), kResNT, 0, s>>>(cap, si, sf, overlap, cell_inv);
+    }
+    e = cudaLaunchKernelEx(&c, k_nms_greedy<KEY_ORDER>, boxes, GL, cap, si, sf, overlap, cell_inv, res, d_kept, diag,
+                           need, cond, has_cond, rest);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
-                             float extent, int cap, int *si, float *sf, float *out, int *d_kept, int *err,
-                             long long *diag, int levels, int *lv_used, int rounds, int *rounds_used, int *need,
-                             int order, cudaStream_t s, cudaStream_t aux) {
-  const float cell_inv = (float)kNmsCells / std::max(extent, 1.0f);
+                             int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
+                             long long *diag, int levels, int *lv_used, int *need, int order, cudaStream_t s,
+                             cudaStream_t aux) {
+  // cells over the image and a margin for boxes that leave it (any value is exact: what is outside shares the edge cells)
+  const float2 cell_inv = make_float2(kNmsCells / (1.15f * std::max(res.img_h, 1)), kNmsCells / (1.15f * std::max(res.img_w, 1)));
   if (n_models <= 0) return cudaSuccess;
-  if (rounds <= 0) rounds = kNmsRounds;
+  auto gather = [&](cudaStream_t q) {
+    k_nms_gather<<<dim3((cap + kPassNT - 1) / kPassNT, n_models), kPassNT, 0, q>>>(boxes, GL, cap, si, sf);
+  };
+  cudaError_t e = cudaSuccess;
   if (order == kNmsOrderQuicksort) {
     launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, nullptr, s);
-    launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, out, d_kept, err, diag, rounds,
-                         rounds_used, nullptr, s);
-    return cudaGetLastError();
+    gather(s);
+    e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, nullptr, 0,
+                             false, s);
+    return e == cudaSuccess ? cudaGetLastError() : e;
   }
-  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, s);
-  launch_greedy<true>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, out, d_kept, err, diag, rounds,
-                      rounds_used, need, s);
   // the models whose kept set could depend on the order inside a run of equal
-  // scores, again in the quicksort's order: in a graph captured with aux, an
-  // if node that runs only when some model needs it; otherwise launches that
-  // do nothing for the models that do not
+  // scores go again in the quicksort's order: in a graph captured with aux, an
+  // if node that runs only when some model needs it (the finishing block of
+  // such a model sets its condition); otherwise launches that do nothing for
+  // the models that do not
+  cudaGraphConditionalHandle h = 0;
+  if (aux && (e = cond_handle(s, 0u, &h)) != cudaSuccess) return e;
+  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, s);
+  if ((e = launch_greedy<true>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, need, h,
+                               aux != nullptr, s)) != cudaSuccess)
+    return e;
   cudaStream_t q = s;
-  cudaError_t e = cudaSuccess;
   if (aux) {
-    cudaGraphConditionalHandle h;
-    if ((e = cond_handle(s, 0u, &h)) != cudaSuccess) return e;
-    k_nms_need<<<1, 1, 0, s>>>(h, need, n_models);
     if ((e = begin_conditional(s, aux, cudaGraphCondTypeIf, h)) != cudaSuccess) return e;
     q = aux;
   }
   launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, need, q);
-  launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, out, d_kept, err, diag, rounds,
-                       rounds_used, need, q);
-  if (aux) e = end_conditional(aux);
+  gather(q);
+  e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, need, 0, false,
+                           q);
+  if (aux) {
+    const cudaError_t e2 = end_conditional(aux);
+    if (e == cudaSuccess) e = e2;
+  }
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 

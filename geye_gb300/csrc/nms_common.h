@@ -12,8 +12,9 @@ constexpr int kNmsNT = 1024;   // threads of the whole-block kernels
 constexpr int kTiny = 32;      // sort segments finished by one thread
 
 struct BatchState {   // greedy rounds
-  int D, nwords, scan_word, npicks;
-  int npb, done, batches, fallback;
+  int D, done;
+  int npicks, batches, next;   // between launches: picks, rounds, the first box not looked at
+  int pad[11];
 };
 
 struct SortState {    // grid-wide partition levels
@@ -22,29 +23,28 @@ struct SortState {    // grid-wide partition levels
   int pad[5];
 };
 
-// per-model scratch: nms_model_words(cap) ints and 5 * cap floats
+// per-model scratch: nms_model_words(cap) ints and 10 * cap floats
 struct Slots {
   float *val;        // sort keys
   int *ord;          // sorted position -> box
-  int *Lpos, *Rpos;  // partition lists; Rpos holds keep flags at the end
+  int *Lpos, *Rpos;  // partition lists; Rpos holds the kept boxes' input indices, ascending, at the end
   int2 *small;       // cap/2 sort segments for the shared-memory kernel
   int *picks;        // sorted positions of the picks, in pick order
   int *flag;         // per pick: it suppressed at least one box
-  unsigned *bits;    // alive bitmap over sorted positions
+  unsigned *bits;    // alive bitmap (nms_batch.cu)
   BatchState *st;
   SortState *ss;
-  float *bp;         // current round's picks: y1, x1, y2, x2, area (kNmsBatch each)
   int2 *big[2];      // nms_big_cap(cap) segments each
   int2 *tiles;       // nms_tile_cap(cap) per-tile (<= key, >= key) counts
-  int *hist;         // 256 * nms_rs_tiles(cap) radix-sort digit counts (nms_radix.cu)
-  unsigned *sbits;   // summary of bits: bit w set while word w has an alive box
-  unsigned *cmask;   // the round's picks by cell: [axis y, x][level][cell][pick word] (nms_batch.cu)
+  int *hist;         // [pass][tile][256] radix-sort digit counts (nms_radix.cu)
   float *y1, *x1, *y2, *x2, *ar;   // boxes in sorted order
+  float4 *pb;        // the picks' boxes y1, x1, y2, x2 and areas, in pick order
+  float *pa;
 };
 
 __device__ __forceinline__ Slots slots(int *si, float *sf, int m, int cap) {
   int *b = si + (size_t)m * nms_model_words(cap);
-  float *f = sf + (size_t)m * 5 * cap;
+  float *f = sf + (size_t)m * 10 * cap;
   Slots S;
   S.val = reinterpret_cast<float *>(b);
   S.ord = b + cap;
@@ -56,21 +56,20 @@ __device__ __forceinline__ Slots slots(int *si, float *sf, int m, int cap) {
   S.bits = reinterpret_cast<unsigned *>(b + 7 * (size_t)cap);
   int *t = b + 8 * (size_t)cap;
   S.st = reinterpret_cast<BatchState *>(t);
-  S.ss = reinterpret_cast<SortState *>(t + 8);
-  S.bp = reinterpret_cast<float *>(t + 64);
-  int *l = t + 64 + 5 * kNmsBatch;
+  S.ss = reinterpret_cast<SortState *>(t + 16);
+  int *l = t + 64;
   const int bc = nms_big_cap(cap);
   S.big[0] = reinterpret_cast<int2 *>(l);
   S.big[1] = reinterpret_cast<int2 *>(l + 2 * bc);
   S.tiles = reinterpret_cast<int2 *>(l + 4 * bc);
   S.hist = l + 4 * bc + 2 * nms_tile_cap(cap);
-  S.sbits = reinterpret_cast<unsigned *>(S.hist + 256 * (size_t)nms_rs_tiles(cap));
-  S.cmask = S.sbits + nms_summary_words(cap);
   S.y1 = f;
   S.x1 = f + cap;
   S.y2 = f + 2 * (size_t)cap;
   S.x2 = f + 3 * (size_t)cap;
   S.ar = f + 4 * (size_t)cap;
+  S.pb = reinterpret_cast<float4 *>(f + 5 * (size_t)cap);
+  S.pa = f + 9 * (size_t)cap;
   return S;
 }
 
@@ -247,22 +246,24 @@ __device__ __forceinline__ void thread_qsort(float *a, int *ord, int lo0, int hi
   }
 }
 
-// suppression test (nms.cpp:141-176); A is the kept box, B the other one
+// suppression test (nms.cpp:141-176) for the pipeline's boxes (score.cu's root_box: both extents, with the
+// + 1 of the widths, are positive): containment is an overlap, so only the ratio
+// of the areas decides.  A is the kept box, B the other one; nms.cpp adds the double 1.0
+// and stores a float: one rounding of the exact sum, which is what the float addition gives.
 __device__ __forceinline__ bool supp(float Ay1, float Ax1, float Ay2, float Ax2, float aA, float By1, float Bx1,
-                                     float By2, float Bx2, float aB, float overlap) {
-  const float yy1 = Ay1 >= By1 ? Ay1 : By1;
-  const float xx1 = Ax1 >= Bx1 ? Ax1 : Bx1;
-  const float yy2 = Ay2 <= By2 ? Ay2 : By2;
-  const float xx2 = Ax2 <= Bx2 ? Ax2 : Bx2;
-  // nms.cpp adds the double 1.0 and stores a float: one rounding of the exact
-  // sum, which is what the float addition gives (no FP64 in the inner loop)
-  const float w = xx2 - xx1 + 1.0f;
-  const float h = yy2 - yy1 + 1.0f;
-  const float R_AREA = aA <= aB ? aA : aB;
-  if (w > 0 && h > 0) return w * h / R_AREA > overlap;
-  if (Ay1 < By1 && Ax1 < Bx1 && Ay2 > By2 && Ax2 > Bx2) return true;
-  if (Ay1 > By1 && Ax1 > Bx1 && Ay2 < By2 && Ax2 < Bx2) return true;
-  return false;
+                                            float By2, float Bx2, float aB, float overlap) {
+  const float w = fminf(Ax2, Bx2) - fmaxf(Ax1, Bx1) + 1.0f;
+  const float h = fminf(Ay2, By2) - fmaxf(Ay1, By1) + 1.0f;
+  const float R_AREA = fminf(aA, aB);
+  // w * h / R_AREA > overlap, without the division where the product with the
+  // overlap decides: with u = 2^-24, q > p (1 + 2^-21) (each side rounded) puts q / R_AREA
+  // above overlap (1 + 2^-22), whose rounding is above overlap; below likewise
+  const float q = w * h, p = R_AREA * overlap;
+  const bool meet = fminf(w, h) > 0.0f;
+  const bool over = q > p * (1.0f + 4.76837158203125e-07f), under = q < p * (1.0f - 4.76837158203125e-07f);
+  bool s = meet & over;
+  if (meet & !((over | under) & (p > 1e-30f) & (p < 1e30f))) s = q / R_AREA > overlap;
+  return s;
 }
 
 // sort stage (nms_sort.cu): leaves val/ord sorted for every model and the

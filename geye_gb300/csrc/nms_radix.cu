@@ -17,16 +17,19 @@
 // kept set is the reference's either way.
 //
 //   k_rs_load     keys (order-preserving transform of the float score, -0 as
-//                 +0, complemented for descending order), indices, the greedy
-//                 state; NaN raises the flag.
-//   four passes of eight bits, three kernels each:
-//     k_rs_count  a block per tile of nms_rs_tile(cap) keys: the digit histogram of its
-//                 tile, stored digit-major (H[digit][tile]);
-//     k_rs_scan   a block per model: exclusive scan of H in that order, which
-//                 is each (digit, tile)'s first output position;
-//     k_rs_scatter a block per tile: each key's rank among the equal digits
-//                 before it in its tile (warp match, then warp prefix), so the
-//                 pass is stable.
+//                 +0, complemented for descending order), indices, the
+//                 greedy state, and the digit counts of the first
+//                 pass per tile of nms_rs_tile(cap) keys; NaN raises the flag.
+//   k_rs_pass     four passes of eight bits, one kernel each: a block per tile
+//                 adds up the tiles' digit counts before it (at most a few
+//                 hundred coalesced rows, so no scan kernel between the
+//                 passes), ranks its keys (warp match, warp prefix: stable),
+//                 writes them out and counts the next pass's digits at the
+//                 tile each key lands in.  The last pass also brings the boxes
+//                 into sorted order.
+// What bounds it is latency: a kernel boundary per pass.  With a count, a scan
+// (one block per model) and a scatter kernel per pass and a gather behind them,
+// 14 launches instead of 5, the 640x480 pair's NMS took 285 us; see nms_batch.cu.
 // Keys ping-pong between (val, ord) and (Lpos, Rpos); after the fourth pass
 // they are back in (val, ord): val holds the transformed keys (equal keys <=>
 // equal scores), ord the input index of each sorted position.
@@ -34,7 +37,7 @@
 
 namespace geye {
 
-constexpr int kRsNT = 512;   // threads of the count and scatter blocks
+constexpr int kRsNT = 512;
 constexpr int kRsWarps = kRsNT / 32;
 
 __device__ __forceinline__ unsigned rs_key(float v, bool &nan) {
@@ -45,30 +48,37 @@ __device__ __forceinline__ unsigned rs_key(float v, bool &nan) {
   return ~asc;   // ascending keys = descending scores
 }
 
-__global__ void __launch_bounds__(256) k_rs_load(const float *__restrict__ boxes_all, const int *__restrict__ d_num,
-                                                 int GL, int cap, int *si, float *sf, int *need) {
-  const int m = blockIdx.y;
+__global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ boxes_all, const int *__restrict__ d_num,
+                                                   int GL, int cap, int *si, float *sf, int *need) {
+  __shared__ int h[256];
+  const int m = blockIdx.y, t = blockIdx.x;
   Slots S = slots(si, sf, m, cap);
   const float *boxes = boxes_all + (size_t)m * cap * GL;
-  const int D = max(0, min(d_num[m], cap));
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  bool nan = false;
-  if (i < D) {
-    const unsigned k = rs_key(boxes[(size_t)i * GL + GL - 2], nan);
-    reinterpret_cast<unsigned *>(S.val)[i] = k;
-    S.ord[i] = i;
-  }
-  if (__any_sync(0xffffffffu, nan) && (threadIdx.x & 31) == 0) need[m] = 1;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  const int D = max(0, min(d_num[m], cap)), T = nms_rs_tile(cap);
+  if (t == 0 && threadIdx.x == 0) {
     BatchState &st = *S.st;
     st.D = D;
-    st.nwords = (D + 31) >> 5;
-    st.scan_word = 0;
-    st.npicks = 0;
-    st.npb = 0;
     st.done = D <= 0;
-    st.batches = 0;
-    st.fallback = 0;
+    st.npicks = st.batches = st.next = 0;
+  }
+  const int e0 = t * T;
+  if (e0 >= D) return;
+  if (threadIdx.x < 256) h[threadIdx.x] = 0;
+  __syncthreads();
+  bool nan = false;
+  for (int i = e0 + threadIdx.x; i < min(e0 + T, D); i += kRsNT) {
+    const unsigned k = rs_key(boxes[(size_t)i * GL + GL - 2], nan);
+    if (nan) need[m] = 1;
+    reinterpret_cast<unsigned *>(S.val)[i] = k;
+    S.ord[i] = i;
+    atomicAdd(&h[k & 255u], 1);
+  }
+  __syncthreads();
+  const size_t pass_words = (size_t)256 * nms_rs_tiles(cap);
+  if (threadIdx.x < 256) {
+    int *H = S.hist + (size_t)256 * t + threadIdx.x;
+    H[0] = h[threadIdx.x];
+    for (int p = 1; p < 4; p++) H[p * pass_words] = 0;
   }
 }
 
@@ -84,12 +94,17 @@ __device__ __forceinline__ void rs_bufs(const Slots &S, int pass, const unsigned
   }
 }
 
-__global__ void __launch_bounds__(kRsNT) k_rs_count(int pass, int cap, int *si, float *sf) {
-  __shared__ int h[256];
-  Slots S = slots(si, sf, blockIdx.y, cap);
-  const int D = S.st->D, T = nms_rs_tile(cap);
-  const int nt = (D + T - 1) / T;
-  const int t = blockIdx.x;
+// IT keys per thread (a tile of kRsNT * IT); pass 3 gathers the boxes
+template <int IT>
+__global__ void __launch_bounds__(kRsNT) k_rs_pass(int pass, const float *__restrict__ boxes_all, int GL, int cap,
+                                                   int *si, float *sf) {
+  constexpr int T = kRsNT * IT;
+  __shared__ int before_s[2][256], total_s[2][256];
+  __shared__ int cnt[kRsWarps][256];
+  __shared__ int wsum[8];
+  const int m = blockIdx.y, t = blockIdx.x;
+  Slots S = slots(si, sf, m, cap);
+  const int D = S.st->D, nt = (D + T - 1) / T;
   if (t >= nt) return;
   const unsigned *sk;
   const int *sidx;
@@ -97,133 +112,97 @@ __global__ void __launch_bounds__(kRsNT) k_rs_count(int pass, int cap, int *si, 
   int *di;
   rs_bufs(S, pass, sk, sidx, dk, di);
   const int shift = 8 * pass;
-  for (int d = threadIdx.x; d < 256; d += kRsNT) h[d] = 0;
-  __syncthreads();
-  const int e0 = t * T, e1 = min(e0 + T, D);
-  for (int e = e0 + threadIdx.x; e < e1; e += kRsNT) atomicAdd(&h[(sk[e] >> shift) & 255u], 1);
-  __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += kRsNT) S.hist[(size_t)d * nt + t] = h[d];
-}
-
-// exclusive scan of H (digit-major) in place, one block per model: chunks of
-// kRsScanNT * kRsScanItems counts staged in shared memory with coalesced
-// loads and stores, each thread scanning kRsScanItems consecutive ones
-constexpr int kRsScanNT = 1024, kRsScanItems = 8, kRsScanPad = kRsScanItems + 1;
-__global__ void __launch_bounds__(kRsScanNT) k_rs_scan(int cap, int *si, float *sf) {
-  __shared__ int buf[kRsScanNT * kRsScanPad];   // thread t's items at t * kRsScanPad (no bank conflicts)
-  __shared__ int wsum[kRsScanNT / 32];
-  __shared__ int carry_s;
-  Slots S = slots(si, sf, blockIdx.x, cap);
-  const int D = S.st->D;
-  if (D <= 0) return;
-  const int n = 256 * ((D + nms_rs_tile(cap) - 1) / nms_rs_tile(cap));
+  const size_t pass_words = (size_t)256 * nms_rs_tiles(cap);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int carry = 0;
-  for (int base = 0; base < n; base += kRsScanItems * kRsScanNT) {
+  // the thread's keys: a warp's 32 * IT are consecutive
+  unsigned key[IT];
+  int idx[IT], rank[IT];
 #pragma unroll
-    for (int k = 0; k < kRsScanItems; k++) {
-      const int e = k * kRsScanNT + threadIdx.x;   // chunk element, coalesced
-      buf[(e / kRsScanItems) * kRsScanPad + e % kRsScanItems] = base + e < n ? S.hist[base + e] : 0;
+  for (int k = 0; k < IT; k++) {
+    const int e = t * T + warp * (32 * IT) + 32 * k + lane;
+    key[k] = e < D ? sk[e] : 0u;
+    idx[k] = e < D ? sidx[e] : -1;
+  }
+  {   // digit counts of the tiles before this one, and of all: two threads per digit, half of the tiles each
+    const int d = threadIdx.x & 255, half = threadIdx.x >> 8, mid = (nt + 1) / 2;
+    const int *H = S.hist + pass * pass_words + d;
+    int before = 0, total = 0;
+#pragma unroll 8
+    for (int u = half ? mid : 0; u < (half ? nt : mid); u++) {
+      const int c = H[(size_t)256 * u];
+      total += c;
+      if (u < t) before += c;
     }
-    __syncthreads();
-    int *mine = buf + threadIdx.x * kRsScanPad;
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < kRsScanItems; k++) s += mine[k];
-    int inc = s;
+    before_s[half][d] = before;
+    total_s[half][d] = total;
+    for (int k = threadIdx.x; k < kRsWarps * 256; k += kRsNT) (&cnt[0][0])[k] = 0;
+  }
+  __syncthreads();
+  int tot = 0, inc = 0;
+  if (threadIdx.x < 256) {   // exclusive scan of the totals
+    tot = total_s[0][threadIdx.x] + total_s[1][threadIdx.x];
+    inc = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += y;
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
     }
     if (lane == 31) wsum[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      int w = wsum[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      wsum[lane] = w;   // inclusive over warps
-      if (lane == 31) carry_s = w;
-    }
-    __syncthreads();
-    int run = carry + (warp ? wsum[warp - 1] : 0) + inc - s;
-#pragma unroll
-    for (int k = 0; k < kRsScanItems; k++) {
-      const int v = mine[k];
-      mine[k] = run;
-      run += v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kRsScanItems; k++) {
-      const int e = k * kRsScanNT + threadIdx.x;
-      if (base + e < n) S.hist[base + e] = buf[(e / kRsScanItems) * kRsScanPad + e % kRsScanItems];
-    }
-    carry += carry_s;
-    __syncthreads();   // buf, wsum and carry_s reused by the next chunk
   }
-}
-
-__global__ void __launch_bounds__(kRsNT) k_rs_scatter(int pass, int cap, int *si, float *sf) {
-  __shared__ int base[256];
-  __shared__ int cnt[kRsWarps][256];
-  Slots S = slots(si, sf, blockIdx.y, cap);
-  const int D = S.st->D, T = nms_rs_tile(cap);
-  const int nt = (D + T - 1) / T;
-  const int t = blockIdx.x;
-  if (t >= nt) return;
-  const unsigned *sk;
-  const int *sidx;
-  unsigned *dk;
-  int *di;
-  rs_bufs(S, pass, sk, sidx, dk, di);
-  const int shift = 8 * pass;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int d = threadIdx.x; d < 256; d += kRsNT) base[d] = S.hist[(size_t)d * nt + t];
   const unsigned lt = (1u << lane) - 1u;
-  for (int e0 = t * T; e0 < min((t + 1) * T, D); e0 += kRsNT) {
-    for (int k = threadIdx.x; k < kRsWarps * 256; k += kRsNT) (&cnt[0][0])[k] = 0;
-    __syncthreads();   // counters clear, base up to date
-    const int e = e0 + threadIdx.x;
-    const bool valid = e < D;
-    const unsigned key = valid ? sk[e] : 0u;
-    const int idx = valid ? sidx[e] : 0;
-    const int digit = (int)((key >> shift) & 255u);
+#pragma unroll
+  for (int k = 0; k < IT; k++) {
+    const int digit = (int)((key[k] >> shift) & 255u);
     // lanes past the end match nobody (a value no digit takes)
-    const unsigned peers = __match_any_sync(0xffffffffu, valid ? digit : 256 + lane);
-    const int rank = __popc(peers & lt);
-    if (valid && rank == 0) cnt[warp][digit] = __popc(peers);
-    __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += kRsNT) {
-      int acc = base[d];
-      for (int w = 0; w < kRsWarps; w++) {
-        const int c = cnt[w][d];
-        cnt[w][d] = acc;
-        acc += c;
-      }
-      base[d] = acc;
+    const unsigned peers = __match_any_sync(0xffffffffu, idx[k] >= 0 ? digit : 256 + lane);
+    const int prev = cnt[warp][digit];
+    __syncwarp();
+    if (idx[k] >= 0 && (peers & lt) == 0u) cnt[warp][digit] = prev + __popc(peers);
+    __syncwarp();
+    rank[k] = prev + __popc(peers & lt);
+  }
+  __syncthreads();
+  if (threadIdx.x < 256) {
+    int acc = inc - tot + before_s[0][threadIdx.x] + before_s[1][threadIdx.x];
+    for (int w = 0; w < warp; w++) acc += wsum[w];
+#pragma unroll
+    for (int w = 0; w < kRsWarps; w++) {
+      const int c = cnt[w][threadIdx.x];
+      cnt[w][threadIdx.x] = acc;
+      acc += c;
     }
-    __syncthreads();
+  }
+  __syncthreads();
+  const float *boxes = boxes_all + (size_t)m * cap * GL;
+  int *Hn = S.hist + (pass + 1) * pass_words;
+#pragma unroll
+  for (int k = 0; k < IT; k++) {
+    const bool valid = idx[k] >= 0;
+    const int p = cnt[warp][(key[k] >> shift) & 255u] + rank[k];
     if (valid) {
-      const int p = cnt[warp][digit] + rank;
-      dk[p] = key;
-      di[p] = idx;
+      dk[p] = key[k];
+      di[p] = idx[k];
     }
-    __syncthreads();   // cnt read before the next clear
+    if (pass < 3) {   // one addition per (tile, digit) of the warp
+      const int q = valid ? (p / T) * 256 + (int)((key[k] >> (shift + 8)) & 255u) : -1 - lane;
+      const unsigned peers = __match_any_sync(0xffffffffu, q);
+      if (valid && (peers & lt) == 0u) atomicAdd(&Hn[q], __popc(peers));
+    } else if (valid) {
+      const float *P = boxes + (size_t)idx[k] * GL;
+      const float y1 = P[0], x1 = P[1], y2 = P[2], x2 = P[3];
+      S.y1[p] = y1; S.x1[p] = x1; S.y2[p] = y2; S.x2[p] = x2;
+      S.ar[p] = (x2 - x1 + 1.0) * (y2 - y1 + 1.0);   // nms.cpp's area expression
+    }
   }
 }
 
 void launch_nms_radix(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
                       int *need, cudaStream_t s) {
-  k_rs_load<<<dim3((cap + 255) / 256, n_models), 256, 0, s>>>(boxes, d_num, GL, cap, si, sf, need);
-  const int tiles = nms_rs_tiles(cap);
+  const dim3 grid(nms_rs_tiles(cap), n_models);
+  k_rs_load<<<grid, kRsNT, 0, s>>>(boxes, d_num, GL, cap, si, sf, need);
   for (int p = 0; p < 4; p++) {
-    k_rs_count<<<dim3(tiles, n_models), kRsNT, 0, s>>>(p, cap, si, sf);
-    k_rs_scan<<<n_models, kRsScanNT, 0, s>>>(cap, si, sf);
-    k_rs_scatter<<<dim3(tiles, n_models), kRsNT, 0, s>>>(p, cap, si, sf);
+    if (nms_rs_tile(cap) == 2 * kRsNT) k_rs_pass<2><<<grid, kRsNT, 0, s>>>(p, boxes, GL, cap, si, sf);
+    else k_rs_pass<8><<<grid, kRsNT, 0, s>>>(p, boxes, GL, cap, si, sf);
   }
 }
 

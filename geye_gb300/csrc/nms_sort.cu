@@ -50,13 +50,8 @@ __global__ void __launch_bounds__(256) k_qs_load(const float *__restrict__ boxes
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     BatchState &st = *S.st;
     st.D = D;
-    st.nwords = (D + 31) >> 5;
-    st.scan_word = 0;
-    st.npicks = 0;
-    st.npb = 0;
     st.done = D <= 0;
-    st.batches = 0;
-    st.fallback = 0;
+    st.npicks = st.batches = st.next = 0;
     SortState &ss = *S.ss;
     ss.big_n[0] = D > kNmsSegS ? 1 : 0;
     ss.big_n[1] = 0;

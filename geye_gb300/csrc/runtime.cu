@@ -615,8 +615,7 @@ static geye_status finish_plan(geye_ctx *ctx, Plan &P, ArenaAlloc &A) {
   P.max_cap = (std::max(cap, 1) + 31) & ~31;
   const size_t nm = std::max<size_t>(P.models.size(), 1);
   GEYE_TRY(P.d_boxes.alloc(ctx, sizeof(float) * nm * P.max_cap * std::max(gl, 1)));
-  GEYE_TRY(P.d_kept_boxes.alloc(ctx, sizeof(float) * nm * P.max_cap * std::max(gl, 1)));
-  GEYE_TRY(P.d_nms_f.alloc(ctx, sizeof(float) * nm * P.max_cap * 6));
+  GEYE_TRY(P.d_nms_f.alloc(ctx, sizeof(float) * nm * P.max_cap * 10));
   GEYE_TRY(P.d_nms_i.alloc(ctx, sizeof(int) * nm * nms_model_words(P.max_cap)));
   GEYE_TRY(P.d_small.alloc(ctx, 4096));
   if (P.width > 0) {
@@ -893,36 +892,28 @@ geye_status run_ascore(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thre
 
 // After a frame of the plan has completed: `used` is the deepest grid-wide
 // quicksort level that had a segment to partition (0 when no model needed the
-// quicksort's order), `rounds` the greedy batches the frame took.
+// quicksort's order).
 // Sort levels: the first frame that sorts launches the default count
 // (nms_sort_levels); if it needed fewer, the plan launches three levels more
 // than it needed from then on (each empty level costs three launches).  A
 // frame whose last launched level still had work left its remaining segments
 // to the single-block fallback (exact, slower): the plan goes back to the
 // default count for good.
-// Rounds: a plan launches kNmsRounds (a round with nothing left is two launches
-// that return at once); a frame that took more batches than were launched (the
-// rest ran in the finish kernel's single block) makes it launch half as many
-// again plus two, so that a few frames settle it (each change costs a graph
-// capture), and the count only grows.
 // The plan's DT tile sizes are tuned here too, once, on this frame's maps
 // (tune_dt).  A change drops the plan's frame graphs after its stream has
 // drained; the next frame captures them again.
-void note_sort_levels(geye_ctx *ctx, Plan &P, int used, int rounds) {
+void note_sort_levels(geye_ctx *ctx, Plan &P, int used) {
   const int full = nms_sort_levels(P.max_cap);
   const int launched = P.sort_levels > 0 ? P.sort_levels : full;
-  const int r_launched = P.nms_rounds > 0 ? P.nms_rounds : kNmsRounds;
-  int next = P.sort_levels, r_next = P.nms_rounds;
+  int next = P.sort_levels;
   if (used >= launched) {
     if (P.sort_levels > 0) { next = 0; P.sort_levels_fixed = true; }
   } else if (!P.sort_levels_fixed && P.sort_levels == 0 && used > 0 && used + 3 < full) {
     next = std::max(4, used + 3);
   }
-  if (rounds > r_launched) r_next = std::min(kNmsMaxRounds, rounds + rounds / 2 + 2);
   const bool dt_changed = P.from_features ? false : tune_dt(ctx, P);   // (behind the frame on its stream)
-  if (next == P.sort_levels && r_next == P.nms_rounds && !dt_changed) return;
+  if (next == P.sort_levels && !dt_changed) return;
   P.sort_levels = next;
-  P.nms_rounds = r_next;
   cudaStreamSynchronize(ctx->stream);
   for (auto &g : P.graphs)
     if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
@@ -933,30 +924,25 @@ geye_status run_nms(geye_ctx *ctx, Plan &P, int n_models, float overlap) {
   int *d_num = P.d_small.as<int>();
   int *d_kept = d_num + 32;
   int *err = d_num + 128;
+  NmsResults res{};
+  for (int mi = 0; mi < n_models; mi++) {
+    geye_model *m = P.models[mi]->model;
+    res.m[mi] = {m->d_coef, m->h.numpart[0], m->h.ratio};
+  }
+  res.out = P.d_result.as<int>();
+  res.img_w = P.width;
+  res.img_h = P.height;
   const cudaError_t ge =
       launch_nms_batch(P.d_boxes.as<float>(), d_num, n_models, P.gl, overlap,
-                       1.25f * (float)std::max(P.width, P.height), P.max_cap, P.d_nms_i.as<int>(),
-                       P.d_nms_f.as<float>(), P.d_kept_boxes.as<float>(), d_kept, err,
-                       reinterpret_cast<long long *>(d_num + 512), P.sort_levels, d_num + kSortLevelsUsed,
-                       P.nms_rounds, d_num + kNmsRoundsUsed, d_num + kNmsNeed, ctx->nms_order, ctx->stream,
-                       (ctx->capturing && ctx->nms_if_node) ? ctx->aux : nullptr);
+                       P.max_cap, P.d_nms_i.as<int>(),
+                       P.d_nms_f.as<float>(), res, d_kept, err, reinterpret_cast<long long *>(d_num + 512),
+                       P.sort_levels, d_num + kSortLevelsUsed, d_num + kNmsNeed, ctx->nms_order,
+                       ctx->stream, (ctx->capturing && ctx->nms_if_node) ? ctx->aux : nullptr);
   if (ge != cudaSuccess) {
     set_error(std::string("nms graph nodes: ") + cudaGetErrorString(ge));
     return GEYE_ERR_CUDA;
   }
-  GEYE_TRY(check_launch(ctx, "nms"));
-  for (int mi = 0; mi < n_models; mi++) {
-    ModelPlan &mp = *P.models[mi];
-    geye_model *m = mp.model;
-    int *res = P.d_result.as<int>() + (size_t)mi * P.max_cap * 11;
-    int *point = res, *or_point = res + 4 * P.max_cap, *type = res + 8 * P.max_cap;
-    float *scale = reinterpret_cast<float *>(res + 9 * P.max_cap), *score = reinterpret_cast<float *>(res + 10 * P.max_cap);
-    launch_new_rects(P.d_kept_boxes.as<float>() + (size_t)mi * P.max_cap * P.gl, d_kept + mi, m->gl(),
-                     m->h.numpart[0], m->d_coef, P.width, P.height, m->h.ratio, point, or_point, type, scale, score,
-                     ctx->stream);
-    GEYE_TRY(check_launch(ctx, "new_rects"));
-  }
-  return GEYE_OK;
+  return check_launch(ctx, "nms");
 }
 
 // Everything after the ingest and the A_SCORE initialisation: plan-static, so

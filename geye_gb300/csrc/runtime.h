@@ -57,12 +57,11 @@ struct ArenaAlloc;
 geye_status plan_tc(geye_ctx *ctx, Plan &P, ArenaAlloc &A);
 geye_status build_tc_plan(geye_ctx *ctx, Plan &P);
 geye_status run_conv_tc(geye_ctx *ctx, Plan &P);
-// d_small[kSortLevelsUsed]: the deepest NMS sort level with work in the frame;
-// d_small[kNmsRoundsUsed]: the greedy batches it took
-constexpr int kSortLevelsUsed = 48, kNmsRoundsUsed = 49;
+// d_small[kSortLevelsUsed]: the deepest NMS sort level with work in the frame
+constexpr int kSortLevelsUsed = 48;
 // d_small[kNmsNeed + m]: model m's kept set was resolved again in the quicksort's order
 constexpr int kNmsNeed = 160;
-void note_sort_levels(geye_ctx *ctx, Plan &P, int used, int rounds);
+void note_sort_levels(geye_ctx *ctx, Plan &P, int used);
 // tensor-core fconvsMT of one feature map (float planes on the device) for the stage entry point
 geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, const float *const *filters,
                          const int *b_dims, int n_filters, float *d_out, const std::vector<int> &out_off,
@@ -194,7 +193,7 @@ struct Plan {
   size_t arena_words = 0, arena16_elems = 0;
   DevBuf arena, arena16;
   DevBuf d_bgr;                          // frame upload buffer
-  DevBuf d_boxes, d_kept_boxes, d_nms_f, d_nms_i, d_small, d_ascore, d_result;
+  DevBuf d_boxes, d_nms_f, d_nms_i, d_small, d_ascore, d_result;
   int gl = 0, max_cap = 0;
   // algorithmic bytes per stage (for roofline reporting)
   double bytes_resize = 0, bytes_hog = 0;
@@ -209,7 +208,6 @@ struct Plan {
   // grid-wide NMS sort levels launched per frame (0: the default for max_cap),
   // adapted once to the depth the plan's frames need (note_sort_levels)
   int sort_levels = 0;
-  int nms_rounds = 0;   // greedy resolve/pass rounds per frame (0: kNmsRounds), adapted to the frames
   bool sort_levels_fixed = false;
   // asynchronous submission (serve.cu): pinned frame staging, pinned result
   // block (counts, then per model kHostRes records) and the completion event

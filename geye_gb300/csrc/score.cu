@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "rects.h"
 
 namespace geye {
 
@@ -289,47 +290,20 @@ void launch_ascore_normalize(float *a_score, int n, const unsigned *max_bits, cu
   k_ascore_norm<<<blocks, 256, 0, s>>>(a_score, n, max_bits);
 }
 
-// get_new_rects on the kept records: coef = [comp][x1, y1, x2, y2][ML]
+// get_new_rects on kept records
 __global__ void k_new_rects(const float *__restrict__ kept, const int *__restrict__ d_kept, int GL, int np,
                             const float *__restrict__ coef, int img_w, int img_h, float ratio, int *point,
                             int *or_point, int *type, float *scale, float *score) {
   const int K = *d_kept;
-  const int ML = 1 + 2 * (1 + np);
-  const int LL = GL - 3;
-  for (int ii = blockIdx.x * blockDim.x + threadIdx.x; ii < K; ii += gridDim.x * blockDim.x) {
-    const float *P = kept + (size_t)ii * GL;
-    const int CNUM = (int)P[GL - 3];
-    const float *x1 = coef + ((size_t)CNUM * 4 + 0) * ML;
-    const float *y1 = coef + ((size_t)CNUM * 4 + 1) * ML;
-    const float *x2 = coef + ((size_t)CNUM * 4 + 2) * ML;
-    const float *y2 = coef + ((size_t)CNUM * 4 + 3) * ML;
-    float XP1 = 0, XP2 = 0, YP1 = 0, YP2 = 0;
-    for (int kk = 0; kk < ML; kk++) {
-      float av;
-      if (kk == 0) av = P[3] - P[1];
-      else {
-        const int q = kk - 1;                 // Avec = [w, (x1, y1) of root and parts]
-        const int box = q >> 1;
-        av = (q & 1) ? P[4 * box] : P[4 * box + 1];
-        if (4 * box >= LL) av = 0.f;
-      }
-      YP1 += av * y1[kk];
-      YP2 += av * y2[kk];
-      XP1 += av * x1[kk];
-      XP2 += av * x2[kk];
-    }
-    int PP[4];
-    PP[0] = XP1 > 0 ? (int)XP1 : 0;
-    PP[1] = YP1 > 0 ? (int)YP1 : 0;
-    PP[2] = XP2 < img_w ? (int)XP2 : img_w;
-    PP[3] = YP2 < img_h ? (int)YP2 : img_h;
-    for (int q = 0; q < 4; q++) {
-      point[4 * ii + q] = PP[q];
-      or_point[4 * ii + q] = (int)((float)PP[q] / ratio);
-    }
-    type[ii] = CNUM;
-    scale[ii] = P[GL - 1];
-    score[ii] = P[GL - 2];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 4 * K; e += gridDim.x * blockDim.x) {
+    const int k = e >> 2, c = e & 3;
+    const float *P = kept + (size_t)k * GL;
+    const int v = new_rect_side(P, GL, np, coef, img_w, img_h, c);
+    point[e] = v;
+    or_point[e] = (int)((float)v / ratio);
+    if (c == 0) type[k] = (int)P[GL - 3];
+    if (c == 1) scale[k] = P[GL - 1];
+    if (c == 2) score[k] = P[GL - 2];
   }
 }
 

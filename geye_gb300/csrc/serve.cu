@@ -94,7 +94,7 @@ static geye_status collect_frame(geye_ctx *ctx, geye_result *out, bool wait = tr
   if (wait) CUDA_TRY(cudaEventSynchronize(P.ev_done));
   const int n_models = (int)P.models.size();
   const int *h = static_cast<const int *>(P.h_res);
-  if (wait) note_sort_levels(ctx, P, h[kSortLevelsUsed], h[kNmsRoundsUsed]);
+  if (wait) note_sort_levels(ctx, P, h[kSortLevelsUsed]);
   geye_status st = GEYE_OK;
   for (int mi = 0; mi < n_models && out; mi++) {
     const int K = h[32 + mi];
@@ -423,7 +423,7 @@ geye_status reap(geye_server *s, bool block) {
 
 namespace geye {
 size_t plan_device_bytes(const Plan &P) {
-  size_t b = P.arena.bytes + P.arena16.bytes + P.d_bgr.bytes + P.d_boxes.bytes + P.d_kept_boxes.bytes +
+  size_t b = P.arena.bytes + P.arena16.bytes + P.d_bgr.bytes + P.d_boxes.bytes +
              P.d_nms_f.bytes + P.d_nms_i.bytes + P.d_small.bytes + P.d_ascore.bytes + P.d_result.bytes;
   b += P.d_conv_jobs.bytes + P.d_conv_blocks.bytes + P.d_conv_bank.bytes;
   b += P.tc.d_bank.bytes + P.tc.d_jobs.bytes + P.tc.d_chunks.bytes + P.tc.d_cols.bytes + P.tc.d_sums.bytes;
