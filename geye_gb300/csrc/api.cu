@@ -18,7 +18,7 @@ namespace geye {
 geye_status run_frame(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step, float thresh, float overlap,
                       const float *const *h_ascore_init);
 geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step);
-geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats);
+geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats, float *ref);
 geye_status run_conv(geye_ctx *ctx, Plan &P);
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp);
 geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh);
@@ -87,6 +87,7 @@ geye_status geye_ctx_create(int device, void *cuda_stream, geye_ctx **out) {
   geye_status s = ctx->d_diag.alloc(ctx, 256);
   if (s != GEYE_OK) { delete ctx; return s; }
   cudaMemset(ctx->d_diag.p, 0, 256);
+  host_pool_ref(1);
   *out = ctx;
   return GEYE_OK;
 }
@@ -110,7 +111,7 @@ geye_status geye_ctx_destroy(geye_ctx *ctx) {
   ctx->d_diag.release();
   for (auto &e : ctx->ev)
     if (e) cudaEventDestroy(e);
-  if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+  ctx->scratch.release();
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
   if (ctx->side) {
@@ -119,6 +120,7 @@ geye_status geye_ctx_destroy(geye_ctx *ctx) {
   }
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
+  host_pool_ref(-1);
   delete ctx;
   return GEYE_OK;
 }
@@ -218,7 +220,7 @@ geye_status geye_score_map(geye_ctx *ctx, const geye_model *m, int level, int co
   return GEYE_ERR_ARG;
 }
 
-void geye_free(void *p) { free(p); }
+void geye_free(void *p) { host_free(p); }
 
 // ---------------------------------------------------------------------------
 // models
@@ -325,43 +327,10 @@ geye_status geye_model_reset_scales(geye_model *m) {
 // ---------------------------------------------------------------------------
 // whole path
 // ---------------------------------------------------------------------------
-static geye_status fetch_model_result(geye_ctx *ctx, Plan &P, int mi, geye_result *out, int *D_out) {
-  int counts[4] = {0, 0, 0, 0};
-  CUDA_TRY(cudaMemcpyAsync(&counts[0], P.d_small.as<int>() + mi, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CUDA_TRY(cudaMemcpyAsync(&counts[1], P.d_small.as<int>() + 32 + mi, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  if (mi == 0)
-    CUDA_TRY(cudaMemcpyAsync(&counts[2], P.d_small.as<int>() + kSortLevelsUsed, sizeof(int), cudaMemcpyDeviceToHost,
-                             ctx->stream));
-  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  const int D = counts[0], K = counts[1];
-  if (mi == 0 && !P.from_features) note_sort_levels(ctx, P, counts[2]);
-  if (D_out) *D_out = D;
-  P.last_D[mi] = D;
-  P.last_K[mi] = K;
-  if (out) {
-    memset(out, 0, sizeof(*out));
-    out->num = K;
-    const size_t k = std::max(K, 1);
-    out->point = (int *)malloc(sizeof(int) * 4 * k);
-    out->or_point = (int *)malloc(sizeof(int) * 4 * k);
-    out->type = (int *)malloc(sizeof(int) * k);
-    out->scale = (float *)malloc(sizeof(float) * k);
-    out->score = (float *)malloc(sizeof(float) * k);
-    if (!out->point || !out->or_point || !out->type || !out->scale || !out->score) {
-      geye_result_free(out);
-      set_error("host allocation failed");
-      return GEYE_ERR_NOMEM;
-    }
-    if (K > 0) {
-      const int *res = P.d_result.as<int>() + (size_t)mi * P.max_cap * 11;
-      CUDA_TRY(cudaMemcpyAsync(out->point, res, sizeof(int) * 4 * K, cudaMemcpyDeviceToHost, ctx->stream));
-      CUDA_TRY(cudaMemcpyAsync(out->or_point, res + 4 * P.max_cap, sizeof(int) * 4 * K, cudaMemcpyDeviceToHost, ctx->stream));
-      CUDA_TRY(cudaMemcpyAsync(out->type, res + 8 * P.max_cap, sizeof(int) * K, cudaMemcpyDeviceToHost, ctx->stream));
-      CUDA_TRY(cudaMemcpyAsync(out->scale, res + 9 * P.max_cap, sizeof(float) * K, cudaMemcpyDeviceToHost, ctx->stream));
-      CUDA_TRY(cudaMemcpyAsync(out->score, res + 10 * P.max_cap, sizeof(float) * K, cudaMemcpyDeviceToHost, ctx->stream));
-    }
-  }
-  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+// the plan's finished frame (the stream has drained): plans adapt to it, then every model's result
+static geye_status read_results(geye_ctx *ctx, Plan &P, geye_result *out) {
+  note_sort_levels(ctx, P, static_cast<const int *>(P.h_res)[kSortLevelsUsed]);
+  for (size_t i = 0; i < P.models.size(); i++) GEYE_TRY(read_result(P, (int)i, &out[i]));
   return GEYE_OK;
 }
 
@@ -380,14 +349,12 @@ geye_status geye_detect_multi(geye_ctx *ctx, geye_model *const *models, int n_mo
   if (a_scores)
     for (int i = 0; i < n_models; i++) init[i] = a_scores[i];
   GEYE_TRY(run_frame(ctx, *P, P->d_bgr.as<uint8_t>(), 3 * width, thresh, overlap, init.data()));
-  for (int i = 0; i < n_models; i++) {
-    GEYE_TRY(fetch_model_result(ctx, *P, i, &out[i], nullptr));
+  for (int i = 0; i < n_models; i++)
     if (a_scores && a_scores[i])
       CUDA_TRY(cudaMemcpyAsync(a_scores[i], P->d_ascore.as<float>() + (size_t)i * width * height,
                                sizeof(float) * (size_t)width * height, cudaMemcpyDeviceToHost, ctx->stream));
-  }
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return GEYE_OK;
+  return read_results(ctx, *P, out);
 }
 
 geye_status geye_car_detection(geye_ctx *ctx, geye_model *model, const uint8_t *bgr, int width, int height,
@@ -418,7 +385,12 @@ geye_status geye_detect_device(geye_ctx *ctx, geye_model *const *models, int n_m
 geye_status geye_fetch_result(geye_ctx *ctx, int model_index, geye_result *out, int *n_boxes_before_nms) {
   ARG_CHECK(ctx && ctx->last_plan, "no device-resident run to fetch");
   ARG_CHECK(model_index >= 0 && model_index < (int)ctx->last_plan->models.size(), "model index out of range");
-  return fetch_model_result(ctx, *ctx->last_plan, model_index, out, n_boxes_before_nms);
+  Plan &P = *ctx->last_plan;
+  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (model_index == 0) note_sort_levels(ctx, P, static_cast<const int *>(P.h_res)[kSortLevelsUsed]);
+  GEYE_TRY(read_result(P, model_index, out));
+  if (n_boxes_before_nms) *n_boxes_before_nms = P.last_D[model_index];
+  return GEYE_OK;
 }
 
 }  // extern "C"

@@ -611,21 +611,6 @@ __global__ void k_feat_planes(const float *__restrict__ feat, int fs0, int fs1, 
 // ---------------------------------------------------------------------------
 // host: the filter bank
 // ---------------------------------------------------------------------------
-static uint16_t to_bf16(float f) {   // round to nearest even
-  uint32_t u;
-  memcpy(&u, &f, 4);
-  if ((u & 0x7f800000u) == 0x7f800000u) return (uint16_t)(u >> 16);   // inf / nan
-  const uint32_t lsb = (u >> 16) & 1u;
-  u += 0x7fffu + lsb;
-  return (uint16_t)(u >> 16);
-}
-static float from_bf16(uint16_t h) {
-  const uint32_t u = (uint32_t)h << 16;
-  float f;
-  memcpy(&f, &u, 4);
-  return f;
-}
-
 static int tc_planes_of(geye_conv_mode mode) { return mode == GEYE_CONV_FP8 ? 2 : 4; }
 static int pad16(int n) { return (n + 15) & ~15; }
 
@@ -641,8 +626,7 @@ static float e4m3_filter_scale(const float *F, size_t n) {
 // from its row y0, column x0 on (a whole filter: 0, 0), or the BF16 remainder of
 // those weights (lo).  Padding rows have no filter.
 struct BankRow {
-  const float *h = nullptr;   // host copy
-  const float *d = nullptr;   // device copy (FP8 banks are converted on the device)
+  const float *d = nullptr;   // on the device
   int fb0 = 0, fb1 = 0, y0 = 0, x0 = 0, lo = 0;
   float scale = 1.f;          // FP8: the filter's power-of-two scale
 };
@@ -651,7 +635,29 @@ struct DevRow {
   const float *f;
   int fb0, fb1, y0, x0;
   float scale;
+  int lo;
 };
+
+// BF16 bank [tap][4][rows][8]: element (tap t = xp*b0 + yp, plane q, row r, lane k) =
+// channel 8q + k of row r's filter at (x0 + xp, y0 + yp), rounded to BF16, or (lo) its
+// remainder; zero outside the filter
+__global__ void k_bank_bf16(const DevRow *__restrict__ rows, int n_rows, int R, int b0, int taps,
+                            __nv_bfloat16 *__restrict__ out) {
+  const size_t total = (size_t)taps * 4 * R * 8;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+    const int k = (int)(e % 8), r = (int)((e / 8) % R), q = (int)((e / (8 * (size_t)R)) % 4);
+    const int t = (int)(e / (32 * (size_t)R));
+    const int c = 8 * q + k, xp = t / b0, yp = t - xp * b0;
+    float v = 0.f;
+    if (r < n_rows && c < kFeat) {
+      const DevRow D = rows[r];
+      const int x = D.x0 + xp, y = D.y0 + yp;
+      if (D.f && x < D.fb1 && y < D.fb0) v = D.f[(size_t)c * D.fb0 * D.fb1 + (size_t)x * D.fb0 + y];
+      if (D.lo) v -= __bfloat162float(__float2bfloat16_rn(v));
+    }
+    out[e] = __float2bfloat16_rn(v);
+  }
+}
 
 // e4m3 bank [tap][2][rows][16]: element (tap t = xp*b0 + yp, plane q, row r, lane k)
 // = channel 16q + k of row r's filter at (x0 + xp, y0 + yp) times its scale, CUDA's
@@ -684,42 +690,24 @@ static size_t layout_bytes(int NQ, int b0, int b1, int n) { return (size_t)b0 * 
 static geye_status upload_bank(geye_ctx *ctx, const std::vector<BankRow> &rows, int NQ, int b0, int b1,
                                const std::vector<BankLayout> &layouts, size_t total, DevBuf &dst) {
   GEYE_TRY(dst.alloc(ctx, std::max<size_t>(total, 16)));
-  if (NQ == 4) {
-    std::vector<uint16_t> bank(total / 2, 0);
-    for (const BankLayout &L : layouts) {
-      uint16_t *out = bank.data() + L.off / 2;
-      for (int xp = 0; xp < b1; xp++)
-        for (int yp = 0; yp < b0; yp++) {
-          const size_t t = (size_t)xp * b0 + yp;
-          for (int r = 0; r < L.n; r++) {
-            const BankRow &B = rows[L.first + r];
-            const int x = B.x0 + xp, y = B.y0 + yp;
-            if (!B.h || x >= B.fb1 || y >= B.fb0) continue;
-            for (int c = 0; c < kFeat; c++) {
-              const float w = B.h[(size_t)c * B.fb0 * B.fb1 + (size_t)x * B.fb0 + y];
-              const uint16_t hi = to_bf16(w);
-              out[((t * 4 + (c >> 3)) * L.n + r) * 8 + (c & 7)] = B.lo ? to_bf16(w - from_bf16(hi)) : hi;
-            }
-          }
-        }
-    }
-    CUDA_TRY(cudaMemcpyAsync(dst.p, bank.data(), total, cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return GEYE_OK;
-  }
   std::vector<DevRow> dr;
-  for (const BankRow &B : rows) dr.push_back(DevRow{B.d, B.fb0, B.fb1, B.y0, B.x0, B.scale});
-  DevBuf d_rows;
+  for (const BankRow &B : rows) dr.push_back(DevRow{B.d, B.fb0, B.fb1, B.y0, B.x0, B.scale, B.lo});
+  DevBuf d_rows(dst.arena);
   GEYE_TRY(upload_bytes(ctx, d_rows, dr.data(), sizeof(DevRow) * std::max<size_t>(dr.size(), 1)));
   const int taps = b0 * b1;
   for (const BankLayout &L : layouts) {
-    const size_t elems = (size_t)taps * 2 * L.n * 16;
-    k_bank_e4m3<<<(int)std::max<size_t>(1, std::min<size_t>((elems + 255) / 256, 2048)), 256, 0, ctx->stream>>>(
-        d_rows.as<DevRow>() + L.first, std::max(0, std::min(L.n, (int)dr.size() - L.first)), L.n, b0, taps,
-        dst.as<uint8_t>() + L.off);
+    const size_t elems = (size_t)taps * 32 * L.n;
+    const int grid = (int)std::max<size_t>(1, std::min<size_t>((elems + 255) / 256, 2048));
+    const DevRow *first = d_rows.as<DevRow>() + L.first;
+    const int n_rows = std::max(0, std::min(L.n, (int)dr.size() - L.first));
+    uint8_t *out = dst.as<uint8_t>() + L.off;
+    if (NQ == 4)
+      k_bank_bf16<<<grid, 256, 0, ctx->stream>>>(first, n_rows, L.n, b0, taps, reinterpret_cast<__nv_bfloat16 *>(out));
+    else
+      k_bank_e4m3<<<grid, 256, 0, ctx->stream>>>(first, n_rows, L.n, b0, taps, out);
     CUDA_TRY(cudaGetLastError());
   }
-  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (!dst.arena) CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // before d_rows is freed
   return GEYE_OK;
 }
 
@@ -1142,7 +1130,6 @@ geye_status build_tc_plan(geye_ctx *ctx, Plan &P) {
     const HostModel &h = m->h;
     const bool root = b.filt < h.NoR;
     BankRow R;
-    R.h = root ? h.rootfilter[b.filt].data() : h.partfilter[b.filt - h.NoR].data();
     R.d = m->d_filters + m->filt_off[b.filt];
     R.fb0 = root ? h.root_size[3 * b.filt] : h.part_size[3 * (b.filt - h.NoR)];
     R.fb1 = root ? h.root_size[3 * b.filt + 1] : h.part_size[3 * (b.filt - h.NoR) + 1];
@@ -1321,10 +1308,10 @@ geye_status run_conv_tc(geye_ctx *ctx, Plan &P) {
 // bank over the largest filter's grid.  Temporary device buffers live in tmp.
 geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, const float *const *filters,
                          const int *b_dims, int n_filters, float *d_out, const std::vector<int> &out_off,
-                         std::vector<std::unique_ptr<DevBuf>> &tmp) {
+                         std::vector<std::unique_ptr<DevBuf>> &tmp, int *err) {
   const geye_conv_mode mode = ctx->conv_mode;
   const int NQ = tc_planes_of(mode);
-  auto buf = [&]() { tmp.push_back(std::make_unique<DevBuf>()); return tmp.back().get(); };
+  auto buf = [&]() { tmp.push_back(std::make_unique<DevBuf>(&ctx->scratch)); return tmp.back().get(); };
   int gb0 = 1, gb1 = 1;
   for (int i = 0; i < n_filters; i++) { gb0 = std::max(gb0, b_dims[2 * i]); gb1 = std::max(gb1, b_dims[2 * i + 1]); }
   const int R = pad16(n_filters);
@@ -1335,14 +1322,18 @@ geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, con
   std::vector<BankRow> rows(R);
   std::vector<TcCol> cols(R);
   int p_valid = 0;
+  std::vector<float> all;   // every filter in one upload
+  for (int i = 0; i < n_filters; i++)
+    all.insert(all.end(), filters[i], filters[i] + (size_t)b_dims[2 * i] * b_dims[2 * i + 1] * kFeat);
+  DevBuf *d_filters = buf();
+  GEYE_TRY(upload_bytes(ctx, *d_filters, all.data(), sizeof(float) * all.size()));
+  size_t at = 0;
   for (int i = 0; i < n_filters; i++) {
     const int fb0 = b_dims[2 * i], fb1 = b_dims[2 * i + 1];
     const size_t n = (size_t)fb0 * fb1 * kFeat;
-    DevBuf *f = buf();
-    GEYE_TRY(upload_bytes(ctx, *f, filters[i], sizeof(float) * n));
     BankRow &B = rows[i];
-    B.h = filters[i];
-    B.d = f->as<float>();
+    B.d = d_filters->as<float>() + at;
+    at += n;
     B.fb0 = fb0;
     B.fb1 = fb1;
     B.scale = mode == GEYE_CONV_FP8 ? e4m3_filter_scale(filters[i], n) : 1.f;
@@ -1398,13 +1389,7 @@ geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, con
   launch_conv_tc(NQ, d_jobs->as<TcJob>(), d_chunks->as<int4>(), (int)chunks.size(), d_cols->as<TcCol>(),
                  planes->as<uint8_t>(), d_bank->as<uint8_t>(), stages, tps, d_out, d_err->as<int>(), smem, ctx->stream);
   CUDA_TRY(cudaGetLastError());
-  int errw = 0;
-  CUDA_TRY(cudaMemcpyAsync(&errw, d_err->p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  if (errw) {
-    set_error("tensor-core conv: a tensor-core wait ran out (error bits " + std::to_string(errw) + ")");
-    return GEYE_ERR_TIMEOUT;
-  }
+  CUDA_TRY(cudaMemcpyAsync(err, d_err->p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   return GEYE_OK;
 }
 

@@ -71,6 +71,7 @@ struct HogJob {
   int hist_off;            // [18][b1*b0] then norm [b1*b0] at hist_off + 18*b1*b0
   int fs0, fs1;            // output cells
   int feat_off;            // float planes (feat_stride)
+  int ref_off;             // the level's place in calc_f_pyramid's output
   int feat16_off;          // tensor-core planes (offset in 2-byte units), -1 = not written
   int feat16lo_off;        // BF16 remainder planes (root levels in BF16 mode), -1 = none
   int fast;                // 1 (tensor-core modes): float normalisation factors computed per cell,
@@ -272,10 +273,11 @@ constexpr int kBatchCells = 256;   // corners / cells per item (a thread each)
 // one stage (phase: the resize phase) over n items
 void launch_batch_front(int stage, const BatchFrame *d_frames, const BatchItem *d_items, int n, int phase,
                         cudaStream_t s);
-// corners: run the corner-factor pass (jobs with fast = 0 read its factors); floats: write the float planes
+// corners: run the corner-factor pass (jobs with fast = 0 read its factors); floats: write the float planes;
+// ref: write the levels there instead, in the reference layout at their ref_off
 void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int n_vote_blocks, int max_b0,
                 int max_b1, const HogPixJob *d_pix, int n_pix, int max_xe, float *arena, void *arena16,
-                bool corners, bool floats, cudaStream_t s);   // arena16: base of the tensor-core planes (bytes)
+                bool corners, bool floats, float *ref, cudaStream_t s);   // arena16: base of the tensor-core planes (bytes)
 void launch_to_ref_layout(const float *feat, int fs0, int fs1, float *out, cudaStream_t s);
 void launch_flip_feat(const float *feat, int n0, int n1, float *out, cudaStream_t s);
 void launch_from_ref_layout(const float *ref, int fs0, int fs1, float *feat, cudaStream_t s);
@@ -336,6 +338,9 @@ struct NmsResults {
     float ratio;
   } m[16];
   int *out;
+  // the frame's result block in pinned host memory (Plan::h_res): counts, then host_cap records a model
+  int *host;
+  int host_cap;
   int img_w, img_h;
 };
 // diag (optional): per model m, diag[8m+1..8m+5] = sort segments left to the fallback, batches, picks,
@@ -344,6 +349,8 @@ struct NmsResults {
 // need: n_models ints, zero on entry; order: kNmsOrderKey (the scores in
 // key order, the quicksort's order only for the models that need it: need[m]
 // raised) or kNmsOrderQuicksort (the quicksort's order for every model)
+// d_small[kSortLevelsUsed] and the same place of the host's result block: the deepest sort level with work in the frame
+constexpr int kSortLevelsUsed = 63;
 constexpr int kNmsOrderKey = 0, kNmsOrderQuicksort = 1;
 // aux: null for plain launches on s; when s is capturing a graph, a second
 // stream that captures the body of the quicksort-order pass's if node

@@ -433,7 +433,8 @@ __device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, in
 template <bool KEY_ORDER>
 __device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int m, int npk, int batches, const float *boxes,
                                              int GL, int cap, const NmsResults &res, int *d_kept, long long *diag,
-                                             int *need, cudaGraphConditionalHandle cond, bool has_cond) {
+                                             const int *lv_used, int *need, cudaGraphConditionalHandle cond,
+                                             bool has_cond) {
   const int D = S.st->D;
   // (the flags are read past L1: other blocks of the cluster have set them)
   const int K = npk - ((npk > 0 && __ldcg(&S.flag[npk - 1]) == 0) ? 1 : 0);
@@ -485,17 +486,26 @@ __device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int 
       diag[8 * m + 5] = need ? *(volatile int *)&need[m] : 1;
     }
   }
-  // the results (get_new_rects), four threads a box
+  // the results (get_new_rects), four threads a box: on the device, and the first of them in the host's block
   const NmsResults::Model &Q = res.m[m];
-  int *out = res.out + (size_t)m * cap * 11;
+  int *out = res.out + (size_t)m * cap * 11, *host = res.host + 64 + (size_t)m * 11 * res.host_cap;
   for (int e = threadIdx.x; e < 4 * K; e += kResNT) {
     const int k = e >> 2, c = e & 3;
     const float *P = boxes + (size_t)keep[k] * GL;
-    const int v = new_rect_side(P, GL, Q.np, Q.coef, res.img_w, res.img_h, c);
-    out[4 * k + c] = v;
-    out[4 * (size_t)cap + 4 * k + c] = (int)((float)v / Q.ratio);
+    const int v = new_rect_side(P, GL, Q.np, Q.coef, res.img_w, res.img_h, c), r = (int)((float)v / Q.ratio);
     // type, scale, score
-    if (c < 3) out[(8 + c) * (size_t)cap + k] = c == 0 ? (int)P[GL - 3] : __float_as_int(P[c == 1 ? GL - 1 : GL - 2]);
+    const int more = c == 0 ? (int)P[GL - 3] : __float_as_int(P[c == 1 ? GL - 1 : GL - 2]);
+    auto put = [&](int *o, size_t stride) {
+      o[e] = v;
+      o[4 * stride + e] = r;
+      if (c < 3) o[(8 + c) * stride + k] = more;
+    };
+    put(out, cap);
+    if (k < res.host_cap) put(host, res.host_cap);
+  }
+  if (threadIdx.x == 0) {
+    res.host[32 + m] = K;
+    if (!KEY_ORDER) res.host[kSortLevelsUsed] = *lv_used;
   }
 }
 
@@ -521,8 +531,8 @@ template <bool KEY_ORDER>
 __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restrict__ boxes_all, int GL, int cap, int *si,
                                                        float *sf, float overlap, float2 cell_inv,
                                                        const __grid_constant__ NmsResults res, int *d_kept,
-                                                       long long *diag, int *need, cudaGraphConditionalHandle cond,
-                                                       bool has_cond, bool rest) {
+                                                       long long *diag, const int *lv_used, int *need,
+                                                       cudaGraphConditionalHandle cond, bool has_cond, bool rest) {
   extern __shared__ __align__(16) unsigned char res_sm[];
   GreedySmem &R = *reinterpret_cast<GreedySmem *>(res_sm);
   cg::cluster_group cluster = cg::this_cluster();
@@ -611,8 +621,8 @@ __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restric
   }
   if (rank == 0) {
     if (threadIdx.x == 0) S.st->done = 1;
-    finish_model<KEY_ORDER>(S, R, m, np, batches, boxes_all + (size_t)m * cap * GL, GL, cap, res, d_kept, diag, need,
-                            cond, has_cond);
+    finish_model<KEY_ORDER>(S, R, m, np, batches, boxes_all + (size_t)m * cap * GL, GL, cap, res, d_kept, diag, lv_used,
+                            need, cond, has_cond);
   }
 }
 
@@ -698,7 +708,7 @@ static int cluster_blocks(K *kernel, size_t smem) {
 // the greedy rounds and the results, in the order the sort left in (val, ord)
 template <bool KEY_ORDER>
 static cudaError_t launch_greedy(const float *boxes, int n_models, int GL, float overlap, float2 cell_inv, int cap, int *si,
-                                 float *sf, const NmsResults &res, int *d_kept, long long *diag, int *need,
+                                 float *sf, const NmsResults &res, int *d_kept, long long *diag, const int *lv_used, int *need,
                                  cudaGraphConditionalHandle cond, bool has_cond, cudaStream_t s) {
   static SmemAttr attr;
   cudaError_t e = raise_smem(attr, k_nms_greedy<KEY_ORDER>, sizeof(GreedySmem));
@@ -720,7 +730,7 @@ static cudaError_t launch_greedy(const float *boxes, int n_models, int GL, float
       k_nms_rest<<<dim3(std::max(304 / n_models, 1), n_models), kResNT, 0, s>>>(cap, si, sf, overlap, cell_inv);
     }
     e = cudaLaunchKernelEx(&c, k_nms_greedy<KEY_ORDER>, boxes, GL, cap, si, sf, overlap, cell_inv, res, d_kept, diag,
-                           need, cond, has_cond, rest);
+                           lv_used, need, cond, has_cond, rest);
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
@@ -738,9 +748,9 @@ cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models,
   };
   cudaError_t e = cudaSuccess;
   if (order == kNmsOrderQuicksort) {
-    launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, nullptr, s);
+    launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, nullptr, res.host, s);
     gather(s);
-    e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, nullptr, 0,
+    e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, lv_used, nullptr, 0,
                              false, s);
     return e == cudaSuccess ? cudaGetLastError() : e;
   }
@@ -751,8 +761,8 @@ cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models,
   // the models that do not
   cudaGraphConditionalHandle h = 0;
   if (aux && (e = cond_handle(s, 0u, &h)) != cudaSuccess) return e;
-  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, s);
-  if ((e = launch_greedy<true>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, need, h,
+  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, res.host, s);
+  if ((e = launch_greedy<true>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, lv_used, need, h,
                                aux != nullptr, s)) != cudaSuccess)
     return e;
   cudaStream_t q = s;
@@ -760,9 +770,9 @@ cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models,
     if ((e = begin_conditional(s, aux, cudaGraphCondTypeIf, h)) != cudaSuccess) return e;
     q = aux;
   }
-  launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, need, q);
+  launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, need, res.host, q);
   gather(q);
-  e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, need, 0, false,
+  e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, lv_used, need, 0, false,
                            q);
   if (aux) {
     const cudaError_t e2 = end_conditional(aux);

@@ -272,11 +272,12 @@ __device__ __forceinline__ bool supp(float Ay1, float Ax1, float Ay2, float Ax2,
 // *lv_used (optional) gets the deepest level that had a segment to partition.
 // need (optional): only the models with need[m] set are sorted; the others
 // are left with an empty, finished state
+// host: the frame's result block; every model's counts start at (D, 0 kept)
 void launch_nms_sort(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
-                     int *err, long long *diag, int levels, int *lv_used, const int *need, cudaStream_t s);
+                     int *err, long long *diag, int levels, int *lv_used, const int *need, int *host, cudaStream_t s);
 // key-order sort (nms_radix.cu): val = transformed keys, ord = input index,
 // BatchState initialised; need[m] set for a NaN score
 void launch_nms_radix(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
-                      int *need, cudaStream_t s);
+                      int *need, int *host, cudaStream_t s);
 
 }  // namespace geye

@@ -49,7 +49,7 @@ __device__ __forceinline__ unsigned rs_key(float v, bool &nan) {
 }
 
 __global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ boxes_all, const int *__restrict__ d_num,
-                                                   int GL, int cap, int *si, float *sf, int *need) {
+                                                   int GL, int cap, int *si, float *sf, int *need, int *host) {
   __shared__ int h[256];
   const int m = blockIdx.y, t = blockIdx.x;
   Slots S = slots(si, sf, m, cap);
@@ -60,6 +60,9 @@ __global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ box
     st.D = D;
     st.done = D <= 0;
     st.npicks = st.batches = st.next = 0;
+    host[m] = D;
+    host[32 + m] = 0;
+    if (m == 0) host[kSortLevelsUsed] = 0;
   }
   const int e0 = t * T;
   if (e0 >= D) return;
@@ -197,9 +200,9 @@ __global__ void __launch_bounds__(kRsNT) k_rs_pass(int pass, const float *__rest
 }
 
 void launch_nms_radix(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
-                      int *need, cudaStream_t s) {
+                      int *need, int *host, cudaStream_t s) {
   const dim3 grid(nms_rs_tiles(cap), n_models);
-  k_rs_load<<<grid, kRsNT, 0, s>>>(boxes, d_num, GL, cap, si, sf, need);
+  k_rs_load<<<grid, kRsNT, 0, s>>>(boxes, d_num, GL, cap, si, sf, need, host);
   for (int p = 0; p < 4; p++) {
     if (nms_rs_tile(cap) == 2 * kRsNT) k_rs_pass<2><<<grid, kRsNT, 0, s>>>(p, boxes, GL, cap, si, sf);
     else k_rs_pass<8><<<grid, kRsNT, 0, s>>>(p, boxes, GL, cap, si, sf);

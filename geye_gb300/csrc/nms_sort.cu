@@ -36,7 +36,7 @@ constexpr int kQ = 1024;         // k_qs_rest's block-tier queue
 // load
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_qs_load(const float *__restrict__ boxes_all, const int *__restrict__ d_num,
-                                                 int GL, int cap, int *si, float *sf, const int *need) {
+                                                 int GL, int cap, int *si, float *sf, const int *need, int *host) {
   const int m = blockIdx.y;
   Slots S = slots(si, sf, m, cap);
   const float *boxes = boxes_all + (size_t)m * cap * GL;
@@ -52,6 +52,11 @@ __global__ void __launch_bounds__(256) k_qs_load(const float *__restrict__ boxes
     st.D = D;
     st.done = D <= 0;
     st.npicks = st.batches = st.next = 0;
+    if (!need) {
+      host[m] = D;
+      host[32 + m] = 0;
+      if (m == 0) host[kSortLevelsUsed] = 0;
+    }
     SortState &ss = *S.ss;
     ss.big_n[0] = D > kNmsSegS ? 1 : 0;
     ss.big_n[1] = 0;
@@ -496,9 +501,9 @@ int nms_sort_levels(int cap) {
 }
 
 void launch_nms_sort(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
-                     int *err, long long *diag, int levels, int *lv_used, const int *need, cudaStream_t s) {
+                     int *err, long long *diag, int levels, int *lv_used, const int *need, int *host, cudaStream_t s) {
   if (levels <= 0) levels = nms_sort_levels(cap);
-  k_qs_load<<<dim3((cap + 255) / 256, n_models), 256, 0, s>>>(boxes, d_num, GL, cap, si, sf, need);
+  k_qs_load<<<dim3((cap + 255) / 256, n_models), 256, 0, s>>>(boxes, d_num, GL, cap, si, sf, need, host);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

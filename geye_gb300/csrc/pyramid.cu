@@ -404,7 +404,7 @@ __global__ void k_hog_norm(const HogJob *__restrict__ jobs, float *__restrict__ 
 
 // output cell i of one level
 __device__ __forceinline__ void hog_feat_one(const HogJob &J, float *__restrict__ arena,
-                                             uint8_t *__restrict__ arena16, int i, bool floats) {
+                                             uint8_t *__restrict__ arena16, int i, bool floats, float *ref) {
   const int ncell = J.fs0 * J.fs1;
   const int b0 = J.b0, nb = J.b0 * J.b1;
   const float *hist = arena + J.hist_off;
@@ -468,8 +468,9 @@ __device__ __forceinline__ void hog_feat_one(const HogJob &J, float *__restrict_
     }
     out[31] = 0.f;
     if (floats) {   // (the tensor-core modes' frames read only the channel planes below)
-      float *dst = arena + J.feat_off + (size_t)x * feat_stride(J.fs0) + y;
-      const size_t plane = (size_t)feat_stride(J.fs0) * J.fs1;
+      const int col = ref ? J.fs0 : feat_stride(J.fs0);
+      float *dst = (ref ? ref + J.ref_off : arena + J.feat_off) + (size_t)x * col + y;
+      const size_t plane = (size_t)col * J.fs1;
 #pragma unroll
       for (int c = 0; c < kFeat; c++) dst[c * plane] = out[c];
     }
@@ -484,11 +485,11 @@ __device__ __forceinline__ void hog_feat_one(const HogJob &J, float *__restrict_
 }
 
 __global__ void k_hog_feat(const HogJob *__restrict__ jobs, float *__restrict__ arena, uint8_t *__restrict__ arena16,
-                           bool floats) {
+                           bool floats, float *__restrict__ ref) {
   const HogJob J = jobs[blockIdx.y];
   const int ncell = J.fs0 * J.fs1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncell; i += gridDim.x * blockDim.x)
-    hog_feat_one(J, arena, arena16, i, floats);
+    hog_feat_one(J, arena, arena16, i, floats, ref);
 }
 
 // ----------------------------------------------------------------------------
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(256) k_batch_front(const BatchFrame *__restric
     } else {
       const HogJob J = F.hog[I.job];
       const int i = I.chunk * kBatchCells + tid;
-      if (i < J.fs0 * J.fs1) hog_feat_one(J, F.arena, F.arena16, i, !J.fast);
+      if (i < J.fs0 * J.fs1) hog_feat_one(J, F.arena, F.arena16, i, !J.fast, nullptr);
     }
   }
 }
@@ -554,7 +555,7 @@ void hog_vote_blocks(const std::vector<HogJob> &jobs, std::vector<int2> &blocks)
 
 void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int n_vote_blocks, int max_b0,
                 int max_b1, const HogPixJob *d_pix, int n_pix, int max_xe, float *arena, void *arena16,
-                bool corners, bool floats, cudaStream_t s) {
+                bool corners, bool floats, float *ref, cudaStream_t s) {
   if (n_jobs <= 0) return;
   dim3 g0((max_xe + kPixWarps - 1) / kPixWarps, n_pix);
   k_hog_pix<<<g0, kPixWarps * 32, 0, s>>>(d_pix, arena);
@@ -564,7 +565,7 @@ void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int
   if (bx > 512) bx = 512;
   dim3 g2(bx, n_jobs);
   if (corners) k_hog_norm<<<g2, 256, 0, s>>>(d_jobs, arena);
-  k_hog_feat<<<g2, 256, 0, s>>>(d_jobs, arena, reinterpret_cast<uint8_t *>(arena16), floats);
+  k_hog_feat<<<g2, 256, 0, s>>>(d_jobs, arena, reinterpret_cast<uint8_t *>(arena16), floats, ref);
 }
 
 // ----------------------------------------------------------------------------

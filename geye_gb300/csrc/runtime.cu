@@ -12,6 +12,7 @@
 //   score assembly inputs                CAR_TRACKING/get_boxes.cpp:1000-1360
 #include <math.h>
 #include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -39,9 +40,16 @@ static bool injected(geye_ctx *ctx, const char *op) {
 
 DevBuf::~DevBuf() { release(); }
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  if (p && !arena) cudaFree(p);
   p = nullptr;
   bytes = 0;
+}
+static geye_status device_alloc(size_t n, void **out) {
+  const cudaError_t e = cudaMalloc(out, n);
+  if (e == cudaSuccess) return GEYE_OK;
+  *out = nullptr;
+  set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  return GEYE_ERR_NOMEM;
 }
 geye_status DevBuf::alloc(geye_ctx *ctx, size_t n) {
   if (n <= bytes && p) return GEYE_OK;
@@ -51,13 +59,112 @@ geye_status DevBuf::alloc(geye_ctx *ctx, size_t n) {
     return GEYE_ERR_INJECTED;
   }
   if (n == 0) n = 16;
-  cudaError_t e = cudaMalloc(&p, n);
-  if (e != cudaSuccess) {
-    p = nullptr;
-    set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  GEYE_TRY(arena ? arena->take(ctx, n, &p) : device_alloc(n, &p));
+  bytes = n;
+  return GEYE_OK;
+}
+
+void ScratchArena::release() {
+  for (auto &c : chunks) cudaFree(c.p);
+  chunks.clear();
+  used = total = 0;
+}
+geye_status ScratchArena::take(geye_ctx *, size_t n, void **out) {
+  n = (n + 255) & ~size_t(255);
+  if (chunks.empty() || chunks.back().bytes - used < n) {
+    const size_t bytes = std::max({n, want, size_t(1) << 20});
+    void *p = nullptr;
+    GEYE_TRY(device_alloc(bytes, &p));
+    chunks.push_back({static_cast<char *>(p), bytes});
+    used = 0;
+  }
+  *out = chunks.back().p + used;
+  used += n;
+  total += n;
+  return GEYE_OK;
+}
+void ScratchArena::reset() {
+  want = std::max(want, total);
+  if (want > kScratchKeep) want = 0;
+  // one chunk that held the whole call stays; several make way for one of their sum
+  if (chunks.size() > 1 || (!chunks.empty() && chunks.back().bytes > kScratchKeep)) release();
+  used = total = 0;
+}
+
+// blocks carry their size in front (a cache line, so that the caller's part stays aligned)
+static std::mutex g_host_mu;
+static std::vector<std::pair<size_t, char *>> g_host_kept;
+static int g_host_refs = 0;
+constexpr size_t kHostHead = 64, kHostBig = 1 << 20, kHostKeep = 256ull << 20;
+void *host_alloc(size_t n) {
+  n = std::max<size_t>(n, 1);
+  if (n >= kHostBig) {
+    std::lock_guard<std::mutex> g(g_host_mu);
+    for (auto it = g_host_kept.begin(); it != g_host_kept.end(); ++it)
+      if (it->first >= n && it->first <= 2 * n) {
+        char *p = it->second;
+        g_host_kept.erase(it);
+        return p + kHostHead;
+      }
+  }
+  char *p = static_cast<char *>(aligned_alloc(kHostHead, (n + 2 * kHostHead - 1) & ~(kHostHead - 1)));
+  if (!p) return nullptr;
+  *reinterpret_cast<size_t *>(p) = n;
+  return p + kHostHead;
+}
+void host_free(void *q) {
+  if (!q) return;
+  char *p = static_cast<char *>(q) - kHostHead;
+  const size_t n = *reinterpret_cast<size_t *>(p);
+  if (n >= kHostBig) {
+    std::lock_guard<std::mutex> g(g_host_mu);
+    size_t kept = n;
+    for (auto &k : g_host_kept) kept += k.first;
+    if (g_host_refs > 0 && kept <= kHostKeep && g_host_kept.size() < 8) {
+      g_host_kept.push_back({n, p});
+      return;
+    }
+  }
+  free(p);
+}
+void host_pool_ref(int d) {
+  std::lock_guard<std::mutex> g(g_host_mu);
+  g_host_refs += d;
+  if (g_host_refs > 0) return;
+  for (auto &k : g_host_kept) free(k.second);
+  g_host_kept.clear();
+}
+
+geye_status read_result(Plan &P, int mi, geye_result *out) {
+  const int *h = static_cast<const int *>(P.h_res);
+  const int K = h[32 + mi];
+  P.last_D[mi] = h[mi];
+  P.last_K[mi] = K;
+  if (!out) return GEYE_OK;
+  memset(out, 0, sizeof(*out));
+  out->num = K;
+  const size_t k = std::max(K, 1);
+  out->point = (int *)malloc(sizeof(int) * 4 * k);
+  out->or_point = (int *)malloc(sizeof(int) * 4 * k);
+  out->type = (int *)malloc(sizeof(int) * k);
+  out->scale = (float *)malloc(sizeof(float) * k);
+  out->score = (float *)malloc(sizeof(float) * k);
+  if (!out->point || !out->or_point || !out->type || !out->scale || !out->score) {
+    geye_result_free(out);
+    set_error("host allocation failed");
     return GEYE_ERR_NOMEM;
   }
-  bytes = n;
+  // field f of `per` ints a record: its place in the pinned block, and (for records past it) on the device
+  const int *src = h + 64 + (size_t)mi * 11 * kHostRes, *res = P.d_result.as<int>() + (size_t)mi * P.max_cap * 11;
+  const int n = std::min(K, kHostRes);
+  struct { void *to; int at, per; } f[5] = {{out->point, 0, 4}, {out->or_point, 4, 4}, {out->type, 8, 1},
+                                            {out->scale, 9, 1}, {out->score, 10, 1}};
+  for (auto &x : f) {
+    memcpy(x.to, src + (size_t)x.at * kHostRes, sizeof(int) * x.per * n);
+    if (K > n)
+      CUDA_TRY(cudaMemcpy(static_cast<int *>(x.to) + x.per * n, res + (size_t)x.at * P.max_cap + x.per * n,
+                          sizeof(int) * x.per * (size_t)(K - n), cudaMemcpyDeviceToHost));
+  }
   return GEYE_OK;
 }
 
@@ -496,6 +603,7 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
   }
   P.bytes_resize += (double)3 * width * height + 12.0 * width * height;   // ingest
   // HOG
+  size_t ref_words = 0;
   for (int l = 0; l < LEN; l++) {
     LevelInfo &L = P.lv[l];
     L.sbin = l < interval ? sbin2 : sbin;
@@ -519,6 +627,7 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
       J.img_off = L.img_off; J.h = L.img_h; J.w = L.img_w; J.sbin = L.sbin; J.b0 = b0; J.b1 = b1;
       J.hist_off = L.hist_off; J.fs0 = L.fs0; J.fs1 = L.fs1; J.feat_off = L.feat_off; J.feat16_off = L.feat16_off;
       J.feat16lo_off = L.feat16lo_off;
+      J.ref_off = (int)ref_words;
       J.tc_planes = tc_planes;
       J.fast = tc_planes ? 1 : 0;
       J.corner_off = A.take((size_t)(L.fs0 + 1) * (L.fs1 + 1));
@@ -528,6 +637,7 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
       P.hog_max_b1 = std::max(P.hog_max_b1, b1);
       P.bytes_hog += 12.0 * L.img_h * L.img_w + 124.0 * L.fs0 * L.fs1;
     }
+    ref_words += (size_t)kFeat * L.fs0 * L.fs1;
   }
   // one (bin, magnitude) buffer per image, covering the widest visible area of its levels
   {
@@ -690,6 +800,7 @@ static geye_status get_frame_plan(geye_ctx *ctx, geye_model *const *models, int 
   // after the arena exists: the tile shapes are tuned on it
   if (ctx->conv_mode != GEYE_CONV_FP32) GEYE_TRY(build_tc_plan(ctx, *P));
   GEYE_TRY(P->d_bgr.alloc(ctx, (size_t)width * height * 3 + 64));
+  CUDA_TRY(cudaMallocHost(&P->h_res, sizeof(int) * res_block_ints(n_models)));
   if (ctx->plans.size() > 32) ctx->plans.clear();
   *out = P.get();
   ctx->plans[key] = std::move(P);
@@ -748,12 +859,12 @@ geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_
   return run_resize(ctx, P);
 }
 
-// floats: also write the float feature planes (the FP32 convolution and calc_f_pyramid read them)
-geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats) {
+// floats: also write the float feature planes (for the FP32 convolution), or (ref) the levels in the reference layout there
+geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats, float *ref) {
   const bool fast = !P.hog_jobs.empty() && P.hog_jobs[0].fast;
   launch_hog(P.d_hog_jobs.as<HogJob>(), (int)P.hog_jobs.size(), P.d_hog_vote_blocks.as<int2>(), P.hog_vote_nblocks,
              P.hog_max_b0, P.hog_max_b1, P.d_pix_jobs.as<HogPixJob>(), (int)P.pix_jobs.size(), P.pix_max_xe,
-             P.arena.as<float>(), P.arena16.p, !fast, floats, ctx->stream);
+             P.arena.as<float>(), P.arena16.p, !fast, floats, ref, ctx->stream);
   ctx->launches += 3;   // pixels, votes, corner norms, features
   return check_launch(ctx, "hog");
 }
@@ -930,6 +1041,8 @@ geye_status run_nms(geye_ctx *ctx, Plan &P, int n_models, float overlap) {
     res.m[mi] = {m->d_coef, m->h.numpart[0], m->h.ratio};
   }
   res.out = P.d_result.as<int>();
+  res.host = static_cast<int *>(P.h_res);
+  res.host_cap = kHostRes;
   res.img_w = P.width;
   res.img_h = P.height;
   const cudaError_t ge =
@@ -951,7 +1064,7 @@ static geye_status run_body(geye_ctx *ctx, Plan &P, float thresh, float overlap)
   StageTimer T(ctx);
   if (!ctx->front_external) GEYE_TRY(run_resize(ctx, P));
   T.mark(1);
-  if (!ctx->front_external) GEYE_TRY(run_hog(ctx, P, ctx->conv_mode == GEYE_CONV_FP32));
+  if (!ctx->front_external) GEYE_TRY(run_hog(ctx, P, ctx->conv_mode == GEYE_CONV_FP32, nullptr));
   T.mark(2);
   const bool tc = ctx->conv_mode != GEYE_CONV_FP32;
   GEYE_TRY(tc ? run_conv_tc(ctx, P) : run_conv(ctx, P));   // every model's filters in one launch

@@ -57,15 +57,13 @@ struct ArenaAlloc;
 geye_status plan_tc(geye_ctx *ctx, Plan &P, ArenaAlloc &A);
 geye_status build_tc_plan(geye_ctx *ctx, Plan &P);
 geye_status run_conv_tc(geye_ctx *ctx, Plan &P);
-// d_small[kSortLevelsUsed]: the deepest NMS sort level with work in the frame
-constexpr int kSortLevelsUsed = 48;
 // d_small[kNmsNeed + m]: model m's kept set was resolved again in the quicksort's order
 constexpr int kNmsNeed = 160;
-void note_sort_levels(geye_ctx *ctx, Plan &P, int used);
+// *err gets the kernel's error word once the stream has drained (0: no wait ran out)
 // tensor-core fconvsMT of one feature map (float planes on the device) for the stage entry point
 geye_status conv_tc_maps(geye_ctx *ctx, const float *d_feat, int a0, int a1, const float *const *filters,
                          const int *b_dims, int n_filters, float *d_out, const std::vector<int> &out_off,
-                         std::vector<std::unique_ptr<DevBuf>> &tmp);
+                         std::vector<std::unique_ptr<DevBuf>> &tmp, int *err);
 
 // Bump allocator of a plan's float arena (128-byte aligned offsets, in words).
 struct ArenaAlloc {
@@ -77,15 +75,53 @@ struct ArenaAlloc {
   }
 };
 
-// Device buffer owned by a plan or context.
+// Device memory of a context's stage calls: handed out piece by piece during a
+// call, all of it free again at its end (reset), and kept for the next one
+// (up to kScratchKeep bytes; cudaMalloc and cudaFree synchronise and cost more than most stages).
+struct ScratchArena {
+  struct Chunk {
+    char *p;
+    size_t bytes;
+  };
+  std::vector<Chunk> chunks;   // the last one is being handed out
+  size_t used = 0;             // of the last chunk
+  size_t total = 0;            // handed out since the last reset
+  size_t want = 0;             // the largest call so far
+  ~ScratchArena() { release(); }
+  void release();
+  geye_status take(geye_ctx *ctx, size_t n, void **out);
+  void reset();                // the stream has drained
+};
+constexpr size_t kScratchKeep = 512ull << 20;
+
+// Device buffer owned by a plan or context, or (arena) a piece of a context's scratch.
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
+  ScratchArena *arena = nullptr;
+  DevBuf() = default;
+  explicit DevBuf(ScratchArena *a) : arena(a) {}
   ~DevBuf();
   geye_status alloc(geye_ctx *ctx, size_t n);
   void release();
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
+
+// Host memory handed to callers (geye_free): blocks of a megabyte and more are kept
+// for the next call (kHostKeep bytes in all, until the last context goes), since fresh
+// pages cost more than the copy into them.
+void *host_alloc(size_t n);
+void host_free(void *p);
+void host_pool_ref(int d);   // contexts come (+1) and go (-1)
+
+// Results of a frame in pinned host memory, written by the NMS kernels: ints [0, 32)
+// boxes before NMS per model, [32, 64) kept per model ([kSortLevelsUsed]: the sort
+// levels used), then per model point[4R], or_point[4R], type[R], scale[R], score[R]
+constexpr int kHostRes = 2048;
+inline size_t res_block_ints(int n_models) { return 64 + (size_t)n_models * 11 * kHostRes; }
+// model mi's result of the plan's finished frame (out: geye_result_free)
+geye_status read_result(Plan &P, int mi, geye_result *out);
+void note_sort_levels(geye_ctx *ctx, Plan &P, int used);
 
 struct LevelInfo {
   int img_h = 0, img_w = 0;   // image of this level (aliases for [interval, 2*interval))
@@ -209,14 +245,11 @@ struct Plan {
   // adapted once to the depth the plan's frames need (note_sort_levels)
   int sort_levels = 0;
   bool sort_levels_fixed = false;
-  // asynchronous submission (serve.cu): pinned frame staging, pinned result
-  // block (counts, then per model kHostRes records) and the completion event
-  void *h_bgr = nullptr, *h_res = nullptr;
-  cudaEvent_t ev_done = nullptr;
+  void *h_res = nullptr;                // pinned result block (kHostRes)
+  cudaEvent_t ev_done = nullptr;        // asynchronous submission (serve.cu): the frame's completion
   ~Plan() {
     for (auto &g : graphs)
       if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
-    if (h_bgr) cudaFreeHost(h_bgr);
     if (h_res) cudaFreeHost(h_res);
     if (ev_done) cudaEventDestroy(ev_done);
   }
@@ -258,9 +291,7 @@ struct geye_ctx {
   int inject_countdown = 0;
   // fallback counters etc. (device)
   geye::DevBuf d_diag;
-  // pinned staging for results
-  void *h_pinned = nullptr;
-  size_t h_pinned_bytes = 0;
+  geye::ScratchArena scratch;   // stage calls
   // last device-resident run
   geye::Plan *last_plan = nullptr;
   // frame submitted with geye_detect_submit and not collected yet

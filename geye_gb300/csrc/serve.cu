@@ -33,27 +33,24 @@ geye_status frame_plan(geye_ctx *ctx, geye_model *const *models, int n, int w, i
 void drop_frame_plans(geye_ctx *ctx, int w, int h);   // the context's whole-path plans for frames of w x h
 size_t plan_device_bytes(const Plan &P);
 
-constexpr int kHostRes = 4096;   // records per model returned through pinned memory
-
-// pinned result block: ints [0, 32) boxes before NMS per model, [32, 64) kept
-// per model, then per model point[4R], or_point[4R], type[R], scale[R], score[R]
-static size_t res_block_ints(int n_models) { return 64 + (size_t)n_models * 11 * kHostRes; }
-
 static long long now_ns() {
   return std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch())
       .count();
 }
 
-// queue everything of one frame on the context's stream (the frame already in P.h_bgr)
-// (from h_src, pinned and kept until the frame completes, when given)
-// (copy_in false: the frame is on the device already)
-static geye_status enqueue_frame(geye_ctx *ctx, Plan &P, float thresh, float overlap, TrackerSet *trk, int stream,
-                                 cudaEvent_t after, cudaEvent_t tracked, bool record_done = true,
-                                 const void *h_src = nullptr, bool copy_in = true) {
-  const int n_models = (int)P.models.size();
-  if (copy_in)
-    CUDA_TRY(cudaMemcpyAsync(P.d_bgr.p, h_src ? h_src : P.h_bgr, (size_t)3 * P.width * P.height,
+// a frame's upload into its plan from `bgr` (pinned memory that outlives it, or the caller's: then it is waited for, on a
+// stream with nothing else to do, so that the buffer is the caller's again)
+static geye_status upload_frame(geye_ctx *ctx, Plan &P, const uint8_t *bgr, int width_step, bool wait) {
+  CUDA_TRY(cudaMemcpy2DAsync(P.d_bgr.p, (size_t)3 * P.width, bgr, width_step, (size_t)3 * P.width, P.height,
                              cudaMemcpyHostToDevice, ctx->stream));
+  if (wait) CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return GEYE_OK;
+}
+
+// queue everything of one uploaded frame on the context's stream; its results arrive in P.h_res
+static geye_status enqueue_frame(geye_ctx *ctx, Plan &P, float thresh, float overlap, TrackerSet *trk, int stream,
+                                 cudaEvent_t after, cudaEvent_t tracked, bool record_done = true) {
+  const int n_models = (int)P.models.size();
   GEYE_TRY(run_frame(ctx, P, P.d_bgr.as<uint8_t>(), 3 * P.width, thresh, overlap, nullptr));
   if (trk) {
     if (after) CUDA_TRY(cudaStreamWaitEvent(ctx->stream, after, 0));
@@ -61,29 +58,11 @@ static geye_status enqueue_frame(geye_ctx *ctx, Plan &P, float thresh, float ove
                             P.d_ascore.as<float>(), P.width, P.height, ctx->stream));
     CUDA_TRY(cudaEventRecord(tracked, ctx->stream));
   }
-  int *h = static_cast<int *>(P.h_res);
-  CUDA_TRY(cudaMemcpyAsync(h, P.d_small.p, sizeof(int) * 64, cudaMemcpyDeviceToHost, ctx->stream));
-  const size_t R = (size_t)std::min(P.max_cap, kHostRes);
-  for (int mi = 0; mi < n_models; mi++) {
-    const int *res = P.d_result.as<int>() + (size_t)mi * P.max_cap * 11;
-    int *dst = h + 64 + (size_t)mi * 11 * kHostRes;
-    CUDA_TRY(cudaMemcpyAsync(dst, res, sizeof(int) * 4 * R, cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_TRY(cudaMemcpyAsync(dst + 4 * kHostRes, res + 4 * (size_t)P.max_cap, sizeof(int) * 4 * R,
-                             cudaMemcpyDeviceToHost, ctx->stream));
-    for (int f = 8; f < 11; f++)   // type, scale, score (max_cap apart on the device, kHostRes apart here)
-      CUDA_TRY(cudaMemcpyAsync(dst + f * kHostRes, res + f * (size_t)P.max_cap, sizeof(int) * R,
-                               cudaMemcpyDeviceToHost, ctx->stream));
+  if (record_done) {
+    if (!P.ev_done) CUDA_TRY(cudaEventCreateWithFlags(&P.ev_done, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(P.ev_done, ctx->stream));
   }
-  if (record_done) CUDA_TRY(cudaEventRecord(P.ev_done, ctx->stream));
   ctx->pending = &P;
-  return GEYE_OK;
-}
-
-static geye_status ensure_staging(Plan &P) {
-  const int n_models = (int)P.models.size();
-  if (!P.h_bgr) CUDA_TRY(cudaMallocHost(&P.h_bgr, (size_t)3 * P.width * P.height));
-  if (!P.h_res) CUDA_TRY(cudaMallocHost(&P.h_res, sizeof(int) * res_block_ints(n_models)));
-  if (!P.ev_done) CUDA_TRY(cudaEventCreateWithFlags(&P.ev_done, cudaEventDisableTiming));
   return GEYE_OK;
 }
 
@@ -92,48 +71,12 @@ static geye_status ensure_staging(Plan &P) {
 static geye_status collect_frame(geye_ctx *ctx, geye_result *out, bool wait = true) {
   Plan &P = *ctx->pending;
   if (wait) CUDA_TRY(cudaEventSynchronize(P.ev_done));
-  const int n_models = (int)P.models.size();
-  const int *h = static_cast<const int *>(P.h_res);
-  if (wait) note_sort_levels(ctx, P, h[kSortLevelsUsed]);
+  if (wait) note_sort_levels(ctx, P, static_cast<const int *>(P.h_res)[kSortLevelsUsed]);
   geye_status st = GEYE_OK;
-  for (int mi = 0; mi < n_models && out; mi++) {
-    const int K = h[32 + mi];
-    geye_result &r = out[mi];
-    memset(&r, 0, sizeof(r));
-    r.num = K;
-    const size_t k = std::max(K, 1);
-    r.point = (int *)malloc(sizeof(int) * 4 * k);
-    r.or_point = (int *)malloc(sizeof(int) * 4 * k);
-    r.type = (int *)malloc(sizeof(int) * k);
-    r.scale = (float *)malloc(sizeof(float) * k);
-    r.score = (float *)malloc(sizeof(float) * k);
-    if (!r.point || !r.or_point || !r.type || !r.scale || !r.score) {
-      set_error("host allocation failed");
-      st = GEYE_ERR_NOMEM;
-      continue;
-    }
-    const int *src = h + 64 + (size_t)mi * 11 * kHostRes;
-    const int n = std::min(K, kHostRes);
-    memcpy(r.point, src, sizeof(int) * 4 * n);
-    memcpy(r.or_point, src + 4 * kHostRes, sizeof(int) * 4 * n);
-    memcpy(r.type, src + 8 * kHostRes, sizeof(int) * n);
-    memcpy(r.scale, src + 9 * kHostRes, sizeof(float) * n);
-    memcpy(r.score, src + 10 * kHostRes, sizeof(float) * n);
-    if (K > n) {   // more kept boxes than the pinned block holds: the rest straight from the device
-      const int *res = P.d_result.as<int>() + (size_t)mi * P.max_cap * 11;
-      const size_t rest = (size_t)(K - n);
-      CUDA_TRY(cudaMemcpy(r.point + 4 * n, res + 4 * n, sizeof(int) * 4 * rest, cudaMemcpyDeviceToHost));
-      CUDA_TRY(cudaMemcpy(r.or_point + 4 * n, res + 4 * (size_t)P.max_cap + 4 * n, sizeof(int) * 4 * rest,
-                          cudaMemcpyDeviceToHost));
-      CUDA_TRY(cudaMemcpy(r.type + n, res + 8 * (size_t)P.max_cap + n, sizeof(int) * rest, cudaMemcpyDeviceToHost));
-      CUDA_TRY(cudaMemcpy(r.scale + n, res + 9 * (size_t)P.max_cap + n, sizeof(float) * rest,
-                          cudaMemcpyDeviceToHost));
-      CUDA_TRY(cudaMemcpy(r.score + n, res + 10 * (size_t)P.max_cap + n, sizeof(float) * rest,
-                          cudaMemcpyDeviceToHost));
-    }
+  for (size_t mi = 0; mi < P.models.size(); mi++) {
+    const geye_status s = read_result(P, (int)mi, out ? &out[mi] : nullptr);
+    if (st == GEYE_OK) st = s;
   }
-  P.last_D.assign(h, h + n_models);
-  P.last_K.assign(h + 32, h + 32 + n_models);
   ctx->last_plan = &P;
   ctx->pending = nullptr;
   return st;
@@ -154,9 +97,7 @@ geye_status geye_detect_submit(geye_ctx *ctx, geye_model *const *models, int n_m
   CUDA_TRY(cudaSetDevice(ctx->device));
   Plan *P = nullptr;
   GEYE_TRY(frame_plan(ctx, models, n_models, width, height, &P));
-  GEYE_TRY(ensure_staging(*P));
-  uint8_t *dst = static_cast<uint8_t *>(P->h_bgr);
-  for (int y = 0; y < height; y++) memcpy(dst + (size_t)y * 3 * width, bgr + (size_t)y * width_step, (size_t)3 * width);
+  GEYE_TRY(upload_frame(ctx, *P, bgr, width_step, true));
   return enqueue_frame(ctx, *P, thresh, overlap, nullptr, 0, nullptr, nullptr);
 }
 
@@ -206,11 +147,14 @@ struct geye_server {
   struct Req {
     long long ticket, t_submit;
     int stream, w, h;
-    uint8_t *bgr;   // pinned (pool below), the H2D copy's source
-    size_t bytes;
+    uint8_t *bgr = nullptr;          // pinned (pool below), the H2D copy's source
+    size_t bytes = 0;
+    const uint8_t *user = nullptr;   // still in the caller's buffer (only during its submit)
+    int step = 0;
   };
-  // pinned frame buffers by size: a submitted frame is copied once, into one of
-  // these, and goes to the device from there.  They are carved from slabs of
+  // pinned frame buffers by size: a submitted frame that no slot takes at once is copied
+  // into one of these, and goes to the device from there (one that a slot takes is
+  // uploaded from the caller's memory: 16 us instead of 36 + 15 at 640x480).  They are carved from slabs of
   // kPinnedSlab bytes (cudaMallocHost is slow and synchronises the device, so
   // it runs once per slab, not once per buffer) and reused, never returned.
   std::map<size_t, std::vector<uint8_t *>> pinned_free;
@@ -342,7 +286,6 @@ geye_status dispatch_one(geye_server *s, bool *dispatched) {
   }
   Plan *P = nullptr;
   GEYE_TRY(frame_plan(sl.ctx, s->models.data(), (int)s->models.size(), r.w, r.h, &P));
-  GEYE_TRY(ensure_staging(*P));
   if (fresh) {
     const size_t b = plan_device_bytes(*P);
     sl.sizes[key] = geye_server::Slot::Held{b, 0};
@@ -353,8 +296,8 @@ geye_status dispatch_one(geye_server *s, bool *dispatched) {
   cudaEvent_t after = nullptr;
   auto it = s->last_tracked.find(r.stream);
   if (it != s->last_tracked.end() && s->stream_busy[r.stream] > 0) after = it->second;
-  GEYE_TRY(enqueue_frame(sl.ctx, *P, s->thresh, s->overlap, s->track ? &s->trk : nullptr, r.stream, after,
-                         sl.tracked, true, r.bgr));
+  GEYE_TRY(upload_frame(sl.ctx, *P, r.user ? r.user : r.bgr, r.user ? r.step : 3 * r.w, r.user != nullptr));
+  GEYE_TRY(enqueue_frame(sl.ctx, *P, s->thresh, s->overlap, s->track ? &s->trk : nullptr, r.stream, after, sl.tracked));
   sl.frame = r.bgr;
   sl.frame_bytes = r.bytes;
   s->last_tracked[r.stream] = sl.tracked;
@@ -492,6 +435,20 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
   r.w = width;
   r.h = height;
   r.bytes = (size_t)3 * width * height;
+  *ticket = r.ticket;
+  GEYE_TRY(reap(s, false));
+  GEYE_TRY(pump(s));
+  if (s->queue.empty()) {   // a slot may take it straight from the caller
+    r.user = bgr;
+    r.step = width_step;
+    s->queue.push_back(r);
+    bool taken = false;
+    const geye_status st = dispatch_one(s, &taken);
+    if (taken) return st;
+    // none free, or an error: the frame waits like any other (and meets the error again)
+    if (!s->queue.empty()) s->queue.pop_back();
+    r.user = nullptr;
+  }
   GEYE_TRY(get_pinned(s, r.bytes, &r.bgr));
   if (width_step == 3 * width) {
     memcpy(r.bgr, bgr, r.bytes);
@@ -499,7 +456,6 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
     for (int y = 0; y < height; y++)
       memcpy(r.bgr + (size_t)y * 3 * width, bgr + (size_t)y * width_step, (size_t)3 * width);
   }
-  *ticket = r.ticket;
   s->queue.push_back(std::move(r));
   if (s->max_queued > 0) {   // the stream's oldest queued frames make way for its newest
     int n = 0;
@@ -802,10 +758,6 @@ geye_status geye_batch_run(geye_batch *b, int n_frames, const uint8_t *const *bg
       b->joins.push_back(j);
     }
     GEYE_TRY(frame_plan(b->lanes[i], b->models.data(), nm, widths[i], heights[i], &plans[i]));
-    GEYE_TRY(ensure_staging(*plans[i]));
-    uint8_t *dst = static_cast<uint8_t *>(plans[i]->h_bgr);
-    for (int y = 0; y < heights[i]; y++)
-      memcpy(dst + (size_t)y * 3 * widths[i], bgr[i] + (size_t)y * width_steps[i], (size_t)3 * widths[i]);
     key += std::to_string(widths[i]) + "x" + std::to_string(heights[i]) + ",";
   }
   {
@@ -831,14 +783,9 @@ geye_status geye_batch_run(geye_batch *b, int n_frames, const uint8_t *const *bg
     CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed));
     geye_status st = GEYE_OK;
     cudaError_t e = cudaSuccess;
-    // every frame in, then the batched front end: one persistent launch per stage for all frames
-    for (int i = 0; i < n_frames && e == cudaSuccess; i++)
-      e = cudaMemcpyAsync(plans[i]->d_bgr.p, plans[i]->h_bgr, (size_t)3 * widths[i] * heights[i],
-                          cudaMemcpyHostToDevice, b->stream);
-    if (e == cudaSuccess) {
-      launch_batch_tables(b, g);
-      e = cudaGetLastError();
-    }
+    // the batched front end: one persistent launch per stage for all frames
+    launch_batch_tables(b, g);
+    e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaEventRecord(b->front_done, b->stream);
     for (int i = 0; i < n_frames && st == GEYE_OK && e == cudaSuccess; i++) {
       geye_ctx *c = b->lanes[i];
@@ -848,7 +795,7 @@ geye_status geye_batch_run(geye_batch *b, int n_frames, const uint8_t *const *bg
       c->use_graphs = false;   // the lane's kernels go straight into the batch graph
       c->capturing = true;
       c->front_external = true;
-      st = enqueue_frame(c, *plans[i], thresh, overlap, nullptr, 0, nullptr, nullptr, false, nullptr, false);
+      st = enqueue_frame(c, *plans[i], thresh, overlap, nullptr, 0, nullptr, nullptr, false);
       c->front_external = false;
       c->capturing = false;
       c->use_graphs = graphs;
@@ -885,6 +832,9 @@ geye_status geye_batch_run(geye_batch *b, int n_frames, const uint8_t *const *bg
     }
     g.kernels = kernels;
   }
+  for (int i = 0; i < n_frames; i++)   // every frame in, from the caller's memory
+    CUDA_TRY(cudaMemcpy2DAsync(plans[i]->d_bgr.p, (size_t)3 * widths[i], bgr[i], width_steps[i], (size_t)3 * widths[i],
+                               heights[i], cudaMemcpyHostToDevice, b->stream));
   CUDA_TRY(cudaEventRecord(b->t0, b->stream));
   CUDA_TRY(cudaGraphLaunch(g.exec, b->stream));
   CUDA_TRY(cudaEventRecord(b->t1, b->stream));

@@ -13,7 +13,7 @@
 
 namespace geye {
 geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step);
-geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats);
+geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats, float *ref);
 geye_status run_conv(geye_ctx *ctx, Plan &P);
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp);
 geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh);
@@ -28,20 +28,18 @@ const char *last_error_cstr();
 using namespace geye;
 
 
-// scoped temporary device buffers for one stage call
+// temporary device buffers of one stage call, from the context's scratch
 struct Scratch {
   geye_ctx *ctx;
-  std::vector<DevBuf *> bufs;
   explicit Scratch(geye_ctx *c) : ctx(c) {}
   ~Scratch() {
     cudaStreamSynchronize(ctx->stream);
-    for (auto *b : bufs) delete b;
+    ctx->scratch.reset();
   }
   template <class T> geye_status get(size_t n, T **out) {
-    DevBuf *b = new DevBuf();
-    bufs.push_back(b);
-    GEYE_TRY(b->alloc(ctx, sizeof(T) * std::max<size_t>(n, 1)));
-    *out = b->as<T>();
+    DevBuf b(&ctx->scratch);
+    GEYE_TRY(b.alloc(ctx, sizeof(T) * std::max<size_t>(n, 1)));
+    *out = b.as<T>();
     return GEYE_OK;
   }
   template <class T> geye_status put(const T *h, size_t n, T **out) {
@@ -49,6 +47,20 @@ struct Scratch {
     if (n) CUDA_TRY(cudaMemcpyAsync(*out, h, sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream));
     return GEYE_OK;
   }
+};
+
+// several small host tables in one upload: add() each, then put(), then at() gives their places
+struct Tables {
+  std::vector<char> bytes;
+  char *d = nullptr;
+  template <class T> size_t add(const T *h, size_t n) {
+    const size_t o = (bytes.size() + 15) & ~size_t(15);
+    bytes.resize(o + sizeof(T) * std::max<size_t>(n, 1));
+    if (n) memcpy(bytes.data() + o, h, sizeof(T) * n);
+    return o;
+  }
+  geye_status put(Scratch &S) { return S.put(bytes.data(), bytes.size(), &d); }
+  template <class T> T *at(size_t o) const { return reinterpret_cast<T *>(d + o); }
 };
 
 static void taps(int sheight, int dheight, std::vector<int> &start, std::vector<int> &si, std::vector<float> &alpha) {
@@ -96,11 +108,6 @@ geye_status geye_resize(geye_ctx *ctx, const float *src, const int *sdims, int *
   const size_t n_src = (size_t)3 * h * w, n_tmp = (size_t)3 * oh * w, n_dst = (size_t)3 * oh * ow;
   GEYE_TRY(S.get(n_src + n_tmp + n_dst, &arena));
   CUDA_TRY(cudaMemcpyAsync(arena, src, sizeof(float) * n_src, cudaMemcpyHostToDevice, ctx->stream));
-  int *d_st, *d_si;
-  float *d_al;
-  GEYE_TRY(S.put(st.data(), st.size(), &d_st));
-  GEYE_TRY(S.put(si.data(), si.size(), &d_si));
-  GEYE_TRY(S.put(al.data(), al.size(), &d_al));
   ResizeJob jv{}, jh{};
   jv.src_off = 0; jv.dst_off = (int)n_src; jv.src_h = h; jv.src_w = w; jv.dst_h = oh; jv.dst_w = w;
   jv.tap_start_off = 0; jv.tap_off = 0;
@@ -108,11 +115,14 @@ geye_status geye_resize(geye_ctx *ctx, const float *src, const int *sdims, int *
   // both tap tables share one start array whose entries index the whole si/alpha arrays
   jh.tap_start_off = h_start; jh.tap_off = 0;
   (void)h_tap;
-  ResizeJob *d_jv, *d_jh;
-  GEYE_TRY(S.put(&jv, 1, &d_jv));
-  GEYE_TRY(S.put(&jh, 1, &d_jh));
-  launch_resize_pass(d_jv, 1, w, 1, d_st, d_si, d_al, arena, ctx->stream);
-  launch_resize_pass(d_jh, 1, ow, 0, d_st, d_si, d_al, arena, ctx->stream);
+  Tables T;
+  const size_t o_st = T.add(st.data(), st.size()), o_si = T.add(si.data(), si.size()),
+               o_al = T.add(al.data(), al.size()), o_v = T.add(&jv, 1), o_h = T.add(&jh, 1);
+  GEYE_TRY(T.put(S));
+  launch_resize_pass(T.at<ResizeJob>(o_v), 1, w, 1, T.at<int>(o_st), T.at<int>(o_si), T.at<float>(o_al), arena,
+                     ctx->stream);
+  launch_resize_pass(T.at<ResizeJob>(o_h), 1, ow, 0, T.at<int>(o_st), T.at<int>(o_si), T.at<float>(o_al), arena,
+                     ctx->stream);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(dst, arena + n_src + n_tmp, sizeof(float) * n_dst, cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -126,9 +136,9 @@ geye_status geye_flip_feat(geye_ctx *ctx, const float *feat, const int *size, fl
   ARG_CHECK(size[0] >= 0 && size[1] >= 0, "negative size");
   const size_t n = (size_t)size[0] * size[1] * kFeat;
   CUDA_TRY(cudaSetDevice(ctx->device));
-  float *h = static_cast<float *>(calloc(n ? n : 1, sizeof(float)));
+  float *h = static_cast<float *>(host_alloc(sizeof(float) * n));
   ARG_CHECK(h, "host allocation failed");
-  if (n == 0) { *out = h; return GEYE_OK; }
+  if (n == 0) { *h = 0.f; *out = h; return GEYE_OK; }
   geye_status st = GEYE_OK;
   {
     Scratch S(ctx);
@@ -144,7 +154,7 @@ geye_status geye_flip_feat(geye_ctx *ctx, const float *feat, const int *size, fl
       }
     }
   }
-  if (st != GEYE_OK) { free(h); return st; }
+  if (st != GEYE_OK) { host_free(h); return st; }
   *out = h;
   return GEYE_OK;
 }
@@ -179,16 +189,13 @@ geye_status geye_calc_feature(geye_ctx *ctx, const float *src, const int *isize,
   J.img_off = 0; J.h = h; J.w = w; J.sbin = sbin; J.b0 = b0; J.b1 = b1; J.hist_off = (int)hist;
   J.fs0 = fs0; J.fs1 = fs1; J.feat_off = (int)feat_off; J.feat16_off = -1; J.feat16lo_off = -1; J.fast = 0;
   J.mag_off = X.mag_off; J.bin_off = X.bin_off; J.pix_Y = X.Y; J.corner_off = (int)corner_off;
-  HogJob *d_j;
-  GEYE_TRY(S.put(&J, 1, &d_j));
-  HogPixJob *d_x;
-  GEYE_TRY(S.put(&X, 1, &d_x));
   std::vector<int2> vb;
   hog_vote_blocks(std::vector<HogJob>{J}, vb);
-  int2 *d_vb;
-  GEYE_TRY(S.put(vb.data(), vb.size(), &d_vb));
-  launch_hog(d_j, 1, d_vb, (int)vb.size(), b0, b1, d_x, 1, X.xe, arena, nullptr, true, true, ctx->stream);
-  launch_to_ref_layout(arena + feat_off, fs0, fs1, out, ctx->stream);
+  Tables T;
+  const size_t o_j = T.add(&J, 1), o_x = T.add(&X, 1), o_vb = T.add(vb.data(), vb.size());
+  GEYE_TRY(T.put(S));
+  launch_hog(T.at<HogJob>(o_j), 1, T.at<int2>(o_vb), (int)vb.size(), b0, b1, T.at<HogPixJob>(o_x), 1, X.xe, arena,
+             nullptr, true, true, out, ctx->stream);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(feat, out, sizeof(float) * (size_t)fs0 * fs1 * kFeat, cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -207,34 +214,32 @@ geye_status geye_calc_f_pyramid(geye_ctx *ctx, geye_model *model, const uint8_t 
   CUDA_TRY(cudaMemcpy2DAsync(P->d_bgr.p, (size_t)3 * width, bgr, width_step, (size_t)3 * width, height,
                              cudaMemcpyHostToDevice, ctx->stream));
   GEYE_TRY(run_pyramid(ctx, *P, P->d_bgr.as<uint8_t>(), 3 * width));
-  GEYE_TRY(run_hog(ctx, *P, true));
   const int LEN = P->models[0]->LEN;
   size_t total = 0;
   for (int l = 0; l < LEN; l++) total += (size_t)P->lv[l].fs0 * P->lv[l].fs1 * kFeat;
   Scratch S(ctx);
   float *d_out;
   GEYE_TRY(S.get(total, &d_out));
-  float *h_feat = (float *)malloc(sizeof(float) * std::max<size_t>(total, 1));
-  int *h_fs = (int *)malloc(sizeof(int) * 2 * LEN);
-  float *h_sc = (float *)malloc(sizeof(float) * LEN);
+  GEYE_TRY(run_hog(ctx, *P, true, d_out));   // the levels back to back in the reference layout
+  float *h_feat = (float *)host_alloc(sizeof(float) * total);
+  int *h_fs = (int *)host_alloc(sizeof(int) * 2 * LEN);
+  float *h_sc = (float *)host_alloc(sizeof(float) * LEN);
+  auto drop = [&]() { host_free(h_feat); host_free(h_fs); host_free(h_sc); };
   if (!h_feat || !h_fs || !h_sc) {
-    free(h_feat); free(h_fs); free(h_sc);
+    drop();
     set_error("host allocation failed");
     return GEYE_ERR_NOMEM;
   }
-  size_t o = 0;
   for (int l = 0; l < LEN; l++) {
     const LevelInfo &L = P->lv[l];
-    launch_to_ref_layout(P->arena.as<float>() + L.feat_off, L.fs0, L.fs1, d_out + o, ctx->stream);
     h_fs[2 * l] = L.fs0;
     h_fs[2 * l + 1] = L.fs1;
     h_sc[l] = L.scale;
-    o += (size_t)L.fs0 * L.fs1 * kFeat;
   }
   cudaError_t e = cudaMemcpyAsync(h_feat, d_out, sizeof(float) * total, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
-    free(h_feat); free(h_fs); free(h_sc);
+    drop();
     set_error(std::string("pyramid readback: ") + cudaGetErrorString(e));
     return GEYE_ERR_CUDA;
   }
@@ -276,7 +281,7 @@ geye_status geye_get_boxes(geye_ctx *ctx, geye_model *model, const float *featur
   CUDA_TRY(cudaMemcpyAsync(&D, P->d_small.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   const int GL = model->gl();
-  float *h = (float *)malloc(sizeof(float) * (size_t)std::max(D, 1) * GL);
+  float *h = (float *)host_alloc(sizeof(float) * (size_t)std::max(D, 1) * GL);
   if (!h) { set_error("host allocation failed"); return GEYE_ERR_NOMEM; }
   cudaError_t e = cudaSuccess;
   if (D > 0) e = cudaMemcpyAsync(h, P->d_boxes.p, sizeof(float) * (size_t)D * GL, cudaMemcpyDeviceToHost, ctx->stream);
@@ -285,7 +290,7 @@ geye_status geye_get_boxes(geye_ctx *ctx, geye_model *model, const float *featur
                         cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
-    free(h);
+    host_free(h);
     set_error(std::string("get_boxes readback: ") + cudaGetErrorString(e));
     return GEYE_ERR_CUDA;
   }
@@ -321,11 +326,11 @@ geye_status geye_nms(geye_ctx *ctx, const float *boxes, float overlap, int *num,
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (res[1]) { set_error("nms sort stack overflow"); return GEYE_ERR_UNSUPPORTED; }
   const int K = res[0];
-  float *h = (float *)malloc(sizeof(float) * (size_t)std::max(K, 1) * GL);
+  float *h = (float *)host_alloc(sizeof(float) * (size_t)std::max(K, 1) * GL);
   if (!h) { set_error("host allocation failed"); return GEYE_ERR_NOMEM; }
   if (K > 0) {
     cudaError_t e = cudaMemcpy(h, d_out, sizeof(float) * (size_t)K * GL, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) { free(h); set_error(cudaGetErrorString(e)); return GEYE_ERR_CUDA; }
+    if (e != cudaSuccess) { host_free(h); set_error(cudaGetErrorString(e)); return GEYE_ERR_CUDA; }
   }
   *out = h;
   *num = K;
@@ -384,14 +389,12 @@ geye_status geye_dt(geye_ctx *ctx, const float *vals, float ax, float bx, float 
   J.in_off = 0; J.d0 = d0; J.d1 = d1;
   J.tmpM_off = (int)np; J.tmpI_off = (int)(2 * np); J.M_off = (int)(3 * np); J.Ix_off = (int)(4 * np); J.Iy_off = (int)(5 * np);
   J.ax = ax; J.bx = bx; J.ay = ay; J.by = by; J.negate = 0;
-  DtJob *d_j;
-  GEYE_TRY(S.put(&J, 1, &d_j));
   std::vector<int2> b1, b2;
   dt_block_lists(std::vector<DtJob>{J}, b1, b2, kDtElems);
-  int2 *d_b1, *d_b2;
-  GEYE_TRY(S.put(b1.data(), b1.size(), &d_b1));
-  GEYE_TRY(S.put(b2.data(), b2.size(), &d_b2));
-  launch_dt(d_j, d_b1, (int)b1.size(), d_b2, (int)b2.size(), d0, d1, arena, reinterpret_cast<int *>(arena),
+  Tables T;
+  const size_t o_j = T.add(&J, 1), o_1 = T.add(b1.data(), b1.size()), o_2 = T.add(b2.data(), b2.size());
+  GEYE_TRY(T.put(S));
+  launch_dt(T.at<DtJob>(o_j), T.at<int2>(o_1), (int)b1.size(), T.at<int2>(o_2), (int)b2.size(), d0, d1, arena, reinterpret_cast<int *>(arena),
             ctx->d_diag.as<int>(), kDtElems, ctx->stream);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(M, arena + 3 * np, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -421,9 +424,10 @@ geye_status geye_fconv(geye_ctx *ctx, const float *feat, const int *a_dims, cons
   }
   GEYE_TRY(S.get(words + out_words, &arena));
   launch_from_ref_layout(d_ref, a0, a1, arena, ctx->stream);
+  int errw = 0;
   if (ctx->conv_mode != GEYE_CONV_FP32) {
     std::vector<std::unique_ptr<DevBuf>> tmp;
-    GEYE_TRY(conv_tc_maps(ctx, arena, a0, a1, filters, b_dims, n_filters, arena, out_off, tmp));
+    GEYE_TRY(conv_tc_maps(ctx, arena, a0, a1, filters, b_dims, n_filters, arena, out_off, tmp, &errw));
   } else {
     std::map<std::pair<int, int>, std::vector<int>> by_size;
     for (int i = 0; i < n_filters; i++) by_size[{b_dims[2 * i], b_dims[2 * i + 1]}].push_back(i);
@@ -442,18 +446,21 @@ geye_status geye_fconv(geye_ctx *ctx, const float *feat, const int *a_dims, cons
     }
     std::vector<int2> blocks;
     const size_t smem = conv_fp32_blocks(jobs, blocks);
-    float *d_bank;
-    ConvJob *d_jobs;
-    int2 *d_blocks;
-    GEYE_TRY(S.put(bank.taps.data(), bank.taps.size(), &d_bank));
-    GEYE_TRY(S.put(jobs.data(), jobs.size(), &d_jobs));
-    GEYE_TRY(S.put(blocks.data(), blocks.size(), &d_blocks));
-    launch_conv_fp32(d_jobs, d_blocks, (int)blocks.size(), smem, d_bank, arena, arena, ctx->stream);
+    Tables T;
+    const size_t o_w = T.add(bank.taps.data(), bank.taps.size()), o_j = T.add(jobs.data(), jobs.size()),
+                 o_b = T.add(blocks.data(), blocks.size());
+    GEYE_TRY(T.put(S));
+    launch_conv_fp32(T.at<ConvJob>(o_j), T.at<int2>(o_b), (int)blocks.size(), smem, T.at<float>(o_w), arena, arena,
+                     ctx->stream);
   }
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(out, arena + words, sizeof(float) * out_words, cudaMemcpyDeviceToHost,
                            ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (errw) {
+    set_error("tensor-core conv: a tensor-core wait ran out (error bits " + std::to_string(errw) + ")");
+    return GEYE_ERR_TIMEOUT;
+  }
   return GEYE_OK;
 }
 

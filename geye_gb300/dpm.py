@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import weakref
 
 import numpy as np
 
@@ -131,17 +132,28 @@ def _p(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
 
 
+def _copied(ptr, n: int, dt) -> np.ndarray:
+    """n values at ptr in an array of their own."""
+    return np.frombuffer(C.string_at(ptr, 4 * n), dt).copy()
+
+
+def _adopted(ptr, n: int) -> np.ndarray:
+    """The n floats of a callee-allocated block as an array that frees the block when it goes."""
+    addr = C.cast(ptr, C.c_void_p).value
+    buf = (C.c_float * max(n, 1)).from_address(addr)
+    weakref.finalize(buf, lib().geye_free, addr)
+    return np.frombuffer(buf, np.float32)[:n]
+
+
 def _result_to_dict(r: _Result) -> dict:
     n = r.num
-
-    def arr(ptr, k, dt):
-        if n <= 0:
-            return np.zeros((0,) if k == 1 else (0, k), dt)
-        a = np.ctypeslib.as_array(ptr, shape=(n * k,)).astype(dt, copy=True)
-        return a if k == 1 else a.reshape(n, k)
-
-    out = dict(num=n, point=arr(r.point, 4, np.int32), or_point=arr(r.or_point, 4, np.int32),
-               type=arr(r.type, 1, np.int32), scale=arr(r.scale, 1, np.float32), score=arr(r.score, 1, np.float32))
+    if n <= 0:
+        out = dict(num=n, point=np.zeros((0, 4), np.int32), or_point=np.zeros((0, 4), np.int32),
+                   type=np.zeros(0, np.int32), scale=np.zeros(0, np.float32), score=np.zeros(0, np.float32))
+    else:
+        out = dict(num=n, point=_copied(r.point, 4 * n, np.int32).reshape(n, 4),
+                   or_point=_copied(r.or_point, 4 * n, np.int32).reshape(n, 4), type=_copied(r.type, n, np.int32),
+                   scale=_copied(r.scale, n, np.float32), score=_copied(r.score, n, np.float32))
     lib().geye_result_free(C.byref(r))
     return out
 
@@ -248,14 +260,14 @@ class Context:
         _check(lib().geye_calc_f_pyramid(self.h, model.h, _p(fr), w, h, 3 * w, C.byref(n), C.byref(fp), C.byref(ip),
                                          C.byref(sp)), "calc_f_pyramid")
         L = n.value
-        fs = np.ctypeslib.as_array(ip, shape=(2 * L,)).reshape(L, 2).copy()
-        sc = np.ctypeslib.as_array(sp, shape=(L,)).copy()
-        total = int(sum(31 * a * b for a, b in fs))
-        flat = np.ctypeslib.as_array(fp, shape=(max(total, 1),))[:total].copy()
-        for q in (fp, ip, sp):
+        fs = _copied(ip, 2 * L, np.int32).reshape(L, 2)
+        sc = _copied(sp, L, np.float32)
+        sizes = fs.tolist()
+        flat = _adopted(fp, sum(31 * a * b for a, b in sizes))
+        for q in (ip, sp):
             lib().geye_free(C.cast(q, C.c_void_p))
         feats, o = [], 0
-        for a, b in fs:
+        for a, b in sizes:
             k = 31 * a * b
             feats.append(flat[o:o + k].reshape(31, b, a))
             o += k
@@ -275,9 +287,7 @@ class Context:
                "get_boxes")
         GL = model.gl
         D = d.value
-        out = np.ctypeslib.as_array(bp, shape=(max(D, 1) * GL,))[:D * GL].reshape(D, GL).copy()
-        lib().geye_free(C.cast(bp, C.c_void_p))
-        return out
+        return _adopted(bp, D * GL).reshape(D, GL)
 
     def nms(self, boxes: np.ndarray, overlap: float, numpart0: int) -> np.ndarray:
         b = np.ascontiguousarray(boxes, np.float32)
@@ -288,9 +298,7 @@ class Context:
         K = num.value
         if not op:
             return np.zeros((0, GL), np.float32)
-        out = np.ctypeslib.as_array(op, shape=(max(K, 1) * GL,))[:K * GL].reshape(K, GL).copy()
-        lib().geye_free(C.cast(op, C.c_void_p))
-        return out
+        return _adopted(op, K * GL).reshape(K, GL)
 
     def get_new_rects(self, img_size: tuple, model: "Model", boxes: np.ndarray) -> dict:
         b = np.ascontiguousarray(boxes, np.float32)
@@ -303,9 +311,9 @@ class Context:
     def dt(self, vals: np.ndarray, ax, bx, ay, by):
         v = np.ascontiguousarray(vals, np.float32)
         d1, d0 = v.shape
-        M = np.zeros_like(v)
-        Ix = np.zeros(v.shape, np.int32)
-        Iy = np.zeros(v.shape, np.int32)
+        M = np.empty_like(v)
+        Ix = np.empty(v.shape, np.int32)
+        Iy = np.empty(v.shape, np.int32)
         dims = np.array([d0, d1], np.int32)
         _check(lib().geye_dt(self.h, _p(v), ax, bx, ay, by, _p(dims), _p(M), _p(Ix), _p(Iy)), "dt")
         return M, Ix, Iy
@@ -317,7 +325,7 @@ class Context:
         ptrs = (C.c_void_p * len(fl))(*[x.ctypes.data for x in fl])
         bd = np.array([[x.shape[2], x.shape[1]] for x in fl], np.int32).ravel()
         sizes = [(a1 - x.shape[1] + 1, a0 - x.shape[2] + 1) for x in fl]
-        out = np.zeros(sum(p * q for p, q in sizes), np.float32)
+        out = np.empty(sum(p * q for p, q in sizes), np.float32)
         _check(lib().geye_fconv(self.h, _p(f), _p(np.array([a0, a1], np.int32)), ptrs, _p(bd), len(fl), _p(out)),
                "fconv")
         res, o = [], 0
@@ -357,9 +365,7 @@ class Context:
         op = C.POINTER(C.c_float)()
         _check(lib().geye_flip_feat(self.h, _p(f), _p(np.array([n0, n1, c], np.int32)), C.byref(op)), "flip_feat")
         n = c * n1 * n0
-        out = np.ctypeslib.as_array(op, shape=(max(n, 1),))[:n].reshape(c, n1, n0).copy()
-        lib().geye_free(C.cast(op, C.c_void_p))
-        return out
+        return _adopted(op, n).reshape(c, n1, n0)
 
     # ---- device-resident path ---------------------------------------------
     def detect_device(self, d_bgr_ptr: int, width: int, height: int, models: list, thresh: float = -0.5,
