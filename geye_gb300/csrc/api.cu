@@ -329,7 +329,7 @@ geye_status geye_model_reset_scales(geye_model *m) {
 // ---------------------------------------------------------------------------
 // the plan's finished frame (the stream has drained): plans adapt to it, then every model's result
 static geye_status read_results(geye_ctx *ctx, Plan &P, geye_result *out) {
-  note_sort_levels(ctx, P, static_cast<const int *>(P.h_res)[kSortLevelsUsed]);
+  tune_plan(ctx, P);
   for (size_t i = 0; i < P.models.size(); i++) GEYE_TRY(read_result(P, (int)i, &out[i]));
   return GEYE_OK;
 }
@@ -387,7 +387,7 @@ geye_status geye_fetch_result(geye_ctx *ctx, int model_index, geye_result *out, 
   ARG_CHECK(model_index >= 0 && model_index < (int)ctx->last_plan->models.size(), "model index out of range");
   Plan &P = *ctx->last_plan;
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  if (model_index == 0) note_sort_levels(ctx, P, static_cast<const int *>(P.h_res)[kSortLevelsUsed]);
+  if (model_index == 0) tune_plan(ctx, P);
   GEYE_TRY(read_result(P, model_index, out));
   if (n_boxes_before_nms) *n_boxes_before_nms = P.last_D[model_index];
   return GEYE_OK;

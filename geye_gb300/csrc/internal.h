@@ -310,13 +310,9 @@ void launch_ascore_normalize(float *a_score, int n, const unsigned *max_bits, cu
 // one block per model; model m uses boxes/out at m*cap*GL, scratch at m*cap*6 floats and m*cap*5 ints
 void launch_nms(const float *boxes, const int *d_num, int n_models, int GL, float overlap, int cap,
                 float *scratch_f, int *scratch_i, float *out, int *d_kept, int *err, cudaStream_t s);
-// pipeline NMS (nms_sort.cu, nms_batch.cu): per model nms_model_words(cap) ints
+// pipeline NMS (nms_radix.cu, nms_batch.cu): per model nms_model_words(cap) ints
 // of scratch and 10 * cap floats (the boxes in sorted order, the picks')
 constexpr int kNmsBatch = 512;     // boxes resolved per round
-constexpr int kNmsSegS = 16384;    // sort segments finished in shared memory (one block, ~203 KB)
-constexpr int kNmsTile = 4096;     // elements per block in the sort's grid-wide partitions
-__host__ __device__ inline int nms_big_cap(int cap) { return cap / kNmsSegS + 2; }
-__host__ __device__ inline int nms_tile_cap(int cap) { return cap / kNmsTile + nms_big_cap(cap) + 1; }
 constexpr int kNmsCells = 64;      // cells per image axis of the greedy's pick masks
 constexpr int kNmsLevels = 7;      // their sparse-table levels (spans of 1..64 cells)
 // elements per block in the key-order radix sort: small tiles spread a frame's
@@ -325,8 +321,7 @@ constexpr int kNmsLevels = 7;      // their sparse-table levels (spans of 1..64 
 __host__ __device__ inline int nms_rs_tile(int cap) { return cap <= (1 << 18) ? 1024 : 4096; }
 __host__ __device__ inline int nms_rs_tiles(int cap) { return (cap + nms_rs_tile(cap) - 1) / nms_rs_tile(cap); }
 __host__ __device__ inline size_t nms_model_words(int cap) {
-  const size_t w = 8 * (size_t)cap + 64 + 4 * (size_t)nms_big_cap(cap) + 2 * (size_t)nms_tile_cap(cap) +
-                   4 * 256 * (size_t)nms_rs_tiles(cap);
+  const size_t w = 32 + 11 * (size_t)cap + cap / 32 + 2 + 4 * 256 * (size_t)nms_rs_tiles(cap);
   return (w + 31) & ~(size_t)31;
 }
 // what the results are made from: per model its regression coefficients [comp][x1, y1, x2, y2][ML],
@@ -343,22 +338,15 @@ struct NmsResults {
   int host_cap;
   int img_w, img_h;
 };
-// diag (optional): per model m, diag[8m+1..8m+5] = sort segments left to the fallback, batches, picks,
-// 0, whether the quicksort order was needed
-// levels, lv_used: as for launch_nms_sort (nms_common.h)
-// need: n_models ints, zero on entry; order: kNmsOrderKey (the scores in
-// key order, the quicksort's order only for the models that need it: need[m]
-// raised) or kNmsOrderQuicksort (the quicksort's order for every model)
-// d_small[kSortLevelsUsed] and the same place of the host's result block: the deepest sort level with work in the frame
-constexpr int kSortLevelsUsed = 63;
+// diag (optional): per model m, diag[8m+2] = rounds, [8m+3] = picks, [8m+5] = whether the quicksort's order was needed
+// need: n_models ints, zero on entry (raised for a NaN score); order: kNmsOrderKey (score order, the quicksort's order
+// among equal scores only where the kept set depends on it) or kNmsOrderQuicksort (the quicksort's order for every model)
 constexpr int kNmsOrderKey = 0, kNmsOrderQuicksort = 1;
 // aux: null for plain launches on s; when s is capturing a graph, a second
-// stream that captures the body of the quicksort-order pass's if node
+// stream that captures the body of the if node for the quicksort's order of all boxes
 cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
                              int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
-                             long long *diag, int levels, int *lv_used, int *need, int order, cudaStream_t s,
-                             cudaStream_t aux);
-int nms_sort_levels(int cap);   // the default number of grid-wide sort levels for cap boxes
+                             long long *diag, int *need, int order, cudaStream_t s, cudaStream_t aux);
 void launch_new_rects(const float *kept, const int *d_kept, int GL, int np, const float *coef, int img_w,
                       int img_h, float ratio, int *point, int *or_point, int *type, float *scale, float *score,
                       cudaStream_t s);

@@ -7,8 +7,10 @@
 //
 //  1. The order: score order from the radix sort (nms_radix.cu), checked for
 //     the cases where the quicksort's order among equal scores could change
-//     the kept set; the models that raise them go through step 2 again in
-//     the quicksort's order (nms_sort.cu, k_nms_gather).
+//     the kept set.  Where a batch's decisions depend on it, the cluster puts the batch's
+//     members of those runs in the quicksort's order (nms_quick.h) and decides the batch again.  What a batch cannot settle
+//     (a run longer than a batch, the last pick of all tied with another, NaN, ties without end)
+//     starts the walk again with every box in the quicksort's order.
 //  2. k_nms_greedy, a cluster of kCluster blocks per model, walks the boxes in
 //     that order, a chunk at a time:
 //       - the cluster tests the chunk's boxes against the picks so far that can
@@ -38,56 +40,38 @@
 // resolved by one block, a pass of all alive boxes over the grid, 285 us; 512
 // members, the pair tests by 32 blocks handing over by a ticket, 155 us; one
 // cluster kernel for all rounds with a pass of all alive boxes each, 147 us;
-// this form 157 us (320x240 car: 135 -> 73, 1280x720: 575 -> 399, 1280x720 trained-like:
-// 280 -> 170, 1920x1080 with a model in the quicksort's order: 2414 -> 1833).
-#include <cooperative_groups.h>
-
+// this form 160 us (320x240 car: 135 -> 70, 1280x720: 575 -> 403, 1280x720 trained-like:
+// 280 -> 170).
+// With the whole quicksort over the grid and a second walk wherever a model needed its order (75 launches, in a batch's
+// lanes on every frame) 1920x1080 took 1830 us when it did, and a batch of eight mixed frames 3630 us; with the few
+// members put in order inside the walk 1010 us, the batch 3140 us.
 #include <algorithm>
 
 #include "nms_common.h"
+#include "nms_quick.h"
 #include "rects.h"
 
 namespace geye {
 
-namespace cg = cooperative_groups;
-
-constexpr int kCluster = 16;         // blocks per model (8 where a device cannot place 16)
-constexpr int kResNT = 512, kResWarps = kResNT / 32;
 constexpr int kBatch = kNmsBatch;
 constexpr int kBW = kBatch / 32;     // words of a suppression row
 constexpr int kPickGroup = 256;      // picks per table of a pass
 constexpr int kGW = kPickGroup / 32;
-constexpr int kPassNT = 256;         // k_nms_gather's blocks
 constexpr int kPrefix = 1 << 16;     // boxes that the first launch takes where there are more than kWhole (the rest
 constexpr int kWhole = 160000;       // of up to 100 000 costs the cluster less than two launches more)
 constexpr int kWinWords = 4 * kResNT;   // words of a chunk's window
 constexpr int kMaxChunk = 32 * (kWinWords - 2);   // with the run at its end
 constexpr int kChunkCap = 60000;
+// Where a batch's tied members are put in order, and where all boxes are, the walk then starting again (1920x1080,
+// 600 000 boxes: 250 us the first time and 150 the next ones, against 1000).  A textured frame ties a few members of one or two
+// runs, far down the order; kSettleHead members or more tied in the first 32nd of the order belong to a frame with
+// large areas of one colour, and more ties follow (a frame of one colour: 3.5 ms with this line, 4.2 without).
+constexpr int kSettle = 4, kSettleHead = 8, kSettleRun = 4096;
 static_assert(kBatch == kResNT, "a thread per member");
-
-// ---------------------------------------------------------------------------
-// the boxes in the quicksort's order (the radix sort brings its own)
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kPassNT) k_nms_gather(const float *__restrict__ boxes_all, int GL, int cap, int *si,
-                                                        float *sf) {
-  const int m = blockIdx.y;
-  Slots S = slots(si, sf, m, cap);
-  const float *boxes = boxes_all + (size_t)m * cap * GL;
-  const int r = blockIdx.x * kPassNT + threadIdx.x;
-  if (r < S.st->D) {
-    const float *P = boxes + (size_t)S.ord[r] * GL;
-    S.y1[r] = P[0]; S.x1[r] = P[1]; S.y2[r] = P[2]; S.x2[r] = P[3];
-    S.ar[r] = (P[3] - P[1] + 1.0) * (P[2] - P[0] + 1.0);   // nms.cpp's area expression
-  }
-}
 
 // cell of a coordinate on one axis of the pick tables (monotone; NaN to cell 0); inv: cells per pixel (.x: y axis, .y: x axis)
 __device__ __forceinline__ int nms_cell(float v, float inv) {
   return (int)fminf(fmaxf(v * inv, 0.0f), (float)(kNmsCells - 1));
-}
-
-__device__ __forceinline__ unsigned sorted_key(const Slots &S, int pos) {
-  return reinterpret_cast<const unsigned *>(S.val)[pos];
 }
 
 struct PickTable {   // see pick_table
@@ -100,6 +84,7 @@ struct GreedySmem {
     unsigned adj[kBatch * kBW];   // the members' rows (the first block's)
     PickTable table;
     int idx[kBatch * kBW];        // at the end: the kept boxes
+    QuickSmem quick;              // while boxes are put in the quicksort's order
   };
   float4 pk[kBatch];              // the tested picks' boxes and areas
   float pka[kBatch];
@@ -110,7 +95,11 @@ struct GreedySmem {
   int pick_any[kBatch];           // the pick removed a member alive at its turn
   int wtot[kResWarps];
   int total[kCluster];            // (the first block's) the blocks' survivors
-  int nb, np, tot;
+  unsigned tied[kBW];             // the batch's runs to be put in order, by their first member
+  SortRuns runs;
+  int nb, np, tot;                // np = -1: the batch depends on the order inside R.runs
+  int n, c0, c1, chunk, npicks, tested, left, batches, settled;   // the walk's place (walk_boxes)
+  int cut, need;                  // a run longer than a batch; a pick that removes a member of its own run
 };
 
 // exclusive block scan of c (kResNT threads); *tot gets the sum
@@ -299,12 +288,10 @@ __device__ __forceinline__ void test_chunk(const Slots &S, PickTable &T, float4 
 // ---------------------------------------------------------------------------
 // The batch: the first kBatch alive items of words [w0, w1] with their boxes, by the whole block (R.nb of them; R.tot:
 // the alive items).  The bitmap is read past L1: other blocks of the cluster have changed it.
-// KEY_ORDER (positions in nms_radix.cu's order): a run of equal scores never straddles two batches (the batch ends
-// before a run that the next alive box continues); a run longer than a batch is cut and raises *need (any block may
-// write it: the value is the same).
-template <bool KEY_ORDER>
-__device__ __forceinline__ void select_members(const Slots &S, GreedySmem &R, const int *list, int w0, int w1, int *need) {
-  constexpr int want = kBatch + (KEY_ORDER ? 1 : 0);   // key order: one more, to see the run at the boundary
+// ordered: the positions are the quicksort's.  Else a run of equal scores never straddles two batches (the batch ends
+// before a run that the next alive box continues); a run longer than a batch raises R.cut.
+__device__ __forceinline__ void select_members(const Slots &S, GreedySmem &R, const int *list, int w0, int w1, bool ordered) {
+  constexpr int want = kBatch + 1;                     // one more, to see the run at the boundary
   const int per = (w1 - w0 + kResNT) / kResNT;         // words per thread: at most four
   unsigned word[4];
   int cnt = 0;
@@ -324,7 +311,7 @@ __device__ __forceinline__ void select_members(const Slots &S, GreedySmem &R, co
   for (int k = threadIdx.x; k < min(want, tot); k += kResNT) {
     const int r = list ? list[R.item[k]] : R.item[k];
     R.pos[k] = r;
-    if (KEY_ORDER) R.key[k] = sorted_key(S, r);
+    R.key[k] = S.key[r];
     if (k < kBatch) {
       R.my[0][k] = S.y1[r];
       R.my[1][k] = S.x1[r];
@@ -336,7 +323,9 @@ __device__ __forceinline__ void select_members(const Slots &S, GreedySmem &R, co
   __syncthreads();
   if (threadIdx.x == 0) {
     int nb = min(kBatch, tot);
-    if (KEY_ORDER && tot > kBatch && R.key[kBatch - 1] == R.key[kBatch]) {   // end before the run that goes on
+    R.cut = 0;
+    R.runs.n = 0;
+    if (!ordered && tot > kBatch && R.key[kBatch - 1] == R.key[kBatch]) {   // end before the run that goes on
       const unsigned kb = R.key[kBatch];
       int lo = 0, hi = kBatch;   // first candidate with key kb (keys ascend)
       while (lo < hi) {
@@ -346,7 +335,7 @@ __device__ __forceinline__ void select_members(const Slots &S, GreedySmem &R, co
       }
       nb = lo;
       if (nb == 0) {   // a run longer than a batch
-        *need = 1;
+        R.cut = 1;
         nb = kBatch;
       }
     }
@@ -372,11 +361,122 @@ __device__ __forceinline__ void pair_row(const GreedySmem &R, int i, float overl
   if (lane < kBW) row[lane] = mine;
 }
 
+// First of the places [lo, hi) with ascending keys that is not below k (kAbove: that is above k), else hi; by a warp
+template <bool kAbove, class F>
+__device__ __forceinline__ int key_bound(F key, int lo, int hi, unsigned k) {
+  const int lane = threadIdx.x & 31;
+  while (lo < hi) {
+    const long long len = hi - lo;
+    const unsigned v = key(lo + (int)(len * lane / 32));
+    const int c = __popc(__ballot_sync(0xffffffffu, kAbove ? v <= k : v < k));   // the first c probes are before it
+    if (c < 32) hi = lo + (int)(len * c / 32);
+    if (c > 0) lo = lo + (int)(len * (c - 1) / 32) + 1;
+  }
+  return lo;
+}
+
+// Whether a sorted position is inside one of the runs
+__device__ __forceinline__ bool in_runs(const SortRuns &runs, int pos) {
+  bool in = false;
+  for (int q = 0; q < runs.n; q++) in |= pos >= runs.r[q].x && pos <= runs.r[q].y;
+  return in;
+}
+
+// The batch's runs in R.tied (a bit for the first member of each) into R.runs (their places in the sorted
+// order); what is more than kRuns goes into the last, which then holds other runs' places too
+__device__ __forceinline__ void tied_runs(GreedySmem &R, const Slots &S, int D) {
+  if (threadIdx.x >= 32) return;
+  auto key = [&](int q) { return S.key[q]; };
+  int n = R.runs.n;
+  for (int w = 0; w < kBW; w++)
+    for (unsigned rem = R.tied[w]; rem; rem &= rem - 1) {
+      const unsigned k = R.key[32 * w + __ffs(rem) - 1];
+      const int lo = key_bound<false>(key, 0, D, k), hi = key_bound<true>(key, 0, D, k) - 1;
+      if (threadIdx.x == 0) {
+        int2 &last = R.runs.r[kRuns - 1];
+        if (n < kRuns) R.runs.r[n] = make_int2(lo, hi);
+        else last = make_int2(min(last.x, lo), max(last.y, hi));
+      }
+      n = min(n + 1, kRuns);
+    }
+  if (threadIdx.x == 0) R.runs.n = n;
+}
+
+// The members of the first block's R.tied and R.runs in the quicksort's order, in every block; false where the order of all boxes
+// is to be taken instead
+__device__ __noinline__ bool settle_members(GreedySmem &R, int *si, float *sf, int m, int cap, int *err) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const Slots S = slots(si, sf, m, cap);
+  const int D = S.st->D;
+  const GreedySmem *R0 = cluster.map_shared_rank(&R, 0);
+  if (cluster.block_rank() == 0) tied_runs(R, S, D);
+  cluster.sync();
+  if (threadIdx.x < sizeof(SortRuns) / sizeof(int))
+    reinterpret_cast<int *>(&R.runs)[threadIdx.x] = reinterpret_cast<const int *>(&R0->runs)[threadIdx.x];
+  if (threadIdx.x == 0) R.settled++;
+  __syncthreads();
+  int places = 0;
+  for (int q = 0; q < R.runs.n; q++) places += R.runs.r[q].y - R.runs.r[q].x + 1;
+  const int tied = __syncthreads_count((int)threadIdx.x < R.nb && in_runs(R.runs, R.pos[threadIdx.x]));
+  if (R.settled > kSettle || places > max(kSettleRun, D / 4) || (tied >= kSettleHead && R.runs.r[0].x < D / 32)) return false;
+  quick_sort(R.quick, R.runs, S, false, err);
+  const int k = threadIdx.x, nb = R.nb;
+  int *rk = R.pick_mem;   // a member's place: a run's members share the run's, the others keep theirs
+  static_assert(kBatch == kResNT, "a thread per member");
+  int pos = 0, item = 0, at = 0;
+  float box[5];
+  if (k < nb) {
+    pos = R.pos[k];
+    item = R.item[k];
+    for (int c = 0; c < 5; c++) box[c] = R.my[c][k];
+    rk[k] = in_runs(R.runs, pos) ? __ldcg(S.place + S.ord[pos]) : pos;
+  }
+  __syncthreads();
+  if (k < nb)
+    for (int j = 0; j < nb; j++) at += rk[j] < rk[k];
+  if (k < nb) {
+    R.pos[at] = pos;
+    R.item[at] = item;
+    for (int c = 0; c < 5; c++) R.my[c][at] = box[c];
+  }
+  __syncthreads();
+  return true;
+}
+
+// The quicksort of all boxes, as far as the cluster takes it
+__device__ __noinline__ void split_boxes(GreedySmem &R, int *si, float *sf, int m, int cap, int *err) {
+  const Slots S = slots(si, sf, m, cap);
+  const int D = S.st->D;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    R.runs.n = 1;
+    R.runs.r[0] = make_int2(0, D - 1);
+  }
+  __syncthreads();
+  quick_sort(R.quick, R.runs, S, true, err);
+}
+
+// The boxes in the quicksort's order, by the cluster
+__device__ __noinline__ void gather_boxes(const float *boxes, int GL, int *si, float *sf, int m, int cap) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const Slots S = slots(si, sf, m, cap);
+  const int D = S.st->D;
+#pragma unroll 4
+  for (int r = (int)cluster.block_rank() * kResNT + threadIdx.x; r < D; r += (int)cluster.num_blocks() * kResNT) {
+    const int i = S.qo[r];
+    const float *P = boxes + (size_t)i * GL;
+    S.ord[r] = i;
+    S.y1[r] = P[0]; S.x1[r] = P[1]; S.y2[r] = P[2]; S.x2[r] = P[3];
+    S.ar[r] = (P[3] - P[1] + 1.0) * (P[2] - P[0] + 1.0);   // nms.cpp's area expression
+  }
+  cluster.sync();
+}
+
 // The batch's decisions from its rows (R.adj), by the first block: R.np picks in R.pick_mem, appended to S.picks
-// and S.pb, the members cleared from the bitmap.  In key order *need is raised where the order inside a run of equal scores
-// matters: a pick that removes a member of its own run.
-template <bool KEY_ORDER>
-__device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, int base, int *need) {
+// and S.pb, the members cleared from the bitmap.  check: where the order inside a run of equal scores
+// matters (a pick that removes a member of its own run, other than the runs in R.runs, which are in order), nothing of
+// that but R.np = -1 and the run in R.tied.
+__device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, int base, bool check) {
   const int nb = R.nb, lane = threadIdx.x & 31;
   if (threadIdx.x < 32) {
     // the undecided members in registers, every lane alike (one wide broadcast read a pick; warp votes in this
@@ -401,21 +501,37 @@ __device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, in
         R.pick_mem[np] = i;
         R.pick_any[np++] = gone != 0u;
       }
-    if (lane == 0) R.np = np;
+    if (lane == 0) {
+      R.np = np;
+      R.need = 0;
+    }
+    if (lane < kBW) R.tied[lane] = 0u;
   }
   __syncthreads();
   const int np = R.np;
-  if (KEY_ORDER)
+  if (check) {
     for (int k = threadIdx.x; k < np; k += kResNT) {
       // members of the pick's own run that it removed: suppressed by it and by no pick before it
       const int i = R.pick_mem[k];
+      if (in_runs(R.runs, R.pos[i])) continue;
       for (int j = i + 1; j < nb && R.key[j] == R.key[i]; j++) {
         if (!((R.adj[i * kBW + (j >> 5)] >> (j & 31)) & 1u)) continue;
         bool alive = true;
         for (int q = 0; q < k && alive; q++) alive = !((R.adj[R.pick_mem[q] * kBW + (j >> 5)] >> (j & 31)) & 1u);
-        if (alive) *need = 1;
+        if (!alive) continue;
+        int first = i;
+        while (first > 0 && R.key[first - 1] == R.key[i]) first--;
+        atomicOr(&R.tied[first >> 5], 1u << (first & 31));
+        R.need = 1;
+        break;
       }
     }
+    __syncthreads();
+    if (R.need) {
+      if (threadIdx.x == 0) R.np = -1;
+      return;
+    }
+  }
   for (int k = threadIdx.x; k < np; k += kResNT) {
     const int i = R.pick_mem[k];
     S.picks[base + k] = R.pos[i];
@@ -430,18 +546,12 @@ __device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, in
 // ---------------------------------------------------------------------------
 // final-pick rule, the kept boxes in input order (whole block, the model done)
 // ---------------------------------------------------------------------------
-template <bool KEY_ORDER>
-__device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int m, int npk, int batches, const float *boxes,
-                                             int GL, int cap, const NmsResults &res, int *d_kept, long long *diag,
-                                             const int *lv_used, int *need, cudaGraphConditionalHandle cond,
-                                             bool has_cond) {
+__device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int m, int npk, int batches, bool quick,
+                                             const float *boxes, int GL, int cap, const NmsResults &res, int *d_kept,
+                                             long long *diag) {
   const int D = S.st->D;
   // (the flags are read past L1: other blocks of the cluster have set them)
   const int K = npk - ((npk > 0 && __ldcg(&S.flag[npk - 1]) == 0) ? 1 : 0);
-  // the last pick shares its score with another pick: which of them is last is the quicksort's call
-  if (KEY_ORDER && threadIdx.x == kResNT - 1 && npk >= 2 &&
-      sorted_key(S, __ldcg(&S.picks[npk - 1])) == sorted_key(S, __ldcg(&S.picks[npk - 2])))
-    need[m] = 1;
   // the kept boxes' input indices (all distinct) in ascending order
   int *keep = S.Rpos;
   int *idx = R.idx;   // the round's buffers are free now
@@ -479,11 +589,10 @@ __device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int 
   __syncthreads();
   if (threadIdx.x == 0) {
     d_kept[m] = K;
-    if (KEY_ORDER && has_cond && *(volatile int *)&need[m]) cudaGraphSetConditional(cond, 1);
     if (diag) {
       diag[8 * m + 2] = batches;
       diag[8 * m + 3] = npk;
-      diag[8 * m + 5] = need ? *(volatile int *)&need[m] : 1;
+      diag[8 * m + 5] = quick;
     }
   }
   // the results (get_new_rects), four threads a box: on the device, and the first of them in the host's block
@@ -503,100 +612,66 @@ __device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int 
     put(out, cap);
     if (k < res.host_cap) put(host, res.host_cap);
   }
-  if (threadIdx.x == 0) {
-    res.host[32 + m] = K;
-    if (!KEY_ORDER) res.host[kSortLevelsUsed] = *lv_used;
-  }
+  if (threadIdx.x == 0) res.host[32 + m] = K;
 }
 
-// The first key-order item at or after c1 whose score differs from the one before it, at most hi (every warp alike)
+// The first item at or after c1 whose score differs from the one before it, at most hi (every warp alike)
 __device__ __forceinline__ int run_end(const Slots &S, const int *list, int c1, int hi) {
-  const int lane = threadIdx.x & 31;
-  const unsigned k = sorted_key(S, list ? list[c1 - 1] : c1 - 1);
-  while (c1 < hi) {
-    const int q = c1 + lane;
-    const unsigned other = __ballot_sync(0xffffffffu, q >= hi || sorted_key(S, list ? list[q] : q) != k);
-    if (other) return c1 + __ffs(other) - 1;
-    c1 += 32;
-  }
-  return hi;
+  auto key = [&](int q) { return S.key[list ? list[q] : q]; };
+  const unsigned k = key(c1 - 1);
+  const int q = c1 + (threadIdx.x & 31);
+  const unsigned other = __ballot_sync(0xffffffffu, q >= hi || key(q) != k);
+  return other ? c1 + __ffs(other) - 1 : key_bound<true>(key, c1 + 32, hi, k);
 }
 
-// The greedy rounds of a model (see the top of the file).  KEY_ORDER: the key-order pass (every model; raises need[m]
-// where the quicksort order could differ).  Otherwise the quicksort-order pass: with need given, only the models that
-// raised it are not done (their result replaces the key-order one); without, every model.
-// rest = false: all the boxes, or the first kPrefix of more than kWhole; true: the survivors that k_nms_rest left of
-// the others.
-template <bool KEY_ORDER>
-__global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restrict__ boxes_all, int GL, int cap, int *si,
-                                                       float *sf, float overlap, float2 cell_inv,
-                                                       const __grid_constant__ NmsResults res, int *d_kept,
-                                                       long long *diag, const int *lv_used, int *need,
-                                                       cudaGraphConditionalHandle cond, bool has_cond, bool rest) {
-  extern __shared__ __align__(16) unsigned char res_sm[];
-  GreedySmem &R = *reinterpret_cast<GreedySmem *>(res_sm);
+// The walk over the items [R.c0, R.n), with R.npicks picks of which R.tested have been tested against all items (list:
+// the items' sorted positions).  kTied: a batch's decisions depend on the order inside runs of equal scores (R.tied of the
+// first block); again with resume kBatchReady once its members are in order.  kCut: a run longer than a batch or a chunk.
+// Every block alike; its place rests in shared memory between the calls.
+enum WalkEnd { kDone, kTied, kCut };
+enum WalkResume { kAnew, kChunkTested, kBatchReady };   // in a chunk that has been tested; with a batch that is selected
+__device__ __forceinline__ WalkEnd walk_boxes(const Slots &S, GreedySmem &R, const int *list, float overlap, float2 cell_inv,
+                                              bool ordered, WalkResume resume) {
   cg::cluster_group cluster = cg::this_cluster();
-  const int m = blockIdx.y, rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
-  const int warp = threadIdx.x >> 5, gw = rank * kResWarps + warp, nw = blocks * kResWarps;
-  Slots S = slots(si, sf, m, cap);
-  const BatchState st = *S.st;
-  if (st.done) return;   // (the same in every block: it is written behind a cluster barrier)
-  int *need_m = need ? need + m : nullptr;
   GreedySmem *R0 = cluster.map_shared_rank(&R, 0);
-  cluster.sync();   // every block has started: its shared memory can be written
-  const int *list = nullptr;
-  int n = st.D, np = st.npicks, tested = 0;
-  if (!rest) {
-    if (st.D > kWhole) n = KEY_ORDER ? run_end(S, nullptr, kPrefix, st.D) : kPrefix;
-  } else {
-    // the alive bits of the words from st.next on as a list of sorted positions, in order: a stretch of words per block
-    const int wa = st.next >> 5, nwords = ((st.D + 31) >> 5) - wa;
-    const int share = (nwords + blocks - 1) / blocks, per = (share + kResNT - 1) / kResNT;
-    const int b0 = wa + rank * share, b1 = min(wa + nwords, b0 + share);
-    const int t0 = b0 + threadIdx.x * per, t1 = min(b1, t0 + per);
-    int cnt = 0, tot;
-    for (int w = t0; w < t1; w++) cnt += __popc(__ldcg(&S.bits[w]));
-    int at = block_excl_scan(cnt, &tot, R.wtot);
-    if (threadIdx.x == 0) R0->total[rank] = tot;
-    cluster.sync();
-    n = 0;
-    for (int b = 0; b < blocks; b++) {
-      const int v = R0->total[b];
-      if (b < rank) at += v;
-      n += v;
-    }
-    for (int w = t0; w < t1; w++)
-      for (unsigned rem = __ldcg(&S.bits[w]); rem; rem &= rem - 1) S.Lpos[at++] = (w << 5) + __ffs(rem) - 1;
-    list = S.Lpos;
-    tested = np;
-    cluster.sync();   // the list is complete, the bitmap free
-  }
-  int chunk = kBatch, batches = st.batches;
-  for (int c0 = 0; c0 < n;) {
-    int c1 = min(c0 + chunk, n);
-    if (KEY_ORDER && c1 < n) {   // not inside a run of equal scores
+  const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
+  const int gw = rank * kResWarps + (threadIdx.x >> 5), nw = blocks * kResWarps;
+  const int n = R.n;
+  int chunk = R.chunk, np = R.npicks, tested = R.tested, batches = R.batches, left = R.left;
+  WalkEnd end = kDone;
+  for (int c0 = R.c0; c0 < n;) {
+    int c1 = resume != kAnew ? R.c1 : min(c0 + chunk, n);
+    if (resume == kAnew && !ordered && c1 < n) {   // not inside a run of equal scores
       const int lim = min(n, c0 + kMaxChunk);
       c1 = run_end(S, list, c1, lim);
-      if (c1 == lim && c1 < n && run_end(S, list, c1, c1 + 1) > c1) {   // a run of that length is cut
-        if (threadIdx.x == 0) *need_m = 1;
-      }
+      if (c1 == lim && c1 < n && run_end(S, list, c1, c1 + 1) > c1) return kCut;   // a run of that length would be cut
     }
     const int w0 = c0 >> 5, w1 = (c1 - 1) >> 5;
-    test_chunk(S, R.table, R.pk, R.pka, tested, np, list, w0, w1, c0, c1, overlap, cell_inv, gw, nw);
-    cluster.sync();   // the bitmap is complete
-    int left = 0;
-    for (int round = 0;; round++) {
-      select_members<KEY_ORDER>(S, R, list, w0, w1, need_m);
-      if (round == 0) left = R.tot;
+    if (resume == kAnew) {
+      test_chunk(S, R.table, R.pk, R.pka, tested, np, list, w0, w1, c0, c1, overlap, cell_inv, gw, nw);
+      cluster.sync();   // the bitmap is complete
+    }
+    for (bool first = resume == kAnew;; first = false) {
+      if (resume != kBatchReady) select_members(S, R, list, w0, w1, ordered);
+      resume = kAnew;
+      if (first) left = R.tot;
       if (R.tot == 0) break;
+      if (R.cut) {
+        end = kCut;
+        break;
+      }
       for (int k = 0; k * nw < R.nb; k++) {   // rows g, then 2G - 1 - g, ...: long and short ones in turn
         const int i = k * nw + ((k & 1) ? nw - 1 - gw : gw);
         if (i < R.nb) pair_row(R, i, overlap, R0->adj + i * kBW);
       }
       cluster.sync();   // the rows are in the first block
-      if (rank == 0) decide_members<KEY_ORDER>(S, R, np, need_m);
+      if (rank == 0) decide_members(S, R, np, !ordered);
       cluster.sync();   // the picks are in the first block and in S, the members cleared
       const int added = R0->np;
+      if (added < 0) {
+        end = kTied;
+        break;
+      }
       batches++;
       if (R.tot > R.nb) {   // the rest of the chunk against the new picks
         test_chunk(S, R.table, R.pk, R.pka, np, np + added, list, w0, w1, 0, 0, overlap, cell_inv, gw, nw, false);
@@ -606,37 +681,223 @@ __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restric
       if (R.tot <= R.nb) break;
     }
     cluster.sync();   // (the first block's picks have been read)
+    if (end != kDone) {
+      if (threadIdx.x == 0) {
+        R.c0 = c0;
+        R.c1 = c1;
+      }
+      break;
+    }
     // the head leaves about a tenth of what follows alive, and the picks thin every next stretch out further:
     // eight times the chunk leaves a batch or two (twice after one that left more)
     chunk = min((left > 2 * kBatch ? 2 : 8) * chunk, kChunkCap);
     c0 = c1;
   }
-  if (!rest && n < st.D) {
-    if (rank == 0 && threadIdx.x == 0) {
-      S.st->npicks = np;
-      S.st->batches = batches;
-      S.st->next = n;
+  if (threadIdx.x == 0) {
+    R.chunk = chunk;
+    R.npicks = np;
+    R.batches = batches;
+    R.left = left;
+  }
+  __syncthreads();
+  return end;
+}
+
+// The greedy rounds of a model (see the top of the file).
+// kFirst: all the boxes, or the first kPrefix of more than kWhole; kRest: the survivors that k_nms_rest left of
+// the others; kOrderedFirst and kOrderedRest: the same in the quicksort's order.
+// kFull = false stops where the quicksort is needed and leaves the model to the kFull instance: with the sort's calls in
+// it, the rounds' code is 8 % slower (same rounds: 1280x720, NMS stage 433 us against 399).
+enum GreedyPass { kFirst, kRest, kOrderedFirst, kOrderedRest };
+template <bool kFull>
+__global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restrict__ boxes_all, int GL, int cap, int *si,
+                                                       float *sf, float overlap, float2 cell_inv,
+                                                       const __grid_constant__ NmsResults res, int *d_kept,
+                                                       long long *diag, const int *need, int *err, bool all_ordered,
+                                                       GreedyPass pass, cudaGraphConditionalHandle cond, bool has_cond) {
+  extern __shared__ __align__(16) unsigned char res_sm[];
+  GreedySmem &R = *reinterpret_cast<GreedySmem *>(res_sm);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int m = blockIdx.y;
+  const float *boxes = boxes_all + (size_t)m * cap * GL;
+  const bool ordered = kFull && pass >= kOrderedFirst, rest = pass & 1;
+  bool whole = false;          // the quicksort's order of all boxes is needed (every block alike)
+  WalkResume resume = kAnew;
+  {
+    const BatchState st = *slots(si, sf, m, cap).st;   // (the same in every block: it is written behind a cluster barrier)
+    if (kFull) {
+      if (pass == kFirst && st.stage == kNmsWhole) whole = true;
+      else if ((pass == kFirst && st.stage == kNmsTied) || (pass == kRest && st.stage == kNmsTiedRest)) resume = kChunkTested;
+      else if (!((pass == kRest && st.stage == kNmsPrefix) || (pass == kOrderedFirst && st.stage == kNmsSplit) ||
+                 (pass == kOrderedRest && st.stage == kNmsOrderedPrefix)))
+        return;
+    } else {
+      if (st.stage != (pass == kFirst ? kNmsStart : kNmsPrefix)) return;
+      whole = pass == kFirst && (all_ordered || need[m]);
+    }
+    if (threadIdx.x == 0) {
+      const bool anew = resume == kAnew;
+      R.n = anew ? st.D : st.n;
+      R.c0 = anew ? 0 : st.c0;
+      R.c1 = anew ? 0 : st.c1;
+      R.chunk = anew ? kBatch : st.chunk;
+      R.npicks = st.npicks;
+      R.tested = anew ? 0 : st.tested;
+      R.left = anew ? 0 : st.left;
+      R.batches = st.batches;
+      R.settled = 0;
+    }
+  }
+  cluster.sync();   // every block has started: its shared memory can be written
+  if (kFull && pass == kOrderedFirst) gather_boxes(boxes, GL, si, sf, m, cap);
+  if (resume != kAnew || whole) {
+  } else if (!rest) {
+    const Slots S = slots(si, sf, m, cap);
+    const int D = R.n, n = D <= kWhole ? D : ordered ? kPrefix : run_end(S, nullptr, kPrefix, D);
+    __syncthreads();
+    if (threadIdx.x == 0) R.n = n;
+  } else {
+    // the alive bits of the words from st.next on as a list of sorted positions, in order: a stretch of words per block
+    const Slots S = slots(si, sf, m, cap);
+    const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
+    GreedySmem *R0 = cluster.map_shared_rank(&R, 0);
+    const int wa = S.st->next >> 5, nwords = ((R.n + 31) >> 5) - wa;
+    const int share = (nwords + blocks - 1) / blocks, per = (share + kResNT - 1) / kResNT;
+    const int b0 = wa + rank * share, b1 = min(wa + nwords, b0 + share);
+    const int t0 = b0 + threadIdx.x * per, t1 = min(b1, t0 + per);
+    int cnt = 0, tot;
+    for (int w = t0; w < t1; w++) cnt += __popc(__ldcg(&S.bits[w]));
+    int at = block_excl_scan(cnt, &tot, R.wtot);
+    if (threadIdx.x == 0) R0->total[rank] = tot;
+    cluster.sync();
+    int n = 0;
+    for (int b = 0; b < blocks; b++) {
+      const int v = R0->total[b];
+      if (b < rank) at += v;
+      n += v;
+    }
+    for (int w = t0; w < t1; w++)
+      for (unsigned rem = __ldcg(&S.bits[w]); rem; rem &= rem - 1) S.Lpos[at++] = (w << 5) + __ffs(rem) - 1;
+    if (threadIdx.x == 0) {
+      R.n = n;
+      R.tested = R.npicks;
+    }
+    cluster.sync();   // the list is complete, the bitmap free
+  }
+  __syncthreads();
+  bool tied = false;
+  while (!whole) {
+    if (kFull) asm volatile("" : "+l"(si), "+l"(sf));   // (nothing formed of them is kept over the settling)
+    const Slots S = slots(si, sf, m, cap);
+    const WalkEnd end = walk_boxes(S, R, rest ? S.Lpos : nullptr, overlap, cell_inv, ordered, resume);
+    if (end == kDone) break;
+    whole = end == kCut;
+    if (!kFull) {
+      tied = !whole;
+      break;
+    }
+    if (!whole) whole = !settle_members(R, si, sf, m, cap, err);
+    resume = kBatchReady;
+  }
+  if (kFull) asm volatile("" : "+l"(si), "+l"(sf));
+  const Slots S = slots(si, sf, m, cap);
+  const int np = R.npicks;
+  const bool more = !rest && R.n < S.st->D;
+  // the last pick of all shares its score with another pick: which of them is last is the quicksort's call
+  if (!whole && !tied && !ordered && !more && np >= 2)
+    whole = S.key[__ldcg(&S.picks[np - 1])] == S.key[__ldcg(&S.picks[np - 2])];
+  if (kFull && whole) split_boxes(R, si, sf, m, cap, err);
+  if (cluster.block_rank() != 0) return;
+  const bool quick = kFull || whole || tied;
+  if (whole || tied || more) {
+    if (threadIdx.x == 0) {
+      BatchState &st = *slots(si, sf, m, cap).st;
+      st.stage = whole ? (kFull ? kNmsSplit : kNmsWhole) : tied ? (rest ? kNmsTiedRest : kNmsTied)
+                 : ordered ? kNmsOrderedPrefix : kNmsPrefix;
+      st.quick |= quick;
+      st.next = rest ? st.next : R.n;
+      st.n = R.n; st.c0 = R.c0; st.c1 = R.c1; st.chunk = R.chunk; st.tested = R.tested; st.left = R.left;
+      st.npicks = whole ? 0 : R.npicks;
+      st.batches = R.batches;
+      if (!kFull && (whole || tied) && has_cond) cudaGraphSetConditional(cond, 1);
     }
     return;
   }
-  if (rank == 0) {
-    if (threadIdx.x == 0) S.st->done = 1;
-    finish_model<KEY_ORDER>(S, R, m, np, batches, boxes_all + (size_t)m * cap * GL, GL, cap, res, d_kept, diag, lv_used,
-                            need, cond, has_cond);
-  }
+  if (threadIdx.x == 0) S.st->stage = kNmsDone;
+  finish_model(S, R, m, np, R.batches, quick || S.st->quick, boxes, GL, cap, res, d_kept, diag);
 }
 
 // The boxes from st.next on against every pick so far, over the grid
-__global__ void __launch_bounds__(kResNT) k_nms_rest(int cap, int *si, float *sf, float overlap, float2 cell_inv) {
+__global__ void __launch_bounds__(kResNT) k_nms_rest(int cap, int *si, float *sf, float overlap, float2 cell_inv, NmsStage stage) {
   __shared__ PickTable T;
   __shared__ float4 pk[kPickGroup];
   __shared__ float pka[kPickGroup];
   Slots S = slots(si, sf, blockIdx.y, cap);
   const BatchState st = *S.st;
-  if (st.done) return;
+  if (st.stage != stage) return;
   const int w0 = st.next >> 5, w1 = (st.D - 1) >> 5;
   test_chunk(S, T, pk, pka, 0, st.npicks, nullptr, w0, w1, st.next, st.D, overlap, cell_inv,
              blockIdx.x * kResWarps + (threadIdx.x >> 5), gridDim.x * kResWarps);
+}
+
+// The quicksort of all boxes of a model that needs it, a block per segment: k_quick_mid takes those that the cluster has
+// left (S.Lpos) down to those for shared memory (S.picks: the picks start anew), which k_quick_small finishes
+__device__ __forceinline__ bool quick_block(const Slots &S, SortRuns &runs) {
+  if (S.st->stage != kNmsSplit) return false;
+  if (threadIdx.x == 0) {
+    runs.n = 1;
+    runs.r[0] = make_int2(0, S.st->D - 1);
+  }
+  __syncthreads();
+  return true;
+}
+
+__global__ void __launch_bounds__(kResNT) k_quick_mid(int cap, int *si, float *sf, int *err) {
+  extern __shared__ __align__(16) unsigned char res_sm[];
+  QuickSmem &Q = *reinterpret_cast<QuickSmem *>(res_sm);
+  __shared__ SortRuns runs;
+  cg::cluster_group cluster = cg::this_cluster();
+  const Slots S = slots(si, sf, blockIdx.y, cap);
+  if (!quick_block(S, runs)) return;
+  const int2 *mid = reinterpret_cast<const int2 *>(S.Lpos);
+  int2 *small = reinterpret_cast<int2 *>(S.picks);   // (disjoint segments of two elements or more: they fit)
+  for (int e = blockIdx.x; e < S.st->n_mid; e += gridDim.x) {
+    auto push = [&](int2 c) {   // by thread 0
+      if (c.y - c.x < kQuickSmall) small[atomicAdd(&S.st->n_small, 1)] = c;
+      else if (Q.nst < 40) Q.stk[Q.nst++] = c;
+      else atomicOr(err, 512);   // impossible: depth <= log2(kQuickMid) + 1
+    };
+    if (threadIdx.x == 0) {
+      Q.nst = 0;
+      push(mid[e]);
+    }
+    __syncthreads();
+    while (Q.nst > 0) {
+      const int2 seg = Q.stk[Q.nst - 1];
+      __syncthreads();   // everyone has read the top entry
+      const int2 ij = quick_partition<false>(cluster, Q, S.qv, S.qo, S.qL, S.qR, seg.x, seg.y);
+      if (threadIdx.x == 0) {
+        Q.nst--;
+        quick_children(runs, 0, seg.x, seg.y, ij.x, ij.y, push, [](int2) {});
+      }
+      __syncthreads();
+    }
+    __syncthreads();   // everyone has seen the stack empty
+  }
+}
+
+__global__ void __launch_bounds__(kResNT) k_quick_small(int cap, int *si, float *sf, int *err) {
+  extern __shared__ __align__(16) unsigned char res_sm[];
+  QuickSmem &Q = *reinterpret_cast<QuickSmem *>(res_sm);
+  __shared__ SortRuns runs;
+  cg::cluster_group cluster = cg::this_cluster();
+  const Slots S = slots(si, sf, blockIdx.y, cap);
+  if (!quick_block(S, runs)) return;
+  const int2 *small = reinterpret_cast<const int2 *>(S.picks);
+  for (int e = blockIdx.x; e < S.st->n_small; e += gridDim.x) {
+    const int2 seg = small[e];
+    quick_small(cluster, Q, runs, S, seg.x, seg.y, false, err);
+  }
 }
 
 // Inside a stream capture: a handle for a conditional node of the graph s is
@@ -705,16 +966,22 @@ static int cluster_blocks(K *kernel, size_t smem) {
   return kCluster;
 }
 
-// the greedy rounds and the results, in the order the sort left in (val, ord)
-template <bool KEY_ORDER>
-static cudaError_t launch_greedy(const float *boxes, int n_models, int GL, float overlap, float2 cell_inv, int cap, int *si,
-                                 float *sf, const NmsResults &res, int *d_kept, long long *diag, const int *lv_used, int *need,
-                                 cudaGraphConditionalHandle cond, bool has_cond, cudaStream_t s) {
-  static SmemAttr attr;
-  cudaError_t e = raise_smem(attr, k_nms_greedy<KEY_ORDER>, sizeof(GreedySmem));
+cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
+                             int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
+                             long long *diag, int *need, int order, cudaStream_t s, cudaStream_t aux) {
+  if (n_models <= 0) return cudaSuccess;
+  // cells over the image and a margin for boxes that leave it (any value is exact: what is outside shares the edge cells)
+  const float2 cell_inv = make_float2(kNmsCells / (1.15f * std::max(res.img_h, 1)), kNmsCells / (1.15f * std::max(res.img_w, 1)));
+  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, res.host, s);
+  static SmemAttr attr[4];
+  cudaError_t e = raise_smem(attr[0], k_nms_greedy<false>, sizeof(GreedySmem));
+  if (e == cudaSuccess) e = raise_smem(attr[1], k_nms_greedy<true>, sizeof(GreedySmem));
+  if (e == cudaSuccess) e = raise_smem(attr[2], k_quick_mid, sizeof(QuickSmem));
+  if (e == cudaSuccess) e = raise_smem(attr[3], k_quick_small, sizeof(QuickSmem));
   if (e != cudaSuccess) return e;
+  const int blocks = std::min(cluster_blocks(k_nms_greedy<false>, sizeof(GreedySmem)),
+                              cluster_blocks(k_nms_greedy<true>, sizeof(GreedySmem)));
   cudaLaunchConfig_t c = {};
-  const int blocks = cluster_blocks(k_nms_greedy<KEY_ORDER>, sizeof(GreedySmem));
   c.gridDim = dim3(blocks, n_models);
   c.blockDim = dim3(kResNT);
   c.dynamicSmemBytes = sizeof(GreedySmem);
@@ -724,56 +991,31 @@ static cudaError_t launch_greedy(const float *boxes, int n_models, int GL, float
   at.val.clusterDim = {(unsigned)blocks, 1, 1};
   c.attrs = &at;
   c.numAttrs = 1;
-  for (const bool rest : {false, true}) {
-    if (rest) {
-      if (cap <= kWhole) break;
-      k_nms_rest<<<dim3(std::max(304 / n_models, 1), n_models), kResNT, 0, s>>>(cap, si, sf, overlap, cell_inv);
-    }
-    e = cudaLaunchKernelEx(&c, k_nms_greedy<KEY_ORDER>, boxes, GL, cap, si, sf, overlap, cell_inv, res, d_kept, diag,
-                           lv_used, need, cond, has_cond, rest);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
-                             int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
-                             long long *diag, int levels, int *lv_used, int *need, int order, cudaStream_t s,
-                             cudaStream_t aux) {
-  // cells over the image and a margin for boxes that leave it (any value is exact: what is outside shares the edge cells)
-  const float2 cell_inv = make_float2(kNmsCells / (1.15f * std::max(res.img_h, 1)), kNmsCells / (1.15f * std::max(res.img_w, 1)));
-  if (n_models <= 0) return cudaSuccess;
-  auto gather = [&](cudaStream_t q) {
-    k_nms_gather<<<dim3((cap + kPassNT - 1) / kPassNT, n_models), kPassNT, 0, q>>>(boxes, GL, cap, si, sf);
-  };
-  cudaError_t e = cudaSuccess;
-  if (order == kNmsOrderQuicksort) {
-    launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, nullptr, res.host, s);
-    gather(s);
-    e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, lv_used, nullptr, 0,
-                             false, s);
-    return e == cudaSuccess ? cudaGetLastError() : e;
-  }
-  // the models whose kept set could depend on the order inside a run of equal
-  // scores go again in the quicksort's order: in a graph captured with aux, an
-  // if node that runs only when some model needs it (the finishing block of
-  // such a model sets its condition); otherwise launches that do nothing for
-  // the models that do not
   cudaGraphConditionalHandle h = 0;
   if (aux && (e = cond_handle(s, 0u, &h)) != cudaSuccess) return e;
-  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, res.host, s);
-  if ((e = launch_greedy<true>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, lv_used, need, h,
-                               aux != nullptr, s)) != cudaSuccess)
-    return e;
-  cudaStream_t q = s;
-  if (aux) {
-    if ((e = begin_conditional(s, aux, cudaGraphCondTypeIf, h)) != cudaSuccess) return e;
-    q = aux;
+  auto greedy = [&](bool full, GreedyPass pass) {
+    if (e != cudaSuccess || ((pass & 1) && cap <= kWhole)) return;
+    if (pass & 1)
+      k_nms_rest<<<dim3(std::max(304 / n_models, 1), n_models), kResNT, 0, c.stream>>>(
+          cap, si, sf, overlap, cell_inv, pass == kRest ? kNmsPrefix : kNmsOrderedPrefix);
+    e = cudaLaunchKernelEx(&c, full ? k_nms_greedy<true> : k_nms_greedy<false>, boxes, GL, cap, si, sf, overlap, cell_inv,
+                           res, d_kept, diag, (const int *)need, err, order == kNmsOrderQuicksort, pass, h, aux != nullptr);
+  };
+  greedy(false, kFirst);
+  greedy(false, kRest);
+  // the models that need the quicksort's order, among a batch's members or of all boxes: in a graph captured with aux, an
+  // if node that runs only when some model needs it; otherwise launches that return at once where none does
+  if (e == cudaSuccess && aux) {
+    e = begin_conditional(s, aux, cudaGraphCondTypeIf, h);
+    c.stream = aux;
   }
-  launch_nms_sort(boxes, d_num, n_models, GL, cap, si, sf, err, diag, levels, lv_used, need, res.host, q);
-  gather(q);
-  e = launch_greedy<false>(boxes, n_models, GL, overlap, cell_inv, cap, si, sf, res, d_kept, diag, lv_used, need, 0, false,
-                           q);
+  if (e != cudaSuccess) return e;
+  greedy(true, kFirst);
+  greedy(true, kRest);
+  k_quick_mid<<<dim3(std::max(152 / n_models, 1), n_models), kResNT, sizeof(QuickSmem), c.stream>>>(cap, si, sf, err);
+  k_quick_small<<<dim3(std::max(456 / n_models, 1), n_models), kResNT, sizeof(QuickSmem), c.stream>>>(cap, si, sf, err);
+  greedy(true, kOrderedFirst);
+  greedy(true, kOrderedRest);
   if (aux) {
     const cudaError_t e2 = end_conditional(aux);
     if (e == cudaSuccess) e = e2;

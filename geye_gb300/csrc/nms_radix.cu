@@ -11,14 +11,13 @@
 //   (b) the last pick's run holds another pick (which of them is last decides
 //       the reference's rule for a box that is alone at its turn),
 // or when a score is NaN (the quicksort places it by its comparisons).  The
-// greedy rounds (nms_batch.cu) check (a) and (b) as they go and raise the
-// model's flag for any of them; a flagged model is then sorted again by the
-// quicksort restatement (nms_sort.cu) and resolved again in that order.  The
-// kept set is the reference's either way.
+// greedy rounds (nms_batch.cu) check (a) and (b) as they go and take the
+// quicksort's order there (nms_quick.h), and from the start for a model whose
+// flag is raised here (NaN).  The kept set is the reference's either way.
 //
 //   k_rs_load     keys (order-preserving transform of the float score, -0 as
 //                 +0, complemented for descending order), indices, the
-//                 greedy state, and the digit counts of the first
+//                 scores in input order (for nms_quick.h), the greedy state, and the digit counts of the first
 //                 pass per tile of nms_rs_tile(cap) keys; NaN raises the flag.
 //   k_rs_pass     four passes of eight bits, one kernel each: a block per tile
 //                 adds up the tiles' digit counts before it (at most a few
@@ -30,8 +29,8 @@
 // What bounds it is latency: a kernel boundary per pass.  With a count, a scan
 // (one block per model) and a scatter kernel per pass and a gather behind them,
 // 14 launches instead of 5, the 640x480 pair's NMS took 285 us; see nms_batch.cu.
-// Keys ping-pong between (val, ord) and (Lpos, Rpos); after the fourth pass
-// they are back in (val, ord): val holds the transformed keys (equal keys <=>
+// Keys ping-pong between (key, ord) and (Lpos, Rpos); after the fourth pass
+// they are back in (key, ord): key holds the transformed keys (equal keys <=>
 // equal scores), ord the input index of each sorted position.
 #include "nms_common.h"
 
@@ -58,11 +57,10 @@ __global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ box
   if (t == 0 && threadIdx.x == 0) {
     BatchState &st = *S.st;
     st.D = D;
-    st.done = D <= 0;
-    st.npicks = st.batches = st.next = 0;
+    st.stage = D > 0 ? kNmsStart : kNmsDone;
+    st.quick = st.next = st.npicks = st.batches = st.n_mid = st.n_small = st.n_left = 0;
     host[m] = D;
     host[32 + m] = 0;
-    if (m == 0) host[kSortLevelsUsed] = 0;
   }
   const int e0 = t * T;
   if (e0 >= D) return;
@@ -70,9 +68,11 @@ __global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ box
   __syncthreads();
   bool nan = false;
   for (int i = e0 + threadIdx.x; i < min(e0 + T, D); i += kRsNT) {
-    const unsigned k = rs_key(boxes[(size_t)i * GL + GL - 2], nan);
+    const float v = boxes[(size_t)i * GL + GL - 2];
+    const unsigned k = rs_key(v, nan);
     if (nan) need[m] = 1;
-    reinterpret_cast<unsigned *>(S.val)[i] = k;
+    S.score[i] = v;
+    S.key[i] = k;
     S.ord[i] = i;
     atomicAdd(&h[k & 255u], 1);
   }
@@ -85,10 +85,10 @@ __global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ box
   }
 }
 
-// pass p reads (val, ord) for even p and (Lpos, Rpos) for odd p
+// pass p reads (key, ord) for even p and (Lpos, Rpos) for odd p
 __device__ __forceinline__ void rs_bufs(const Slots &S, int pass, const unsigned *&sk, const int *&si_, unsigned *&dk,
                                         int *&di) {
-  unsigned *a_k = reinterpret_cast<unsigned *>(S.val), *b_k = reinterpret_cast<unsigned *>(S.Lpos);
+  unsigned *a_k = S.key, *b_k = reinterpret_cast<unsigned *>(S.Lpos);
   int *a_i = S.ord, *b_i = S.Rpos;
   if (pass & 1) {
     sk = b_k; si_ = b_i; dk = a_k; di = a_i;

@@ -1001,30 +1001,11 @@ geye_status run_ascore(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thre
   return ascore_compute(ctx, P, mp, mi, thresh, ctx->stream);
 }
 
-// After a frame of the plan has completed: `used` is the deepest grid-wide
-// quicksort level that had a segment to partition (0 when no model needed the
-// quicksort's order).
-// Sort levels: the first frame that sorts launches the default count
-// (nms_sort_levels); if it needed fewer, the plan launches three levels more
-// than it needed from then on (each empty level costs three launches).  A
-// frame whose last launched level still had work left its remaining segments
-// to the single-block fallback (exact, slower): the plan goes back to the
-// default count for good.
-// The plan's DT tile sizes are tuned here too, once, on this frame's maps
+// After a plan's first frame has completed: its DT tile sizes are tuned, once, on that frame's maps
 // (tune_dt).  A change drops the plan's frame graphs after its stream has
 // drained; the next frame captures them again.
-void note_sort_levels(geye_ctx *ctx, Plan &P, int used) {
-  const int full = nms_sort_levels(P.max_cap);
-  const int launched = P.sort_levels > 0 ? P.sort_levels : full;
-  int next = P.sort_levels;
-  if (used >= launched) {
-    if (P.sort_levels > 0) { next = 0; P.sort_levels_fixed = true; }
-  } else if (!P.sort_levels_fixed && P.sort_levels == 0 && used > 0 && used + 3 < full) {
-    next = std::max(4, used + 3);
-  }
-  const bool dt_changed = P.from_features ? false : tune_dt(ctx, P);   // (behind the frame on its stream)
-  if (next == P.sort_levels && !dt_changed) return;
-  P.sort_levels = next;
+void tune_plan(geye_ctx *ctx, Plan &P) {
+  if (P.from_features || !tune_dt(ctx, P)) return;   // (behind the frame on its stream)
   cudaStreamSynchronize(ctx->stream);
   for (auto &g : P.graphs)
     if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
@@ -1049,8 +1030,8 @@ geye_status run_nms(geye_ctx *ctx, Plan &P, int n_models, float overlap) {
       launch_nms_batch(P.d_boxes.as<float>(), d_num, n_models, P.gl, overlap,
                        P.max_cap, P.d_nms_i.as<int>(),
                        P.d_nms_f.as<float>(), res, d_kept, err, reinterpret_cast<long long *>(d_num + 512),
-                       P.sort_levels, d_num + kSortLevelsUsed, d_num + kNmsNeed, ctx->nms_order,
-                       ctx->stream, (ctx->capturing && ctx->nms_if_node) ? ctx->aux : nullptr);
+                       d_num + kNmsNeed, ctx->nms_order, ctx->stream,
+                       (ctx->capturing && ctx->nms_if_node) ? ctx->aux : nullptr);
   if (ge != cudaSuccess) {
     set_error(std::string("nms graph nodes: ") + cudaGetErrorString(ge));
     return GEYE_ERR_CUDA;

@@ -115,13 +115,12 @@ void host_free(void *p);
 void host_pool_ref(int d);   // contexts come (+1) and go (-1)
 
 // Results of a frame in pinned host memory, written by the NMS kernels: ints [0, 32)
-// boxes before NMS per model, [32, 64) kept per model ([kSortLevelsUsed]: the sort
-// levels used), then per model point[4R], or_point[4R], type[R], scale[R], score[R]
+// boxes before NMS per model, [32, 64) kept per model, then per model point[4R], or_point[4R], type[R], scale[R], score[R]
 constexpr int kHostRes = 2048;
 inline size_t res_block_ints(int n_models) { return 64 + (size_t)n_models * 11 * kHostRes; }
 // model mi's result of the plan's finished frame (out: geye_result_free)
 geye_status read_result(Plan &P, int mi, geye_result *out);
-void note_sort_levels(geye_ctx *ctx, Plan &P, int used);
+void tune_plan(geye_ctx *ctx, Plan &P);
 
 struct LevelInfo {
   int img_h = 0, img_w = 0;   // image of this level (aliases for [interval, 2*interval))
@@ -241,10 +240,6 @@ struct Plan {
     int kernels = 0;
   };
   std::map<std::string, FrameGraph> graphs;
-  // grid-wide NMS sort levels launched per frame (0: the default for max_cap),
-  // adapted once to the depth the plan's frames need (note_sort_levels)
-  int sort_levels = 0;
-  bool sort_levels_fixed = false;
   void *h_res = nullptr;                // pinned result block (kHostRes)
   cudaEvent_t ev_done = nullptr;        // asynchronous submission (serve.cu): the frame's completion
   ~Plan() {
@@ -264,7 +259,7 @@ struct geye_ctx {
   // A_SCORE runs beside NMS on this stream (forked after the score stage,
   // joined before the frame ends)
   cudaStream_t side = nullptr;
-  // captures the bodies of the frame graph's conditional nodes (NMS rounds, quicksort pass)
+  // captures the body of the frame graph's conditional node (NMS in the quicksort's order)
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   geye_conv_mode conv_mode = GEYE_CONV_FP32;
@@ -279,8 +274,8 @@ struct geye_ctx {
   int launches = 0;
   bool use_graphs = true;   // replay the frame as a CUDA graph (GEYE_NO_GRAPHS=1 at creation: plain launches)
   int nms_order = geye::kNmsOrderKey;   // geye_ctx_set_nms_order
-  // the frame graph runs the NMS quicksort-order pass as an if node (a lone
-  // frame skips its launches when no model needs it); server slots and batch
+  // the frame graph runs the NMS in the quicksort's order of all boxes as an if node (a lone
+  // frame skips its launches when no model needs it); batch
   // lanes launch it plainly (its kernels return at once there), which measured
   // faster with frames of other contexts in flight
   bool nms_if_node = true;

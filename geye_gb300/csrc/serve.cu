@@ -66,12 +66,12 @@ static geye_status enqueue_frame(geye_ctx *ctx, Plan &P, float thresh, float ove
   return GEYE_OK;
 }
 
-// wait: the frame's own graph (submit and server slots; the plan's sort level
-// count may then adapt); false: a lane of a batch graph, already complete
+// wait: the frame's own graph (submit and server slots; the plan may then be
+// tuned); false: a lane of a batch graph, already complete
 static geye_status collect_frame(geye_ctx *ctx, geye_result *out, bool wait = true) {
   Plan &P = *ctx->pending;
   if (wait) CUDA_TRY(cudaEventSynchronize(P.ev_done));
-  if (wait) note_sort_levels(ctx, P, static_cast<const int *>(P.h_res)[kSortLevelsUsed]);
+  if (wait) tune_plan(ctx, P);
   geye_status st = GEYE_OK;
   for (size_t mi = 0; mi < P.models.size(); mi++) {
     const geye_status s = read_result(P, (int)mi, out ? &out[mi] : nullptr);
