@@ -1416,7 +1416,7 @@ geye_status geye_dt_tuning(geye_ctx *ctx, const geye_model *m, int *elems, float
   ARG_CHECK(ctx->last_plan, "no run yet");
   for (auto &mp : ctx->last_plan->models)
     if (mp->model == m) {
-      *elems = mp->dt_elems;
+      *elems = mp->dt->elems;
       for (int c = 0; c < 3; c++) ms[c] = mp->dt_ms[c];
       return GEYE_OK;
     }

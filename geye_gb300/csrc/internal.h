@@ -157,6 +157,8 @@ struct DtJob {             // one part map: DT of the negated map
   // ((x - par_x) / 2) * cm0 + (y - par_y) / 2, Ix/Iy likewise with the other
   // parity and ci0 rows (cm0 / ci0 = the class's rows; 0: full layout)
   int cm0, ci0;
+  int rng, n_rng;          // its chunks' value ranges (dt_block_lists)
+  int rows, parts;         // rows of a strip (dt_strip_rows); blocks of the map
 };
 
 struct ScoreJob {          // one (level, component) score map
@@ -290,13 +292,21 @@ size_t conv_fp32_blocks(std::vector<ConvJob> &jobs, std::vector<int2> &blocks);
 void launch_conv_fp32(const ConvJob *d_jobs, const int2 *d_blocks, int n_blocks, size_t smem, const float *d_bank,
                       const float *arena_in, float *arena_out, cudaStream_t s);
 // (job, first line) of every DT block, pass 1 (columns) and pass 2 (rows), largest maps first
-// DT tiles of about `elems` outputs per block (kDtElems by default; a plan
+// DT strips of about 2 * `elems` outputs per block (kDtElems by default; a plan
 // tunes it on its first frame's maps among kDtElemsChoices)
 constexpr int kDtElems = 2048;
 constexpr int kDtElemsChoices[3] = {1024, 2048, 4096};
-void dt_block_lists(const std::vector<DtJob> &jobs, std::vector<int2> &b1, std::vector<int2> &b2, int elems);
-void launch_dt(const DtJob *d_jobs, const int2 *d_b1, int n_b1, const int2 *d_b2, int n_b2, int max_d0, int max_d1,
-               float *arena, int *arena_i, int *fallback_count, int elems, cudaStream_t s);
+constexpr int kDtStageElems = 512;   // dt() itself: one map, over as many blocks as its strips allow
+struct DtBlocks {
+  std::vector<int2> chunks, strips;   // (job, first value), (job, first row)
+  int blocks = 0, rest_blocks = 0;    // the strips and, of a lone map, helpers in the general form; its second pass
+  size_t smem = 0, smem_rest = 0;     // shared memory of the strips, of the general form
+};
+void dt_strip_sizes(std::vector<DtJob> &jobs, int elems);   // the jobs' strips
+void dt_block_lists(std::vector<DtJob> &jobs, DtBlocks &B); // the blocks (their place among the chunks into the jobs)
+size_t dt_work_words(const DtBlocks &B);                    // ints of scratch, 16-byte aligned (without chunks the first is 0)
+cudaError_t launch_dt(const DtJob *d_jobs, const int2 *d_chunks, const int2 *d_strips, const DtBlocks &B, float *arena,
+                      int *arena_i, int *work, int *fallback_count, cudaStream_t s);
 // (job, block of 256 positions) of every score map, in job order
 void score_block_list(const std::vector<ScoreJob> &jobs, std::vector<int2> &blocks);
 void launch_score(const ScoreJob *d_jobs, const int2 *d_blocks, int n_blocks, float thresh, float *arena,

@@ -391,6 +391,25 @@ static geye_status conv_level(geye_ctx *ctx, Plan &P, ModelPlan &mp, ArenaAlloc 
   return GEYE_OK;
 }
 
+static geye_status plan_dt(geye_ctx *ctx, const ModelPlan &mp, int elems, std::unique_ptr<DtPlan> &out) {
+  auto D = std::make_unique<DtPlan>();
+  D->elems = elems;
+  D->jobs = mp.dt_jobs;
+  dt_strip_sizes(D->jobs, elems);
+  dt_block_lists(D->jobs, D->blocks);
+  GEYE_TRY(upload(ctx, D->d_jobs, D->jobs));
+  GEYE_TRY(upload(ctx, D->d_chunks, D->blocks.chunks));
+  GEYE_TRY(upload(ctx, D->d_strips, D->blocks.strips));
+  GEYE_TRY(D->d_work.alloc(ctx, sizeof(int) * dt_work_words(D->blocks)));
+  out = std::move(D);
+  return GEYE_OK;
+}
+
+static cudaError_t launch_plan_dt(geye_ctx *ctx, Plan &P, const DtPlan &D) {
+  return launch_dt(D.d_jobs.as<DtJob>(), D.d_chunks.as<int2>(), D.d_strips.as<int2>(), D.blocks, P.arena.as<float>(),
+                   P.arena.as<int>(), D.d_work.as<int>(), ctx->d_diag.as<int>(), ctx->stream);
+}
+
 static geye_status build_model_plan(geye_ctx *ctx, Plan &P, geye_model *mdl, int LEN_m, ArenaAlloc &A) {
   const HostModel &m = mdl->h;
   auto mp = std::make_unique<ModelPlan>();
@@ -493,15 +512,7 @@ static geye_status build_model_plan(geye_ctx *ctx, Plan &P, geye_model *mdl, int
     }
   }
   if (mp->dt_max_d0 > 1100 || mp->dt_max_d1 > 1100) { set_error("frame too large for the DT kernels"); return GEYE_ERR_UNSUPPORTED; }
-  GEYE_TRY(upload(ctx, mp->d_dt_jobs, mp->dt_jobs));
-  {
-    std::vector<int2> b1, b2;
-    dt_block_lists(mp->dt_jobs, b1, b2, mp->dt_elems);
-    mp->dt_nblocks1 = (int)b1.size();
-    mp->dt_nblocks2 = (int)b2.size();
-    GEYE_TRY(upload(ctx, mp->d_dt_blocks1, b1));
-    GEYE_TRY(upload(ctx, mp->d_dt_blocks2, b2));
-  }
+  GEYE_TRY(plan_dt(ctx, *mp, kDtElems, mp->dt));
   GEYE_TRY(upload(ctx, mp->d_score_jobs, mp->score_jobs));
   {
     std::vector<int2> sb;
@@ -879,9 +890,10 @@ geye_status run_conv(geye_ctx *ctx, Plan &P) {
 
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp) {
   if (mp.dt_jobs.empty()) return GEYE_OK;
-  launch_dt(mp.d_dt_jobs.as<DtJob>(), mp.d_dt_blocks1.as<int2>(), mp.dt_nblocks1, mp.d_dt_blocks2.as<int2>(),
-            mp.dt_nblocks2, mp.dt_max_d0, mp.dt_max_d1, P.arena.as<float>(),
-            P.arena.as<int>(), ctx->d_diag.as<int>(), mp.dt_elems, ctx->stream);
+  if (launch_plan_dt(ctx, P, *mp.dt) != cudaSuccess) {
+    set_error("dt launch");
+    return GEYE_ERR_CUDA;
+  }
   ctx->launches++;
   return check_launch(ctx, "dt");
 }
@@ -905,46 +917,26 @@ static bool tune_dt(geye_ctx *ctx, Plan &P) {
       return changed;
     }
     int best = -1;
-    float best_ms = 0.f;
-    std::vector<int2> keep1, keep2;
+    std::unique_ptr<DtPlan> trial[3];
     for (int c = 0; c < 3; c++) {
-      const int elems = kDtElemsChoices[c];
-      std::vector<int2> b1, b2;
-      dt_block_lists(mp.dt_jobs, b1, b2, elems);
-      DevBuf t1, t2;
-      if (upload(ctx, t1, b1) != GEYE_OK || upload(ctx, t2, b2) != GEYE_OK) break;
+      const bool own = kDtElemsChoices[c] == mp.dt->elems;
+      if (!own && plan_dt(ctx, mp, kDtElemsChoices[c], trial[c]) != GEYE_OK) break;
       float ms = 0.f;
-      for (int rep = 0; rep < 4; rep++) {
+      cudaError_t e = cudaSuccess;
+      for (int rep = 0; rep < 4 && e == cudaSuccess; rep++) {
         if (rep == 1) cudaEventRecord(e0, ctx->stream);
-        launch_dt(mp.d_dt_jobs.as<DtJob>(), t1.as<int2>(), (int)b1.size(), t2.as<int2>(), (int)b2.size(),
-                  mp.dt_max_d0, mp.dt_max_d1, P.arena.as<float>(), P.arena.as<int>(), ctx->d_diag.as<int>(), elems,
-                  ctx->stream);
+        e = launch_plan_dt(ctx, P, own ? *mp.dt : *trial[c]);
       }
       cudaEventRecord(e1, ctx->stream);
-      if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) break;
+      if (cudaEventSynchronize(e1) != cudaSuccess || e != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) break;
       mp.dt_ms[c] = ms / 3.0f;
-      if (best < 0 || mp.dt_ms[c] < best_ms) {
-        best = c;
-        best_ms = mp.dt_ms[c];
-        keep1 = b1;
-        keep2 = b2;
-      }
+      if (best < 0 || mp.dt_ms[c] < mp.dt_ms[best]) best = c;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaGetLastError();
-    if (best >= 0 && kDtElemsChoices[best] != mp.dt_elems) {
-      if (upload(ctx, mp.d_dt_blocks1, keep1) != GEYE_OK || upload(ctx, mp.d_dt_blocks2, keep2) != GEYE_OK) {
-        // the old lists may be gone: rebuild them for the old size
-        std::vector<int2> b1, b2;
-        dt_block_lists(mp.dt_jobs, b1, b2, mp.dt_elems);
-        upload(ctx, mp.d_dt_blocks1, b1);
-        upload(ctx, mp.d_dt_blocks2, b2);
-        continue;
-      }
-      mp.dt_elems = kDtElemsChoices[best];
-      mp.dt_nblocks1 = (int)keep1.size();
-      mp.dt_nblocks2 = (int)keep2.size();
+    if (best >= 0 && trial[best]) {
+      mp.dt = std::move(trial[best]);
       changed = true;
     }
   }

@@ -135,6 +135,14 @@ struct LevelInfo {
   int hist_off = -1;
 };
 
+// a model's distance transforms in strips of one size (tuned on the plan's first frame, tune_dt)
+struct DtPlan {
+  int elems = 0;
+  std::vector<DtJob> jobs;
+  DtBlocks blocks;
+  DevBuf d_jobs, d_chunks, d_strips, d_work;
+};
+
 struct ModelPlan {
   geye_model *model = nullptr;
   int LEN = 0;                          // levels this model uses
@@ -144,10 +152,8 @@ struct ModelPlan {
   int score_max_r = 0;
   int cap = 0;                          // max detections (sum of root map sizes)
   // device copies
-  DevBuf d_dt_jobs, d_score_jobs, d_counts;
-  DevBuf d_dt_blocks1, d_dt_blocks2;    // DT tiles of every map (dt_block_lists)
-  int dt_nblocks1 = 0, dt_nblocks2 = 0;
-  int dt_elems = kDtElems;              // outputs per DT block: tuned on the plan's first frame (tune_dt)
+  DevBuf d_score_jobs, d_counts;
+  std::unique_ptr<DtPlan> dt;
   bool dt_tuned = false;
   float dt_ms[3] = {0, 0, 0};           // the timed launch per kDtElemsChoices entry
   DevBuf d_score_blocks;                // score / box blocks of every map (score_block_list)

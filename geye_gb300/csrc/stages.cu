@@ -389,13 +389,17 @@ geye_status geye_dt(geye_ctx *ctx, const float *vals, float ax, float bx, float 
   J.in_off = 0; J.d0 = d0; J.d1 = d1;
   J.tmpM_off = (int)np; J.tmpI_off = (int)(2 * np); J.M_off = (int)(3 * np); J.Ix_off = (int)(4 * np); J.Iy_off = (int)(5 * np);
   J.ax = ax; J.bx = bx; J.ay = ay; J.by = by; J.negate = 0;
-  std::vector<int2> b1, b2;
-  dt_block_lists(std::vector<DtJob>{J}, b1, b2, kDtElems);
+  std::vector<DtJob> jobs{J};
+  DtBlocks B;
+  dt_strip_sizes(jobs, kDtStageElems);
+  dt_block_lists(jobs, B);
+  const std::vector<int> work(dt_work_words(B), 0);
   Tables T;
-  const size_t o_j = T.add(&J, 1), o_1 = T.add(b1.data(), b1.size()), o_2 = T.add(b2.data(), b2.size());
+  const size_t o_j = T.add(jobs.data(), 1), o_1 = T.add(B.chunks.data(), B.chunks.size()), o_2 = T.add(B.strips.data(), B.strips.size()),
+               o_w = T.add(work.data(), work.size());
   GEYE_TRY(T.put(S));
-  launch_dt(T.at<DtJob>(o_j), T.at<int2>(o_1), (int)b1.size(), T.at<int2>(o_2), (int)b2.size(), d0, d1, arena, reinterpret_cast<int *>(arena),
-            ctx->d_diag.as<int>(), kDtElems, ctx->stream);
+  CUDA_TRY(launch_dt(T.at<DtJob>(o_j), T.at<int2>(o_1), T.at<int2>(o_2), B, arena, reinterpret_cast<int *>(arena), T.at<int>(o_w),
+                     ctx->d_diag.as<int>(), ctx->stream));
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(M, arena + 3 * np, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaMemcpyAsync(Ix, arena + 4 * np, sizeof(int) * n, cudaMemcpyDeviceToHost, ctx->stream));
