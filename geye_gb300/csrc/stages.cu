@@ -67,6 +67,7 @@ static void taps(int sheight, int dheight, std::vector<int> &start, std::vector<
   // resize.cc:68-105, grouped by destination index (same as the plan builder)
   float scale = (float)dheight / (float)sheight;
   float invscale = (float)sheight / (float)dheight;
+  const size_t first = si.size();
   for (int dy = 0; dy < dheight; dy++) {
     start.push_back((int)si.size());
     float fsy1 = dy * invscale;
@@ -80,7 +81,8 @@ static void taps(int sheight, int dheight, std::vector<int> &start, std::vector<
   start.push_back((int)si.size());
   // float rounding could name a source row one past the end (the reference
   // would read past its buffer); keep every read inside the image
-  for (auto &v : si) v = std::min(std::max(v, 0), sheight - 1);
+  // (of this call's taps: si may hold another axis's before them)
+  for (size_t k = first; k < si.size(); k++) si[k] = std::min(std::max(si[k], 0), sheight - 1);
 }
 
 extern "C" {
