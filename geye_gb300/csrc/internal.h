@@ -54,13 +54,13 @@ inline cudaError_t raise_smem(SmemAttr &A, K *kernel, size_t smem) {
 // ----------------------------------------------------------------------------
 // job descriptors (device-readable, plain structs)
 // ----------------------------------------------------------------------------
-struct ResizeJob {         // one 1-D resize pass of one level
-  int src_off;             // float offset of the source planes
+struct ResizeJob {         // one level from its source image: along y, then along x
+  int src_off;             // float offset of the source planes [3][src_w][src_h]
   int dst_off;             // float offset of the destination planes
-  int src_h, src_w;        // source dims (rows, cols)
-  int dst_h, dst_w;        // destination dims of this pass
-  int tap_start_off;       // int offset of tap_start[dst_len + 1] in the tap-index table
-  int tap_off;             // offset of the tap (si, alpha) arrays
+  int src_h, src_w;
+  int dst_h, dst_w;
+  int v_start_off, v_tap_off;   // offsets of tap_start[dst_h + 1] and of the tap (si, alpha) arrays, along y
+  int h_start_off, h_tap_off;   // along x
 };
 
 struct HogJob {
@@ -242,8 +242,12 @@ namespace geye {
 // ----------------------------------------------------------------------------
 void launch_fill(float *p, size_t n, float v, cudaStream_t s);
 void launch_ingest(const uint8_t *bgr, int width, int height, int width_step, float *planes, cudaStream_t s);
-void launch_resize_pass(const ResizeJob *d_jobs, int n_jobs, int max_cols, int vertical, const int *d_tap_start,
-                        const int *d_tap_si, const float *d_tap_alpha, float *arena, cudaStream_t s);
+// the blocks of a job's resize (kResizeWarps warps each)
+int resize_blocks(const ResizeJob &J);
+int resize_items(const ResizeJob &J);   // its tiles, a warp each
+// max_blocks: the largest of the jobs' resize_blocks
+void launch_resize(const ResizeJob *d_jobs, int n_jobs, int max_blocks, const int *d_tap_start,
+                   const int *d_tap_si, const float *d_tap_alpha, float *arena, cudaStream_t s);
 // (job, block of histogram blocks) of every level's vote kernel
 void hog_vote_blocks(const std::vector<HogJob> &jobs, std::vector<int2> &blocks);
 
@@ -259,7 +263,7 @@ struct BatchFrame {
   uint8_t *arena16;
   int img0_off;            // level-0 image planes (ingest output)
   int n_phases;
-  const ResizeJob *vjobs[kBatchMaxPhases], *hjobs[kBatchMaxPhases];
+  const ResizeJob *rjobs[kBatchMaxPhases];
   const int *tap_start, *tap_si;
   const float *tap_alpha;
   const HogPixJob *pix;
@@ -269,8 +273,9 @@ struct BatchFrame {
 struct BatchItem {
   int frame, job, chunk, pad;
 };
-enum BatchStage { kBatchIngest = 0, kBatchResizeV, kBatchResizeH, kBatchPix, kBatchVote, kBatchNorm, kBatchFeat };
-constexpr int kBatchColumns = 8;   // resize / pixel columns per item (a warp each)
+enum BatchStage { kBatchIngest = 0, kBatchResize, kBatchPix, kBatchVote, kBatchNorm, kBatchFeat };
+constexpr int kBatchColumns = 8;   // pixel columns per item (a warp each)
+constexpr int kBatchTiles = 8;     // resize tiles per item (a warp each)
 constexpr int kBatchCells = 256;   // corners / cells per item (a thread each)
 // one stage (phase: the resize phase) over n items
 void launch_batch_front(int stage, const BatchFrame *d_frames, const BatchItem *d_items, int n, int phase,
@@ -291,7 +296,6 @@ bool conv_fp32_jobs(ConvJob J, const std::vector<const float *> &filters, const 
 size_t conv_fp32_blocks(std::vector<ConvJob> &jobs, std::vector<int2> &blocks);
 void launch_conv_fp32(const ConvJob *d_jobs, const int2 *d_blocks, int n_blocks, size_t smem, const float *d_bank,
                       const float *arena_in, float *arena_out, cudaStream_t s);
-// (job, first line) of every DT block, pass 1 (columns) and pass 2 (rows), largest maps first
 // DT strips of about 2 * `elems` outputs per block (kDtElems by default; a plan
 // tunes it on its first frame's maps among kDtElemsChoices)
 constexpr int kDtElems = 2048;

@@ -63,110 +63,144 @@ void launch_ingest(const uint8_t *bgr, int width, int height, int width_step, fl
 }
 
 // ----------------------------------------------------------------------------
-// resize: one 1-D pass over all jobs of a phase.  Taps for destination index d
-// are tap_si/tap_alpha[tap_start[d] .. tap_start[d+1]) in the reference's order.
-// vertical: out[c][x][d] = sum alpha * src[c][x][si]     (src h -> dst h, same w)
-// horizontal: out[c][d][y] = sum alpha * src[c][si][y]   (src w -> dst w, same h)
-// A warp owns one column x of the output (all three channels), lanes along y:
-// no index division per element, and each tap is loaded once for the three
-// channels (vertical) or once per column (horizontal).
+// resize: all levels of a phase, the pass along y and the one along x together.
+// Taps for destination index d are tap_si/tap_alpha[tap_start[d] .. tap_start[d+1])
+// in the reference's order:
+//   v[c][x][d] = sum alpha * src[c][x][si]   (src h -> dst h),
+//   out[c][d][y] = sum alpha * v[c][si][y]   (src w -> dst w).
+// A warp owns 32 rows of kResizeCols output columns, a row per lane: a row's taps
+// along y stay in registers, the source columns are walked in order, each one's
+// sum along y is formed once and goes to the outputs that it belongs to (two, at a
+// boundary), and the taps along x, the same for all lanes, are held one per lane.  Four columns'
+// loads are in flight.  What bounds it is latency, and the L1 in large frames.
+// As two kernels, with v through memory and every lane reading the taps of each of its
+// outputs, ingest and resize took 36 us for 320x240 (28 so), 640x480 73 (57),
+// 1280x720 150 (96), 1920x1080 267 (172); one column at a time in flight 36, 71, 117, 192.
 // ----------------------------------------------------------------------------
 constexpr int kResizeWarps = 4;
+constexpr int kResizeCols = 8;
+constexpr int kResizeTaps = 3;    // a row's taps along y in registers (scales of a half and more)
+constexpr int kResizeAhead = 4;   // source columns in flight
 
-// output column x of one pass (all three channels) by one warp
-__device__ __forceinline__ void resize_column(const ResizeJob &J, int vertical, const int *__restrict__ tap_start,
-                                              const int *__restrict__ tap_si, const float *__restrict__ tap_alpha,
-                                              float *__restrict__ arena, int x) {
-  const float *src = arena + J.src_off;
-  float *dst = arena + J.dst_off;
-  const int *ts = tap_start + J.tap_start_off;
-  const int *si = tap_si + J.tap_off;
-  const float *al = tap_alpha + J.tap_off;
+// the item'th (32 rows, kResizeCols columns) of a job, by one warp
+__device__ __forceinline__ void resize_tile(const ResizeJob &J, const int *__restrict__ tap_start,
+                                            const int *__restrict__ tap_si, const float *__restrict__ tap_alpha,
+                                            float *__restrict__ arena, int item) {
   const int lane = threadIdx.x & 31;
-  const size_t src_plane = (size_t)J.src_w * J.src_h, dst_plane = (size_t)J.dst_w * J.dst_h;
-  {
-    float *out = dst + (size_t)x * J.dst_h;
-    if (vertical) {
-      const float *col = src + (size_t)x * J.src_h;
-      for (int y = lane; y < J.dst_h; y += 64) {   // two outputs per lane in flight
-        const int y2 = y + 32;
-        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
-        const int t1 = ts[y + 1];
-        const int u0 = y2 < J.dst_h ? ts[y2] : 0, u1 = y2 < J.dst_h ? ts[y2 + 1] : 0;
-#pragma unroll 4
-        for (int t = ts[y]; t < t1; t++) {
-          const float w = al[t];
-          const float *p = col + si[t];
-          a0 += w * p[0];
-          a1 += w * p[src_plane];
-          a2 += w * p[2 * src_plane];
-        }
-#pragma unroll 4
-        for (int t = u0; t < u1; t++) {
-          const float w = al[t];
-          const float *p = col + si[t];
-          c0 += w * p[0];
-          c1 += w * p[src_plane];
-          c2 += w * p[2 * src_plane];
-        }
-        out[y] = a0;
-        out[dst_plane + y] = a1;
-        out[2 * dst_plane + y] = a2;
-        if (y2 < J.dst_h) {
-          out[y2] = c0;
-          out[dst_plane + y2] = c1;
-          out[2 * dst_plane + y2] = c2;
-        }
-      }
-    } else {
-      // taps are uniform along the column: two outputs per lane in flight
-      const int t0 = ts[x], t1 = ts[x + 1];
-      for (int y = lane; y < J.dst_h; y += 64) {
-        const bool two = y + 32 < J.dst_h;
-        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f;
-        for (int t = t0; t < t1; t++) {
-          const float w = al[t];
-          const float *p = src + (size_t)si[t] * J.src_h + y;
-          a0 += w * p[0];
-          a1 += w * p[src_plane];
-          a2 += w * p[2 * src_plane];
-          if (two) {
-            b0 += w * p[32];
-            b1 += w * p[src_plane + 32];
-            b2 += w * p[2 * src_plane + 32];
+  const int ny = (J.dst_h + 31) >> 5, xs = item / ny, y = 32 * (item - xs * ny) + lane;
+  const int x0 = xs * kResizeCols, x1 = min(x0 + kResizeCols, J.dst_w);
+  if (x0 >= J.dst_w) return;
+  const float *src = arena + J.src_off;
+  float *out = arena + J.dst_off + (size_t)x0 * J.dst_h + y;
+  const size_t plane = (size_t)J.src_w * J.src_h, dst_plane = (size_t)J.dst_w * J.dst_h;
+  const bool live = y < J.dst_h;
+  const int *vsi = tap_si + J.v_tap_off, *hsi = tap_si + J.h_tap_off;
+  const float *val = tap_alpha + J.v_tap_off, *hal = tap_alpha + J.h_tap_off;
+  const int *vs = tap_start + J.v_start_off + min(y, J.dst_h - 1), *hs = tap_start + J.h_start_off;
+  const int t0 = vs[0], n = vs[1] - t0, u0 = hs[x0], nu = hs[x1] - u0;   // (every output has a tap)
+  float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+  auto store = [&]() {   // an output column is complete
+    if (live) {
+      out[0] = a0;
+      out[dst_plane] = a1;
+      out[2 * dst_plane] = a2;
+    }
+    out += J.dst_h;
+    a0 = a1 = a2 = 0.0f;
+  };
+  // the columns' taps along x, one per lane; their source columns ascend (the last one again beyond them)
+  const int ts = hsi[u0 + max(min(lane, nu - 1), 0)], te = hs[min(x0 + lane + 1, x1)] - u0;
+  const int ts_before = __shfl_up_sync(0xffffffffu, ts, 1), te_before = __shfl_up_sync(0xffffffffu, te, 1);
+  const bool in_order = (lane == 0 || ts_before <= ts) && (lane >= x1 - x0 || te > (lane == 0 ? 0 : te_before));
+  if (nu <= 32 && __all_sync(0xffffffffu, n <= kResizeTaps && in_order)) {
+    const float ta = lane < nu ? hal[u0 + lane] : 0.0f;
+    int o[kResizeTaps];
+    float w[kResizeTaps];
+#pragma unroll
+    for (int k = 0; k < kResizeTaps; k++) {
+      o[k] = k < n ? vsi[t0 + k] : 0;
+      w[k] = k < n ? val[t0 + k] : 0.0f;
+    }
+    const int s1 = __shfl_sync(0xffffffffu, ts, nu - 1);
+    int x = 0, t = 0, end = __shfl_sync(0xffffffffu, te, 0), next = __shfl_sync(0xffffffffu, ts, 0);
+    for (int s = next; s <= s1; s += kResizeAhead) {
+      float p[kResizeAhead][kResizeTaps][3];
+#pragma unroll
+      for (int b = 0; b < kResizeAhead; b++) {
+        const float *col = src + (size_t)min(s + b, s1) * J.src_h;
+#pragma unroll
+        for (int k = 0; k < kResizeTaps; k++)
+          if (k < n) {
+            p[b][k][0] = col[o[k]];
+            p[b][k][1] = col[plane + o[k]];
+            p[b][k][2] = col[2 * plane + o[k]];
           }
-        }
-        out[y] = a0;
-        out[dst_plane + y] = a1;
-        out[2 * dst_plane + y] = a2;
-        if (two) {
-          out[y + 32] = b0;
-          out[dst_plane + y + 32] = b1;
-          out[2 * dst_plane + y + 32] = b2;
+      }
+#pragma unroll
+      for (int b = 0; b < kResizeAhead; b++) {
+        float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+#pragma unroll
+        for (int k = 0; k < kResizeTaps; k++)
+          if (k < n) {
+            v0 += w[k] * p[b][k][0];
+            v1 += w[k] * p[b][k][1];
+            v2 += w[k] * p[b][k][2];
+          }
+        while (t < nu && next == s + b) {   // the taps on this column (every lane alike)
+          const float wx = __shfl_sync(0xffffffffu, ta, t);
+          a0 += wx * v0;
+          a1 += wx * v1;
+          a2 += wx * v2;
+          next = __shfl_sync(0xffffffffu, ts, ++t & 31);
+          if (t == end) {
+            store();
+            end = __shfl_sync(0xffffffffu, te, ++x & 31);
+          }
         }
       }
     }
+    return;
+  }
+  for (int x = x0; x < x1; x++) {   // any scale
+    const int ue = hs[x + 1];
+    for (int u = hs[x]; u < ue; u++) {
+      const float *col = src + (size_t)hsi[u] * J.src_h;
+      const float wx = hal[u];
+      float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+      for (int k = t0; k < t0 + n; k++) {
+        const float *p = col + vsi[k];
+        const float wk = val[k];
+        v0 += wk * p[0];
+        v1 += wk * p[plane];
+        v2 += wk * p[2 * plane];
+      }
+      a0 += wx * v0;
+      a1 += wx * v1;
+      a2 += wx * v2;
+    }
+    store();
   }
 }
 
-__global__ void __launch_bounds__(kResizeWarps * 32) k_resize_pass(const ResizeJob *__restrict__ jobs, int vertical,
-                                                                   const int *__restrict__ tap_start,
-                                                                   const int *__restrict__ tap_si,
-                                                                   const float *__restrict__ tap_alpha,
-                                                                   float *__restrict__ arena) {
+__global__ void __launch_bounds__(kResizeWarps * 32) k_resize(const ResizeJob *__restrict__ jobs,
+                                                              const int *__restrict__ tap_start,
+                                                              const int *__restrict__ tap_si,
+                                                              const float *__restrict__ tap_alpha,
+                                                              float *__restrict__ arena) {
   const ResizeJob J = jobs[blockIdx.y];
-  for (int x = blockIdx.x * kResizeWarps + (threadIdx.x >> 5); x < J.dst_w; x += gridDim.x * kResizeWarps)
-    resize_column(J, vertical, tap_start, tap_si, tap_alpha, arena, x);
+  resize_tile(J, tap_start, tap_si, tap_alpha, arena, blockIdx.x * kResizeWarps + (threadIdx.x >> 5));
 }
 
-// max_cols: the largest output column count (dst_w) of the phase's jobs
-void launch_resize_pass(const ResizeJob *d_jobs, int n_jobs, int max_cols, int vertical, const int *d_tap_start,
-                        const int *d_tap_si, const float *d_tap_alpha, float *arena, cudaStream_t s) {
-  if (n_jobs <= 0) return;
-  int bx = (max_cols + kResizeWarps - 1) / kResizeWarps;
-  if (bx > 1024) bx = 1024;
-  dim3 grid(bx, n_jobs);
-  k_resize_pass<<<grid, kResizeWarps * 32, 0, s>>>(d_jobs, vertical, d_tap_start, d_tap_si, d_tap_alpha, arena);
+int resize_items(const ResizeJob &J) {
+  return ((J.dst_h + 31) / 32) * ((J.dst_w + kResizeCols - 1) / kResizeCols);
+}
+
+int resize_blocks(const ResizeJob &J) { return (resize_items(J) + kResizeWarps - 1) / kResizeWarps; }
+
+void launch_resize(const ResizeJob *d_jobs, int n_jobs, int max_blocks, const int *d_tap_start, const int *d_tap_si,
+                   const float *d_tap_alpha, float *arena, cudaStream_t s) {
+  if (n_jobs <= 0 || max_blocks <= 0) return;
+  k_resize<<<dim3(max_blocks, n_jobs), kResizeWarps * 32, 0, s>>>(d_jobs, d_tap_start, d_tap_si, d_tap_alpha, arena);
 }
 
 // ----------------------------------------------------------------------------
@@ -506,10 +540,9 @@ __global__ void __launch_bounds__(256) k_batch_front(const BatchFrame *__restric
     if (STAGE == kBatchIngest) {
       ingest_tile(F.bgr, F.width, F.height, F.width_step, F.arena + F.img0_off, 32 * I.job, 32 * I.chunk, tid & 31,
                   warp, reinterpret_cast<float (*)[32][33]>(sm));
-    } else if (STAGE == kBatchResizeV || STAGE == kBatchResizeH) {
-      const ResizeJob J = (STAGE == kBatchResizeV ? F.vjobs[phase] : F.hjobs[phase])[I.job];
-      const int x = I.chunk * kBatchColumns + warp;
-      if (x < J.dst_w) resize_column(J, STAGE == kBatchResizeV, F.tap_start, F.tap_si, F.tap_alpha, F.arena, x);
+    } else if (STAGE == kBatchResize) {
+      const ResizeJob J = F.rjobs[phase][I.job];
+      resize_tile(J, F.tap_start, F.tap_si, F.tap_alpha, F.arena, I.chunk * kBatchTiles + warp);   // (past the job's last one: nothing)
     } else if (STAGE == kBatchPix) {
       const HogPixJob J = F.pix[I.job];
       const int x = 1 + I.chunk * kBatchColumns + warp;
@@ -538,8 +571,7 @@ void launch_batch_front(int stage, const BatchFrame *d_frames, const BatchItem *
   const int grid = std::max(1, std::min(n, 4 * std::max(sms, 1)));   // persistent: a few CTAs per SM
   switch (stage) {
     case kBatchIngest: k_batch_front<kBatchIngest><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;
-    case kBatchResizeV: k_batch_front<kBatchResizeV><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;
-    case kBatchResizeH: k_batch_front<kBatchResizeH><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;
+    case kBatchResize: k_batch_front<kBatchResize><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;
     case kBatchPix: k_batch_front<kBatchPix><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;
     case kBatchVote: k_batch_front<kBatchVote><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;
     case kBatchNorm: k_batch_front<kBatchNorm><<<grid, 256, 0, s>>>(d_frames, d_items, n, phase); break;

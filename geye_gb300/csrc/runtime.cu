@@ -566,51 +566,43 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
   // resize phases: phase 0 = base levels 1..interval-1 from level 0; phase k>=1 = octave k+1
   std::vector<int> tstart, tsi;
   std::vector<float> talpha;
-  auto add_job = [&](std::vector<ResizeJob> &vj, std::vector<ResizeJob> &hj, int &vmax, int &hmax, int src_level,
-                     int dst_level) {
-    const LevelInfo &S = P.lv[src_level];
-    LevelInfo &D = P.lv[dst_level];
-    const int tmp = A.take((size_t)3 * D.img_h * S.img_w);
-    ResizeJob v{};
-    v.src_off = S.img_off; v.dst_off = tmp; v.src_h = S.img_h; v.src_w = S.img_w; v.dst_h = D.img_h; v.dst_w = S.img_w;
-    v.tap_start_off = (int)tstart.size(); v.tap_off = (int)tsi.size();
-    {
-      std::vector<int> st, si; std::vector<float> al;
-      build_taps(S.img_h, D.img_h, st, si, al);
-      for (auto &x : st) tstart.push_back(x);
-      tsi.insert(tsi.end(), si.begin(), si.end());
-      talpha.insert(talpha.end(), al.begin(), al.end());
-    }
-    ResizeJob h{};
-    h.src_off = tmp; h.dst_off = D.img_off; h.src_h = D.img_h; h.src_w = S.img_w; h.dst_h = D.img_h; h.dst_w = D.img_w;
-    h.tap_start_off = (int)tstart.size(); h.tap_off = (int)tsi.size();
-    {
-      std::vector<int> st, si; std::vector<float> al;
-      build_taps(S.img_w, D.img_w, st, si, al);
-      for (auto &x : st) tstart.push_back(x);
-      tsi.insert(tsi.end(), si.begin(), si.end());
-      talpha.insert(talpha.end(), al.begin(), al.end());
-    }
-    vj.push_back(v);
-    hj.push_back(h);
-    vmax = std::max(vmax, v.dst_w);   // output columns: one warp each
-    hmax = std::max(hmax, h.dst_w);
-    P.bytes_resize += 4.0 * 3 * (S.img_h * S.img_w + D.img_h * S.img_w) + 4.0 * 3 * (D.img_h * S.img_w + D.img_h * D.img_w);
+  auto add_taps = [&](int src, int dst, int &start_off, int &tap_off) {
+    start_off = (int)tstart.size();
+    tap_off = (int)tsi.size();
+    std::vector<int> st, si;
+    std::vector<float> al;
+    build_taps(src, dst, st, si, al);
+    tstart.insert(tstart.end(), st.begin(), st.end());
+    tsi.insert(tsi.end(), si.begin(), si.end());
+    talpha.insert(talpha.end(), al.begin(), al.end());
+  };
+  auto add_job = [&](std::vector<ResizeJob> &jobs, int src_level, int dst_level) {
+    const LevelInfo &S = P.lv[src_level], &D = P.lv[dst_level];
+    ResizeJob J{};
+    J.src_off = S.img_off; J.dst_off = D.img_off; J.src_h = S.img_h; J.src_w = S.img_w; J.dst_h = D.img_h; J.dst_w = D.img_w;
+    add_taps(S.img_h, D.img_h, J.v_start_off, J.v_tap_off);
+    add_taps(S.img_w, D.img_w, J.h_start_off, J.h_tap_off);
+    jobs.push_back(J);
+    P.bytes_resize += 4.0 * 3 * (S.img_h * S.img_w + D.img_h * D.img_w);
+  };
+  auto add_phase = [&](const std::vector<ResizeJob> &jobs) {
+    int most = 0;
+    for (const ResizeJob &J : jobs) most = std::max(most, resize_blocks(J));
+    P.rjobs.push_back(jobs);
+    P.r_max_blocks.push_back(most);
   };
   {
-    std::vector<ResizeJob> vj, hj;
-    int vm = 0, hm = 0;
+    std::vector<ResizeJob> jobs;
     for (int ii = 1; ii < interval && ii < LEN; ii++) {
       if (P.lv[ii].img_h == P.lv[0].img_h && P.lv[ii].img_w == P.lv[0].img_w && 1.0 / pow(sc, ii) == 1.0) continue;
-      add_job(vj, hj, vm, hm, 0, ii);
+      add_job(jobs, 0, ii);
     }
-    P.vjobs.push_back(vj); P.hjobs.push_back(hj); P.v_max_items.push_back(vm); P.h_max_items.push_back(hm);
+    add_phase(jobs);
   }
   for (int base = 2 * interval; base < LEN; base += interval) {
-    std::vector<ResizeJob> vj, hj;
-    int vm = 0, hm = 0;
-    for (int l = base; l < std::min(base + interval, LEN); l++) add_job(vj, hj, vm, hm, P.lv[l - interval].img_level, l);
-    P.vjobs.push_back(vj); P.hjobs.push_back(hj); P.v_max_items.push_back(vm); P.h_max_items.push_back(hm);
+    std::vector<ResizeJob> jobs;
+    for (int l = base; l < std::min(base + interval, LEN); l++) add_job(jobs, P.lv[l - interval].img_level, l);
+    add_phase(jobs);
   }
   P.bytes_resize += (double)3 * width * height + 12.0 * width * height;   // ingest
   // HOG
@@ -682,12 +674,8 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
   GEYE_TRY(upload(ctx, P.d_tap_start, tstart));
   GEYE_TRY(upload(ctx, P.d_tap_si, tsi));
   GEYE_TRY(upload(ctx, P.d_tap_alpha, talpha));
-  P.d_vjobs.resize(P.vjobs.size());
-  P.d_hjobs.resize(P.hjobs.size());
-  for (size_t i = 0; i < P.vjobs.size(); i++) {
-    GEYE_TRY(upload(ctx, P.d_vjobs[i], P.vjobs[i]));
-    GEYE_TRY(upload(ctx, P.d_hjobs[i], P.hjobs[i]));
-  }
+  P.d_rjobs.resize(P.rjobs.size());
+  for (size_t i = 0; i < P.rjobs.size(); i++) GEYE_TRY(upload(ctx, P.d_rjobs[i], P.rjobs[i]));
   GEYE_TRY(upload(ctx, P.d_hog_jobs, P.hog_jobs));
   {
     std::vector<int2> vb;
@@ -853,14 +841,11 @@ geye_status run_ingest(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_s
 geye_status run_resize(geye_ctx *ctx, Plan &P) {
   cudaStream_t s = ctx->stream;
   float *arena = P.arena.as<float>();
-  for (size_t ph = 0; ph < P.vjobs.size(); ph++) {
-    if (P.vjobs[ph].empty()) continue;
-    launch_resize_pass(P.d_vjobs[ph].as<ResizeJob>(), (int)P.vjobs[ph].size(), P.v_max_items[ph], 1,
-                       P.d_tap_start.as<int>(), P.d_tap_si.as<int>(), P.d_tap_alpha.as<float>(), arena, s);
-    GEYE_TRY(check_launch(ctx, "resize (vertical)"));
-    launch_resize_pass(P.d_hjobs[ph].as<ResizeJob>(), (int)P.hjobs[ph].size(), P.h_max_items[ph], 0,
-                       P.d_tap_start.as<int>(), P.d_tap_si.as<int>(), P.d_tap_alpha.as<float>(), arena, s);
-    GEYE_TRY(check_launch(ctx, "resize (horizontal)"));
+  for (size_t ph = 0; ph < P.rjobs.size(); ph++) {
+    if (P.rjobs[ph].empty()) continue;
+    launch_resize(P.d_rjobs[ph].as<ResizeJob>(), (int)P.rjobs[ph].size(), P.r_max_blocks[ph], P.d_tap_start.as<int>(),
+                  P.d_tap_si.as<int>(), P.d_tap_alpha.as<float>(), arena, s);
+    GEYE_TRY(check_launch(ctx, "resize"));
   }
   return GEYE_OK;
 }

@@ -210,9 +210,9 @@ struct Plan {
   bool from_features = false;
   std::vector<LevelInfo> lv;
   // resize phases: each phase is two passes (vertical then horizontal)
-  std::vector<std::vector<ResizeJob>> vjobs, hjobs;
-  std::vector<int> v_max_items, h_max_items;   // per phase: largest output column count
-  std::vector<DevBuf> d_vjobs, d_hjobs;
+  std::vector<std::vector<ResizeJob>> rjobs;
+  std::vector<int> r_max_blocks;       // per phase: the largest job's
+  std::vector<DevBuf> d_rjobs;
   DevBuf d_tap_start, d_tap_si, d_tap_alpha;
   std::vector<HogJob> hog_jobs;
   DevBuf d_hog_jobs;

@@ -575,24 +575,23 @@ namespace {
 
 // The batched front end's tables for one batch key: every frame's plan
 // pointers and, per stage, the ragged list of (frame, job, chunk) items,
-// in one device buffer that the batch graph reads.  Lists: ingest, vertical
-// and horizontal resize per phase, pixels, votes, corner norms, features.
+// in one device buffer that the batch graph reads.  Lists: ingest,
+// resize per phase, pixels, votes, corner norms, features.
 int front_list(int stage, int phase) {   // list index of a stage (resize: per phase)
   if (stage == kBatchIngest) return 0;
-  if (stage == kBatchResizeV) return 1 + 2 * phase;
-  if (stage == kBatchResizeH) return 2 + 2 * phase;
-  return 1 + 2 * kBatchMaxPhases + (stage - kBatchPix);
+  if (stage == kBatchResize) return 1 + phase;
+  return 1 + kBatchMaxPhases + (stage - kBatchPix);
 }
 
 geye_status batch_front_tables(geye_batch *b, const std::vector<Plan *> &plans, geye_batch::Graph &g) {
   const int nf = (int)plans.size();
-  const int n_lists = 1 + 2 * kBatchMaxPhases + 4;
+  const int n_lists = 1 + kBatchMaxPhases + 4;
   std::vector<std::vector<BatchItem>> L(n_lists);
   std::vector<BatchFrame> fr(nf);
   int max_ph = 0;
   for (int f = 0; f < nf; f++) {
     const Plan &P = *plans[f];
-    ARG_CHECK((int)P.vjobs.size() <= kBatchMaxPhases, "batch: too many resize phases");
+    ARG_CHECK((int)P.rjobs.size() <= kBatchMaxPhases, "batch: too many resize phases");
     BatchFrame &F = fr[f];
     F = BatchFrame{};
     F.bgr = P.d_bgr.as<uint8_t>();
@@ -602,11 +601,8 @@ geye_status batch_front_tables(geye_batch *b, const std::vector<Plan *> &plans, 
     F.arena = P.arena.as<float>();
     F.arena16 = static_cast<uint8_t *>(P.arena16.p);
     F.img0_off = P.lv[0].img_off;
-    F.n_phases = (int)P.vjobs.size();
-    for (int ph = 0; ph < F.n_phases; ph++) {
-      F.vjobs[ph] = P.d_vjobs[ph].as<ResizeJob>();
-      F.hjobs[ph] = P.d_hjobs[ph].as<ResizeJob>();
-    }
+    F.n_phases = (int)P.rjobs.size();
+    for (int ph = 0; ph < F.n_phases; ph++) F.rjobs[ph] = P.d_rjobs[ph].as<ResizeJob>();
     F.tap_start = P.d_tap_start.as<int>();
     F.tap_si = P.d_tap_si.as<int>();
     F.tap_alpha = P.d_tap_alpha.as<float>();
@@ -617,12 +613,9 @@ geye_status batch_front_tables(geye_batch *b, const std::vector<Plan *> &plans, 
     for (int ty = 0; ty < (P.height + 31) / 32; ty++)
       for (int tx = 0; tx < (P.width + 31) / 32; tx++) L[0].push_back(BatchItem{f, tx, ty, 0});
     for (int ph = 0; ph < F.n_phases; ph++)
-      for (size_t j = 0; j < P.vjobs[ph].size(); j++) {
-        for (int c = 0; c * kBatchColumns < P.vjobs[ph][j].dst_w; c++)
-          L[front_list(kBatchResizeV, ph)].push_back(BatchItem{f, (int)j, c, 0});
-        for (int c = 0; c * kBatchColumns < P.hjobs[ph][j].dst_w; c++)
-          L[front_list(kBatchResizeH, ph)].push_back(BatchItem{f, (int)j, c, 0});
-      }
+      for (size_t j = 0; j < P.rjobs[ph].size(); j++)
+        for (int c = 0; c * kBatchTiles < resize_items(P.rjobs[ph][j]); c++)
+          L[front_list(kBatchResize, ph)].push_back(BatchItem{f, (int)j, c, 0});
     for (size_t j = 0; j < P.pix_jobs.size(); j++)
       for (int c = 0; 1 + c * kBatchColumns < P.pix_jobs[j].xe; c++)
         L[front_list(kBatchPix, 0)].push_back(BatchItem{f, (int)j, c, 0});
@@ -671,10 +664,7 @@ void launch_batch_tables(geye_batch *b, geye_batch::Graph &g) {
     launch_batch_front(stage, frames, items + g.offset[l], g.count[l], phase, b->stream);
   };
   run(kBatchIngest, 0);
-  for (int ph = 0; ph < g.n_phases; ph++) {
-    run(kBatchResizeV, ph);
-    run(kBatchResizeH, ph);
-  }
+  for (int ph = 0; ph < g.n_phases; ph++) run(kBatchResize, ph);
   run(kBatchPix, 0);
   run(kBatchVote, 0);
   run(kBatchNorm, 0);

@@ -104,29 +104,24 @@ geye_status geye_resize(geye_ctx *ctx, const float *src, const int *sdims, int *
   std::vector<int> st, si;
   std::vector<float> al;
   taps(h, oh, st, si, al);
-  const int h_start = (int)st.size(), h_tap = (int)si.size();
+  const int h_start = (int)st.size();
   taps(w, ow, st, si, al);
   float *arena;
-  const size_t n_src = (size_t)3 * h * w, n_tmp = (size_t)3 * oh * w, n_dst = (size_t)3 * oh * ow;
-  GEYE_TRY(S.get(n_src + n_tmp + n_dst, &arena));
+  const size_t n_src = (size_t)3 * h * w, n_dst = (size_t)3 * oh * ow;
+  GEYE_TRY(S.get(n_src + n_dst, &arena));
   CUDA_TRY(cudaMemcpyAsync(arena, src, sizeof(float) * n_src, cudaMemcpyHostToDevice, ctx->stream));
-  ResizeJob jv{}, jh{};
-  jv.src_off = 0; jv.dst_off = (int)n_src; jv.src_h = h; jv.src_w = w; jv.dst_h = oh; jv.dst_w = w;
-  jv.tap_start_off = 0; jv.tap_off = 0;
-  jh.src_off = (int)n_src; jh.dst_off = (int)(n_src + n_tmp); jh.src_h = oh; jh.src_w = w; jh.dst_h = oh; jh.dst_w = ow;
+  ResizeJob J{};
+  J.src_off = 0; J.dst_off = (int)n_src; J.src_h = h; J.src_w = w; J.dst_h = oh; J.dst_w = ow;
   // both tap tables share one start array whose entries index the whole si/alpha arrays
-  jh.tap_start_off = h_start; jh.tap_off = 0;
-  (void)h_tap;
+  J.h_start_off = h_start;
   Tables T;
   const size_t o_st = T.add(st.data(), st.size()), o_si = T.add(si.data(), si.size()),
-               o_al = T.add(al.data(), al.size()), o_v = T.add(&jv, 1), o_h = T.add(&jh, 1);
+               o_al = T.add(al.data(), al.size()), o_j = T.add(&J, 1);
   GEYE_TRY(T.put(S));
-  launch_resize_pass(T.at<ResizeJob>(o_v), 1, w, 1, T.at<int>(o_st), T.at<int>(o_si), T.at<float>(o_al), arena,
-                     ctx->stream);
-  launch_resize_pass(T.at<ResizeJob>(o_h), 1, ow, 0, T.at<int>(o_st), T.at<int>(o_si), T.at<float>(o_al), arena,
-                     ctx->stream);
+  launch_resize(T.at<ResizeJob>(o_j), 1, resize_blocks(J), T.at<int>(o_st), T.at<int>(o_si), T.at<float>(o_al), arena,
+                ctx->stream);
   CUDA_TRY(cudaGetLastError());
-  CUDA_TRY(cudaMemcpyAsync(dst, arena + n_src + n_tmp, sizeof(float) * n_dst, cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_TRY(cudaMemcpyAsync(dst, arena + n_src, sizeof(float) * n_dst, cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return GEYE_OK;
 }
