@@ -86,7 +86,7 @@ struct HogPixJob {         // (bin, magnitude) of the pixels of one image
   int img_off;             // image planes [3][w][h]
   int h, w;
   int xe, ye;              // pixels 1 <= x < xe, 1 <= y < ye
-  int Y;                   // row stride of the outputs
+  int Y;                   // column length of the outputs, a multiple of four; columns 0 .. xe
   int mag_off, bin_off;    // float magnitudes; u8 bins at (uint8_t *)(arena + bin_off)
 };
 

@@ -659,7 +659,7 @@ static geye_status build_pyramid_plan(geye_ctx *ctx, Plan &P, int width, int hei
       X.ye = std::max(X.ye, J.b0 * J.sbin - 1);
     }
     for (auto &X : P.pix_jobs) {
-      X.Y = X.ye + 1;
+      X.Y = (X.ye + 4) & ~3;
       const size_t n = (size_t)(X.xe + 1) * X.Y;
       X.mag_off = A.take(n);
       X.bin_off = A.take((n + 3) / 4);

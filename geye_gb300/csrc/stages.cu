@@ -172,7 +172,7 @@ geye_status geye_calc_feature(geye_ctx *ctx, const float *src, const int *isize,
   const size_t hist = ((n_img + 31) & ~size_t(31));
   const size_t feat_off = ((hist + (size_t)19 * b0 * b1 + 31) & ~size_t(31));
   HogPixJob X{};
-  X.img_off = 0; X.h = h; X.w = w; X.xe = b1 * sbin - 1; X.ye = b0 * sbin - 1; X.Y = X.ye + 1;
+  X.img_off = 0; X.h = h; X.w = w; X.xe = b1 * sbin - 1; X.ye = b0 * sbin - 1; X.Y = (X.ye + 4) & ~3;
   const size_t n_pix = (size_t)(X.xe + 1) * X.Y;
   const size_t mag_off = ((feat_off + feat_words(fs0, fs1) + 31) & ~size_t(31));
   const size_t bin_off = ((mag_off + n_pix + 31) & ~size_t(31));
