@@ -21,7 +21,7 @@ geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_
 geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats, float *ref);
 geye_status run_conv(geye_ctx *ctx, Plan &P);
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp);
-geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh);
+geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, float *records);
 geye_status run_ascore(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, const float *h_init);
 geye_status collect_stage_times(geye_ctx *ctx);
 geye_status frame_plan(geye_ctx *ctx, geye_model *const *models, int n, int w, int h, Plan **out);

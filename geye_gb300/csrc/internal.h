@@ -161,6 +161,8 @@ struct DtJob {             // one part map: DT of the negated map
   int rows, parts;         // rows of a strip (dt_strip_rows); blocks of the map
 };
 
+constexpr int kScoreThreads = 256;   // positions per score block
+
 struct ScoreJob {          // one (level, component) score map
   int root_off;            // root conv map
   int r0, r1;
@@ -317,6 +319,14 @@ void launch_score(const ScoreJob *d_jobs, const int2 *d_blocks, int n_blocks, fl
                   int *block_counts, cudaStream_t s);
 void launch_boxes(const ScoreJob *d_jobs, const int2 *d_blocks, int n_blocks, float thresh, const float *arena,
                   const int *arena_i, const int *block_offsets, int GL, float *boxes, cudaStream_t s);
+// the pipeline's detections of a model: root box (y1, x1, y2, x2), score, and score block * kScoreThreads + thread
+struct NmsCandidates {
+  float4 *box;
+  float *score;
+  int *ref;
+};
+void launch_candidates(const ScoreJob *d_jobs, const int2 *d_blocks, int n_blocks, float thresh, const float *arena,
+                       const int *block_offsets, const NmsCandidates &out, cudaStream_t s);
 void launch_scan_counts(int *counts, int n, int *total, cudaStream_t s);
 void launch_ascore(const int *col, const int *row, int n_jobs, const float *arena, float *a_score, int im_w,
                   int im_h, float thresh, unsigned *max_bits, cudaStream_t s);
@@ -325,7 +335,7 @@ void launch_ascore_normalize(float *a_score, int n, const unsigned *max_bits, cu
 void launch_nms(const float *boxes, const int *d_num, int n_models, int GL, float overlap, int cap,
                 float *scratch_f, int *scratch_i, float *out, int *d_kept, int *err, cudaStream_t s);
 // pipeline NMS (nms_radix.cu, nms_batch.cu): per model nms_model_words(cap) ints
-// of scratch and 10 * cap floats (the boxes in sorted order, the picks')
+// of scratch and 16 * cap floats (the boxes in sorted order, the picks', the candidates)
 constexpr int kNmsBatch = 512;     // boxes resolved per round
 constexpr int kNmsCells = 64;      // cells per image axis of the greedy's pick masks
 constexpr int kNmsLevels = 7;      // their sparse-table levels (spans of 1..64 cells)
@@ -335,17 +345,24 @@ constexpr int kNmsLevels = 7;      // their sparse-table levels (spans of 1..64 
 __host__ __device__ inline int nms_rs_tile(int cap) { return cap <= (1 << 18) ? 1024 : 4096; }
 __host__ __device__ inline int nms_rs_tiles(int cap) { return (cap + nms_rs_tile(cap) - 1) / nms_rs_tile(cap); }
 __host__ __device__ inline size_t nms_model_words(int cap) {
-  const size_t w = 32 + 11 * (size_t)cap + cap / 32 + 2 + 4 * 256 * (size_t)nms_rs_tiles(cap);
+  const size_t w = 32 + 10 * (size_t)cap + cap / 32 + 2 + 4 * 256 * (size_t)nms_rs_tiles(cap);
   return (w + 31) & ~(size_t)31;
 }
+inline NmsCandidates nms_candidates(float *sf, int m, int cap) {   // cap: a multiple of four
+  float *f = sf + (size_t)m * 16 * cap + 10 * (size_t)cap;
+  return {reinterpret_cast<float4 *>(f), f + 4 * (size_t)cap, reinterpret_cast<int *>(f + 5 * (size_t)cap)};
+}
 // what the results are made from: per model its regression coefficients [comp][x1, y1, x2, y2][ML],
-// part count and ratio; out: 11 * cap ints per model (point, or_point, type, scale, score)
+// part count, ratio, score maps and their blocks; arena_i: the frame's maps; out: 11 * cap ints per model (point, or_point, type, scale, score)
 struct NmsResults {
   struct Model {
     const float *coef;
     int np;
     float ratio;
+    const ScoreJob *jobs;
+    const int2 *blocks;
   } m[16];
+  const int *arena_i;
   int *out;
   // the frame's result block in pinned host memory (Plan::h_res): counts, then host_cap records a model
   int *host;
@@ -358,7 +375,7 @@ struct NmsResults {
 constexpr int kNmsOrderKey = 0, kNmsOrderQuicksort = 1;
 // aux: null for plain launches on s; when s is capturing a graph, a second
 // stream that captures the body of the if node for the quicksort's order of all boxes
-cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
+cudaError_t launch_nms_batch(const int *d_num, int n_models, float overlap,
                              int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
                              long long *diag, int *need, int order, cudaStream_t s, cudaStream_t aux);
 void launch_new_rects(const float *kept, const int *d_kept, int GL, int np, const float *coef, int img_w,

@@ -457,17 +457,17 @@ __device__ __noinline__ void split_boxes(GreedySmem &R, int *si, float *sf, int 
 }
 
 // The boxes in the quicksort's order, by the cluster
-__device__ __noinline__ void gather_boxes(const float *boxes, int GL, int *si, float *sf, int m, int cap) {
+__device__ __noinline__ void gather_boxes(int *si, float *sf, int m, int cap) {
   cg::cluster_group cluster = cg::this_cluster();
   const Slots S = slots(si, sf, m, cap);
   const int D = S.st->D;
 #pragma unroll 4
   for (int r = (int)cluster.block_rank() * kResNT + threadIdx.x; r < D; r += (int)cluster.num_blocks() * kResNT) {
     const int i = S.qo[r];
-    const float *P = boxes + (size_t)i * GL;
+    const float4 b = S.box[i];
     S.ord[r] = i;
-    S.y1[r] = P[0]; S.x1[r] = P[1]; S.y2[r] = P[2]; S.x2[r] = P[3];
-    S.ar[r] = (P[3] - P[1] + 1.0) * (P[2] - P[0] + 1.0);   // nms.cpp's area expression
+    S.y1[r] = b.x; S.x1[r] = b.y; S.y2[r] = b.z; S.x2[r] = b.w;
+    S.ar[r] = (b.w - b.y + 1.0) * (b.z - b.x + 1.0);   // nms.cpp's area expression
   }
   cluster.sync();
 }
@@ -544,18 +544,17 @@ __device__ __forceinline__ void decide_members(const Slots &S, GreedySmem &R, in
 }
 
 // ---------------------------------------------------------------------------
-// final-pick rule, the kept boxes in input order (whole block, the model done)
+// final-pick rule, the kept boxes in input order (the model done)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int m, int npk, int batches, bool quick,
-                                             const float *boxes, int GL, int cap, const NmsResults &res, int *d_kept,
-                                             long long *diag) {
+// The kept boxes' input indices, by the first block: R.tot of them, in R.idx + kRankMax, or in S.Rpos where they are more
+constexpr int kRankMax = 2 * kResNT;
+__device__ __forceinline__ void rank_kept(const Slots &S, GreedySmem &R, int npk) {
   const int D = S.st->D;
   // (the flags are read past L1: other blocks of the cluster have set them)
   const int K = npk - ((npk > 0 && __ldcg(&S.flag[npk - 1]) == 0) ? 1 : 0);
   // the kept boxes' input indices (all distinct) in ascending order
   int *keep = S.Rpos;
   int *idx = R.idx;   // the round's buffers are free now
-  constexpr int kRankMax = 2 * kResNT;
   if (K <= kRankMax) {   // ranked in shared memory
     for (int k = threadIdx.x; k < ((K + 3) & ~3); k += kResNT) idx[k] = k < K ? S.ord[__ldcg(&S.picks[k])] : 0x7fffffff;
     __syncthreads();
@@ -586,33 +585,64 @@ __device__ __forceinline__ void finish_model(const Slots &S, GreedySmem &R, int 
       written += tot;
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    d_kept[m] = K;
-    if (diag) {
-      diag[8 * m + 2] = batches;
-      diag[8 * m + 3] = npk;
-      diag[8 * m + 5] = quick;
-    }
-  }
-  // the results (get_new_rects), four threads a box: on the device, and the first of them in the host's block
+  if (threadIdx.x == 0) R.tot = K;
+}
+
+// The results (get_new_rects) of the kept boxes, by the cluster, four threads a box: its parts' corners looked up anew,
+// then a side each; on the device, and the first of them in the host's block
+__device__ __forceinline__ void write_results(const Slots &S, GreedySmem &R, int m, int cap, const NmsResults &res) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const GreedySmem *R0 = cluster.map_shared_rank(&R, 0);
   const NmsResults::Model &Q = res.m[m];
+  const int K = R0->tot, np = Q.np, ML = 1 + 2 * (1 + np);
   int *out = res.out + (size_t)m * cap * 11, *host = res.host + 64 + (size_t)m * 11 * res.host_cap;
-  for (int e = threadIdx.x; e < 4 * K; e += kResNT) {
-    const int k = e >> 2, c = e & 3;
-    const float *P = boxes + (size_t)keep[k] * GL;
-    const int v = new_rect_side(P, GL, Q.np, Q.coef, res.img_w, res.img_h, c), r = (int)((float)v / Q.ratio);
-    // type, scale, score
-    const int more = c == 0 ? (int)P[GL - 3] : __float_as_int(P[c == 1 ? GL - 1 : GL - 2]);
-    auto put = [&](int *o, size_t stride) {
-      o[e] = v;
-      o[4 * stride + e] = r;
-      if (c < 3) o[(8 + c) * stride + k] = more;
-    };
-    put(out, cap);
-    if (k < res.host_cap) put(host, res.host_cap);
+  static_assert(sizeof(R.idx) >= (2 * kRankMax + (kResNT / 4) * (1 + 2 * (1 + kMaxParts))) * sizeof(int) ||
+                    sizeof(QuickSmem) >= (2 * kRankMax + (kResNT / 4) * (1 + 2 * (1 + kMaxParts))) * sizeof(int),
+                "the ranks and a block's records");
+  // [w, (x1, y1) of root and parts] of the thread's box, behind the ranks
+  float *vec = reinterpret_cast<float *>(R.idx) + 2 * kRankMax + (threadIdx.x >> 2) * ML;
+  const int step = (int)cluster.num_blocks() * kResNT, first = (int)cluster.block_rank() * kResNT;
+  for (int e0 = first; e0 < 4 * K; e0 += step) {
+    const int e = e0 + threadIdx.x, k = e >> 2, c = e & 3;
+    const bool in = k < K;
+    int comp = 0, more = 0;
+    if (in) {
+      const int box = K <= kRankMax ? R0->idx[kRankMax + k] : __ldcg(&S.Rpos[k]), ref = S.ref[box];
+      const int2 blk = Q.blocks[ref / kScoreThreads];
+      const ScoreJob &J = Q.jobs[blk.x];
+      const int i = blk.y * kScoreThreads + ref % kScoreThreads, y = i % J.r0, x = i / J.r0;
+      comp = J.comp;
+      for (int p = c; p < np; p += 4) {
+        const float2 q = part_corner(J, p, x, y, res.arena_i);
+        vec[3 + 2 * p] = q.y;
+        vec[4 + 2 * p] = q.x;
+      }
+      if (c == 0) {
+        const float4 b = S.box[box];
+        vec[0] = b.w - b.y;
+        vec[1] = b.y;
+        vec[2] = b.x;
+      }
+      // type, scale, score
+      more = c == 0 ? comp : __float_as_int(c == 1 ? J.scale : S.score[box]);
+    }
+    __syncwarp();
+    if (in) {
+      const float *w = Q.coef + ((size_t)comp * 4 + c) * ML;
+      float sum = 0;
+#pragma unroll 8
+      for (int q = 0; q < ML; q++) sum += vec[q] * w[q];
+      const int v = rect_bound(sum, res.img_w, res.img_h, c), r = (int)((float)v / Q.ratio);
+      auto put = [&](int *o, size_t stride) {
+        o[e] = v;
+        o[4 * stride + e] = r;
+        if (c < 3) o[(8 + c) * stride + k] = more;
+      };
+      put(out, cap);
+      if (k < res.host_cap) put(host, res.host_cap);
+    }
+    __syncwarp();
   }
-  if (threadIdx.x == 0) res.host[32 + m] = K;
 }
 
 // The first item at or after c1 whose score differs from the one before it, at most hi (every warp alike)
@@ -710,7 +740,7 @@ __device__ __forceinline__ WalkEnd walk_boxes(const Slots &S, GreedySmem &R, con
 // it, the rounds' code is 8 % slower (same rounds: 1280x720, NMS stage 433 us against 399).
 enum GreedyPass { kFirst, kRest, kOrderedFirst, kOrderedRest };
 template <bool kFull>
-__global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restrict__ boxes_all, int GL, int cap, int *si,
+__global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(int cap, int *si,
                                                        float *sf, float overlap, float2 cell_inv,
                                                        const __grid_constant__ NmsResults res, int *d_kept,
                                                        long long *diag, const int *need, int *err, bool all_ordered,
@@ -719,7 +749,6 @@ __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restric
   GreedySmem &R = *reinterpret_cast<GreedySmem *>(res_sm);
   cg::cluster_group cluster = cg::this_cluster();
   const int m = blockIdx.y;
-  const float *boxes = boxes_all + (size_t)m * cap * GL;
   const bool ordered = kFull && pass >= kOrderedFirst, rest = pass & 1;
   bool whole = false;          // the quicksort's order of all boxes is needed (every block alike)
   WalkResume resume = kAnew;
@@ -749,7 +778,7 @@ __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restric
     }
   }
   cluster.sync();   // every block has started: its shared memory can be written
-  if (kFull && pass == kOrderedFirst) gather_boxes(boxes, GL, si, sf, m, cap);
+  if (kFull && pass == kOrderedFirst) gather_boxes(si, sf, m, cap);
   if (resume != kAnew || whole) {
   } else if (!rest) {
     const Slots S = slots(si, sf, m, cap);
@@ -807,10 +836,9 @@ __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restric
   if (!whole && !tied && !ordered && !more && np >= 2)
     whole = S.key[__ldcg(&S.picks[np - 1])] == S.key[__ldcg(&S.picks[np - 2])];
   if (kFull && whole) split_boxes(R, si, sf, m, cap, err);
-  if (cluster.block_rank() != 0) return;
-  const bool quick = kFull || whole || tied;
+  const bool quick = kFull || whole || tied, first = cluster.block_rank() == 0;
   if (whole || tied || more) {
-    if (threadIdx.x == 0) {
+    if (first && threadIdx.x == 0) {
       BatchState &st = *slots(si, sf, m, cap).st;
       st.stage = whole ? (kFull ? kNmsSplit : kNmsWhole) : tied ? (rest ? kNmsTiedRest : kNmsTied)
                  : ordered ? kNmsOrderedPrefix : kNmsPrefix;
@@ -823,8 +851,19 @@ __global__ void __launch_bounds__(kResNT, 1) k_nms_greedy(const float *__restric
     }
     return;
   }
-  if (threadIdx.x == 0) S.st->stage = kNmsDone;
-  finish_model(S, R, m, np, R.batches, quick || S.st->quick, boxes, GL, cap, res, d_kept, diag);
+  if (first) rank_kept(S, R, np);
+  cluster.sync();   // the kept boxes are in order
+  write_results(S, R, m, cap, res);
+  if (first && threadIdx.x == 0) {
+    S.st->stage = kNmsDone;
+    d_kept[m] = res.host[32 + m] = R.tot;
+    if (diag) {
+      diag[8 * m + 2] = R.batches;
+      diag[8 * m + 3] = np;
+      diag[8 * m + 5] = quick || S.st->quick;
+    }
+  }
+  cluster.sync();   // (the first block's ranks have been read)
 }
 
 // The boxes from st.next on against every pick so far, over the grid
@@ -966,13 +1005,13 @@ static int cluster_blocks(K *kernel, size_t smem) {
   return kCluster;
 }
 
-cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models, int GL, float overlap,
+cudaError_t launch_nms_batch(const int *d_num, int n_models, float overlap,
                              int cap, int *si, float *sf, const NmsResults &res, int *d_kept, int *err,
                              long long *diag, int *need, int order, cudaStream_t s, cudaStream_t aux) {
   if (n_models <= 0) return cudaSuccess;
   // cells over the image and a margin for boxes that leave it (any value is exact: what is outside shares the edge cells)
   const float2 cell_inv = make_float2(kNmsCells / (1.15f * std::max(res.img_h, 1)), kNmsCells / (1.15f * std::max(res.img_w, 1)));
-  launch_nms_radix(boxes, d_num, n_models, GL, cap, si, sf, need, res.host, s);
+  launch_nms_radix(d_num, n_models, cap, si, sf, need, res.host, s);
   static SmemAttr attr[4];
   cudaError_t e = raise_smem(attr[0], k_nms_greedy<false>, sizeof(GreedySmem));
   if (e == cudaSuccess) e = raise_smem(attr[1], k_nms_greedy<true>, sizeof(GreedySmem));
@@ -998,7 +1037,7 @@ cudaError_t launch_nms_batch(const float *boxes, const int *d_num, int n_models,
     if (pass & 1)
       k_nms_rest<<<dim3(std::max(304 / n_models, 1), n_models), kResNT, 0, c.stream>>>(
           cap, si, sf, overlap, cell_inv, pass == kRest ? kNmsPrefix : kNmsOrderedPrefix);
-    e = cudaLaunchKernelEx(&c, full ? k_nms_greedy<true> : k_nms_greedy<false>, boxes, GL, cap, si, sf, overlap, cell_inv,
+    e = cudaLaunchKernelEx(&c, full ? k_nms_greedy<true> : k_nms_greedy<false>, cap, si, sf, overlap, cell_inv,
                            res, d_kept, diag, (const int *)need, err, order == kNmsOrderQuicksort, pass, h, aux != nullptr);
   };
   greedy(false, kFirst);

@@ -29,12 +29,11 @@ struct BatchState {   // greedy rounds, between launches
   int pad[1];
 };
 
-// per-model scratch: nms_model_words(cap) ints and 10 * cap floats
+// per-model scratch: nms_model_words(cap) ints and 16 * cap floats
 struct Slots {
   unsigned *key;     // sort keys (nms_radix.cu)
   int *ord;          // sorted position -> box
   int *Lpos, *Rpos;  // the radix sort's second buffers; then Lpos the list of items, Rpos the kept boxes' input indices
-  float *score;      // the scores in input order
   float *qv;         // the quicksort's values, boxes and partition lists
   int *qo, *qL, *qR;
   int *place;        // box -> its place in the quicksort's order
@@ -46,11 +45,14 @@ struct Slots {
   float *y1, *x1, *y2, *x2, *ar;   // boxes in sorted order
   float4 *pb;        // the picks' boxes y1, x1, y2, x2 and areas, in pick order
   float *pa;
+  const float4 *box;   // the candidates in input order (NmsCandidates)
+  const float *score;
+  const int *ref;
 };
 
 __device__ __forceinline__ Slots slots(int *si, float *sf, int m, int cap) {
   int *b = si + (size_t)m * nms_model_words(cap);
-  float *f = sf + (size_t)m * 10 * cap;
+  float *f = sf + (size_t)m * 16 * cap;
   const size_t n = cap;
   Slots S;
   S.st = reinterpret_cast<BatchState *>(b);
@@ -59,23 +61,25 @@ __device__ __forceinline__ Slots slots(int *si, float *sf, int m, int cap) {
   S.ord = b + n;
   S.Lpos = b + 2 * n;
   S.Rpos = b + 3 * n;
-  S.score = reinterpret_cast<float *>(b + 4 * n);
-  S.qv = reinterpret_cast<float *>(b + 5 * n);
-  S.qo = b + 6 * n;
-  S.qL = b + 7 * n;
+  S.qv = reinterpret_cast<float *>(b + 4 * n);
+  S.qo = b + 5 * n;
+  S.qL = b + 6 * n;
   S.qR = S.Rpos;
-  S.picks = b + 8 * n;
-  S.flag = b + 9 * n;
-  S.place = b + 10 * n;
-  S.bits = reinterpret_cast<unsigned *>(b + 11 * n);
-  S.hist = b + ((11 * n + n / 32 + 2) & ~(size_t)1);
+  S.picks = b + 7 * n;
+  S.flag = b + 8 * n;
+  S.place = b + 9 * n;
+  S.bits = reinterpret_cast<unsigned *>(b + 10 * n);
+  S.hist = b + ((10 * n + n / 32 + 2) & ~(size_t)1);
   S.y1 = f;
   S.x1 = f + cap;
   S.y2 = f + 2 * (size_t)cap;
   S.x2 = f + 3 * (size_t)cap;
   S.ar = f + 4 * (size_t)cap;
   S.pb = reinterpret_cast<float4 *>(f + 5 * (size_t)cap);
-  S.pa = f + 9 * (size_t)cap;
+  S.pa = f + 9 * n;
+  S.box = reinterpret_cast<const float4 *>(f + 10 * n);
+  S.score = f + 14 * n;
+  S.ref = reinterpret_cast<const int *>(f + 15 * n);
   return S;
 }
 
@@ -101,7 +105,7 @@ __device__ __forceinline__ bool supp(float Ay1, float Ax1, float Ay2, float Ax2,
 
 // key-order sort (nms_radix.cu): key = transformed scores, ord = input index,
 // BatchState initialised; need[m] set for a NaN score
-void launch_nms_radix(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
+void launch_nms_radix(const int *d_num, int n_models, int cap, int *si, float *sf,
                       int *need, int *host, cudaStream_t s);
 
 }  // namespace geye

@@ -17,7 +17,7 @@
 //
 //   k_rs_load     keys (order-preserving transform of the float score, -0 as
 //                 +0, complemented for descending order), indices, the
-//                 scores in input order (for nms_quick.h), the greedy state, and the digit counts of the first
+//                 greedy state, and the digit counts of the first
 //                 pass per tile of nms_rs_tile(cap) keys; NaN raises the flag.
 //   k_rs_pass     four passes of eight bits, one kernel each: a block per tile
 //                 adds up the tiles' digit counts before it (at most a few
@@ -47,12 +47,10 @@ __device__ __forceinline__ unsigned rs_key(float v, bool &nan) {
   return ~asc;   // ascending keys = descending scores
 }
 
-__global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ boxes_all, const int *__restrict__ d_num,
-                                                   int GL, int cap, int *si, float *sf, int *need, int *host) {
+__global__ void __launch_bounds__(kRsNT) k_rs_load(const int *__restrict__ d_num, int cap, int *si, float *sf, int *need, int *host) {
   __shared__ int h[256];
   const int m = blockIdx.y, t = blockIdx.x;
   Slots S = slots(si, sf, m, cap);
-  const float *boxes = boxes_all + (size_t)m * cap * GL;
   const int D = max(0, min(d_num[m], cap)), T = nms_rs_tile(cap);
   if (t == 0 && threadIdx.x == 0) {
     BatchState &st = *S.st;
@@ -68,10 +66,8 @@ __global__ void __launch_bounds__(kRsNT) k_rs_load(const float *__restrict__ box
   __syncthreads();
   bool nan = false;
   for (int i = e0 + threadIdx.x; i < min(e0 + T, D); i += kRsNT) {
-    const float v = boxes[(size_t)i * GL + GL - 2];
-    const unsigned k = rs_key(v, nan);
+    const unsigned k = rs_key(S.score[i], nan);
     if (nan) need[m] = 1;
-    S.score[i] = v;
     S.key[i] = k;
     S.ord[i] = i;
     atomicAdd(&h[k & 255u], 1);
@@ -99,7 +95,7 @@ __device__ __forceinline__ void rs_bufs(const Slots &S, int pass, const unsigned
 
 // IT keys per thread (a tile of kRsNT * IT); pass 3 gathers the boxes
 template <int IT>
-__global__ void __launch_bounds__(kRsNT) k_rs_pass(int pass, const float *__restrict__ boxes_all, int GL, int cap,
+__global__ void __launch_bounds__(kRsNT) k_rs_pass(int pass, int cap,
                                                    int *si, float *sf) {
   constexpr int T = kRsNT * IT;
   __shared__ int before_s[2][256], total_s[2][256];
@@ -176,7 +172,6 @@ __global__ void __launch_bounds__(kRsNT) k_rs_pass(int pass, const float *__rest
     }
   }
   __syncthreads();
-  const float *boxes = boxes_all + (size_t)m * cap * GL;
   int *Hn = S.hist + (pass + 1) * pass_words;
 #pragma unroll
   for (int k = 0; k < IT; k++) {
@@ -191,21 +186,21 @@ __global__ void __launch_bounds__(kRsNT) k_rs_pass(int pass, const float *__rest
       const unsigned peers = __match_any_sync(0xffffffffu, q);
       if (valid && (peers & lt) == 0u) atomicAdd(&Hn[q], __popc(peers));
     } else if (valid) {
-      const float *P = boxes + (size_t)idx[k] * GL;
-      const float y1 = P[0], x1 = P[1], y2 = P[2], x2 = P[3];
+      const float4 b = S.box[idx[k]];
+      const float y1 = b.x, x1 = b.y, y2 = b.z, x2 = b.w;
       S.y1[p] = y1; S.x1[p] = x1; S.y2[p] = y2; S.x2[p] = x2;
       S.ar[p] = (x2 - x1 + 1.0) * (y2 - y1 + 1.0);   // nms.cpp's area expression
     }
   }
 }
 
-void launch_nms_radix(const float *boxes, const int *d_num, int n_models, int GL, int cap, int *si, float *sf,
+void launch_nms_radix(const int *d_num, int n_models, int cap, int *si, float *sf,
                       int *need, int *host, cudaStream_t s) {
   const dim3 grid(nms_rs_tiles(cap), n_models);
-  k_rs_load<<<grid, kRsNT, 0, s>>>(boxes, d_num, GL, cap, si, sf, need, host);
+  k_rs_load<<<grid, kRsNT, 0, s>>>(d_num, cap, si, sf, need, host);
   for (int p = 0; p < 4; p++) {
-    if (nms_rs_tile(cap) == 2 * kRsNT) k_rs_pass<2><<<grid, kRsNT, 0, s>>>(p, boxes, GL, cap, si, sf);
-    else k_rs_pass<8><<<grid, kRsNT, 0, s>>>(p, boxes, GL, cap, si, sf);
+    if (nms_rs_tile(cap) == 2 * kRsNT) k_rs_pass<2><<<grid, kRsNT, 0, s>>>(p, cap, si, sf);
+    else k_rs_pass<8><<<grid, kRsNT, 0, s>>>(p, cap, si, sf);
   }
 }
 

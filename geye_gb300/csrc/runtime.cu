@@ -714,17 +714,12 @@ static geye_status finish_plan(geye_ctx *ctx, Plan &P, ArenaAlloc &A) {
     // plane tails are read (and their outputs discarded) but never written: keep them zero
     CUDA_TRY(cudaMemsetAsync(P.arena16.p, 0, P.arena16_elems * 2, ctx->stream));
   }
-  int gl = 0, cap = 0;
-  for (auto &mp : P.models) {
-    gl = std::max(gl, mp->model->gl());
-    cap = std::max(cap, mp->cap);
-  }
-  P.gl = gl;
+  int cap = 0;
+  for (auto &mp : P.models) cap = std::max(cap, mp->cap);
   // multiple of 32: per-model NMS scratch (int2 queues) stays 8-byte aligned
   P.max_cap = (std::max(cap, 1) + 31) & ~31;
   const size_t nm = std::max<size_t>(P.models.size(), 1);
-  GEYE_TRY(P.d_boxes.alloc(ctx, sizeof(float) * nm * P.max_cap * std::max(gl, 1)));
-  GEYE_TRY(P.d_nms_f.alloc(ctx, sizeof(float) * nm * P.max_cap * 10));
+  GEYE_TRY(P.d_nms_f.alloc(ctx, sizeof(float) * nm * P.max_cap * 16));
   GEYE_TRY(P.d_nms_i.alloc(ctx, sizeof(int) * nm * nms_model_words(P.max_cap)));
   GEYE_TRY(P.d_small.alloc(ctx, 4096));
   if (P.width > 0) {
@@ -928,8 +923,8 @@ static bool tune_dt(geye_ctx *ctx, Plan &P) {
   return changed;
 }
 
-// score maps, detection records; model index mi writes boxes at mi*cap*GL and its count at d_small[mi]
-geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh) {
+// score maps and detections: the count at d_small[mi], the NMS candidates, or (records) the whole records there
+geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, float *records) {
   int *counts = mp.d_counts.as<int>();
   int *d_num = P.d_small.as<int>() + mi;
   const int nj = (int)mp.score_jobs.size();
@@ -942,9 +937,12 @@ geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thres
   GEYE_TRY(check_launch(ctx, "score"));
   launch_scan_counts(counts, mp.score_nblocks, d_num, ctx->stream);
   GEYE_TRY(check_launch(ctx, "scan"));
-  float *boxes = P.d_boxes.as<float>() + (size_t)mi * P.max_cap * P.gl;
-  launch_boxes(mp.d_score_jobs.as<ScoreJob>(), mp.d_score_blocks.as<int2>(), mp.score_nblocks, thresh,
-               P.arena.as<float>(), P.arena.as<int>(), counts, mp.model->gl(), boxes, ctx->stream);
+  if (records)
+    launch_boxes(mp.d_score_jobs.as<ScoreJob>(), mp.d_score_blocks.as<int2>(), mp.score_nblocks, thresh,
+                 P.arena.as<float>(), P.arena.as<int>(), counts, mp.model->gl(), records, ctx->stream);
+  else
+    launch_candidates(mp.d_score_jobs.as<ScoreJob>(), mp.d_score_blocks.as<int2>(), mp.score_nblocks, thresh,
+                      P.arena.as<float>(), counts, nms_candidates(P.d_nms_f.as<float>(), mi, P.max_cap), ctx->stream);
   return check_launch(ctx, "boxes");
 }
 
@@ -996,15 +994,17 @@ geye_status run_nms(geye_ctx *ctx, Plan &P, int n_models, float overlap) {
   NmsResults res{};
   for (int mi = 0; mi < n_models; mi++) {
     geye_model *m = P.models[mi]->model;
-    res.m[mi] = {m->d_coef, m->h.numpart[0], m->h.ratio};
+    res.m[mi] = {m->d_coef, m->h.numpart[0], m->h.ratio, P.models[mi]->d_score_jobs.as<ScoreJob>(),
+                 P.models[mi]->d_score_blocks.as<int2>()};
   }
+  res.arena_i = P.arena.as<int>();
   res.out = P.d_result.as<int>();
   res.host = static_cast<int *>(P.h_res);
   res.host_cap = kHostRes;
   res.img_w = P.width;
   res.img_h = P.height;
   const cudaError_t ge =
-      launch_nms_batch(P.d_boxes.as<float>(), d_num, n_models, P.gl, overlap,
+      launch_nms_batch(d_num, n_models, overlap,
                        P.max_cap, P.d_nms_i.as<int>(),
                        P.d_nms_f.as<float>(), res, d_kept, err, reinterpret_cast<long long *>(d_num + 512),
                        d_num + kNmsNeed, ctx->nms_order, ctx->stream,
@@ -1030,7 +1030,7 @@ static geye_status run_body(geye_ctx *ctx, Plan &P, float thresh, float overlap)
     T.mark(3);
     for (auto &mp : P.models) GEYE_TRY(run_dt(ctx, P, *mp));
     T.mark(4);
-    for (size_t mi = 0; mi < P.models.size(); mi++) GEYE_TRY(run_score(ctx, P, *P.models[mi], (int)mi, thresh));
+    for (size_t mi = 0; mi < P.models.size(); mi++) GEYE_TRY(run_score(ctx, P, *P.models[mi], (int)mi, thresh, nullptr));
   } else {
     // each model's DT -> score chain reads only the conv maps and writes only its
     // own maps and records: models 1.. run on the side stream beside model 0
@@ -1038,7 +1038,7 @@ static geye_status run_body(geye_ctx *ctx, Plan &P, float thresh, float overlap)
     // joined before NMS
     auto chain = [&](size_t mi) -> geye_status {
       GEYE_TRY(run_dt(ctx, P, *P.models[mi]));
-      return run_score(ctx, P, *P.models[mi], (int)mi, thresh);
+      return run_score(ctx, P, *P.models[mi], (int)mi, thresh, nullptr);
     };
     CUDA_TRY(cudaEventRecord(ctx->ev_fork, ctx->stream));
     CUDA_TRY(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));

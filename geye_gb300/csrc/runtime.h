@@ -234,8 +234,8 @@ struct Plan {
   size_t arena_words = 0, arena16_elems = 0;
   DevBuf arena, arena16;
   DevBuf d_bgr;                          // frame upload buffer
-  DevBuf d_boxes, d_nms_f, d_nms_i, d_small, d_ascore, d_result;
-  int gl = 0, max_cap = 0;
+  DevBuf d_nms_f, d_nms_i, d_small, d_ascore, d_result;
+  int max_cap = 0;
   // algorithmic bytes per stage (for roofline reporting)
   double bytes_resize = 0, bytes_hog = 0;
   // last-run results (host)

@@ -17,7 +17,6 @@
 
 namespace geye {
 
-constexpr int kScoreThreads = 256;
 
 __global__ void k_fill(float *__restrict__ p, size_t n, float v) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
@@ -121,34 +120,16 @@ void launch_scan_counts(int *counts, int n, int *total, cudaStream_t s) {
 // then rank order), so they are built in shared memory and written out with
 // coalesced stores.
 //
-// partbox (get_boxes.cpp:243-258) is written in double; every step of it is
-// exact except the final rounding to float, so it is restated in float and
-// integer arithmetic with that one rounding (the FP64 pipe is narrow here):
-//   q0 = ((py - 2)/2 + 1) * scale  ==  (py * 0.5f) * scale   (exact product, one rounding)
-//   q2 = q0 + psize*scale/2 - 1     ==  one rounding of the exact sum (below)
-
-// float(q + h - 1) with the sum taken exactly.  For q, h in [0.5, 2^23) the
-// double expression is exact before its rounding to float.  In float:
-// s + e = q + h exactly (TwoSum; no contraction), s - 1 is exact for
-// 1 <= s < 2^24 (1 is a multiple of s's unit in the last place), so
-// (s - 1) + e is one correctly rounded addition of the exact q + h - 1.
-// (64-bit integer conversions would run on the narrow FP64 pipe.)
-__device__ __forceinline__ float sum_minus_one(float q, float h) {
-  if (q >= 0.5f && h >= 0.5f && q < 8388608.0f && h < 8388608.0f) {
-    const float s = q + h;
-    const float bb = s - q;
-    const float e = (q - (s - bb)) + (h - bb);
-    return (s - 1.0f) + e;
-  }
-  return (float)((double)q + (double)h - 1.0);
-}
-
+// kRecords: whole records (get_boxes itself).  Otherwise what the pipeline's NMS looks at (the root box and the score) and
+// the position, from which the records of the few kept ones are formed at the end (nms_batch.cu): 24 bytes a
+// detection instead of 156.  Score stage: 640x480 car+person 41 -> 25 us, 1920x1080 139 -> 45 us
+template <bool kRecords>
 __global__ void __launch_bounds__(kScoreThreads) k_boxes(const ScoreJob *__restrict__ jobs,
                                                          const int2 *__restrict__ blocks, float thresh,
                                                          const float *__restrict__ arena,
                                                          const int *__restrict__ arena_i,
                                                          const int *__restrict__ block_offsets, int GL,
-                                                         float *__restrict__ boxes) {
+                                                         float *__restrict__ boxes, NmsCandidates cand) {
   extern __shared__ float rec_s[];   // [count][GL]
   __shared__ int warp_cnt[kScoreThreads / 32];
   const int2 blk = blocks[blockIdx.x];
@@ -171,36 +152,26 @@ __global__ void __launch_bounds__(kScoreThreads) k_boxes(const ScoreJob *__restr
     count += warp_cnt[w];
   }
   if (count == 0) return;
+  if (!kRecords) {
+    if (flag) {
+      const int o = block_offsets[blockIdx.x] + rank;
+      float P[4];
+      root_box(i / J.r0, i % J.r0, J.scale, J.rsize0, J.rsize1, P);
+      cand.box[o] = make_float4(P[0], P[1], P[2], P[3]);
+      cand.score[o] = s;
+      cand.ref[o] = blockIdx.x * kScoreThreads + threadIdx.x;
+    }
+    return;
+  }
   if (flag) {
     const int y = i % J.r0, x = i / J.r0;
     float *P = rec_s + rank * GL;
-    const float scale = J.scale;
-    root_box(x, y, scale, J.rsize0, J.rsize1, P);
-    float *Q = P + 4;
-    for (int k = 0; k < J.np; k++) {
-      const int probex = (x - 1) * 2 + J.ax[k];
-      const int probey = (y - 1) * 2 + J.ay[k];
-      long Pi;
-      if (const int ci0 = J.part_ci0[k]) {   // compact: every probe is inside and in the stored class
-        Pi = (long)(probex >> 1) * ci0 + (probey >> 1);
-      } else {
-        Pi = probey + (long)probex * J.part_d0[k];
-        // the reference reads outside the map here (undefined); use entry 0 instead
-        if (Pi < 0 || Pi >= (long)J.part_d0[k] * J.part_d1[k]) Pi = 0;
-      }
-      const float px = (float)arena_i[J.part_Ix[k] + Pi] + 1.0f;   // an integer: exact
-      const float py = (float)arena_i[J.part_Iy[k] + Pi] + 1.0f;
-      const float q0 = (py * 0.5f) * scale;
-      const float q1 = (px * 0.5f) * scale;
-      Q[0] = q0;
-      Q[1] = q1;
-      Q[2] = sum_minus_one(q0, ((float)J.psize0[k] * scale) * 0.5f);
-      Q[3] = sum_minus_one(q1, ((float)J.psize1[k] * scale) * 0.5f);
-      Q += 4;
-    }
+    root_box(x, y, J.scale, J.rsize0, J.rsize1, P);
+    for (int k = 0; k < J.np; k++) part_box(J, k, x, y, arena_i, P + 4 * (k + 1));
+    float *Q = P + 4 * (J.np + 1);
     Q[0] = (float)J.comp;
     Q[1] = s;
-    Q[2] = scale;
+    Q[2] = J.scale;
   }
   __syncthreads();
   float *out = boxes + (size_t)block_offsets[blockIdx.x] * GL;
@@ -212,8 +183,15 @@ void launch_boxes(const ScoreJob *d_jobs, const int2 *d_blocks, int n_blocks, fl
   if (n_blocks <= 0) return;
   const size_t smem = sizeof(float) * kScoreThreads * GL;
   static SmemAttr attr;
-  raise_smem(attr, k_boxes, smem);
-  k_boxes<<<n_blocks, kScoreThreads, smem, s>>>(d_jobs, d_blocks, thresh, arena, arena_i, block_offsets, GL, boxes);
+  raise_smem(attr, k_boxes<true>, smem);
+  k_boxes<true><<<n_blocks, kScoreThreads, smem, s>>>(d_jobs, d_blocks, thresh, arena, arena_i, block_offsets, GL, boxes,
+                                                     NmsCandidates{});
+}
+
+void launch_candidates(const ScoreJob *d_jobs, const int2 *d_blocks, int n_blocks, float thresh, const float *arena,
+                       const int *block_offsets, const NmsCandidates &out, cudaStream_t s) {
+  if (n_blocks <= 0) return;
+  k_boxes<false><<<n_blocks, kScoreThreads, 0, s>>>(d_jobs, d_blocks, thresh, arena, nullptr, block_offsets, 0, nullptr, out);
 }
 
 // A_SCORE in gather form: target pixel (X, Y) takes the max over every

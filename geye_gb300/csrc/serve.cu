@@ -366,7 +366,7 @@ geye_status reap(geye_server *s, bool block) {
 
 namespace geye {
 size_t plan_device_bytes(const Plan &P) {
-  size_t b = P.arena.bytes + P.arena16.bytes + P.d_bgr.bytes + P.d_boxes.bytes +
+  size_t b = P.arena.bytes + P.arena16.bytes + P.d_bgr.bytes +
              P.d_nms_f.bytes + P.d_nms_i.bytes + P.d_small.bytes + P.d_ascore.bytes + P.d_result.bytes;
   b += P.d_conv_jobs.bytes + P.d_conv_blocks.bytes + P.d_conv_bank.bytes;
   b += P.tc.d_bank.bytes + P.tc.d_jobs.bytes + P.tc.d_chunks.bytes + P.tc.d_cols.bytes + P.tc.d_sums.bytes;

@@ -16,7 +16,7 @@ geye_status run_pyramid(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_
 geye_status run_hog(geye_ctx *ctx, Plan &P, bool floats, float *ref);
 geye_status run_conv(geye_ctx *ctx, Plan &P);
 geye_status run_dt(geye_ctx *ctx, Plan &P, ModelPlan &mp);
-geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh);
+geye_status run_score(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, float *records);
 geye_status run_ascore(geye_ctx *ctx, Plan &P, ModelPlan &mp, int mi, float thresh, const float *h_init);
 geye_status frame_plan(geye_ctx *ctx, geye_model *const *models, int n, int w, int h, Plan **out);
 geye_status features_plan(geye_ctx *ctx, geye_model *model, const int *ftsize, const float *scales, int n_levels,
@@ -272,7 +272,9 @@ geye_status geye_get_boxes(geye_ctx *ctx, geye_model *model, const float *featur
   CUDA_TRY(cudaMemsetAsync(P->d_small.p, 0, 4096, ctx->stream));
   GEYE_TRY(run_conv(ctx, *P));
   GEYE_TRY(run_dt(ctx, *P, mp));
-  GEYE_TRY(run_score(ctx, *P, mp, 0, thresh));
+  float *d_records;
+  GEYE_TRY(S.get((size_t)mp.cap * model->gl(), &d_records));
+  GEYE_TRY(run_score(ctx, *P, mp, 0, thresh, d_records));
   if (a_score && img_width > 0 && img_height > 0) GEYE_TRY(run_ascore(ctx, *P, mp, 0, thresh, a_score));
   int D = 0;
   CUDA_TRY(cudaMemcpyAsync(&D, P->d_small.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -281,7 +283,7 @@ geye_status geye_get_boxes(geye_ctx *ctx, geye_model *model, const float *featur
   float *h = (float *)host_alloc(sizeof(float) * (size_t)std::max(D, 1) * GL);
   if (!h) { set_error("host allocation failed"); return GEYE_ERR_NOMEM; }
   cudaError_t e = cudaSuccess;
-  if (D > 0) e = cudaMemcpyAsync(h, P->d_boxes.p, sizeof(float) * (size_t)D * GL, cudaMemcpyDeviceToHost, ctx->stream);
+  if (D > 0) e = cudaMemcpyAsync(h, d_records, sizeof(float) * (size_t)D * GL, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess && a_score && img_width > 0 && img_height > 0)
     e = cudaMemcpyAsync(a_score, P->d_ascore.p, sizeof(float) * (size_t)img_width * img_height,
                         cudaMemcpyDeviceToHost, ctx->stream);
