@@ -57,8 +57,11 @@ constexpr int kBatch = kNmsBatch;
 constexpr int kBW = kBatch / 32;     // words of a suppression row
 constexpr int kPickGroup = 256;      // picks per table of a pass
 constexpr int kGW = kPickGroup / 32;
-constexpr int kPrefix = 1 << 16;     // boxes that the first launch takes where there are more than kWhole (the rest
-constexpr int kWhole = 160000;       // of up to 100 000 costs the cluster less than two launches more)
+// Boxes that the first launch takes where there are more than kWhole: its first three chunks, after which nearly every pick
+// is made; the others meet the picks on all of the chip instead of the cluster's 16 SMs, for two launches more.
+// 1013x571 (140 000 boxes) NMS stage 264 us in one launch, 236 so; 1280x720 (240 000) 397 with a prefix of 65 536, 341 so
+// and 364 with 4608; 640x480 (66 000) 160 either way.
+constexpr int kPrefix = 512 + 4096 + 32768, kWhole = 70000;
 constexpr int kWinWords = 4 * kResNT;   // words of a chunk's window
 constexpr int kMaxChunk = 32 * (kWinWords - 2);   // with the run at its end
 constexpr int kChunkCap = 60000;
@@ -671,6 +674,7 @@ __device__ __forceinline__ WalkEnd walk_boxes(const Slots &S, GreedySmem &R, con
   WalkEnd end = kDone;
   for (int c0 = R.c0; c0 < n;) {
     int c1 = resume != kAnew ? R.c1 : min(c0 + chunk, n);
+    if (resume == kAnew && n - c1 < chunk / 8 && n - c0 <= kMaxChunk) c1 = n;   // (no round for a short rest: 4 us)
     if (resume == kAnew && !ordered && c1 < n) {   // not inside a run of equal scores
       const int lim = min(n, c0 + kMaxChunk);
       c1 = run_end(S, list, c1, lim);
