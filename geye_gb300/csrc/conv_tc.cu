@@ -736,12 +736,22 @@ struct TcShape {
   size_t budget;    // dynamic shared memory per CTA, at most
   int stages;       // bank stages in the ring
   int col;          // a stage holds -1: every tap of a phase (the bank resident), 1: a filter column, 0: one tap
+  int phased;       // 1: a wide slab is walked in column phases before tiles are given up for it
 };
-static const TcShape kTcShapes[] = {{4, 110 * 1024, 2, 1},  {2, 72 * 1024, 3, 0},  {4, 220 * 1024, 1, -1},
-                                    {2, 220 * 1024, 1, -1}, {8, 220 * 1024, 1, -1}, {2, 110 * 1024, 1, -1},
-                                    {1, 72 * 1024, 4, 0},   {4, 220 * 1024, 8, 0},  {4, 110 * 1024, 8, 0},
-                                    {4, 110 * 1024, 4, 0}};
+// The columns of a slab beyond its tiles' are a filter's width times the level's rows: at 1920x1080 they are three times the four
+// tiles themselves, and one CTA takes an SM.  Walked in phases of a few filter columns the slab is reloaded (the same bytes
+// in all, or less) and two CTAs share an SM again.  Conv stage: 1920x1080 car+person 402 -> 228 us, 1280x720
+// trained-like (a grid of 10 x 10 taps) 375 -> 193, 640x480 49 -> 45 (five tiles a CTA), 1013x571 FP8 57 -> 51.
+// Three or four CTAs an SM (72 and 56 KB) 269 to 511 at 1920x1080, eight tiles and one CTA 269.
+static const TcShape kTcShapes[] = {{4, 110 * 1024, 2, 1, 0},  {2, 72 * 1024, 3, 0, 0},  {4, 220 * 1024, 1, -1, 0},
+                                    {2, 220 * 1024, 1, -1, 0}, {8, 220 * 1024, 1, -1, 0}, {2, 110 * 1024, 1, -1, 0},
+                                    {1, 72 * 1024, 4, 0, 0},   {4, 220 * 1024, 8, 0, 0},  {4, 110 * 1024, 8, 0, 0},
+                                    {4, 110 * 1024, 4, 0, 0},  {4, 110 * 1024, 2, 1, 1},  {4, 110 * 1024, 1, -1, 1},
+                                    {8, 110 * 1024, 2, 1, 1},  {8, 110 * 1024, 1, -1, 1}};
 constexpr int kTcNumShapes = (int)(sizeof(kTcShapes) / sizeof(kTcShapes[0]));
+// a plan's candidates: the shapes, and in between, where it has always been, the persistent form
+constexpr int kTcPersistent = 10;
+static const TcShape &tc_shape(int candidate) { return kTcShapes[candidate - (candidate > kTcPersistent)]; }
 
 // taps a stage holds for a phase of cs columns: one, a column (b0), or the whole phase
 static int taps_per_stage(const TcJob &J, const TcShape &sh, int cs) {
@@ -769,10 +779,15 @@ static bool chunk_jobs(const std::vector<TcJob> &jobs, int NQ, const TcShape &sh
   max_smem = 0;
   for (size_t j = 0; j < jobs.size(); j++) {
     const TcJob &J = jobs[j];
-    const int t_max = std::max(1, std::min(sh.t_cap, kTcTmemCols / J.n));
+    int t_max = std::max(1, std::min(sh.t_cap, kTcTmemCols / J.n));
+    if (sh.phased)   // as many as the accumulators of the CTAs that share an SM leave room for
+      while (t_max > 1 && (size_t)tmem_cols(t_max * J.n) * std::max<size_t>(1, (228u * 1024u) / (sh.budget + 1024)) >
+                              (size_t)kTcTmemCols)
+        t_max--;
     int T = 0, cs = 0;
     for (int Tc = t_max; Tc >= 1 && !T; Tc--)
-      if (tc_need(J, NQ, Tc, J.b1, sh) <= sh.budget) { T = Tc; cs = J.b1; }
+      for (int c = J.b1; c >= (sh.phased ? 1 : J.b1) && !T; c--)
+        if (tc_need(J, NQ, Tc, c, sh) <= sh.budget) { T = Tc; cs = c; }
     for (int c = J.b1 - 1; c >= 1 && !T; c--)
       if (tc_need(J, NQ, 1, c, sh) <= sh.budget) { T = 1; cs = c; }
     if (!T) return false;
@@ -1152,7 +1167,7 @@ geye_status build_tc_plan(geye_ctx *ctx, Plan &P) {
                     std::to_string((int)ctx->conv_mode);
   for (auto &mp : P.models) key += ":" + std::to_string(mp->model->id);
   geye_model *m0 = P.models[0]->model;
-  int first = 0, last = kTcNumShapes + 1;   // the tile shapes, then the persistent form
+  int first = 0, last = kTcNumShapes + 1;   // (tc_shape)
   float best_ms = 0.f;
   {
     std::lock_guard<std::mutex> lk(m0->tc_mu);
@@ -1176,7 +1191,7 @@ geye_status build_tc_plan(geye_ctx *ctx, Plan &P) {
   int sms = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   for (int si = first; si < last; si++) {
-    if (si == kTcNumShapes) {
+    if (si == kTcPersistent) {
       TcpLayout L;
       if (!tcp_layout(T.jobs, NQ, sms, cells_total, L)) continue;
       DevBuf d_units, d_ranges;
@@ -1216,7 +1231,7 @@ geye_status build_tc_plan(geye_ctx *ctx, Plan &P) {
     }
     std::vector<int4> chunks;
     size_t smem = 0;
-    if (!chunk_jobs(T.jobs, NQ, kTcShapes[si], cells_total, chunks, smem)) continue;
+    if (!chunk_jobs(T.jobs, NQ, tc_shape(si), cells_total, chunks, smem)) continue;
     if (!timed) {
       best = std::move(chunks);
       best_smem = smem;
@@ -1227,8 +1242,8 @@ geye_status build_tc_plan(geye_ctx *ctx, Plan &P) {
     GEYE_TRY(upload_bytes(ctx, d_chunks, chunks.data(), sizeof(int4) * chunks.size()));
     auto launch = [&]() {
       launch_conv_tc(NQ, T.d_jobs.as<TcJob>(), d_chunks.as<int4>(), (int)chunks.size(), T.d_cols.as<TcCol>(),
-                     P.arena16.as<uint8_t>(), T.d_bank.as<uint8_t>(), kTcShapes[si].stages,
-                     tps_arg(kTcShapes[si]), P.arena.as<float>(), err, smem, ctx->stream);
+                     P.arena16.as<uint8_t>(), T.d_bank.as<uint8_t>(), tc_shape(si).stages,
+                     tps_arg(tc_shape(si)), P.arena.as<float>(), err, smem, ctx->stream);
     };
     launch();
     CUDA_TRY(cudaEventRecord(e0, ctx->stream));
@@ -1259,9 +1274,9 @@ geye_status build_tc_plan(geye_ctx *ctx, Plan &P) {
   T.smem = best_smem;
   T.n_chunks = (int)best.size();
   T.shape = best_shape;
-  if (best_shape < kTcNumShapes) {
-    T.stages = kTcShapes[best_shape].stages;
-    T.tps = tps_arg(kTcShapes[best_shape]);
+  if (best_shape != kTcPersistent) {
+    T.stages = tc_shape(best_shape).stages;
+    T.tps = tps_arg(tc_shape(best_shape));
     T.d_units.release();
     T.d_ranges.release();
     T.tcp_ctas = 0;
@@ -1277,7 +1292,7 @@ geye_status run_conv_tc(geye_ctx *ctx, Plan &P) {
     set_error("tensor-core conv: the plan has no feature planes");
     return GEYE_ERR_UNSUPPORTED;
   }
-  if (T.shape == kTcNumShapes) {
+  if (T.shape == kTcPersistent) {
     launch_conv_tcp(T.planes, T.d_jobs.as<TcJob>(), T.d_units.as<int4>(), T.d_ranges.as<int4>(), T.tcp_ctas,
                     T.d_cols.as<TcCol>(), P.arena16.as<uint8_t>(), T.d_bank.as<uint8_t>(), T.tcp_colbuf,
                     P.arena.as<float>(), P.d_small.as<int>() + 130, T.smem, ctx->stream);
@@ -1403,9 +1418,9 @@ geye_status geye_conv_tuning(geye_ctx *ctx, const geye_model *m, int shape[3], f
   for (auto &mp : P.models) in_plan |= mp->model == m;
   ARG_CHECK(in_plan, "the last run has no such model");
   ARG_CHECK(P.tc.shape >= 0, "the last run's plan has no tensor-core convolution");
-  const bool persistent = P.tc.shape == geye::kTcNumShapes;
-  shape[0] = persistent ? 0 : geye::kTcShapes[P.tc.shape].t_cap;
-  shape[1] = (int)((persistent ? P.tc.smem : geye::kTcShapes[P.tc.shape].budget) / 1024);
+  const bool persistent = P.tc.shape == geye::kTcPersistent;
+  shape[0] = persistent ? 0 : geye::tc_shape(P.tc.shape).t_cap;
+  shape[1] = (int)((persistent ? P.tc.smem : geye::tc_shape(P.tc.shape).budget) / 1024);
   shape[2] = persistent ? P.tc.tcp_ctas : P.tc.n_chunks;
   *ms = P.tc.tuned_ms;
   return GEYE_OK;
