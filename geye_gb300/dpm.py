@@ -418,8 +418,8 @@ class Context:
         return {"tiles_per_cta": int(shape[0]), "smem_kb": int(shape[1]), "ctas": int(shape[2]), "ms": float(ms[0])}
 
     def dt_tuning(self, model: "Model") -> dict:
-        """DT tile size (outputs per block) the plan of the last run chose for the model, and the
-        timed launch of each candidate (1024, 2048, 4096 outputs per block; zeros before tuning)."""
+        """DT strip size (half the outputs a block takes, about) the plan of the last run chose for the model,
+        and the timed launch of each candidate (1024, 2048, 4096; zeros before tuning)."""
         elems = C.c_int()
         ms = np.zeros(3, np.float32)
         _check(lib().geye_dt_tuning(self.h, model.h, C.byref(elems), _p(ms)), "dt_tuning")
