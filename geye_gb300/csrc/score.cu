@@ -199,44 +199,90 @@ void launch_candidates(const ScoreJob *d_jobs, const int2 *d_blocks, int n_block
 // loop maps from source pixel (X - RX, Y - RY) -- looked up in the plan's
 // per-map column and row tables -- then the threshold/offset of
 // get_boxes.cpp:1765-1776 and a running maximum for the normalisation.
-// A block owns a 16 x 16 pixel tile and stages the tile's table entries of
-// every map in shared memory, so only the score gathers touch global memory.
-// The maximum is exact in any order.
-constexpr int kAsTile = 16;
+// A block owns a tile of kAsX columns of kAsY pixels and stages the tile's table entries of
+// every map (kAsJobs at a time) in shared memory, so only the score gathers touch global memory.  The maximum is exact
+// in any order.  A thread takes four pixels of a column: a cell is four pixels or more in every map but those of models with
+// small cells, so the four lie in two cells at most and two gathers serve them; where a quad of the tile has a third
+// cell between (found while staging), the block looks every pixel up.
+// What bounds it alone is latency (12 us a model at 640x480, with a thread per pixel too), but it runs beside NMS and, in a
+// server or batch, beside other frames, where the instructions and warps it takes count: with a thread per pixel (a gather
+// and nine instructions each) 16 served frames of 640x480 took 3434 us, 3351 so; eight mixed frames 2265 and 2205;
+// 1920x1080 1771 and 1744.
+constexpr int kAsX = 16, kAsY = 32, kAsThreads = kAsX * kAsY / 4, kAsJobs = 128;
 
-__global__ void __launch_bounds__(kAsTile *kAsTile) k_ascore(const int *__restrict__ col, const int *__restrict__ row,
-                                                             int n_jobs, const float *__restrict__ arena,
-                                                             float *__restrict__ a_score, int im_w, int im_h,
-                                                             float thresh, unsigned *max_bits) {
-  extern __shared__ int tab_s[];   // [job][16] column bases, then [job][16] rows
-  const int X0 = blockIdx.y * kAsTile, Y0 = blockIdx.x * kAsTile;
-  for (int i = threadIdx.x; i < n_jobs * kAsTile; i += blockDim.x) {
-    const int j = i / kAsTile, k = i % kAsTile;
-    tab_s[i] = X0 + k < im_w ? col[(size_t)j * im_w + X0 + k] : -1;
-    tab_s[n_jobs * kAsTile + i] = Y0 + k < im_h ? row[(size_t)j * im_h + Y0 + k] : -1;
-  }
-  __syncthreads();
-  const int tx = threadIdx.x / kAsTile, ty = threadIdx.x % kAsTile;
-  const int X = X0 + tx, Y = Y0 + ty;
-  unsigned local_max = 0;
-  if (X < im_w && Y < im_h) {
-    const size_t idx = (size_t)X * im_h + Y;
-    float a = a_score[idx];
-    const int *tc = tab_s + tx, *tr = tab_s + n_jobs * kAsTile + ty;
-#pragma unroll 8   // eight gathers in flight per thread (the maximum is exact in any order)
-    for (int j = 0; j < n_jobs; j++) {
-      const int c = tc[j * kAsTile], r = tr[j * kAsTile];
-      if ((c | r) >= 0) {
-        const float sc = arena[c + r];
-        if (sc > a) a = sc;
+__global__ void __launch_bounds__(kAsThreads) k_ascore(const int *__restrict__ col, const int *__restrict__ row,
+                                                       int n_jobs, const float *__restrict__ arena,
+                                                       float *__restrict__ a_score, int im_w, int im_h,
+                                                       float thresh, unsigned *max_bits) {
+  __shared__ int4 row_s[kAsJobs * (kAsY / 4)];
+  __shared__ int col_s[kAsJobs * kAsX];
+  const int X0 = blockIdx.y * kAsX, Y0 = blockIdx.x * kAsY;
+  const int tx = threadIdx.x / (kAsY / 4), ty = threadIdx.x % (kAsY / 4);
+  const int X = X0 + tx, Y = Y0 + 4 * ty;
+  const size_t idx = (size_t)X * im_h + Y;
+  const int n = X < im_w ? min(4, im_h - Y) : 0;   // pixels of this thread
+  float a[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) a[k] = k < n ? a_score[idx + k] : 0.f;
+  const float none = -INFINITY;   // never above a score
+  for (int j0 = 0; j0 < n_jobs; j0 += kAsJobs) {
+    const int nj = min(kAsJobs, n_jobs - j0);
+    if (j0) __syncthreads();
+    for (int i = threadIdx.x; i < nj * kAsY; i += kAsThreads) {
+      const int j = j0 + i / kAsY, k = i % kAsY;
+      reinterpret_cast<int *>(row_s)[i] = Y0 + k < im_h ? row[(size_t)j * im_h + Y0 + k] : -1;
+    }
+    for (int i = threadIdx.x; i < nj * kAsX; i += kAsThreads) {
+      const int j = j0 + i / kAsX, k = i % kAsX;
+      col_s[i] = X0 + k < im_w ? col[(size_t)j * im_w + X0 + k] : -1;
+    }
+    __syncthreads();
+    bool third = false;
+    for (int i = threadIdx.x; i < nj * (kAsY / 4); i += kAsThreads) {
+      const int4 r = row_s[i];
+      third |= (r.y != r.x && r.y != r.w) || (r.z != r.x && r.z != r.w);
+    }
+    third = __syncthreads_or(third);
+    if (n <= 0) continue;
+    const int *tc = col_s + tx;
+    const int4 *tr = row_s + ty;
+    if (!third) {
+#pragma unroll 8   // sixteen gathers in flight per thread
+      for (int j = 0; j < nj; j++) {
+        const int c = tc[j * kAsX];
+        const int4 r = tr[j * (kAsY / 4)];
+        const float u = (c | r.x) >= 0 ? arena[c + r.x] : none, v = (c | r.w) >= 0 ? arena[c + r.w] : none;
+        const float s1 = r.y == r.x ? u : v, s2 = r.z == r.x ? u : v;
+        if (u > a[0]) a[0] = u;
+        if (s1 > a[1]) a[1] = s1;
+        if (s2 > a[2]) a[2] = s2;
+        if (v > a[3]) a[3] = v;
+      }
+    } else {
+#pragma unroll 2
+      for (int j = 0; j < nj; j++) {
+        const int c = tc[j * kAsX];
+        const int4 r = tr[j * (kAsY / 4)];
+        const int e[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const float sc = (c | e[k]) >= 0 ? arena[c + e[k]] : none;
+          if (sc > a[k]) a[k] = sc;
+        }
       }
     }
+  }
+  unsigned local_max = 0;
+  if (n > 0) {
     const float AS_OFF = fabsf(thresh);
-    if (a < thresh) a = 0.0;
-    else a += AS_OFF;
-    a_score[idx] = a;
-    const unsigned bits = __float_as_uint(a);
-    if (a > 0.0f) local_max = bits;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (k >= n) break;
+      if (a[k] < thresh) a[k] = 0.0;
+      else a[k] += AS_OFF;
+      a_score[idx + k] = a[k];
+      if (a[k] > 0.0f) local_max = max(local_max, __float_as_uint(a[k]));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) local_max = max(local_max, __shfl_xor_sync(0xffffffffu, local_max, o));
@@ -255,11 +301,8 @@ __global__ void k_ascore_norm(float *__restrict__ a_score, int n, const unsigned
 
 void launch_ascore(const int *col, const int *row, int n_jobs, const float *arena, float *a_score, int im_w,
                   int im_h, float thresh, unsigned *max_bits, cudaStream_t s) {
-  dim3 grid((im_h + kAsTile - 1) / kAsTile, (im_w + kAsTile - 1) / kAsTile);
-  const size_t smem = sizeof(int) * 2 * kAsTile * (size_t)std::max(n_jobs, 1);
-  static SmemAttr attr;
-  raise_smem(attr, k_ascore, smem);
-  k_ascore<<<grid, kAsTile * kAsTile, smem, s>>>(col, row, n_jobs, arena, a_score, im_w, im_h, thresh, max_bits);
+  dim3 grid((im_h + kAsY - 1) / kAsY, (im_w + kAsX - 1) / kAsX);
+  k_ascore<<<grid, kAsThreads, 0, s>>>(col, row, n_jobs, arena, a_score, im_w, im_h, thresh, max_bits);
 }
 
 void launch_ascore_normalize(float *a_score, int n, const unsigned *max_bits, cudaStream_t s) {
