@@ -417,7 +417,7 @@ __device__ __noinline__ bool settle_members(GreedySmem &R, int *si, float *sf, i
   if (threadIdx.x < sizeof(SortRuns) / sizeof(int))
     reinterpret_cast<int *>(&R.runs)[threadIdx.x] = reinterpret_cast<const int *>(&R0->runs)[threadIdx.x];
   if (threadIdx.x == 0) R.settled++;
-  __syncthreads();
+  cluster.sync();   // every block has its copy: the first block's may be overwritten (split_boxes)
   int places = 0;
   for (int q = 0; q < R.runs.n; q++) places += R.runs.r[q].y - R.runs.r[q].x + 1;
   const int tied = __syncthreads_count((int)threadIdx.x < R.nb && in_runs(R.runs, R.pos[threadIdx.x]));
