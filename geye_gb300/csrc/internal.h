@@ -310,7 +310,7 @@ struct DtBlocks {
 };
 void dt_strip_sizes(std::vector<DtJob> &jobs, int elems);   // the jobs' strips
 void dt_block_lists(std::vector<DtJob> &jobs, DtBlocks &B); // the blocks (their place among the chunks into the jobs)
-size_t dt_work_words(const DtBlocks &B);                    // ints of scratch, 16-byte aligned (without chunks the first is 0)
+size_t dt_work_words(const DtBlocks &B);                    // ints of scratch, 16-byte aligned (without chunks the first is 0 before every launch)
 cudaError_t launch_dt(const DtJob *d_jobs, const int2 *d_chunks, const int2 *d_strips, const DtBlocks &B, float *arena,
                       int *arena_i, int *work, int *fallback_count, cudaStream_t s);
 // (job, block of 256 positions) of every score map, in job order

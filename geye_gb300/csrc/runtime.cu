@@ -406,6 +406,10 @@ static geye_status plan_dt(geye_ctx *ctx, const ModelPlan &mp, int elems, std::u
 }
 
 static cudaError_t launch_plan_dt(geye_ctx *ctx, Plan &P, const DtPlan &D) {
+  if (D.blocks.chunks.empty()) {   // a lone map's strips have no k_dt_range before them to clear the count of those left
+    const cudaError_t e = cudaMemsetAsync(D.d_work.p, 0, sizeof(int), ctx->stream);
+    if (e != cudaSuccess) return e;
+  }
   return launch_dt(D.d_jobs.as<DtJob>(), D.d_chunks.as<int2>(), D.d_strips.as<int2>(), D.blocks, P.arena.as<float>(),
                    P.arena.as<int>(), D.d_work.as<int>(), ctx->d_diag.as<int>(), ctx->stream);
 }
