@@ -386,9 +386,10 @@ bool conv_fp32_jobs(ConvJob J, const std::vector<const float *> &filters, const 
       }
       fits = conv_shape(C, true) || conv_shape(C, true, kConvSmemMax);
       if (fits) {   // every level's group of these filters shares one bank
-        auto it = bank.at.find(w);
+        const auto key = std::make_pair(std::make_pair(C.b0, C.b1), w);
+        auto it = bank.at.find(key);
         if (it == bank.at.end()) {
-          it = bank.at.emplace(w, (int)bank.taps.size()).first;
+          it = bank.at.emplace(key, (int)bank.taps.size()).first;
           conv_bank(C, w, bank.taps);
         }
         C.bank_off = it->second;

@@ -107,7 +107,8 @@ struct ConvJob {           // FP32 maps of one level for up to kConvGroup filter
 };
 struct ConvBank {          // the groups' taps as the FP32 kernel reads them, built with the jobs
   std::vector<float> taps;
-  std::map<std::vector<const float *>, int> at;   // a group's filters (host) -> its place, in pairs
+  // a group's filter size (b0, b1) and filters (host) -> its place; one buffer may serve filters of several sizes
+  std::map<std::pair<std::pair<int, int>, std::vector<const float *>>, int> at;
 };
 
 // tensor-core convolution (conv_tc.cu)
