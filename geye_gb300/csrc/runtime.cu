@@ -135,8 +135,20 @@ void host_pool_ref(int d) {
   g_host_kept.clear();
 }
 
-geye_status read_result(Plan &P, int mi, geye_result *out) {
-  const int *h = static_cast<const int *>(P.h_res);
+geye_status park_pending(geye_ctx *ctx, Plan &P) {
+  if (ctx->pending != &P || P.parked) return GEYE_OK;
+  const size_t bytes = P.models.size() * (size_t)P.max_cap * 11 * sizeof(int);
+  GEYE_TRY(P.d_parked.alloc(ctx, bytes));
+  if (!P.h_parked) CUDA_TRY(cudaMallocHost(&P.h_parked, 64 * sizeof(int)));
+  CUDA_TRY(cudaMemcpyAsync(P.h_parked, P.d_small.p, 64 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_TRY(cudaMemcpyAsync(P.d_parked.p, P.d_result.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+  CUDA_TRY(cudaEventRecord(P.ev_done, ctx->stream));   // the submitted frame is done when they are there
+  P.parked = true;
+  return GEYE_OK;
+}
+
+geye_status read_result(Plan &P, int mi, geye_result *out, bool parked) {
+  const int *h = static_cast<const int *>(parked ? P.h_parked : P.h_res);
   const int K = h[32 + mi];
   P.last_D[mi] = h[mi];
   P.last_K[mi] = K;
@@ -155,12 +167,13 @@ geye_status read_result(Plan &P, int mi, geye_result *out) {
     return GEYE_ERR_NOMEM;
   }
   // field f of `per` ints a record: its place in the pinned block, and (for records past it) on the device
-  const int *src = h + 64 + (size_t)mi * 11 * kHostRes, *res = P.d_result.as<int>() + (size_t)mi * P.max_cap * 11;
-  const int n = std::min(K, kHostRes);
+  const int *src = h + 64 + (size_t)mi * 11 * kHostRes;
+  const int *res = (parked ? P.d_parked : P.d_result).as<int>() + (size_t)mi * P.max_cap * 11;
+  const int n = parked ? 0 : std::min(K, kHostRes);
   struct { void *to; int at, per; } f[5] = {{out->point, 0, 4}, {out->or_point, 4, 4}, {out->type, 8, 1},
                                             {out->scale, 9, 1}, {out->score, 10, 1}};
   for (auto &x : f) {
-    memcpy(x.to, src + (size_t)x.at * kHostRes, sizeof(int) * x.per * n);
+    if (n) memcpy(x.to, src + (size_t)x.at * kHostRes, sizeof(int) * x.per * n);
     if (K > n)
       CUDA_TRY(cudaMemcpy(static_cast<int *>(x.to) + x.per * n, res + (size_t)x.at * P.max_cap + x.per * n,
                           sizeof(int) * x.per * (size_t)(K - n), cudaMemcpyDeviceToHost));
@@ -1124,6 +1137,7 @@ static geye_status run_body_graph(geye_ctx *ctx, Plan &P, float thresh, float ov
 // Whole path for n models on a frame already on the device.
 geye_status run_frame(geye_ctx *ctx, Plan &P, const uint8_t *d_bgr, int width_step, float thresh, float overlap,
                       const float *const *h_ascore_init) {
+  GEYE_TRY(park_pending(ctx, P));
   StageTimer T(ctx);
   ctx->launches = 0;
   CUDA_TRY(cudaMemsetAsync(P.d_small.p, 0, 4096, ctx->stream));

@@ -118,8 +118,11 @@ void host_pool_ref(int d);   // contexts come (+1) and go (-1)
 // boxes before NMS per model, [32, 64) kept per model, then per model point[4R], or_point[4R], type[R], scale[R], score[R]
 constexpr int kHostRes = 2048;
 inline size_t res_block_ints(int n_models) { return 64 + (size_t)n_models * 11 * kHostRes; }
-// model mi's result of the plan's finished frame (out: geye_result_free)
-geye_status read_result(Plan &P, int mi, geye_result *out);
+// model mi's result of the plan's finished frame (out: geye_result_free); parked: of the frame put aside by park_pending
+geye_status read_result(Plan &P, int mi, geye_result *out, bool parked = false);
+// A submitted frame's results put aside, in stream order, before another frame runs on its plan (and writes the plan's
+// result block) while they have not been collected
+geye_status park_pending(geye_ctx *ctx, Plan &P);
 void tune_plan(geye_ctx *ctx, Plan &P);
 
 struct LevelInfo {
@@ -248,10 +251,15 @@ struct Plan {
   std::map<std::string, FrameGraph> graphs;
   void *h_res = nullptr;                // pinned result block (kHostRes)
   cudaEvent_t ev_done = nullptr;        // asynchronous submission (serve.cu): the frame's completion
+  // park_pending: whether the pending frame's results are there, its counts (pinned) and records
+  bool parked = false;
+  void *h_parked = nullptr;
+  DevBuf d_parked;
   ~Plan() {
     for (auto &g : graphs)
       if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
     if (h_res) cudaFreeHost(h_res);
+    if (h_parked) cudaFreeHost(h_parked);
     if (ev_done) cudaEventDestroy(ev_done);
   }
 };

@@ -70,15 +70,17 @@ static geye_status enqueue_frame(geye_ctx *ctx, Plan &P, float thresh, float ove
 // tuned); false: a lane of a batch graph, already complete
 static geye_status collect_frame(geye_ctx *ctx, geye_result *out, bool wait = true) {
   Plan &P = *ctx->pending;
+  const bool parked = P.parked;
   if (wait) CUDA_TRY(cudaEventSynchronize(P.ev_done));
   if (wait) tune_plan(ctx, P);
   geye_status st = GEYE_OK;
   for (size_t mi = 0; mi < P.models.size(); mi++) {
-    const geye_status s = read_result(P, (int)mi, out ? &out[mi] : nullptr);
+    const geye_status s = read_result(P, (int)mi, out ? &out[mi] : nullptr, parked);
     if (st == GEYE_OK) st = s;
   }
   ctx->last_plan = &P;
   ctx->pending = nullptr;
+  P.parked = false;
   return st;
 }
 
