@@ -447,8 +447,9 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
     bool taken = false;
     const geye_status st = dispatch_one(s, &taken);
     if (taken) return st;
+    if (s->queue.empty()) return st;   // too old already (what came before it took time): dropped and reported
     // none free, or an error: the frame waits like any other (and meets the error again)
-    if (!s->queue.empty()) s->queue.pop_back();
+    s->queue.pop_back();
     r.user = nullptr;
   }
   GEYE_TRY(get_pinned(s, r.bytes, &r.bgr));
