@@ -438,20 +438,20 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
   r.h = height;
   r.bytes = (size_t)3 * width * height;
   *ticket = r.ticket;
-  GEYE_TRY(reap(s, false));
-  GEYE_TRY(pump(s));
-  if (s->queue.empty()) {   // a slot may take it straight from the caller
+  geye_status st = reap(s, false);
+  if (st == GEYE_OK) st = pump(s);
+  if (st == GEYE_OK && s->queue.empty()) {   // a slot may take it straight from the caller
     r.user = bgr;
     r.step = width_step;
     s->queue.push_back(r);
     bool taken = false;
-    const geye_status st = dispatch_one(s, &taken);
-    if (taken) return st;
-    if (s->queue.empty()) return st;   // too old already (what came before it took time): dropped and reported
-    // none free, or an error: the frame waits like any other (and meets the error again)
+    st = dispatch_one(s, &taken);
+    // (the queue is empty too when it is too old already, since what came before took time: dropped and reported)
+    if (taken || s->queue.empty()) return st;
     s->queue.pop_back();
     r.user = nullptr;
   }
+  // none free, or an error, of this frame or of one before it: the frame waits like any other, and the error is returned
   GEYE_TRY(get_pinned(s, r.bytes, &r.bgr));
   if (width_step == 3 * width) {
     memcpy(r.bgr, bgr, r.bytes);
@@ -473,6 +473,7 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
       }
     }
   }
+  GEYE_TRY(st);
   GEYE_TRY(reap(s, false));
   return pump(s);
 }
