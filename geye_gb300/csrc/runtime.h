@@ -250,6 +250,7 @@ struct Plan {
   };
   std::map<std::string, FrameGraph> graphs;
   void *h_res = nullptr;                // pinned result block (kHostRes)
+  void *h_bgr = nullptr;                // pinned copy of a submitted frame (where its upload is not waited for)
   cudaEvent_t ev_done = nullptr;        // asynchronous submission (serve.cu): the frame's completion
   // park_pending: whether the pending frame's results are there, its counts (pinned) and records
   bool parked = false;
@@ -259,6 +260,7 @@ struct Plan {
     for (auto &g : graphs)
       if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
     if (h_res) cudaFreeHost(h_res);
+    if (h_bgr) cudaFreeHost(h_bgr);
     if (h_parked) cudaFreeHost(h_parked);
     if (ev_done) cudaEventDestroy(ev_done);
   }

@@ -99,7 +99,18 @@ geye_status geye_detect_submit(geye_ctx *ctx, geye_model *const *models, int n_m
   CUDA_TRY(cudaSetDevice(ctx->device));
   Plan *P = nullptr;
   GEYE_TRY(frame_plan(ctx, models, n_models, width, height, &P));
-  GEYE_TRY(upload_frame(ctx, *P, bgr, width_step, true));
+  // from the caller's memory where that needs no wait but for the copy itself: the context's own stream, idle. Else (the
+  // caller's stream, earlier frames under way) from a pinned copy, and the call returns while the stream works
+  const bool idle = ctx->own_stream && cudaStreamQuery(ctx->stream) == cudaSuccess;
+  if (!idle) {
+    cudaGetLastError();   // (cudaErrorNotReady)
+    if (!P->h_bgr) CUDA_TRY(cudaMallocHost(&P->h_bgr, (size_t)3 * width * height));
+    uint8_t *to = static_cast<uint8_t *>(P->h_bgr);
+    for (int y = 0; y < height; y++) memcpy(to + (size_t)y * 3 * width, bgr + (size_t)y * width_step, (size_t)3 * width);
+    bgr = to;
+    width_step = 3 * width;
+  }
+  GEYE_TRY(upload_frame(ctx, *P, bgr, width_step, idle));
   return enqueue_frame(ctx, *P, thresh, overlap, nullptr, 0, nullptr, nullptr);
 }
 
