@@ -10,6 +10,7 @@
 //   feature sizes        CAR_TRACKING/featurepyramid.cpp:277-281
 //   level skip, conv and part-map sizes  CAR_TRACKING/fconvsMT.cpp:420-470
 //   score assembly inputs                CAR_TRACKING/get_boxes.cpp:1000-1360
+#include <malloc.h>
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -91,31 +92,27 @@ void ScratchArena::reset() {
   used = total = 0;
 }
 
-// blocks carry their size in front (a cache line, so that the caller's part stays aligned)
+// malloc's blocks (a C caller may free() them); the kept ones with their usable sizes
 static std::mutex g_host_mu;
-static std::vector<std::pair<size_t, char *>> g_host_kept;
+static std::vector<std::pair<size_t, void *>> g_host_kept;
 static int g_host_refs = 0;
-constexpr size_t kHostHead = 64, kHostBig = 1 << 20, kHostKeep = 256ull << 20;
+constexpr size_t kHostBig = 1 << 20, kHostKeep = 256ull << 20;
 void *host_alloc(size_t n) {
   n = std::max<size_t>(n, 1);
   if (n >= kHostBig) {
     std::lock_guard<std::mutex> g(g_host_mu);
     for (auto it = g_host_kept.begin(); it != g_host_kept.end(); ++it)
-      if (it->first >= n && it->first <= 2 * n) {
-        char *p = it->second;
+      if (it->first >= n && it->first / 2 <= n) {
+        void *p = it->second;
         g_host_kept.erase(it);
-        return p + kHostHead;
+        return p;
       }
   }
-  char *p = static_cast<char *>(aligned_alloc(kHostHead, (n + 2 * kHostHead - 1) & ~(kHostHead - 1)));
-  if (!p) return nullptr;
-  *reinterpret_cast<size_t *>(p) = n;
-  return p + kHostHead;
+  return malloc(n);
 }
-void host_free(void *q) {
-  if (!q) return;
-  char *p = static_cast<char *>(q) - kHostHead;
-  const size_t n = *reinterpret_cast<size_t *>(p);
+void host_free(void *p) {
+  if (!p) return;
+  const size_t n = malloc_usable_size(p);
   if (n >= kHostBig) {
     std::lock_guard<std::mutex> g(g_host_mu);
     size_t kept = n;

@@ -107,9 +107,10 @@ struct DevBuf {
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
-// Host memory handed to callers (geye_free): blocks of a megabyte and more are kept
-// for the next call (kHostKeep bytes in all, until the last context goes), since fresh
-// pages cost more than the copy into them.
+// Host memory handed to callers, who free it with geye_free, or with free() like the reference's
+// results: blocks of a megabyte and more that come back through geye_free are kept for the next
+// call (kHostKeep bytes in all, until the last context goes), since fresh pages cost more than
+// the copy into them.
 void *host_alloc(size_t n);
 void host_free(void *p);
 void host_pool_ref(int d);   // contexts come (+1) and go (-1)
