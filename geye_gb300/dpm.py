@@ -141,7 +141,7 @@ def _adopted(ptr, n: int) -> np.ndarray:
     """The n floats of a callee-allocated block as an array that frees the block when it goes."""
     addr = C.cast(ptr, C.c_void_p).value
     buf = (C.c_float * max(n, 1)).from_address(addr)
-    weakref.finalize(buf, lib().geye_free, addr)
+    weakref.finalize(buf, lib().geye_free, addr).atexit = False   # (arrays that live to the exit stay whole)
     return np.frombuffer(buf, np.float32)[:n]
 
 
