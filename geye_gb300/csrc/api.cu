@@ -252,9 +252,10 @@ geye_status geye_model_load_csv(geye_ctx *ctx, const char *comp_csv, const char 
       coef[((size_t)c * 4 + 3) * ML + j] = m->h.y2[c][j];
     }
   cudaSetDevice(ctx->device);
-  cudaError_t e = cudaMalloc(&m->d_filters, sizeof(float) * std::max<size_t>(all.size(), 1));
-  if (e == cudaSuccess) e = cudaMalloc(&m->d_filt_off, sizeof(int) * std::max<size_t>(off.size(), 1));
-  if (e == cudaSuccess) e = cudaMalloc(&m->d_coef, sizeof(float) * std::max<size_t>(coef.size(), 1));
+  auto room = [](auto **p, size_t n) { return device_malloc(reinterpret_cast<void **>(p), sizeof(**p) * std::max<size_t>(n, 1)); };
+  cudaError_t e = room(&m->d_filters, all.size());
+  if (e == cudaSuccess) e = room(&m->d_filt_off, off.size());
+  if (e == cudaSuccess) e = room(&m->d_coef, coef.size());
   if (e == cudaSuccess) e = cudaMemcpy(m->d_filters, all.data(), sizeof(float) * all.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(m->d_filt_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(m->d_coef, coef.data(), sizeof(float) * coef.size(), cudaMemcpyHostToDevice);

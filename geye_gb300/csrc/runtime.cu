@@ -10,7 +10,6 @@
 //   feature sizes        CAR_TRACKING/featurepyramid.cpp:277-281
 //   level skip, conv and part-map sizes  CAR_TRACKING/fconvsMT.cpp:420-470
 //   score assembly inputs                CAR_TRACKING/get_boxes.cpp:1000-1360
-#include <malloc.h>
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -30,106 +29,13 @@ void set_error(const std::string &msg) { g_err = msg; }
 
 
 
-static bool injected(geye_ctx *ctx, const char *op) {
+bool injected(geye_ctx *ctx, const char *op) {
   if (!ctx || ctx->inject_countdown <= 0 || ctx->inject_op != op) return false;
   if (--ctx->inject_countdown == 0) {
     ctx->inject_op.clear();
     return true;
   }
   return false;
-}
-
-DevBuf::~DevBuf() { release(); }
-void DevBuf::release() {
-  if (p && !arena) cudaFree(p);
-  p = nullptr;
-  bytes = 0;
-}
-static geye_status device_alloc(size_t n, void **out) {
-  const cudaError_t e = cudaMalloc(out, n);
-  if (e == cudaSuccess) return GEYE_OK;
-  *out = nullptr;
-  set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  return GEYE_ERR_NOMEM;
-}
-geye_status DevBuf::alloc(geye_ctx *ctx, size_t n) {
-  if (n <= bytes && p) return GEYE_OK;
-  release();
-  if (injected(ctx, "alloc")) {
-    set_error("injected allocation failure");
-    return GEYE_ERR_INJECTED;
-  }
-  if (n == 0) n = 16;
-  GEYE_TRY(arena ? arena->take(ctx, n, &p) : device_alloc(n, &p));
-  bytes = n;
-  return GEYE_OK;
-}
-
-void ScratchArena::release() {
-  for (auto &c : chunks) cudaFree(c.p);
-  chunks.clear();
-  used = total = 0;
-}
-geye_status ScratchArena::take(geye_ctx *, size_t n, void **out) {
-  n = (n + 255) & ~size_t(255);
-  if (chunks.empty() || chunks.back().bytes - used < n) {
-    const size_t bytes = std::max({n, want, size_t(1) << 20});
-    void *p = nullptr;
-    GEYE_TRY(device_alloc(bytes, &p));
-    chunks.push_back({static_cast<char *>(p), bytes});
-    used = 0;
-  }
-  *out = chunks.back().p + used;
-  used += n;
-  total += n;
-  return GEYE_OK;
-}
-void ScratchArena::reset() {
-  want = std::max(want, total);
-  if (want > kScratchKeep) want = 0;
-  // one chunk that held the whole call stays; several make way for one of their sum
-  if (chunks.size() > 1 || (!chunks.empty() && chunks.back().bytes > kScratchKeep)) release();
-  used = total = 0;
-}
-
-// malloc's blocks (a C caller may free() them); the kept ones with their usable sizes
-static std::mutex g_host_mu;
-static std::vector<std::pair<size_t, void *>> g_host_kept;
-static int g_host_refs = 0;
-constexpr size_t kHostBig = 1 << 20, kHostKeep = 256ull << 20;
-void *host_alloc(size_t n) {
-  n = std::max<size_t>(n, 1);
-  if (n >= kHostBig) {
-    std::lock_guard<std::mutex> g(g_host_mu);
-    for (auto it = g_host_kept.begin(); it != g_host_kept.end(); ++it)
-      if (it->first >= n && it->first / 2 <= n) {
-        void *p = it->second;
-        g_host_kept.erase(it);
-        return p;
-      }
-  }
-  return malloc(n);
-}
-void host_free(void *p) {
-  if (!p) return;
-  const size_t n = malloc_usable_size(p);
-  if (n >= kHostBig) {
-    std::lock_guard<std::mutex> g(g_host_mu);
-    size_t kept = n;
-    for (auto &k : g_host_kept) kept += k.first;
-    if (g_host_refs > 0 && kept <= kHostKeep && g_host_kept.size() < 8) {
-      g_host_kept.push_back({n, p});
-      return;
-    }
-  }
-  free(p);
-}
-void host_pool_ref(int d) {
-  std::lock_guard<std::mutex> g(g_host_mu);
-  g_host_refs += d;
-  if (g_host_refs > 0) return;
-  for (auto &k : g_host_kept) free(k.second);
-  g_host_kept.clear();
 }
 
 geye_status park_pending(geye_ctx *ctx, Plan &P) {

@@ -75,9 +75,16 @@ struct ArenaAlloc {
   }
 };
 
+// the n-th call of `op` fails by request (geye_debug_inject_fault)
+bool injected(geye_ctx *ctx, const char *op);
+
+// cudaMalloc; where there is not enough, the device's idle scratch (below) is given back and it is tried again
+cudaError_t device_malloc(void **out, size_t n);
+
 // Device memory of a context's stage calls: handed out piece by piece during a
 // call, all of it free again at its end (reset), and kept for the next one
 // (up to kScratchKeep bytes; cudaMalloc and cudaFree synchronise and cost more than most stages).
+// Between two calls any context's allocation that fails may take it (device_malloc), from any thread.
 struct ScratchArena {
   struct Chunk {
     char *p;
@@ -87,6 +94,8 @@ struct ScratchArena {
   size_t used = 0;             // of the last chunk
   size_t total = 0;            // handed out since the last reset
   size_t want = 0;             // the largest call so far
+  int device = 0;
+  bool busy = false;           // a call has memory of it (changed and, by other threads, read under the list's mutex)
   ~ScratchArena() { release(); }
   void release();
   geye_status take(geye_ctx *ctx, size_t n, void **out);
@@ -109,8 +118,8 @@ struct DevBuf {
 
 // Host memory handed to callers, who free it with geye_free, or with free() like the reference's
 // results: blocks of a megabyte and more that come back through geye_free are kept for the next
-// call (kHostKeep bytes in all, until the last context goes), since fresh pages cost more than
-// the copy into them.
+// call (kHostKeep bytes in all, until the last context goes or an allocation fails), since fresh
+// pages cost more than the copy into them.
 void *host_alloc(size_t n);
 void host_free(void *p);
 void host_pool_ref(int d);   // contexts come (+1) and go (-1)

@@ -664,7 +664,7 @@ geye_status batch_front_tables(geye_batch *b, const std::vector<Plan *> &plans, 
   }
   if (g.d_tables) cudaFree(g.d_tables);
   g.d_tables = nullptr;
-  CUDA_TRY(cudaMalloc(&g.d_tables, host.size()));
+  CUDA_TRY(device_malloc(&g.d_tables, host.size()));
   CUDA_TRY(cudaMemcpy(g.d_tables, host.data(), host.size(), cudaMemcpyHostToDevice));
   (void)b;
   return GEYE_OK;

@@ -264,7 +264,7 @@ geye_status tracker_update(TrackerSet &T, int stream, const int *d_result, int m
   TrackState *S = nullptr;
   auto it = T.d.find(stream);
   if (it == T.d.end()) {
-    CUDA_TRY(cudaMalloc(&S, sizeof(TrackState)));
+    CUDA_TRY(device_malloc(reinterpret_cast<void **>(&S), sizeof(TrackState)));
     k_track_clear<<<64, 256, 0, s>>>(S);
     T.d[stream] = S;
   } else {
