@@ -794,8 +794,8 @@ def run_batch(args, wl):
             "config": {"workload": args.workload, "frames_per_batch": B,
                        "sizes": {f"{a}x{b}": sizes.count((a, b)) for a, b in sorted(set(sizes))},
                        "models": list(wl["models"]), "conv": wl["conv"], "thresh": -0.5, "overlap": 0.5,
-                       "step": "one batch: one CUDA graph with a branch per frame (frame upload from pinned "
-                               "memory inside the graph)", "parallelism": f"replicas{world}",
+                       "step": "one batch: the frames' uploads from the caller's memory, then one CUDA graph with a "
+                               "branch per frame", "parallelism": f"replicas{world}",
                        "l2": "working set (frames + per-frame arenas) larger than L2"},
             "e2e": {"value": world * B * args.steps / t_wall, "unit": "frames/s", "api": "geye_batch_run (host frames in, host results out)",
                     "h2d_bytes_per_step": int(sum(w * h * 3 for w, h in sizes)),

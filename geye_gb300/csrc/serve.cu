@@ -583,7 +583,7 @@ struct geye_batch {
   };
   std::map<std::string, Graph> graphs;   // by lane sizes, thresh, overlap
   int last_kernels = 0;
-  cudaEvent_t t0 = nullptr, t1 = nullptr;   // around the last graph launch
+  cudaEvent_t t0 = nullptr, t1 = nullptr;   // around the last batch's uploads and graph
 };
 
 namespace {
@@ -837,10 +837,10 @@ geye_status geye_batch_run(geye_batch *b, int n_frames, const uint8_t *const *bg
     }
     g.kernels = kernels;
   }
+  CUDA_TRY(cudaEventRecord(b->t0, b->stream));
   for (int i = 0; i < n_frames; i++)   // every frame in, from the caller's memory
     CUDA_TRY(cudaMemcpy2DAsync(plans[i]->d_bgr.p, (size_t)3 * widths[i], bgr[i], width_steps[i], (size_t)3 * widths[i],
                                heights[i], cudaMemcpyHostToDevice, b->stream));
-  CUDA_TRY(cudaEventRecord(b->t0, b->stream));
   CUDA_TRY(cudaGraphLaunch(g.exec, b->stream));
   CUDA_TRY(cudaEventRecord(b->t1, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));

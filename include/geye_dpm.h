@@ -265,8 +265,8 @@ geye_status geye_batch_destroy(geye_batch *b);
 geye_status geye_batch_run(geye_batch *b, int n_frames, const uint8_t *const *bgr, const int *widths,
                            const int *heights, const int *width_steps, float thresh, float overlap,
                            geye_result *results);
-/* out = {lanes, graphs built, kernels in the last graph, 0}; last_ms = device
- * time of the last graph launch (CUDA events on the batch stream). */
+/* out = {lanes, graphs built, kernels in the last graph, 0}; last_ms = time of the
+ * last batch on its stream, its frames' uploads and its graph (CUDA events). */
 geye_status geye_batch_stats(geye_batch *b, int out[4], float *last_ms);
 
 /* ---- measurement ---------------------------------------------------------- */
