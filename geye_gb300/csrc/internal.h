@@ -288,7 +288,6 @@ void launch_batch_front(int stage, const BatchFrame *d_frames, const BatchItem *
 void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int n_vote_blocks, int max_b0,
                 int max_b1, const HogPixJob *d_pix, int n_pix, int max_xe, float *arena, void *arena16,
                 bool corners, bool floats, float *ref, cudaStream_t s);   // arena16: base of the tensor-core planes (bytes)
-void launch_to_ref_layout(const float *feat, int fs0, int fs1, float *out, cudaStream_t s);
 void launch_flip_feat(const float *feat, int n0, int n1, float *out, cudaStream_t s);
 void launch_from_ref_layout(const float *ref, int fs0, int fs1, float *feat, cudaStream_t s);
 // jobs for filters of one size [31][b1][b0] (host memory) over one level (J: its features and the

@@ -622,15 +622,9 @@ void launch_hog(const HogJob *d_jobs, int n_jobs, const int2 *d_vote_blocks, int
 }
 
 // ----------------------------------------------------------------------------
-// between the device feature planes and the reference layout [31][fs1][fs0]
-// (stage entry points only): they differ in the columns' padding
+// from the reference layout [31][fs1][fs0] to the device feature planes (stage
+// entry points only): they differ in the columns' padding
 // ----------------------------------------------------------------------------
-__global__ void k_to_ref(const float *__restrict__ feat, int fs0, int ncols, float *__restrict__ out) {
-  const int S0 = feat_stride(fs0), n = ncols * fs0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[i] = feat[(size_t)(i / fs0) * S0 + i % fs0];
-}
-
 __global__ void k_from_ref(const float *__restrict__ ref, int fs0, int ncols, float *__restrict__ feat) {
   const int S0 = feat_stride(fs0), n = ncols * fs0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -657,12 +651,6 @@ void launch_flip_feat(const float *feat, int n0, int n1, float *out, cudaStream_
   const size_t total = (size_t)n0 * n1 * kFeat;
   const int blocks = (int)std::min<size_t>((total + 255) / 256, 4096);
   k_flip_feat<<<blocks, 256, 0, s>>>(feat, n0, n1, out);
-}
-
-void launch_to_ref_layout(const float *feat, int fs0, int fs1, float *out, cudaStream_t s) {
-  int n = fs0 * fs1 * kFeat;
-  if (n <= 0) return;
-  k_to_ref<<<std::min((n + 255) / 256, 2048), 256, 0, s>>>(feat, fs0, fs1 * kFeat, out);
 }
 
 void launch_from_ref_layout(const float *ref, int fs0, int fs1, float *feat, cudaStream_t s) {
