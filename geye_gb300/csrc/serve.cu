@@ -448,7 +448,6 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
   r.w = width;
   r.h = height;
   r.bytes = (size_t)3 * width * height;
-  *ticket = r.ticket;
   geye_status st = reap(s, false);
   if (st == GEYE_OK) st = pump(s);
   if (st == GEYE_OK && s->queue.empty()) {   // a slot may take it straight from the caller
@@ -458,7 +457,10 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
     bool taken = false;
     st = dispatch_one(s, &taken);
     // (the queue is empty too when it is too old already, since what came before took time: dropped and reported)
-    if (taken || s->queue.empty()) return st;
+    if (taken || s->queue.empty()) {
+      *ticket = r.ticket;
+      return st;
+    }
     s->queue.pop_back();
     r.user = nullptr;
   }
@@ -470,6 +472,7 @@ geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, i
     for (int y = 0; y < height; y++)
       memcpy(r.bgr + (size_t)y * 3 * width, bgr + (size_t)y * width_step, (size_t)3 * width);
   }
+  *ticket = r.ticket;
   s->queue.push_back(std::move(r));
   if (s->max_queued > 0) {   // the stream's oldest queued frames make way for its newest
     int n = 0;

@@ -224,7 +224,10 @@ geye_status geye_server_create(int device, geye_model *const *models, int n_mode
                                size_t hbm_budget, int max_slots, float thresh, float overlap, int track,
                                geye_server **out);
 geye_status geye_server_destroy(geye_server *s);
-/* Copies the frame and queues it; dispatches whatever fits.  *ticket identifies it. */
+/* Takes the frame over (the caller's buffer is free on return: uploaded from it where a
+ * slot is free, else copied) and queues it; dispatches whatever fits.  *ticket identifies it.
+ * Where the frame has been queued and it or one before it then meets an error, *ticket is set
+ * and the error returned. */
 geye_status geye_server_submit(geye_server *s, int stream, const uint8_t *bgr, int width, int height,
                                int width_step, long long *ticket);
 /* Completes finished frames and dispatches queued ones without blocking; up to
