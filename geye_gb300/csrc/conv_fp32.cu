@@ -85,7 +85,7 @@ __device__ __forceinline__ void conv_zero(float (&v)[G][kCX][CR]) {
 
 // N taps of a filter column: val[g][j][h] holds rows 2h, 2h + 1 of column j.  Ax: the
 // features under the first tap at the thread's first row and column (jx floats between
-// its columns); Bx: the taps in pairs (b0p between filters).
+// its columns); Bx: the taps (b0p between filters).
 template <int G, int CR, int N>
 __device__ __forceinline__ void conv_column(float (&val)[G][kCX][CR], const float *__restrict__ Ax, int jx,
                                             const float *__restrict__ Bx, int b0p) {
@@ -125,7 +125,7 @@ __device__ __forceinline__ void conv_columns(float (&val)[G][kCX][CR], const flo
     conv_column<G, CR, N>(val, Ax + xp * RP, jx, Bx + xp * G * b0p, b0p);
 }
 
-// One warp's channel of a chunk over xb filter columns, tap by tap (Ac: [x][RP] floats, Bc: [xp][g][b0p] pairs);
+// One warp's channel of a chunk over xb filter columns, tap by tap (Ac: [x][RP] floats, Bc: [xp][g][b0p] floats);
 // columns of 4 to 10 taps are unrolled, others take four at a time
 template <int G, int CR>
 __device__ __forceinline__ void conv_taps(float (&val)[G][kCX][CR], const float *__restrict__ Ac, int RP, int jx,
@@ -164,7 +164,7 @@ __device__ __forceinline__ void conv_tile(const ConvJob &J, int tile, const floa
   const int WY = J.wy, WX = SPLIT ? 1 : kCWarps / WY;       // warps' tiles along y and x
   const int ty0 = (tile % J.tiles_y) * (WY * TY * CR), tx0 = (tile / J.tiles_y) * (WX * kCX * TX);
   const int cols = WX * kCX * TX + J.xb - 1, chan = cols * RP;   // staged columns; floats of a channel
-  const int bcol = G * b0p;                                 // taps (pairs) of a filter column
+  const int bcol = G * b0p;                                 // taps of a filter column
   const size_t bchan = (size_t)J.b1 * bcol;                 // of a channel in the bank
   float *A_s = sm;                                          // [2][kChunk][cols][RP]
   float *B_s = A_s + 2 * kChunk * chan;                     // [2][kChunk][xb][G][b0p]
@@ -356,7 +356,7 @@ static bool conv_shape(ConvJob &J, bool split, size_t limit = kConvSmem) {
   return best >= 0;
 }
 
-// The bank of a group: [channel, padded to whole chunks][filter column][filter][b0p] taps, each twice.
+// The bank of a group: [channel, padded to whole chunks][filter column][filter][b0p] taps.
 static void conv_bank(const ConvJob &J, const std::vector<const float *> &w, std::vector<float> &bank) {
   const size_t at = bank.size();
   bank.resize(at + (size_t)kChunks * kChunk * J.b1 * J.n_filt * J.b0p, 0.f);

@@ -95,7 +95,7 @@ constexpr int kConvGroup = 4;   // filters per FP32 convolution job
 struct ConvJob {           // FP32 maps of one level for up to kConvGroup filters of one size
   int feat_off, a0, a1;    // feature level, dims
   int n_filt;
-  int bank_off;            // the group's taps in the bank (in pairs)
+  int bank_off;            // the group's taps in the bank (floats)
   int out_off[kConvGroup];    // float offset of each output map
   int b0, b1;              // filter dims
   int c0, c1;              // output dims

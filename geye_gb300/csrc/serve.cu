@@ -2,9 +2,10 @@
 // server (no counterpart in the reference, whose car_detection handles one
 // frame at a time from main.cpp's loop).
 //
-// A context is a slot: geye_detect_submit stages a frame through pinned
-// memory, replays the frame graph on the context's stream and queues the
-// result copies; a completion event tells when it is done.  The server keeps a
+// A context is a slot: geye_detect_submit uploads a frame (from the caller's
+// memory on an idle stream of the context's own, else through a pinned copy) and
+// replays the frame graph on the context's stream, whose NMS kernels write the
+// results into pinned memory; a completion event tells when it is done.  The server keeps a
 // pool of slots and a FIFO of submitted frames.  A frame goes to a free slot
 // that already holds a plan for its size, else to a new slot while the device
 // memory held by slots stays within the budget, else to any free slot, which

@@ -151,6 +151,7 @@ geye_status geye_flip_feat(geye_ctx *ctx, const float *feat, const int *size, fl
  * partner is 0).  Any pointer may be NULL. */
 geye_status geye_model_sym(const geye_model *model, int *rootsym, int *part_partner, int *part_sym);
 
+/* Frees what a stage entry point has allocated (malloc's blocks: free() takes them too). */
 void geye_free(void *p);
 
 /* ---- device-resident path (benchmarks, batching) ------------------------ */
@@ -186,9 +187,10 @@ geye_status geye_nms_noalloc(const float *d_boxes, int num, int numpart0, float 
                              int *d_kept, void *cuda_stream);
 
 /* ---- asynchronous submission (no counterpart in the reference) ------------ */
-/* The work of geye_detect_multi without waiting: the frame is copied (the
- * caller's buffer is free on return), staged through pinned memory, run on the
- * context's stream and its results copied back into pinned memory.  One frame
+/* The work of geye_detect_multi without waiting for it: the frame is taken over
+ * (the caller's buffer is free on return: uploaded from it on an idle stream of the
+ * context's own, else copied into pinned memory first) and run on the context's
+ * stream, its results written into pinned memory.  One frame
  * per context may be outstanding; geye_detect_query returns GEYE_OK when it is
  * done and GEYE_BUSY while it runs; geye_detect_collect waits for it and fills
  * out[0..n_models) (free each with geye_result_free).  Several contexts on one
@@ -257,8 +259,8 @@ geye_status geye_server_tracks(geye_server *s, int stream, int max, float *boxes
 /* Several frames of any sizes as one CUDA graph: each frame gets a lane (its own
  * context, stream and plan per size, created on first use) and the lanes run as
  * parallel branches of one graph between a fork and a join, the graph kept per
- * combination of lane sizes, thresh and overlap.  geye_batch_run copies the
- * frames into the lanes' pinned buffers, launches the graph, waits, and fills
+ * combination of lane sizes, thresh and overlap.  geye_batch_run uploads the
+ * frames from the caller's memory, launches the graph, waits, and fills
  * results[i * n_models + m] (free each with geye_result_free); every result is
  * the one geye_detect_multi gives for that frame alone. */
 typedef struct geye_batch geye_batch;     /* the models must outlive the batch */
