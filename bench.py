@@ -542,11 +542,11 @@ def run_served(args, wl):
     # ---- e2e: the server API with host frames, S streams kept busy (closed loop)
     n_frames = args.steps * S
     srv = g.Server(models, conv=g.CONV_BF16, max_slots=S)
-    for _ in range(2):   # warm the slots' plans and graphs (the second round runs the refitted graphs)
+    for _ in range(2):   # warm the slots' plans and graphs (the second round runs the tuned ones)
         for k in range(S):
             srv.submit(k, frames[k])
         srv.drain()
-        srv.poll(4 * S)
+        res_bytes = sum(_result_bytes(d["results"]) for d in srv.poll(4 * S))   # of the S frames of a step
     lat = []
     submitted = done = 0
     t0 = time.perf_counter()
@@ -568,7 +568,6 @@ def run_served(args, wl):
     srv.close()
     e2e_t = max_over_ranks(pg, e2e_t)
     e2e_fps = world * n_frames / e2e_t
-    res_bytes = 4 * (64 + len(models) * 11 * 4096)
 
     # ---- the plain FP32 drop-in on the same frame, stage breakdown and roofline of the conv
     plain = _plain_fp32(paths, frames[0], 30)
@@ -610,7 +609,7 @@ def run_served(args, wl):
                        "l2": "flushed between steps (256 MiB write, outside the timed events)"},
             "p50_ms": float(np.percentile(lat, 50)), "p99_ms": float(np.percentile(lat, 99)),
             "e2e": {"value": e2e_fps, "unit": "frames/s", "api": "geye_server_submit/poll (host frames in, host results out)",
-                    "h2d_bytes_per_step": int(S * W * H * 3), "d2h_bytes_per_step": int(S * res_bytes),
+                    "h2d_bytes_per_step": int(S * W * H * 3), "d2h_bytes_per_step": int(res_bytes),
                     "p50_ms": float(np.percentile(lat, 50)), "p99_ms": float(np.percentile(lat, 99)),
                     "slots": srv_stats["slots"]},
             "plain_fp32": plain,
@@ -647,13 +646,14 @@ def serve_sim(wl, models, max_slots):
     base = {(sz, k): synth.make_frame(*sz, seed=1000 * j + k) for j, sz in enumerate(sorted(set(sizes))) for k in range(4)}
     frames = {(s, k): base[(sizes[s], (s + k) % 4)] for s in range(n) for k in range(2)}
     srv = g.Server(models, conv=g.CONV_BF16, hbm_budget=40 << 30, max_slots=max_slots, track=True)
+    d2h = {}                        # result bytes of a frame of each size
     for sz in sorted(set(sizes)):   # slots, plans and graphs for every resolution before the clock starts
         s0 = sizes.index(sz)
-        for rnd in range(3):        # later rounds run the graphs refitted to the frames' NMS depth
+        for rnd in range(3):        # later rounds run the tuned graphs
             for k in range(max_slots):
                 srv.submit(s0, base[(sz, (rnd + k) % 4)])
             srv.drain()
-            srv.poll(1024)
+            d2h[sz] = np.mean([_result_bytes(d["results"]) for d in srv.poll(1024)])
         # the pinned frame pool for as many frames of this size as can be queued and in flight at once
         for k in range(max_slots + 2 * sizes.count(sz)):
             srv.submit(s0, base[(sz, k % 4)])
@@ -703,7 +703,8 @@ def serve_sim(wl, models, max_slots):
             "slots": st["slots"], "max_slots": max_slots, "bytes_held": st["bytes_held"], "live_tracks_end": tracks,
             "admission": {"max_waiting_per_stream": adm[0], "max_wait_ms": adm[1]},
             "sizes": {f"{a}x{b}": sizes.count((a, b)) for a, b in sorted(set(sizes))},
-            "h2d_bytes_per_frame": int(np.mean([a * b * 3 for a, b in sizes])), "clocks": clk.summary()}
+            "h2d_bytes_per_frame": int(np.mean([a * b * 3 for a, b in sizes])),
+            "d2h_bytes_per_frame": int(np.mean([d2h[sz] for sz in sizes])), "clocks": clk.summary()}
 
 
 def run_serve_sim(args, wl):
@@ -731,7 +732,7 @@ def run_serve_sim(args, wl):
                    "models": list(wl["models"]), "conv": "bf16", "admission": r["admission"]},
         "p50_ms": r["p50_ms"], "p99_ms": r["p99_ms"],
         "e2e": {"value": r["served_fps"], "unit": "frames/s", "api": "geye_server_submit/poll",
-                "h2d_bytes_per_step": r["h2d_bytes_per_frame"], "d2h_bytes_per_step": 4 * (64 + 2 * 11 * 4096),
+                "h2d_bytes_per_step": r["h2d_bytes_per_frame"], "d2h_bytes_per_step": r["d2h_bytes_per_frame"],
                 "p50_ms": r["p50_ms"], "p99_ms": r["p99_ms"]},
         "offered_fps": r["offered_fps"], "dropped_fps": r["dropped_fps"],
         "server": {"slots": r["slots"], "max_slots": r["max_slots"], "bytes_held": r["bytes_held"],
@@ -740,6 +741,11 @@ def run_serve_sim(args, wl):
     }
     print(json.dumps(line), flush=True)
     return 0
+
+
+def _result_bytes(results):
+    """Bytes a frame's results take to the host: per model two counts and eleven words a kept box."""
+    return sum(4 * (2 + 11 * r["num"]) for r in results)
 
 
 def run_batch(args, wl):
@@ -799,7 +805,7 @@ def run_batch(args, wl):
                        "l2": "working set (frames + per-frame arenas) larger than L2"},
             "e2e": {"value": world * B * args.steps / t_wall, "unit": "frames/s", "api": "geye_batch_run (host frames in, host results out)",
                     "h2d_bytes_per_step": int(sum(w * h * 3 for w, h in sizes)),
-                    "d2h_bytes_per_step": int(B * 4 * (64 + len(models) * 11 * 4096))},
+                    "d2h_bytes_per_step": int(sum(_result_bytes(fr) for fr in res))},
             "gpu_launches": st["kernels"], "graph_launches_per_step": 1,
             "detections_kept": kept[:4],
             "clocks": clk.summary(),
